@@ -494,10 +494,26 @@ struct SortBuffers {
     }
 };
 
-// Sort + bucket construction.  On return ix holds cand/bucket arrays; if want_i2b the
-// (row, table) -> bucket map is filled.  Returns the device error word read at the one
+// Lists of a self-join from the finished buckets.  Cleared and filled a few tables at a time: the
+// strips are still in the L2 when the scattered words arrive, so that no half-written sector has
+// to be read back from memory.
+void fill_self_bounds(const culsh_index& ix, const int32_t* cand, const uint32_t* tile_base, bool pairs, uint32_t* packed) {
+    const CtxPtr& c = ix.ctx;
+    const int n = ix.n, tpt = (int)ceil_div(n, IB_TILE);
+    const int group = std::max(1, (int)std::min<size_t>((size_t)ix.L, ((size_t)32 << 20) / (sizeof(uint32_t) * (size_t)n)));
+    for (int t0 = 0; t0 < ix.L; t0 += group) {
+        const int nt = std::min(group, ix.L - t0);
+        CU_CHECK(cudaMemsetAsync(packed + (size_t)t0 * n, 0, sizeof(uint32_t) * (size_t)nt * n, c->stream));
+        bucket_bounds_kernel<<<(unsigned)(nt * tpt), IB_THREADS, 0, c->stream>>>(
+            ix.bucket_offsets.p, cand, n, t0, tpt, tile_base, packed_bounds(n), pairs, packed);
+        KERNEL_CHECK();
+    }
+}
+
+// Sort + bucket construction.  On return ix holds cand/bucket arrays; a self-join's `bounds` hold
+// the list of every (table, row).  Returns the device error word read at the one
 // host synchronisation of the build.
-int build_index(culsh_index& ix, SortBuffers& sb, Scratch<int32_t>* item_to_bucket, StageTimer& tm) {
+int build_index(culsh_index& ix, SortBuffers& sb, Scratch<uint32_t>* bounds, StageTimer& tm) {
     const CtxPtr& c = ix.ctx;
     const int n = ix.n, L = ix.L, NW = ix.ks.key_words;
     HostTrace tr;
@@ -547,19 +563,12 @@ int build_index(culsh_index& ix, SortBuffers& sb, Scratch<int32_t>* item_to_buck
     ix.bucket_keys.alloc(c, (size_t)B * NW);
     ix.bucket_offsets.alloc(c, (size_t)B + 1);
     ix.table_offsets.alloc(c, (size_t)L + 1);
-    Scratch<int32_t> i2b_tm;  // (table, row) -> bucket, transposed to (row, table) below
-    if (item_to_bucket) {
-        item_to_bucket->reserve(c, SL_I2B, (size_t)n * L);
-        i2b_tm.reserve(c, SL_I2B_TM, (size_t)n * L);
-    }
     tr.lap("alloc bucket arrays");
-    CULSH_DISPATCH_NW(NW, launch_bucket_write<NW>(c->stream, kp[cur], vp[cur], n, L, tile_base.p,
-                                                  ix.bucket_keys.p, ix.bucket_offsets.p,
-                                                  ix.table_offsets.p, i2b_tm.p));
-    if (item_to_bucket) {
-        dim3 grid((unsigned)ceil_div(n, 32), (unsigned)ceil_div(L, 32));
-        transpose_table_major_kernel<<<grid, 256, 0, c->stream>>>(i2b_tm.p, n, L, item_to_bucket->p);
-        KERNEL_CHECK();
+    CULSH_DISPATCH_NW(NW, launch_bucket_write<NW>(c->stream, kp[cur], n, L, tile_base.p, ix.bucket_keys.p,
+                                                  ix.bucket_offsets.p, ix.table_offsets.p));
+    if (bounds) {
+        bounds->reserve(c, SL_BOUNDS, (size_t)n * L);
+        fill_self_bounds(ix, reinterpret_cast<const int32_t*>(vp[cur]), tile_base.p, true, bounds->p);
     }
     // the sorted row ids are the candidate array: adopt the buffer
     static_assert(sizeof(int32_t) == sizeof(uint32_t), "");
@@ -593,7 +602,7 @@ void validate_shape(int n, int d, int L, int k) {
 
 // Hash + sort + build.  `hash_fn(ks, keys)` fills the key array for a given key layout.
 template <typename HashFn>
-void fit_common(culsh_index& ix, HashFn&& hash_fn, Scratch<int32_t>* item_to_bucket) {
+void fit_common(culsh_index& ix, HashFn&& hash_fn, Scratch<uint32_t>* bounds) {
     const CtxPtr& c = ix.ctx;
     c->stats = culsh_stats{};
     c->stats.params_ms = c->last_params_ms;
@@ -613,7 +622,7 @@ void fit_common(culsh_index& ix, HashFn&& hash_fn, Scratch<int32_t>* item_to_buc
         tm.mark();
         hash_fn(ix.ks, sb.keys[0].p);
         tm.mark();
-        int err = build_index(ix, sb, item_to_bucket, tm);
+        int err = build_index(ix, sb, bounds, tm);
         if (err & DEV_ERR_NARROW_OVERFLOW) {  // p-stable values do not fit: widen and redo
             if (eb >= 4) fail(CULSH_ERR_INTERNAL, "overflow reported at full width");
             eb *= 2;
@@ -635,8 +644,13 @@ void fit_common(culsh_index& ix, HashFn&& hash_fn, Scratch<int32_t>* item_to_buc
     }
 }
 
+BoundsView query_bounds(const int2* pair, int n_q) { return BoundsView{pair, nullptr, nullptr, nullptr, PackedBounds{}, n_q}; }
+BoundsView self_bounds(const culsh_index& ix, const uint32_t* packed) {
+    return BoundsView{nullptr, packed, ix.bucket_offsets.p, ix.table_offsets.p, packed_bounds(ix.n), ix.n};
+}
+
 // -----------------------------------------------------------------------------------------
-// Query from matched bucket ids (matched[q*L + t])
+// Query from the matched buckets' lists (bounds[t*n_q + q])
 // -----------------------------------------------------------------------------------------
 int bitmap_window_bits(const CtxPtr& c, int n_rows) {
     size_t fixed = bitmap_smem_bytes(0) + 1024;
@@ -672,11 +686,11 @@ int chain_window_bits(int n_rows, int* n_win) {
     return (int)(ceil_div(ceil_div(n, wins), (size_t)4096) * 4096);
 }
 
-void query_from_matched(const culsh_index& ix, const int32_t* matched, int n_q, culsh_candidates& out,
+void query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool self_join, culsh_candidates& out,
                         StageTimer& tm) {
     const CtxPtr& c = ix.ctx;
     cudaStream_t s = c->stream;
-    const int L = ix.L;
+    const int L = ix.L, n_q = bounds.n_q;
     HostTrace tr;
     bool dedupe_timed = false;
     out.ctx = c;
@@ -685,32 +699,33 @@ void query_from_matched(const culsh_index& ix, const int32_t* matched, int n_q, 
     out.offsets.alloc(c, (size_t)n_q + 1);
     Scratch<uint64_t> raw_cnt(c, SL_RAW_CNT, n_q), raw_off(c, SL_RAW_OFF, (size_t)n_q + 1),
         scratch(c, SL_SCAN, scan_scratch_elems(n_q));
-    Scratch<uint32_t> big_list(c, SL_BIG_LIST, 2 * (size_t)n_q), n_big(c, SL_NBIG, 2);
+    Scratch<uint32_t> big_list(c, SL_BIG_LIST, 2 * (size_t)n_q), n_big(c, SL_NBIG, 4);
     uint32_t* mid_list = big_list.p + n_q;
     const int wbits = bitmap_window_bits(c, ix.n);
     // with more rows than two bitmap windows, mid-sized candidate sets are sorted in shared memory
     const int mid_max = (size_t)ix.n > 2 * (size_t)wbits ? MID_MAX : 0;
-    CU_CHECK(cudaMemsetAsync(n_big.p, 0, 2 * sizeof(uint32_t), s));
-    // The count pass keeps the list bounds it reads for the warp path (one coalesced read there
-    // instead of two dependent scattered ones), when the table is worth it and fits 8 GB.
-    Scratch<int2> bounds;
-    const size_t pairs = (size_t)n_q * L;
-    if (pairs >= ((size_t)1 << 22) && pairs <= ((size_t)1 << 30)) bounds.reserve(c, SL_BOUNDS, pairs);
-    raw_count_kernel<<<(unsigned)ceil_div(n_q, 256), 256, 0, s>>>(matched, ix.bucket_offsets.p, n_q, L,
-                                                                 raw_cnt.p, big_list.p, mid_list, n_big.p,
-                                                                 mid_max, bounds.p);
+    CU_CHECK(cudaMemsetAsync(n_big.p, 0, 4 * sizeof(uint32_t), s));
+    const uint32_t self_lists = self_join ? (uint32_t)L : 0u;
+    raw_count_kernel<<<(unsigned)ceil_div(n_q, 256), 256, 0, s>>>(bounds, n_q, L, self_join, raw_cnt.p, big_list.p,
+                                                                 mid_list, n_big.p, mid_max);
     KERNEL_CHECK();
     exclusive_scan<uint64_t, uint64_t>(s, raw_cnt.p, n_q, raw_off.p, scratch.p);
     uint64_t raw_total = 0;
-    uint32_t nb = 0, nm = 0;
+    uint32_t nc[3] = {0, 0, 0};
     CU_CHECK(cudaMemcpyAsync(c->pinned, raw_off.p + n_q, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-    CU_CHECK(cudaMemcpyAsync(c->pinned + 1, n_big.p, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    CU_CHECK(cudaMemcpyAsync(c->pinned + 1, n_big.p, sizeof(nc), cudaMemcpyDeviceToHost, s));
     CU_CHECK(cudaStreamSynchronize(s));
     std::memcpy(&raw_total, c->pinned, sizeof(uint64_t));
-    std::memcpy(&nb, c->pinned + 1, sizeof(uint32_t));
-    std::memcpy(&nm, reinterpret_cast<const char*>(c->pinned + 1) + sizeof(uint32_t), sizeof(uint32_t));
+    std::memcpy(nc, c->pinned + 1, sizeof(nc));
+    const uint32_t nb = nc[0], nm = nc[1];
     tr.lap("count+scan+sync");
-    c->stats.raw_candidates += raw_total;
+    // The bitmap and sort paths walk lists: a self-join with rows for them takes its pairs as lists too
+    // (the tile bases of the build are still in their slot).
+    if (self_join && (nb || nm))
+        fill_self_bounds(ix, ix.cand.p, static_cast<const uint32_t*>(c->slot_ptr[SL_TILE_BASE]), false,
+                         const_cast<uint32_t*>(bounds.packed));
+    // upstream's raw count: a self-join counts the own row once per table
+    c->stats.raw_candidates += raw_total + (self_join ? (uint64_t)n_q * (uint64_t)(L - 1) : 0ull);
     if (raw_total == 0) {
         CU_CHECK(cudaMemsetAsync(out.counts.p, 0, out.counts.bytes(), s));
         CU_CHECK(cudaMemsetAsync(out.offsets.p, 0, out.offsets.bytes(), s));
@@ -735,18 +750,24 @@ void query_from_matched(const culsh_index& ix, const int32_t* matched, int n_q, 
     if (!(chained && n_other == 0 && nm == 0)) tmp.reserve(c, SL_TMP, raw_total);
     tr.lap("alloc tmp");
     if (n_other) {
-        size_t blocks = std::min<size_t>(ceil_div(n_q, SM_WARPS), (size_t)c->sm_count * 16);
-        dedupe_small_kernel<<<(unsigned)blocks, SM_THREADS, 0, s>>>(
-            matched, ix.bucket_offsets.p, ix.cand.p, raw_cnt.p, raw_off.p, n_q, L, tmp.p, out.counts.p, bounds.p);
-        KERNEL_CHECK();
+        // Short lists in a form that fits twice as many warps on an SM, the rest in a second launch; a
+        // set that one launch takes in a wave or two is not worth a second one.
+        const size_t blocks = std::min<size_t>(ceil_div(n_q, SM_WARPS), (size_t)c->sm_count * 32);
+        auto launch = [&](auto kernel, int above) {
+            kernel<<<(unsigned)blocks, SM_THREADS, 0, s>>>(bounds, ix.cand.p, raw_cnt.p, raw_off.p, L, above, tmp.p, out.counts.p);
+            KERNEL_CHECK();
+        };
+        const bool both = nc[2] && n_q < (1 << 15);
+        if (n_other > nc[2] && !both) launch(self_join ? dedupe_small_kernel<SHORT_MAX, true> : dedupe_small_kernel<SHORT_MAX, false>, 0);
+        if (nc[2]) launch(self_join ? dedupe_small_kernel<SMALL_MAX, true> : dedupe_small_kernel<SMALL_MAX, false>, both ? 0 : SHORT_MAX);
     }
     if (nm) {
         int id_bytes = 1;
         while (id_bytes < 4 && ((uint64_t)ix.n - 1) >> (8 * id_bytes)) ++id_bytes;
         size_t smem = sort_path_smem_bytes();
         CU_CHECK(cudaFuncSetAttribute(dedupe_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        dedupe_sort_kernel<<<nm, MS_THREADS, smem, s>>>(mid_list, matched, ix.bucket_offsets.p, ix.cand.p,
-                                                       raw_cnt.p, raw_off.p, L, id_bytes, tmp.p, out.counts.p);
+        dedupe_sort_kernel<<<nm, MS_THREADS, smem, s>>>(mid_list, bounds, ix.cand.p, raw_off.p, L,
+                                                       id_bytes, tmp.p, out.counts.p);
         KERNEL_CHECK();
     }
     if (chained) {
@@ -760,7 +781,7 @@ void query_from_matched(const culsh_index& ix, const int32_t* matched, int n_q, 
         if (env_long("CULSH_CHAIN_SLICES", 1) && n_win > 1 && n_tk * (size_t)L <= ((size_t)32 << 20)) {
             slices.reserve(c, SL_SLICES, n_tk * (size_t)L);
             slice_lists_kernel<<<(unsigned)ceil_div(n_tk * (size_t)L, 256), 256, 0, s>>>(
-                matched, ix.bucket_offsets.p, ix.cand.p, raw_cnt.p, n_q, L, cbits, n_win, mid_max, slices.p);
+                bounds, ix.cand.p, raw_cnt.p, n_q, L, cbits, n_win, mid_max, self_lists, slices.p);
             KERNEL_CHECK();
         }
         auto launch = [&](auto nt_tag, auto mk_tag) {
@@ -770,8 +791,8 @@ void query_from_matched(const culsh_index& ix, const int32_t* matched, int n_q, 
             CU_CHECK(cudaFuncSetAttribute(dedupe_chained_rank_kernel<NT, MK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CU_CHECK(cudaFuncSetAttribute(dedupe_chained_rank_kernel<NT, MK>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
             dedupe_chained_rank_kernel<NT, MK><<<(unsigned)n_tk, NT, smem, s>>>(
-                matched, ix.bucket_offsets.p, ix.cand.p, raw_cnt.p, raw_off.p, n_q, L, ix.n, cbits, n_win, stage_ids,
-                mid_max, slices.p, tmp.p, status.p, ticket, out.indices.p, out.counts.p, out.offsets.p, c->d_error);
+                bounds, ix.cand.p, raw_cnt.p, raw_off.p, n_q, L, ix.n, cbits, n_win, stage_ids, mid_max, self_lists,
+                slices.p, tmp.p, status.p, ticket, out.indices.p, out.counts.p, out.offsets.p, c->d_error);
         };
         const long cw_threads = env_long("CULSH_CHAIN_THREADS", 384);
         const long cw_mk = env_long("CULSH_CHAIN_LOADS", 16);
@@ -807,9 +828,8 @@ void query_from_matched(const culsh_index& ix, const int32_t* matched, int n_q, 
             size_t smem = bitmap_smem_bytes(wbits);
             CU_CHECK(cudaFuncSetAttribute(dedupe_bitmap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             if (c->profiling) cudaEventRecord(c->ev_dedupe[0], s);
-            dedupe_bitmap_kernel<<<nb, BM_THREADS, smem, s>>>(big_list.p, matched, ix.bucket_offsets.p,
-                                                              ix.cand.p, raw_off.p, L, ix.n, wbits, tmp.p,
-                                                              out.counts.p);
+            dedupe_bitmap_kernel<<<nb, BM_THREADS, smem, s>>>(big_list.p, bounds, ix.cand.p, raw_off.p,
+                                                              L, ix.n, wbits, tmp.p, out.counts.p);
             KERNEL_CHECK();
             if (c->profiling) { cudaEventRecord(c->ev_dedupe[1], s); dedupe_timed = true; }
         }
@@ -822,9 +842,10 @@ void query_from_matched(const culsh_index& ix, const int32_t* matched, int n_q, 
         if (total) {
             out.indices.alloc(c, total);
             tr.lap("alloc indices");
-            size_t blocks = std::min<size_t>(ceil_div((size_t)n_q * 32, 256), (size_t)c->sm_count * 32);
+            const int per = n_q >= (1 << 17) ? 32 : CS_ROWS;  // from here on full warps still fill the chip
+            const size_t blocks = std::min<size_t>(ceil_div(ceil_div((size_t)n_q, per) * 32, 256), (size_t)c->sm_count * 32);
             compact_small_kernel<<<(unsigned)blocks, 256, 0, s>>>(tmp.p, raw_cnt.p, raw_off.p, out.counts.p,
-                                                                 out.offsets.p, n_q, out.indices.p);
+                                                                 out.offsets.p, n_q, per, out.indices.p);
             KERNEL_CHECK();
             if (nb) {
                 compact_big_kernel<<<nb, 256, 0, s>>>(big_list.p, tmp.p, raw_off.p, out.counts.p,
@@ -858,15 +879,15 @@ void query_batch(const culsh_index& ix, int n_q, HashFn&& hash_fn, culsh_candida
     Scratch<uint32_t> qkeys(c, SL_QKEYS, pairs * NW);
     Scratch<uint8_t> ovf;
     if (ix.family == CULSH_PSLSH && ix.ks.elem_bytes < 4) ovf.reserve(c, SL_QOVF, pairs);
-    Scratch<int32_t> matched(c, SL_MATCHED, pairs);
+    Scratch<int2> bounds(c, SL_BOUNDS, pairs);
     tm.mark();
     hash_fn(ix.ks, qkeys.p, ovf.p);
     tm.mark();
     CULSH_DISPATCH_NW(NW, (lookup_kernel<NW><<<(unsigned)ceil_div(pairs, 256), 256, 0, c->stream>>>(
-                              qkeys.p, ovf.p, n_q, ix.L, ix.bucket_keys.p, ix.table_offsets.p, matched.p)));
+                              qkeys.p, ovf.p, n_q, ix.L, ix.bucket_keys.p, ix.bucket_offsets.p, ix.table_offsets.p, bounds.p)));
     KERNEL_CHECK();
     tm.mark();
-    query_from_matched(ix, matched.p, n_q, out, tm);
+    query_from_matched(ix, query_bounds(bounds.p, n_q), false, out, tm);
     c->stats.hash_ms += tm.between(0, 1);
     c->stats.lookup_ms += tm.between(1, 2);
     c->stats.gather_ms += tm.between(2, 3);
@@ -961,14 +982,14 @@ void fit_query_dense(culsh_handle* h, int family, const T* X, int n, int d, int 
     if (!X) fail(CULSH_ERR_INVALID, "X is null");
     DeviceGuard g(h->ctx->device);
     auto ix = new_dense_index<T>(h, family, n, d, L, k, window, seed);
-    Scratch<int32_t> i2b;
+    Scratch<uint32_t> bounds;
     fit_common(*ix, [&](const KeySpec& ks, uint32_t* keys) {
         hash_dense<T>(*ix, ks, X, n, keys, nullptr, n, 0);
-    }, &i2b);
+    }, &bounds);
     auto res = std::make_unique<culsh_candidates>();
     StageTimer tm(h->ctx);
     tm.mark();
-    query_from_matched(*ix, i2b.p, n, *res, tm);
+    query_from_matched(*ix, self_bounds(*ix, bounds.p), true, *res, tm);
     h->ctx->stats.gather_ms = tm.between(0, 1);
     check_error_word(read_error_word(h->ctx));  // the gather's bounded waits report here
     *out = res.release();
@@ -1244,14 +1265,14 @@ int culsh_minhash_fit_query(culsh_handle* h, const int32_t* indices, const int32
         if (!indptr) fail(CULSH_ERR_INVALID, "indptr is null");
         DeviceGuard g(h->ctx->device);
         auto ix = new_minhash_index(h, n, d, L, k, seed);
-        Scratch<int32_t> i2b;
+        Scratch<uint32_t> bounds;
         fit_common(*ix, [&](const KeySpec& ks, uint32_t* keys) {
             hash_csr(*ix, ks, indices, indptr, n, keys, n, 0);
-        }, &i2b);
+        }, &bounds);
         auto res = std::make_unique<culsh_candidates>();
         StageTimer tm(h->ctx);
         tm.mark();
-        query_from_matched(*ix, i2b.p, n, *res, tm);
+        query_from_matched(*ix, self_bounds(*ix, bounds.p), true, *res, tm);
         h->ctx->stats.gather_ms = tm.between(0, 1);
         check_error_word(read_error_word(h->ctx));  // the gather's bounded waits report here
         *out = res.release();
@@ -1343,13 +1364,13 @@ int culsh_index_query_keys(culsh_handle* h, const culsh_index* ix, const uint32_
         const int NW = ix->ks.key_words;
         const size_t pairs = (size_t)n_q * ix->L;
         StageTimer tm(c);
-        Scratch<int32_t> matched(c, SL_MATCHED, pairs);
+        Scratch<int2> bounds(c, SL_BOUNDS, pairs);
         tm.mark();
         CULSH_DISPATCH_NW(NW, (lookup_kernel<NW><<<(unsigned)ceil_div(pairs, 256), 256, 0, c->stream>>>(
-                                  keys, nullptr, n_q, ix->L, ix->bucket_keys.p, ix->table_offsets.p, matched.p)));
+                                  keys, nullptr, n_q, ix->L, ix->bucket_keys.p, ix->bucket_offsets.p, ix->table_offsets.p, bounds.p)));
         KERNEL_CHECK();
         tm.mark();
-        query_from_matched(*ix, matched.p, n_q, *res, tm);
+        query_from_matched(*ix, query_bounds(bounds.p, n_q), false, *res, tm);
         c->stats.lookup_ms = tm.between(0, 1);
         c->stats.gather_ms = tm.between(1, 2);
         c->stats.total_ms = tm.between(0, 2);

@@ -3,8 +3,8 @@
 // (core/fit.cuh:97-208, 285-363).  The sorted keys sit next to each other, so a boundary
 // is a compare of two adjacent keys (no gather of signatures through the permutation),
 // the sorted row ids already are all_candidate_indices, and one count pass + one write
-// pass produce bucket keys, bucket offsets, table offsets and (for fit_query) the
-// (row, table) -> bucket map.
+// pass produce bucket keys, bucket offsets and table offsets; a self-join takes the list of every
+// (table, row) from the finished buckets (bucket_bounds_kernel).
 #pragma once
 
 #include "common.cuh"
@@ -53,14 +53,13 @@ bucket_count_kernel(const uint32_t* __restrict__ keys, int n, int tiles_per_tabl
 // Items are visited in warp-coalesced order twice: the first sweep records the head flags of
 // the tile as one ballot word per 32 consecutive items, a prefix over those words then gives
 // every item its bucket id, and the second sweep writes bucket keys / offsets (consecutive
-// heads -> consecutive addresses) and the optional (table, row) -> bucket map [L][n].
+// heads -> consecutive addresses).
 template <int NW>
 __global__ void __launch_bounds__(IB_THREADS)
-bucket_write_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ rows, int n,
-                    int L, int tiles_per_table, const uint32_t* __restrict__ tile_base,
-                    uint32_t n_tiles, uint32_t* __restrict__ bucket_keys,
-                    int32_t* __restrict__ bucket_offsets, int32_t* __restrict__ table_offsets,
-                    int32_t* __restrict__ item_to_bucket) {
+bucket_write_kernel(const uint32_t* __restrict__ keys, int n, int L, int tiles_per_table,
+                    const uint32_t* __restrict__ tile_base, uint32_t n_tiles,
+                    uint32_t* __restrict__ bucket_keys, int32_t* __restrict__ bucket_offsets,
+                    int32_t* __restrict__ table_offsets) {
     constexpr int WORDS = IB_TILE / 32;
     __shared__ uint32_t s_bits[WORDS];
     __shared__ uint32_t s_pref[WORDS];
@@ -117,9 +116,6 @@ bucket_write_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restric
             store_key<NW>(bucket_keys + (size_t)bid * NW, kk);
             bucket_offsets[bid] = (int32_t)(tbase + li);
         }
-        // table-major: the writes of one table stay inside its n*4-byte strip, which the L2 merges
-        // into full lines (row-major would touch a separate sector per item)
-        if (item_to_bucket) item_to_bucket[tbase + rows[tbase + li]] = (int32_t)bid;
     }
 }
 
@@ -132,39 +128,126 @@ inline void launch_bucket_count(cudaStream_t s, const uint32_t* keys, int n, int
 }
 
 template <int NW>
-inline void launch_bucket_write(cudaStream_t s, const uint32_t* keys, const uint32_t* rows, int n,
-                                int L, const uint32_t* tile_base, uint32_t* bucket_keys,
-                                int32_t* bucket_offsets, int32_t* table_offsets,
-                                int32_t* item_to_bucket) {
+inline void launch_bucket_write(cudaStream_t s, const uint32_t* keys, int n, int L, const uint32_t* tile_base,
+                                uint32_t* bucket_keys, int32_t* bucket_offsets, int32_t* table_offsets) {
     int tpt = (int)ceil_div(n, IB_TILE);
     uint32_t n_tiles = (uint32_t)((size_t)tpt * L);
-    bucket_write_kernel<NW><<<n_tiles, IB_THREADS, 0, s>>>(keys, rows, n, L, tpt, tile_base, n_tiles,
-                                                          bucket_keys, bucket_offsets, table_offsets,
-                                                          item_to_bucket);
+    bucket_write_kernel<NW><<<n_tiles, IB_THREADS, 0, s>>>(keys, n, L, tpt, tile_base, n_tiles, bucket_keys,
+                                                          bucket_offsets, table_offsets);
     KERNEL_CHECK();
 }
 
-// [L][n] -> [n][L]: 32 x 32 tiles through shared memory, coalesced on both sides.
-__global__ void __launch_bounds__(256)
-transpose_table_major_kernel(const int32_t* __restrict__ src, int n, int L, int32_t* __restrict__ dst) {
-    __shared__ int32_t tile[32][33];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-    const size_t row0 = (size_t)blockIdx.x * 32;
-    const int t0 = blockIdx.y * 32;
+// Self-join: the list of every (table, row), packed into one word, packed[t * n + row]:
+//   0                          the row is alone in its bucket
+//   PB_PAIR | other row        the bucket has two rows (only if asked for)
+//   position | rows << pos_bits  position of the list inside the table; the largest number of rows
+//                              stands for "that many or more", and the reader looks the end up
+// Half of the lists that are worth a look hold two rows: with the other one at hand the gather
+// leaves the random read of the list out.
+constexpr uint32_t PB_PAIR = 0x80000000u;
+struct PackedBounds {
+    int pos_bits;       // bits of n - 1, at most 30
+    uint32_t max_len;   // 2^(31 - pos_bits) - 1
+};
+inline PackedBounds packed_bounds(int n) {
+    int bits = 1;
+    while (bits < 29 && ((uint32_t)(n - 1) >> bits)) ++bits;
+    if ((uint32_t)(n - 1) >> bits) ++bits;
+    return PackedBounds{bits, 0x7FFFFFFFu >> bits};
+}
+
+// `packed` comes zeroed and buckets of one row are left out: they add nothing but the row itself,
+// which the gather supplies, and they are the larger part (10M x 48 tables: 250M of 480M items).
+// A CTA takes the same IB_TILE consecutive items as bucket_write_kernel: the offsets of the buckets
+// that meet the tile come in one coalesced read, their heads are marked in a bit per item, and the
+// pop-count up to an item is its bucket.  Scattered stores bound the kernel: those of a table go to
+// its strip of 4 n bytes, tiles in table order, which the L2 merges into full lines.  (A thread per
+// bucket that walks the bucket's rows waits for one load after another: 11.6 ms at 10M x 48.)
+__global__ void __launch_bounds__(IB_THREADS)
+bucket_bounds_kernel(const int32_t* __restrict__ bucket_offsets, const int32_t* __restrict__ cand, int n, int t0,
+                     int tiles_per_table, const uint32_t* __restrict__ tile_base, PackedBounds pb,
+                     bool pairs, uint32_t* __restrict__ packed) {
+    constexpr int WORDS = IB_TILE / 32;
+    __shared__ int32_t s_off[IB_TILE + 2];  // [0] the bucket before the tile's first head, then its heads, then the next head
+    __shared__ uint32_t s_bits[WORDS];
+    __shared__ uint32_t s_pref[WORDS];
+    const int table = blockIdx.x / tiles_per_table, t = t0 + table;
+    const int lt = blockIdx.x - table * tiles_per_table;
+    const int tile = t * tiles_per_table + lt;
+    const int tbase = t * n;
+    const int first = tbase + lt * IB_TILE, count = min(IB_TILE, n - lt * IB_TILE);
+    const int lane = threadIdx.x & 31;
+    int32_t row[IB_IPT];
 #pragma unroll
-    for (int j = ty; j < 32; j += 8) {
-        const int t = t0 + j;
-        const size_t row = row0 + tx;
-        if (t < L && row < (size_t)n) tile[j][tx] = src[(size_t)t * n + row];
+    for (int i = 0; i < IB_IPT; ++i) {
+        const int local = i * IB_THREADS + threadIdx.x;
+        row[i] = local < count ? cand[first + local] : 0;
+    }
+    const int b0 = (int)tile_base[tile], heads = (int)tile_base[tile + 1] - b0;
+    if (threadIdx.x < WORDS) s_bits[threadIdx.x] = 0;
+    for (int j = threadIdx.x; j < heads + 2; j += IB_THREADS) s_off[j] = b0 - 1 + j >= 0 ? bucket_offsets[b0 - 1 + j] : 0;
+    __syncthreads();
+    for (int j = 1 + threadIdx.x; j <= heads; j += IB_THREADS) {
+        const int local = s_off[j] - first;
+        atomicOr(&s_bits[local >> 5], 1u << (local & 31));
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        uint32_t run = 0;
+        for (int w0 = 0; w0 < WORDS; w0 += 32) {
+            const uint32_t c = __popc(s_bits[w0 + lane]);
+            uint32_t inc = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+                if (lane >= o) inc += x;
+            }
+            s_pref[w0 + lane] = run + inc - c;
+            run += __shfl_sync(0xFFFFFFFFu, inc, 31);
+        }
     }
     __syncthreads();
 #pragma unroll
-    for (int j = ty; j < 32; j += 8) {
-        const size_t row = row0 + j;
-        const int t = t0 + tx;
-        if (row < (size_t)n && t < L) dst[row * L + t] = tile[tx][j];
+    for (int i = 0; i < IB_IPT; ++i) {
+        const int local = i * IB_THREADS + threadIdx.x;
+        if (local >= count) continue;
+        const int j = (int)(s_pref[local >> 5] + __popc(s_bits[local >> 5] & (0xFFFFFFFFu >> (31 - lane))));
+        const int lo = s_off[j], hi = s_off[j + 1];
+        if (hi - lo > 1) {
+            uint32_t word = (uint32_t)(lo - tbase) | (min((uint32_t)(hi - lo), pb.max_len) << pb.pos_bits);
+            if (pairs && hi - lo == 2) word = PB_PAIR | (uint32_t)cand[lo == first + local ? hi - 1 : lo];
+            packed[(size_t)tbase + row[i]] = word;
+        }
     }
 }
+
+// The lists of a set of queries: an array of [x, y) per (table, query), table major, or the packed
+// form of a self-join.
+struct BoundsView {
+    const int2* pair;                // or null: packed
+    const uint32_t* packed;
+    const int32_t* bucket_offsets;   // packed: to find the end of a list that is too long for its word
+    const int32_t* table_offsets;
+    PackedBounds pb;
+    int n_q;                         // queries (a self-join: rows)
+    __device__ __forceinline__ int2 get(int t, int q) const {
+        if (pair) return pair[(size_t)t * n_q + q];
+        return unpack(t, packed[(size_t)t * n_q + q]);
+    }
+    // not for PB_PAIR words
+    __device__ __forceinline__ int2 unpack(int t, uint32_t w) const {
+        if (w == 0) return make_int2(0, 0);
+        const int lo = t * n_q + (int)(w & ((1u << pb.pos_bits) - 1u));
+        const uint32_t len = w >> pb.pos_bits;
+        if (len < pb.max_len) return make_int2(lo, lo + (int)len);
+        int a = table_offsets[t], b = table_offsets[t + 1] - 1;  // the bucket that starts at lo
+        while (a < b) {
+            const int mid = a + ((b - a) >> 1);
+            if (bucket_offsets[mid] < lo) a = mid + 1; else b = mid;
+        }
+        return make_int2(lo, bucket_offsets[a + 1]);
+    }
+};
 
 #define CULSH_DISPATCH_NW(NWVAL, ...)                                         \
     switch (NWVAL) {                                                          \

@@ -8,13 +8,13 @@
 #pragma once
 
 #include "common.cuh"
+#include "index_build.cuh"
 #include "radix_sort.cuh"
 
 namespace culsh_b200 {
 
 // ---------------------------------------------------------------------------------------
 // Lookup: one thread per (table, query); binary search over the table's sorted bucket keys.
-// matched[q*L + t] = bucket id or -1 (same layout as upstream's matched_bucket_indices).
 // ---------------------------------------------------------------------------------------
 template <int NW>
 __device__ __forceinline__ int compare_keys(const uint32_t* __restrict__ a,
@@ -26,82 +26,103 @@ __device__ __forceinline__ int compare_keys(const uint32_t* __restrict__ a,
     return 0;
 }
 
+// bounds[t*n_q + q] = the matched bucket's list [x, y) in `cand`, (0, 0) when there is none.  Table
+// major, like the query keys: neighbouring threads (queries) read and write neighbouring words here,
+// in the count and in the warp path, and a self-join writes the same array from its buckets.
 template <int NW>
 __global__ void __launch_bounds__(256)
 lookup_kernel(const uint32_t* __restrict__ qkeys, const uint8_t* __restrict__ q_ovf, int n_q, int L,
-              const uint32_t* __restrict__ bucket_keys, const int32_t* __restrict__ table_offsets,
-              int32_t* __restrict__ matched) {
+              const uint32_t* __restrict__ bucket_keys, const int32_t* __restrict__ bucket_offsets,
+              const int32_t* __restrict__ table_offsets, int2* __restrict__ bounds) {
     size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)n_q * L) return;
     const int t = (int)(idx / n_q);
-    const int q = (int)(idx - (size_t)t * n_q);
     uint32_t key[NW];
     load_key<NW>(qkeys + idx * NW, key);
     int lo = table_offsets[t], hi = table_offsets[t + 1] - 1;
-    int found = -1;
+    int2 found = make_int2(0, 0);
     if (q_ovf && q_ovf[idx]) hi = lo - 1;  // value outside the index's narrow range: no bucket
     while (lo <= hi) {
         int mid = lo + ((hi - lo) >> 1);
         int c = compare_keys<NW>(key, bucket_keys + (size_t)mid * NW);
-        if (c == 0) { found = mid; break; }
+        if (c == 0) { found = make_int2(bucket_offsets[mid], bucket_offsets[mid + 1]); break; }
         if (c < 0) hi = mid - 1; else lo = mid + 1;
     }
-    matched[(size_t)q * L + t] = found;
+    bounds[idx] = found;
 }
 
 // ---------------------------------------------------------------------------------------
 // Raw (pre-dedupe) candidate count per query; queries above the small-path limit are
-// appended to big_list.
+// appended to big_list.  In a self-join every list of two or more rows holds the query's own row
+// and lists of that row alone are not in `bounds` at all, so the row is counted once and taken
+// off every list: the count is what the result can hold at most.
 // ---------------------------------------------------------------------------------------
 // largest raw count handled by the warp path (1024: 32 ids per lane in the sort network; with 512
 // the queries of 513 - 1024 ids of a 12.5M-row shard took a CTA each on the sort path: 0.77 -> 0.50 ms
 // per 10k queries, the 10M-row self-join, all below 512, is unchanged)
 constexpr int SMALL_MAX = 1024;
+// ... and by its short form (4 ids per lane: 512 bytes of shared memory and 40 registers, so that all
+// of an SM's warp slots are filled; the long form runs at half of that)
+constexpr int SHORT_MAX = 128;
 
-constexpr int RC_BATCH = 8;  // sixteen measured no faster on the 10M-row self-join
+// rows of a packed list other than the query's own
+__device__ __forceinline__ uint32_t packed_count(const BoundsView& bounds, int t, uint32_t w) {
+    if (w == 0) return 0;
+    if (w & PB_PAIR) return 1;
+    const int2 b = bounds.unpack(t, w);
+    return (uint32_t)(b.y - b.x) - 1u;
+}
+
+constexpr int RC_BATCH = 8;
 // counters[0] = queries for the bitmap path (big_list), counters[1] = queries for the
-// shared-memory sort path (mid_list; only used when mid_max > SMALL_MAX)
+// shared-memory sort path (mid_list; only used when mid_max > SMALL_MAX), counters[2] = queries for
+// the long form of the warp path
 __global__ void __launch_bounds__(256)
-raw_count_kernel(const int32_t* __restrict__ matched, const int32_t* __restrict__ bucket_offsets,
-                 int n_q, int L, uint64_t* __restrict__ raw_cnt, uint32_t* __restrict__ big_list,
-                 uint32_t* __restrict__ mid_list, uint32_t* __restrict__ counters, int mid_max,
-                 int2* __restrict__ bounds /* or null: [n_q][L] list bounds for the warp path */) {
+raw_count_kernel(BoundsView bounds, int n_q, int L, bool self_join, uint64_t* __restrict__ raw_cnt,
+                 uint32_t* __restrict__ big_list, uint32_t* __restrict__ mid_list, uint32_t* __restrict__ counters,
+                 int mid_max) {
     int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n_q) return;
-    int2* bq = bounds ? bounds + (size_t)q * L : nullptr;
-    // RC_BATCH tables at a time, branch-free, so that the dependent loads (bucket id -> bounds) of
-    // different tables are in flight together
-    uint64_t c = 0;
-    const int32_t* mq = matched + (size_t)q * L;
+    uint32_t c = self_join ? 1u : 0u;  // at most n * L < 2^31
     int t = 0;
-    for (; t + RC_BATCH <= L; t += RC_BATCH) {
-        int b[RC_BATCH], lo[RC_BATCH], hi[RC_BATCH];
+    for (; t + RC_BATCH <= L; t += RC_BATCH) {  // RC_BATCH loads in flight
+        if (bounds.pair) {
+            int2 b[RC_BATCH];
 #pragma unroll
-        for (int j = 0; j < RC_BATCH; ++j) b[j] = mq[t + j];
+            for (int j = 0; j < RC_BATCH; ++j) b[j] = bounds.pair[(size_t)(t + j) * n_q + q];
 #pragma unroll
-        for (int j = 0; j < RC_BATCH; ++j) {
-            const int bb = max(b[j], 0);
-            lo[j] = bucket_offsets[bb];
-            hi[j] = bucket_offsets[bb + 1];
-        }
+            for (int j = 0; j < RC_BATCH; ++j) c += (uint32_t)(b[j].y - b[j].x);
+        } else {
+            uint32_t w[RC_BATCH];
 #pragma unroll
-        for (int j = 0; j < RC_BATCH; ++j) {
-            c += b[j] >= 0 ? (uint64_t)(hi[j] - lo[j]) : 0ull;
-            if (bq) bq[t + j] = b[j] >= 0 ? make_int2(lo[j], hi[j]) : make_int2(0, 0);
+            for (int j = 0; j < RC_BATCH; ++j) w[j] = bounds.packed[(size_t)(t + j) * n_q + q];
+#pragma unroll
+            for (int j = 0; j < RC_BATCH; ++j) {
+                c += packed_count(bounds, t + j, w[j]);
+            }
         }
     }
     for (; t < L; ++t) {
-        const int b = mq[t];
-        int lo = 0, hi = 0;
-        if (b >= 0) { lo = bucket_offsets[b]; hi = bucket_offsets[b + 1]; }
-        c += (uint64_t)(hi - lo);
-        if (bq) bq[t] = make_int2(lo, hi);
+        if (bounds.pair) {
+            const int2 b = bounds.pair[(size_t)t * n_q + q];
+            c += (uint32_t)(b.y - b.x);
+        } else {
+            c += packed_count(bounds, t, bounds.packed[(size_t)t * n_q + q]);
+        }
     }
     raw_cnt[q] = c;
     if (c > SMALL_MAX) {
-        if (c <= (uint64_t)mid_max) mid_list[atomicAdd(&counters[1], 1u)] = (uint32_t)q;
+        // the sort path gathers a self-join's lists with the own row in each
+        if (c + (self_join ? (uint32_t)L : 0u) <= (uint32_t)mid_max) mid_list[atomicAdd(&counters[1], 1u)] = (uint32_t)q;
         else big_list[atomicAdd(&counters[0], 1u)] = (uint32_t)q;
+    } else if (c > SHORT_MAX) {
+        atomicAdd(&counters[2], 1u);
     }
+}
+
+// A query is on the bitmap / chained path when neither the warp nor the sort path takes it.
+__device__ __forceinline__ bool is_big(uint64_t raw, int mid_max, uint32_t self_lists) {
+    return raw > (uint64_t)SMALL_MAX && raw + self_lists > (uint64_t)mid_max;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -112,129 +133,183 @@ raw_count_kernel(const int32_t* __restrict__ matched, const int32_t* __restrict_
 constexpr int SM_THREADS = 256;
 constexpr int SM_WARPS = SM_THREADS / 32;
 
-// Bitonic sort of 32*E ids held E per lane (position p = 32*e + lane lives in v[e] of `lane`),
-// then adjacent-unique and ballot compaction to out[]; returns the number of unique ids.
-// Exchanges at distance >= 32 stay inside a lane, shorter ones are one shuffle each; everything
-// is unrolled at compile time, so the ids never leave registers.
+// Bitonic sort of 32*E ids, position p = E*lane + e in v[e] of `lane`, then adjacent-unique and
+// ballot compaction to out[]; returns the number of unique ids.  Exchanges at distance < E stay
+// inside a lane, the others are one shuffle and one min / max each.  Every merge starts with the
+// reversing step (partner p ^ (size - 1)), after which all steps go upwards, so that which of the
+// two a lane keeps is one bit of its number.  The network is what the warp path spends its
+// instructions on: with the striped layout (p = 32*e + lane) and alternating directions it took 190
+// instructions for 64 ids instead of 80 and the gather of the 10M-row self-join 8.9 ms instead of 6.3.
 template <int E>
 __device__ __forceinline__ int warp_sort_unique(const int32_t* __restrict__ buf, int r, int lane,
                                                 int32_t* __restrict__ out) {
     int32_t v[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
+    for (int e = 0; e < E; ++e) {  // which id starts where does not matter: the striped read has no bank conflicts
         const int p = 32 * e + lane;
         v[e] = p < r ? buf[p] : 0x7FFFFFFF;
     }
 #pragma unroll
     for (int ksz = 2; ksz <= 32 * E; ksz <<= 1) {
+        if (ksz <= E) {  // reversing step inside the lane
 #pragma unroll
-        for (int j = ksz >> 1; j > 0; j >>= 1) {
-            if (j >= 32) {
-                const int je = j >> 5;
+            for (int e = 0; e < E; ++e) {
+                const int f = e ^ (ksz - 1);
+                if (e < f) {
+                    const int32_t a = v[e], b = v[f];
+                    v[e] = min(a, b);
+                    v[f] = max(a, b);
+                }
+            }
+        } else {  // partner lane ^ (ksz / E - 1), its ids in reverse order
+            const bool low = (lane & (ksz / (2 * E))) == 0;
+            int32_t o[E];
+#pragma unroll
+            for (int e = 0; e < E; ++e) o[e] = __shfl_xor_sync(0xFFFFFFFFu, v[E - 1 - e], ksz / E - 1);
+#pragma unroll
+            for (int e = 0; e < E; ++e) v[e] = low ? min(v[e], o[e]) : max(v[e], o[e]);
+        }
+#pragma unroll
+        for (int j = ksz >> 2; j > 0; j >>= 1) {
+            if (j >= E) {
+                const bool low = (lane & (j / E)) == 0;
 #pragma unroll
                 for (int e = 0; e < E; ++e) {
-                    if ((e & je) == 0) {
-                        const bool up = ((32 * e + lane) & ksz) == 0;
-                        const int32_t a = v[e], b = v[e | je];
-                        const bool sw = (a > b) == up;
-                        v[e] = sw ? b : a;
-                        v[e | je] = sw ? a : b;
-                    }
+                    const int32_t other = __shfl_xor_sync(0xFFFFFFFFu, v[e], j / E);
+                    v[e] = low ? min(v[e], other) : max(v[e], other);
                 }
             } else {
 #pragma unroll
                 for (int e = 0; e < E; ++e) {
-                    const bool up = ((32 * e + lane) & ksz) == 0;
-                    const int32_t other = __shfl_xor_sync(0xFFFFFFFFu, v[e], j);
-                    const bool keep_min = ((lane & j) == 0) == up;
-                    v[e] = keep_min ? min(v[e], other) : max(v[e], other);
+                    if ((e & j) == 0) {
+                        const int32_t a = v[e], b = v[e | j];
+                        v[e] = min(a, b);
+                        v[e | j] = max(a, b);
+                    }
                 }
             }
         }
     }
-    int written = 0;
+    // ids below the first padding value that differ from their predecessor
+    int32_t prev = __shfl_up_sync(0xFFFFFFFFu, v[E - 1], 1);
+    if (lane == 0) prev = -1;
+    int mine = 0;
+    uint32_t keep = 0;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-        int32_t prev = __shfl_up_sync(0xFFFFFFFFu, v[e], 1);
-        if (e > 0) {
-            const int32_t last = __shfl_sync(0xFFFFFFFFu, v[e - 1], 31);
-            if (lane == 0) prev = last;
-        }
-        const int p = 32 * e + lane;
-        const bool keep = p < r && (p == 0 || prev != v[e]);
-        const uint32_t mask = __ballot_sync(0xFFFFFFFFu, keep);
-        if (keep) out[written + __popc(mask & ((1u << lane) - 1))] = v[e];
-        written += __popc(mask);
+        if (v[e] != prev && v[e] != 0x7FFFFFFF) { keep |= 1u << e; ++mine; }
+        prev = v[e];
     }
-    return written;
+    int inc = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if (lane >= o) inc += x;
+    }
+    int32_t* dst = out + (inc - mine);
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+        if (keep & (1u << e)) *dst++ = v[e];
+    return __shfl_sync(0xFFFFFFFFu, inc, 31);
 }
 
-__global__ void __launch_bounds__(SM_THREADS)
-dedupe_small_kernel(const int32_t* __restrict__ matched, const int32_t* __restrict__ bucket_offsets,
-                    const int32_t* __restrict__ cand, const uint64_t* __restrict__ raw_cnt,
-                    const uint64_t* __restrict__ raw_off, int n_q, int L, int32_t* __restrict__ tmp,
-                    uint64_t* __restrict__ uniq_cnt,
-                    const int2* __restrict__ bounds /* or null: list bounds kept by raw_count_kernel */) {
-    __shared__ int32_t s_buf[SM_WARPS][SMALL_MAX];
+// Ids of one list of a lane into the warp's buffer at dst: the first four with independent loads,
+// longer lists by the whole warp.  SELF: without the query's own row, which the list holds once (the
+// ids behind it move up by one).
+template <bool SELF>
+__device__ __forceinline__ void put_id(int32_t* __restrict__ buf, int dst, int32_t x, int q) {
+    if (!SELF) buf[dst] = x;
+    else if (x != q) buf[dst - (x > q ? 1 : 0)] = x;
+}
+
+// Takes the queries with `above` < raw <= CAP (and with `above` = 0 the empty ones).
+template <int CAP, bool SELF>
+__global__ void __launch_bounds__(SM_THREADS, CAP == SHORT_MAX ? 6 : 4)
+dedupe_small_kernel(BoundsView bounds, const int32_t* __restrict__ cand, const uint64_t* __restrict__ raw_cnt,
+                    const uint64_t* __restrict__ raw_off, int L, int above, int32_t* __restrict__ tmp,
+                    uint64_t* __restrict__ uniq_cnt) {
+    __shared__ int32_t s_buf[SM_WARPS][CAP];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n_q = bounds.n_q;
     int32_t* buf = s_buf[warp];
     for (int q = blockIdx.x * SM_WARPS + warp; q < n_q; q += gridDim.x * SM_WARPS) {
         const uint64_t r64 = raw_cnt[q];
-        if (r64 > SMALL_MAX) continue;  // the block path owns it
+        if (r64 > CAP) continue;  // another launch owns it
         const int r = (int)r64;
+        if (above && r <= above) continue;
         if (r == 0) {
             if (lane == 0) uniq_cnt[q] = 0;
             continue;
         }
-        int m = 32;
-        while (m < r) m <<= 1;
-        // gather the bucket lists: 32 tables at a time, one lane per table, so the dependent loads
-        // (bucket id -> list bounds -> ids) of all tables overlap.  A lane copies up to four ids
-        // of its own list with independent loads; longer lists are copied by the whole warp.
+        // Gather the bucket lists: 64 tables at a time, two per lane, so that the dependent loads
+        // (bounds -> ids) of all tables overlap.  A self-join keeps the query's own row out of the
+        // lists and puts it in front: a row of the 10M-row self-join has 91 ids in its 48 lists,
+        // 48 of them its own.
         int fill = 0;
-        for (int t0 = 0; t0 < L; t0 += 32) {
-            const int t = t0 + lane;
-            int s = 0, e = 0;
-            if (bounds) {  // one coalesced read instead of two dependent, scattered ones
-                if (t < L) { const int2 be = bounds[(size_t)q * L + t]; s = be.x; e = be.y; }
-            } else {
-                const int b = t < L ? matched[(size_t)q * L + t] : -1;
-                if (b >= 0) { s = bucket_offsets[b]; e = bucket_offsets[b + 1]; }
+        if (SELF) {
+            if (lane == 0) buf[0] = q;
+            fill = 1;
+        }
+        for (int t0 = 0; t0 < L; t0 += 64) {
+            int s[2], len[2], keep[2];
+            uint32_t w[2] = {0, 0};
+            int2 be[2] = {make_int2(0, 0), make_int2(0, 0)};
+            // neighbouring warps (queries) share the sectors of these table-major reads
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int t = t0 + 32 * h + lane;
+                if (t < L) {
+                    if (SELF) w[h] = bounds.packed[(size_t)t * n_q + q];
+                    else be[h] = bounds.pair[(size_t)t * n_q + q];
+                }
             }
-            const int len = e - s;
-            int inc = len;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (SELF && !(w[h] & PB_PAIR)) be[h] = bounds.unpack(t0 + 32 * h + lane, w[h]);
+                s[h] = be[h].x;
+                len[h] = be[h].y - be[h].x;
+                keep[h] = SELF ? ((w[h] & PB_PAIR) ? 1 : max(len[h] - 1, 0)) : len[h];
+            }
+            int inc = keep[0] | (keep[1] << 16);  // both prefixes in one scan: at most CAP ids each
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
                 if (lane >= o) inc += x;
             }
-            const int dst0 = fill + inc - len;
-            int32_t v[4];
+            const int tot = __shfl_sync(0xFFFFFFFFu, inc, 31);
+            const int dst[2] = {fill + (inc & 0xFFFF) - keep[0], fill + (tot & 0xFFFF) + (inc >> 16) - keep[1]};
+            int32_t v[2][4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) v[i] = i < len ? cand[s + i] : 0;
+            for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (i < len) buf[dst0 + i] = v[i];
-            uint32_t longer = __ballot_sync(0xFFFFFFFFu, len > 4);
-            while (longer) {
-                const int src = __ffs(longer) - 1;
-                longer &= longer - 1;
-                const int ls = __shfl_sync(0xFFFFFFFFu, s, src);
-                const int ll = __shfl_sync(0xFFFFFFFFu, len, src);
-                const int ld = __shfl_sync(0xFFFFFFFFu, dst0, src);
-                for (int i = 4 + lane; i < ll; i += 32) buf[ld + i] = cand[ls + i];
+                for (int i = 0; i < 4; ++i) v[h][i] = i < len[h] ? cand[s[h] + i] : 0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (SELF && (w[h] & PB_PAIR)) buf[dst[h]] = (int32_t)(w[h] & ~PB_PAIR);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (i < len[h]) put_id<SELF>(buf, dst[h] + i, v[h][i], q);
+                uint32_t longer = __ballot_sync(0xFFFFFFFFu, len[h] > 4);
+                while (longer) {
+                    const int src = __ffs(longer) - 1;
+                    longer &= longer - 1;
+                    const int ls = __shfl_sync(0xFFFFFFFFu, s[h], src);
+                    const int ll = __shfl_sync(0xFFFFFFFFu, len[h], src);
+                    const int ld = __shfl_sync(0xFFFFFFFFu, dst[h], src);
+                    for (int i = 4 + lane; i < ll; i += 32) put_id<SELF>(buf, ld + i, cand[ls + i], q);
+                }
             }
-            fill += __shfl_sync(0xFFFFFFFFu, inc, 31);
+            fill += (tot & 0xFFFF) + (tot >> 16);
         }
         __syncwarp();
         int32_t* out = tmp + raw_off[q];
         int written;
-        if (m <= 32) written = warp_sort_unique<1>(buf, r, lane, out);
-        else if (m <= 64) written = warp_sort_unique<2>(buf, r, lane, out);
-        else if (m <= 128) written = warp_sort_unique<4>(buf, r, lane, out);
-        else if (m <= 256) written = warp_sort_unique<8>(buf, r, lane, out);
-        else if (m <= 512) written = warp_sort_unique<16>(buf, r, lane, out);
-        else written = warp_sort_unique<32>(buf, r, lane, out);
+        if (r <= 32) written = warp_sort_unique<1>(buf, r, lane, out);
+        else if (r <= 64) written = warp_sort_unique<2>(buf, r, lane, out);
+        else if (CAP <= 128 || r <= 128) written = warp_sort_unique<4>(buf, r, lane, out);
+        else if (r <= 256) written = warp_sort_unique<CAP <= 128 ? 1 : 8>(buf, r, lane, out);
+        else if (r <= 512) written = warp_sort_unique<CAP <= 128 ? 1 : 16>(buf, r, lane, out);
+        else written = warp_sort_unique<CAP <= 128 ? 1 : 32>(buf, r, lane, out);
         if (lane == 0) uniq_cnt[q] = (uint64_t)written;
         __syncwarp();
     }
@@ -256,10 +331,8 @@ inline size_t sort_path_smem_bytes() {
 }
 
 __global__ void __launch_bounds__(MS_THREADS)
-dedupe_sort_kernel(const uint32_t* __restrict__ mid_list, const int32_t* __restrict__ matched,
-                   const int32_t* __restrict__ bucket_offsets, const int32_t* __restrict__ cand,
-                   const uint64_t* __restrict__ raw_cnt, const uint64_t* __restrict__ raw_off, int L,
-                   int id_bytes, int32_t* __restrict__ tmp, uint64_t* __restrict__ uniq_cnt) {
+dedupe_sort_kernel(const uint32_t* __restrict__ mid_list, BoundsView bounds,
+                   const int32_t* __restrict__ cand, const uint64_t* __restrict__ raw_off, int L, int id_bytes, int32_t* __restrict__ tmp, uint64_t* __restrict__ uniq_cnt) {
     extern __shared__ __align__(16) uint32_t s_ms[];
     uint32_t* bufA = s_ms;
     uint32_t* bufB = bufA + MID_MAX;
@@ -268,16 +341,15 @@ dedupe_sort_kernel(const uint32_t* __restrict__ mid_list, const int32_t* __restr
     uint32_t* s_misc = s_binstart + 256;      // [64]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int q = (int)mid_list[blockIdx.x];
-    const int r = (int)raw_cnt[q];
     // gather the bucket lists one after another
     int fill = 0;
     for (int t = 0; t < L; ++t) {
-        const int b = matched[(size_t)q * L + t];
-        if (b < 0) continue;
-        const int s = bucket_offsets[b], e = bucket_offsets[b + 1];
+        const int2 be = bounds.get(t, q);
+        const int s = be.x, e = be.y;
         for (int i = s + tid; i < e; i += MS_THREADS) bufA[fill + (i - s)] = (uint32_t)cand[i];
         fill += e - s;
     }
+    const int r = fill;  // at most MID_MAX: the count that chose this path allows for it
     __syncthreads();
     const int n_iter = (r + MS_THREADS - 1) / MS_THREADS;  // uniform
     uint32_t* src = bufA;
@@ -460,9 +532,8 @@ __device__ __forceinline__ void mark_lists_flat(uint32_t* __restrict__ bitmap, c
 }
 
 __global__ void __launch_bounds__(BM_THREADS)
-dedupe_bitmap_kernel(const uint32_t* __restrict__ big_list, const int32_t* __restrict__ matched,
-                     const int32_t* __restrict__ bucket_offsets, const int32_t* __restrict__ cand,
-                     const uint64_t* __restrict__ raw_off, int L, int n_rows, int window_bits,
+dedupe_bitmap_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds,
+                     const int32_t* __restrict__ cand, const uint64_t* __restrict__ raw_off, int L, int n_rows, int window_bits,
                      int32_t* __restrict__ tmp, uint64_t* __restrict__ uniq_cnt) {
     extern __shared__ __align__(16) uint32_t s_dyn[];
     uint32_t* bitmap = s_dyn;                                       // [window_bits / 32]
@@ -490,10 +561,10 @@ dedupe_bitmap_kernel(const uint32_t* __restrict__ big_list, const int32_t* __res
             if (tid == 0) s_any = 0;
             __syncthreads();
             for (int t = tid; t < Lg; t += BM_THREADS) {
-                int b = matched[(size_t)q * L + g0 + t];
+                const int2 be = bounds.get(g0 + t, q);
                 int lo = 0, hi = 0, we = 0;
-                if (b >= 0) {
-                    int s = bucket_offsets[b], e = bucket_offsets[b + 1];
+                if (be.y > be.x) {
+                    int s = be.x, e = be.y;
                     if (n_rows <= window_bits) { lo = s; we = e; }
                     else {
                         lo = lower_bound_i32(cand, s, e, win_lo);
@@ -751,19 +822,17 @@ struct ListWalk {
 // with a million independent searches in flight the dependent loads cost nothing, whereas
 // inside the chained kernel they would sit on the critical path of every CTA.
 __global__ void __launch_bounds__(256)
-slice_lists_kernel(const int32_t* __restrict__ matched, const int32_t* __restrict__ bucket_offsets,
-                   const int32_t* __restrict__ cand, const uint64_t* __restrict__ raw_cnt, int n_q, int L,
-                   int window_bits, int n_win, int mid_max, int2* __restrict__ slices) {
+slice_lists_kernel(BoundsView bounds, const int32_t* __restrict__ cand,
+                   const uint64_t* __restrict__ raw_cnt, int n_q, int L, int window_bits, int n_win, int mid_max,
+                   uint32_t self_lists, int2* __restrict__ slices) {
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)n_q * L * n_win) return;
     const int w = (int)(idx % n_win);
     const size_t pair = idx / n_win;  // q * L + t
     const int q = (int)(pair / L), t = (int)(pair - (size_t)q * L);
-    const uint64_t raw = raw_cnt[q];
-    if (!(raw > (uint64_t)SMALL_MAX && raw > (uint64_t)mid_max)) return;  // not a bitmap-path query
-    const int b = matched[pair];
-    int lo = 0, we = 0;
-    if (b >= 0) { lo = bucket_offsets[b]; we = bucket_offsets[b + 1]; }
+    if (!is_big(raw_cnt[q], mid_max, self_lists)) return;
+    const int2 be = bounds.get(t, q);
+    const int lo = be.x, we = be.y;
     int* flat = reinterpret_cast<int*>(slices);
     const size_t mine = (((size_t)q * n_win + w) * L + t) * 2;
     int a = lo;
@@ -778,10 +847,9 @@ slice_lists_kernel(const int32_t* __restrict__ matched, const int32_t* __restric
 
 template <int NT, int MK>
 __global__ void __launch_bounds__(NT)
-dedupe_chained_rank_kernel(const int32_t* __restrict__ matched, const int32_t* __restrict__ bucket_offsets,
-                           const int32_t* __restrict__ cand, const uint64_t* __restrict__ raw_cnt,
+dedupe_chained_rank_kernel(BoundsView bounds, const int32_t* __restrict__ cand, const uint64_t* __restrict__ raw_cnt,
                            const uint64_t* __restrict__ raw_off, int n_q, int L, int n_rows, int window_bits,
-                           int n_win, int stage_ids, int mid_max, const int2* __restrict__ slices /* or null */,
+                           int n_win, int stage_ids, int mid_max, uint32_t self_lists, const int2* __restrict__ slices /* or null */,
                            const int32_t* __restrict__ tmp,
                            unsigned long long* __restrict__ status, uint32_t* __restrict__ ticket,
                            int32_t* __restrict__ out_indices, uint64_t* __restrict__ counts,
@@ -809,8 +877,7 @@ dedupe_chained_rank_kernel(const int32_t* __restrict__ matched, const int32_t* _
     if (tk >= n_tk) return;
     const int q = tk / n_win, w = tk - q * n_win;
     const bool last_ticket = tk == n_tk - 1;
-    const uint64_t raw = raw_cnt[q];
-    const bool big = raw > (uint64_t)SMALL_MAX && raw > (uint64_t)mid_max;
+    const bool big = is_big(raw_cnt[q], mid_max, self_lists);
 
     if (!big) {  // count and ids are in tmp already: window 0 joins the chain with them and copies
         if (w > 0 && !last_ticket) {
@@ -848,10 +915,8 @@ dedupe_chained_rank_kernel(const int32_t* __restrict__ matched, const int32_t* _
         }
     } else {
         if (tid < L) {
-            const int b = matched[(size_t)q * L + tid];
-            int lo = 0, we = 0;
-            if (b >= 0) { lo = bucket_offsets[b]; we = bucket_offsets[b + 1]; }
-            s_lo[tid] = lo; s_we[tid] = we;
+            const int2 be = bounds.get(tid, q);
+            s_lo[tid] = be.x; s_we[tid] = be.y;
         }
         if (n_win > 1) {
             __syncthreads();
@@ -1060,20 +1125,53 @@ compact_big_kernel(const uint32_t* __restrict__ big_list, const int32_t* __restr
     for (uint64_t i = threadIdx.x; i < c; i += blockDim.x) dst[i] = src[i];
 }
 
-// Small queries only (big ones are copied by compact_big_kernel).
+// Small queries only (big ones are copied by compact_big_kernel).  A warp takes `per` <= 32 queries
+// (few for a small set, which would leave the chip idle otherwise), reads
+// their descriptors with one coalesced load each and copies CS_ROWS segments at a time, two words
+// per lane each, so that 2 * CS_ROWS independent loads are in flight; one segment after another
+// left the copy of the 10M-row self-join's 1.8 GB at 1.6 TB/s.
+constexpr int CS_ROWS = 4;
 __global__ void __launch_bounds__(256)
 compact_small_kernel(const int32_t* __restrict__ tmp, const uint64_t* __restrict__ raw_cnt,
                      const uint64_t* __restrict__ raw_off, const uint64_t* __restrict__ uniq_cnt,
-                     const uint64_t* __restrict__ offsets, int n_q, int32_t* __restrict__ out) {
+                     const uint64_t* __restrict__ offsets, int n_q, int per, int32_t* __restrict__ out) {
     const int lane = threadIdx.x & 31;
     const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const size_t n_warps = ((size_t)gridDim.x * blockDim.x) >> 5;
-    for (size_t q = warp; q < (size_t)n_q; q += n_warps) {
-        if (raw_cnt[q] > SMALL_MAX) continue;
-        const uint64_t c = uniq_cnt[q];
-        const int32_t* src = tmp + raw_off[q];
-        int32_t* dst = out + offsets[q];
-        for (uint64_t i = lane; i < c; i += 32) dst[i] = src[i];
+    for (size_t q0 = warp * per; q0 < (size_t)n_q; q0 += n_warps * per) {
+        const size_t q = q0 + lane;
+        uint64_t from = 0, to = 0;
+        int cnt = 0;
+        if (lane < per && q < (size_t)n_q && raw_cnt[q] <= SMALL_MAX) {
+            cnt = (int)uniq_cnt[q];
+            from = raw_off[q];
+            to = offsets[q];
+        }
+        for (int i = 0; i < per; i += CS_ROWS) {
+            const int32_t* src[CS_ROWS];
+            int32_t* dst[CS_ROWS];
+            int c[CS_ROWS], most = 0;
+#pragma unroll
+            for (int j = 0; j < CS_ROWS; ++j) {
+                src[j] = tmp + __shfl_sync(0xFFFFFFFFu, from, i + j);
+                dst[j] = out + __shfl_sync(0xFFFFFFFFu, to, i + j);
+                c[j] = __shfl_sync(0xFFFFFFFFu, cnt, i + j);
+                most = max(most, c[j]);
+            }
+            for (int e = lane; e - lane < most; e += 64) {
+                int32_t a[CS_ROWS], b[CS_ROWS];
+#pragma unroll
+                for (int j = 0; j < CS_ROWS; ++j) {
+                    a[j] = e < c[j] ? src[j][e] : 0;
+                    b[j] = e + 32 < c[j] ? src[j][e + 32] : 0;
+                }
+#pragma unroll
+                for (int j = 0; j < CS_ROWS; ++j) {
+                    if (e < c[j]) dst[j][e] = a[j];
+                    if (e + 32 < c[j]) dst[j][e + 32] = b[j];
+                }
+            }
+        }
     }
 }
 
