@@ -2,6 +2,7 @@
 #include "common.cuh"
 #include "index_build.cuh"
 #include "minhash.cuh"
+#include "project_f64.cuh"
 #include "project_simt.cuh"
 #include "project_tc.cuh"
 #include "query.cuh"
@@ -347,6 +348,13 @@ void hash_dense(const culsh_index& ix, const KeySpec& ks, const T* X, int n, uin
         if (!tc) {
             if (c->projection_path == 2 && !allow_fallback)
                 fail(CULSH_ERR_UNSUPPORTED, "tensor-core projection path is not available for this shape");
+            if constexpr (std::is_same<T, double>::value) {
+                if (c->projection_path != 1 &&
+                    launch_project_f64(c, s, ix.family, Xd, P, bias, rows, ix.d, ix.L, ix.k, ks, keys, ovf_rows, off, n_total)) {
+                    c->stats.hash_path = 0;
+                    return;
+                }
+            }
             launch_project_simt<T>(c, s, ix.family, Xd, P, bias, rows, ix.d, ix.L, ix.k, ks, keys,
                                    ovf_rows, off, n_total);
         }

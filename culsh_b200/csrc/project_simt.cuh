@@ -74,13 +74,37 @@ __device__ __forceinline__ void assemble_key(const int32_t* __restrict__ hv, int
     }
 }
 
+// Pack and store the hash values of `rows` rows and `tables_here` tables in shared memory: consecutive
+// threads -> consecutive rows of one table.
+template <int FAMILY>
+__device__ __forceinline__ void pack_hash_values(const ProjectArgs& a, const int32_t* __restrict__ hbuf, int pitch,
+                                                 int row0, int rows, int first_table, int tables_here, int threads) {
+    const int NW = a.key_words;
+    for (int idx = threadIdx.x; idx < rows * tables_here; idx += threads) {
+        int r = idx % rows, g = idx / rows;
+        int row = row0 + r;
+        if (row >= a.n) continue;
+        int t = first_table + g;
+        uint32_t w[16];
+        bool ovf;
+        assemble_key<FAMILY>(hbuf + r * pitch + g * a.k, a.k, NW, a.elem_bytes, w, ovf);
+        size_t item = (size_t)t * a.n_total + a.row_offset + row;
+        uint32_t* dst = a.keys + item * NW;
+        for (int wi = 0; wi < NW; ++wi) dst[wi] = w[wi];
+        if (FAMILY == CULSH_PSLSH) {
+            if (a.ovf_rows) a.ovf_rows[item] = ovf ? 1 : 0;
+            else if (ovf) atomicOr(a.d_error, DEV_ERR_NARROW_OVERFLOW);
+        }
+    }
+}
+
 template <typename T, int FAMILY>
 __global__ void __launch_bounds__(PS_THREADS)
 project_simt_kernel(ProjectArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* Xs = reinterpret_cast<T*>(smem_raw);                 // [BK][PS_XS]
     T* Ps = Xs + PS_BK * PS_XS;                              // [BK][PS_PS]
-    int32_t* hbuf = reinterpret_cast<int32_t*>(Ps + PS_BK * PS_PS);  // [BM][GC]
+    int32_t* hbuf = reinterpret_cast<int32_t*>(Ps + PS_BK * PS_PS);  // [BM][GC | 1]
 
     const T* __restrict__ X = static_cast<const T*>(a.X);
     const T* __restrict__ P = static_cast<const T*>(a.P);
@@ -92,7 +116,7 @@ project_simt_kernel(ProjectArgs a) {
     const int n_groups = (a.L + G - 1) / G;
     const int group = blockIdx.x % n_groups;  // fastest: the groups of one row block share X in L2
     const int row0 = (blockIdx.x / n_groups) * PS_BM;
-    const int GC = G * a.k;
+    const int GC = G * a.k, pitch = GC | 1;  // odd: the packing threads read one column of many rows
     const int H = a.L * a.k;
     const int col_base = group * GC;
     const int gc_valid = min(GC, H - col_base);
@@ -158,32 +182,14 @@ project_simt_kernel(ProjectArgs a) {
                     } else {
                         q = static_cast<int32_t>(floor(acc[i][j] + bv));  // pslsh/hash.cuh:46
                     }
-                    hbuf[(ty * 8 + i) * GC + lc] = q;
+                    hbuf[(ty * 8 + i) * pitch + lc] = q;
                 }
             }
         }
     }
     __syncthreads();
 
-    // pack and store: consecutive threads -> consecutive rows of one table
-    const int NW = a.key_words;
-    const int tables_here = gc_valid / a.k;
-    for (int idx = tid; idx < PS_BM * tables_here; idx += PS_THREADS) {
-        int r = idx % PS_BM, g = idx / PS_BM;
-        int row = row0 + r;
-        if (row >= a.n) continue;
-        int t = group * G + g;
-        uint32_t w[8];
-        bool ovf;
-        assemble_key<FAMILY>(hbuf + r * GC + g * a.k, a.k, NW, a.elem_bytes, w, ovf);
-        size_t item = (size_t)t * a.n_total + a.row_offset + row;
-        uint32_t* dst = a.keys + item * NW;
-        for (int wi = 0; wi < NW; ++wi) dst[wi] = w[wi];
-        if (FAMILY == CULSH_PSLSH) {
-            if (a.ovf_rows) a.ovf_rows[item] = ovf ? 1 : 0;
-            else if (ovf) atomicOr(a.d_error, DEV_ERR_NARROW_OVERFLOW);
-        }
-    }
+    pack_hash_values<FAMILY>(a, hbuf, pitch, row0, PS_BM, group * G, gc_valid / a.k, PS_THREADS);
 }
 
 inline int simt_tables_per_group(int L, int k) {
@@ -195,7 +201,7 @@ inline int simt_tables_per_group(int L, int k) {
 
 template <typename T>
 inline size_t simt_smem_bytes(int G, int k) {
-    return sizeof(T) * (PS_BK * PS_XS + PS_BK * PS_PS) + sizeof(int32_t) * PS_BM * (size_t)G * k;
+    return sizeof(T) * (PS_BK * PS_XS + PS_BK * PS_PS) + sizeof(int32_t) * PS_BM * (size_t)((G * k) | 1);
 }
 
 // Host launcher.  X may be a chunk (n rows starting at row_offset of an n_total-row index).
