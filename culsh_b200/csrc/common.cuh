@@ -140,6 +140,10 @@ enum ScratchSlot {
     SL_SLICES, SL_BOUNDS, SL_COUNT
 };
 
+// Pinned ring that pageable host arrays go through on their way to the device.
+constexpr int FEED_SLOTS = 16;
+constexpr size_t FEED_PIECE = (size_t)2 << 20;
+
 struct Ctx {
     int device = 0;
     // hash parameters already generated on this handle (they depend only on the key): the
@@ -158,6 +162,8 @@ struct Ctx {
     cudaEvent_t copy_done[2] = {};
     cudaEvent_t chunk_free[2] = {};
     uint64_t* pinned = nullptr;       // 64 x u64 words of pinned host memory
+    void* feed_ring = nullptr;        // pinned ring for pageable host inputs (host_feed.cuh), made on first use
+    cudaEvent_t feed_free[FEED_SLOTS] = {};  // the last copy out of a slot
     int* d_error = nullptr;           // device-side self-check word
     unsigned long long* d_mma = nullptr;  // tensor-core projection: K-blocks issued / with the low-part MMA
     bool profiling = false;
@@ -186,6 +192,8 @@ struct Ctx {
         for (auto& q : slot_ptr) if (q) cudaFree(q);
         for (auto& b : big_free) cudaFree(b.p);
         if (pinned) cudaFreeHost(pinned);
+        for (auto& e : feed_free) if (e) cudaEventDestroy(e);
+        if (feed_ring) cudaFreeHost(feed_ring);
         if (d_error) cudaFree(d_error);
         if (d_mma) cudaFree(d_mma);
         if (copy_stream) cudaStreamDestroy(copy_stream);

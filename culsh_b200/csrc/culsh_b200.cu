@@ -1,5 +1,6 @@
 // Host orchestration and the C ABI of the engine (see include/culsh_b200.h).
 #include "common.cuh"
+#include "host_feed.cuh"
 #include "index_build.cuh"
 #include "minhash.cuh"
 #include "project_f64.cuh"
@@ -377,11 +378,15 @@ void hash_dense(const culsh_index& ix, const KeySpec& ks, const T* X, int n, uin
     CU_CHECK(cudaEventRecord(c->chunk_free[0], c->stream));
     CU_CHECK(cudaEventRecord(c->chunk_free[1], c->stream));
     int slot = 0;
+    HostFeed feed(c, X, (size_t)n * row_bytes);
     for (size_t r0 = 0; r0 < (size_t)n; r0 += chunk_rows, slot ^= 1) {
         const int rows = (int)std::min(chunk_rows, (size_t)n - r0);
         CU_CHECK(cudaStreamWaitEvent(c->copy_stream, c->chunk_free[slot], 0));
-        CU_CHECK(cudaMemcpyAsync(stage[slot].p, reinterpret_cast<const uint8_t*>(X) + r0 * row_bytes,
-                                 rows * row_bytes, cudaMemcpyHostToDevice, c->copy_stream));
+        if (feed.active())
+            feed.copy(stage[slot].p, r0 * row_bytes, rows * row_bytes);
+        else
+            CU_CHECK(cudaMemcpyAsync(stage[slot].p, reinterpret_cast<const uint8_t*>(X) + r0 * row_bytes,
+                                     rows * row_bytes, cudaMemcpyHostToDevice, c->copy_stream));
         CU_CHECK(cudaEventRecord(c->copy_done[slot], c->copy_stream));
         CU_CHECK(cudaStreamWaitEvent(c->stream, c->copy_done[slot], 0));
         launch(c->stream, reinterpret_cast<const T*>(stage[slot].p), rows, row_offset + (int)r0);
@@ -428,6 +433,9 @@ void hash_csr(const culsh_index& ix, const KeySpec& ks, const int32_t* indices, 
         CU_CHECK(cudaEventRecord(c->chunk_free[0], c->stream));
         CU_CHECK(cudaEventRecord(c->chunk_free[1], c->stream));
         int slot = 0;
+        // entries in front of row 0 (indptr[0] > 0) belong to no row
+        const int64_t first = indptr[0];
+        HostFeed feed(c, indices ? indices + first : nullptr, sizeof(int32_t) * (size_t)std::max<int64_t>(nnz - first, 0));
         for (size_t i = 0; i + 1 < cuts.size(); ++i, slot ^= 1) {
             const int r0 = cuts[i], rows = cuts[i + 1] - r0;
             const int64_t e0 = indptr[r0], cnt = indptr[r0 + rows] - e0;
@@ -435,7 +443,9 @@ void hash_csr(const culsh_index& ix, const KeySpec& ks, const int32_t* indices, 
             CU_CHECK(cudaStreamWaitEvent(c->copy_stream, c->chunk_free[slot], 0));
             CU_CHECK(cudaMemcpyAsync(st_ptr[slot].p, indptr + r0, sizeof(int32_t) * ((size_t)rows + 1),
                                      cudaMemcpyHostToDevice, c->copy_stream));
-            if (cnt)
+            if (cnt && feed.active())
+                feed.copy(st_idx[slot].p, sizeof(int32_t) * (size_t)(e0 - first), sizeof(int32_t) * (size_t)cnt);
+            else if (cnt)
                 CU_CHECK(cudaMemcpyAsync(st_idx[slot].p, indices + e0, sizeof(int32_t) * (size_t)cnt,
                                          cudaMemcpyHostToDevice, c->copy_stream));
             CU_CHECK(cudaEventRecord(c->copy_done[slot], c->copy_stream));
@@ -1143,6 +1153,10 @@ int culsh_trim_scratch(culsh_handle* h, uint64_t keep_bytes) {
         DeviceGuard g(c->device);
         CU_CHECK(cudaStreamSynchronize(c->stream));
         CU_CHECK(cudaStreamSynchronize(c->copy_stream));
+        if (c->feed_ring && FEED_SLOTS * FEED_PIECE > keep_bytes) {
+            CU_CHECK(cudaFreeHost(c->feed_ring));
+            c->feed_ring = nullptr;
+        }
         for (int i = 0; i < SL_COUNT; ++i) {
             if (c->slot_ptr[i] && c->slot_cap[i] > keep_bytes) {
                 CU_CHECK(cudaFree(c->slot_ptr[i]));
