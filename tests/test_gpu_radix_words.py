@@ -1,0 +1,41 @@
+"""Keys of four words and more are sorted word by word: row counts on both sides of the 4096-item tile
+and of the 512 tiles from which tile offsets are scanned in chunks, key lengths that end inside a word (16 to 64
+bytes), and collections where the rows agree in the leading, the trailing or all hashes, so that
+the order depends on every word and equal keys keep their row order."""
+import numpy as np
+import pytest
+
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,k", [(1, 3), (31, 16), (4095, 3), (4096, 4), (4097, 5), (8193, 8), (12_289, 9), (20_000, 16), (2_097_153, 3)])
+def test_index_equals_oracle_order(n, k):
+    from culsh_b200 import _culsh_core as core_mod
+    rng = np.random.default_rng(n)
+    L = 2
+    # row r of block b has b's set of ids with a few of the positions changed: many equal hashes
+    sets = rng.integers(0, 400, (max(1, n // 50), 6))
+    rows = sets[rng.integers(0, len(sets), n)]
+    hit = rng.random(n) < 0.3
+    rows[hit, rng.integers(0, 6, int(hit.sum()))] = rng.integers(0, 400, int(hit.sum()))
+    indices = np.ascontiguousarray(rows.astype(np.int32)).ravel()
+    indptr = (6 * np.arange(n + 1)).astype(np.int32)
+    core = core_mod.MinHashCore(L, k, 7)
+    ix = core.fit(indices, indptr, n, 400)
+    sig = core.hash(indices, indptr, n, ix)  # [L][n][k]
+    # the order of the engine: unsigned bytes in memory order, ties by row
+    got_c, got_b = ix.get_candidate_indices(), ix.get_bucket_signatures().reshape(-1, 4 * k)
+    off, tab = ix.get_bucket_candidate_offsets(), ix.get_table_bucket_offsets()
+    for t in range(L):
+        raw = np.ascontiguousarray(sig[t]).view(np.uint8).reshape(n, 4 * k)
+        big = np.ascontiguousarray(raw).view(">u4")
+        order = np.lexsort(tuple(big[:, j] for j in range(k - 1, -1, -1)))
+        assert np.array_equal(got_c[t * n:(t + 1) * n], order)
+        srt = raw[order]
+        head = np.concatenate([[True], (srt[1:] != srt[:-1]).any(axis=1)])
+        assert np.array_equal(got_b[tab[t]:tab[t + 1]], srt[head])
+        assert np.array_equal(off[tab[t]:tab[t + 1]], t * n + np.flatnonzero(head))
+    want = oracle.minhash_signatures(indices[:600], indptr[:min(n, 100) + 1], ix.get_hash_a(), ix.get_hash_b())
+    assert np.array_equal(sig[:, :min(n, 100)].transpose(1, 0, 2).reshape(-1, L * k), want)
