@@ -136,7 +136,7 @@ struct ParamKey {
 enum ScratchSlot {
     SL_STAGE0, SL_STAGE1, SL_CSR_INDPTR, SL_CSR_INDICES, SL_KEYS0, SL_KEYS1, SL_VALS, SL_GHIST,
     SL_STATUS, SL_COUNTER, SL_TILE_HEADS, SL_TILE_BASE, SL_SCAN, SL_RAW_CNT, SL_RAW_OFF,
-    SL_BIG_LIST, SL_NBIG, SL_TMP, SL_QKEYS, SL_QOVF, SL_MISC0, SL_MISC1, SL_MISC2, SL_CHAIN,
+    SL_BIG_LIST, SL_TMP, SL_QKEYS, SL_QOVF, SL_MISC0, SL_MISC1, SL_MISC2, SL_CHAIN,
     SL_SLICES, SL_BOUNDS, SL_COUNT
 };
 
@@ -165,6 +165,7 @@ struct Ctx {
     void* feed_ring = nullptr;        // pinned ring for pageable host inputs (host_feed.cuh), made on first use
     cudaEvent_t feed_free[FEED_SLOTS] = {};  // the last copy out of a slot
     int* d_error = nullptr;           // device-side self-check word
+    int seen_error = 0;               // its value behind the last query
     unsigned long long* d_mma = nullptr;  // tensor-core projection: K-blocks issued / with the low-part MMA
     bool profiling = false;
     int projection_path = 0;
