@@ -134,7 +134,7 @@ inline long env_long_early(const char* name, long dflt) {
 }
 
 void reset_error_word(const CtxPtr& c) {
-    CU_CHECK(cudaMemsetAsync(c->d_error, 0, sizeof(int), c->stream));
+    CU_CHECK(cudaMemsetAsync(c->d_error, 0, 4 * sizeof(int), c->stream));
 }
 
 
@@ -537,20 +537,14 @@ int build_index(culsh_index& ix, SortBuffers& sb, Scratch<uint32_t>* bounds, Sta
     bool compressed = false;
     KeyComp kc{0u, 0u};
     if (SortBuffers::may_compress(ix.ks) && !getenv("CULSH_SORT_PLAIN_KEYS")) {
-        static const uint32_t init[2] = {0u, 256u};
-        Scratch<uint32_t> range(c, SL_MISC1, 2);
-        CU_CHECK(cudaMemcpyAsync(range.p, init, sizeof(init), cudaMemcpyHostToDevice, c->stream));
-        const size_t n_words = (size_t)n * L * NW;
-        key_byte_range_kernel<<<(unsigned)std::min<size_t>(ceil_div(n_words, 1024), (size_t)c->sm_count * 16), 256, 0,
-                                c->stream>>>(sb.keys[0].p, n_words, range.p);
-        KERNEL_CHECK();
-        uint32_t r[2] = {0, 256};
-        read_words(c, range.p, sizeof(r), r);
-        const uint32_t n_pos = r[0] + 1, n_neg = 256 - r[1];
+        int w[4] = {0, 0, 0, 0};
+        read_words(c, c->d_error, sizeof(w), w);
+        if (w[0]) return w[0];  // values that do not fit a byte: no need to sort them
+        const uint32_t n_pos = (uint32_t)w[3] + 1, n_neg = (uint32_t)-w[2];
         if (n_pos + n_neg <= 32 && radix_sort_passes(ix.ks.key_bytes, true) < ix.ks.key_bytes) {
             compressed = true;
             kc.n_pos = n_pos;
-            kc.sub = n_neg ? r[1] - n_pos : 0u;
+            kc.sub = n_neg ? 256u - n_neg - n_pos : 0u;
         }
     }
     const int passes = radix_sort_passes(ix.ks.key_bytes, compressed);
@@ -1128,8 +1122,8 @@ int culsh_create(int device, culsh_handle** out) {
         for (auto& e : c->copy_done) CU_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         for (auto& e : c->chunk_free) CU_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         CU_CHECK(cudaMallocHost(&c->pinned, 64 * sizeof(uint64_t)));
-        CU_CHECK(cudaMalloc(&c->d_error, sizeof(int)));
-        CU_CHECK(cudaMemset(c->d_error, 0, sizeof(int)));
+        CU_CHECK(cudaMalloc(&c->d_error, 4 * sizeof(int)));
+        CU_CHECK(cudaMemset(c->d_error, 0, 4 * sizeof(int)));
         CU_CHECK(cudaMalloc(&c->d_mma, 2 * sizeof(unsigned long long)));
         CU_CHECK(cudaMemset(c->d_mma, 0, 2 * sizeof(unsigned long long)));
         cudaDeviceProp prop{};

@@ -170,6 +170,7 @@ inline bool launch_project_f64(const CtxPtr& c, cudaStream_t stream, int family,
     ProjectArgs a{};
     a.X = X; a.P = P; a.bias = bias; a.keys = keys; a.ovf_rows = ovf_rows;
     a.d_error = c->d_error;
+    a.range = family == CULSH_PSLSH && ks.elem_bytes == 1 && !ovf_rows ? c->d_error + 2 : nullptr;
     a.n = n; a.d = d; a.L = L; a.k = k;
     a.tables_per_group = (int)ceil_div(L, groups);
     a.key_words = ks.key_words;

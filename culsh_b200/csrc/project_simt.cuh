@@ -25,6 +25,7 @@ struct ProjectArgs {
     uint32_t* keys;      // [L][n][NW]
     uint8_t* ovf_rows;   // [L][n] query mode: 1 where a value does not fit elem_bytes; or null
     int* d_error;        // fit mode: NARROW_OVERFLOW is OR-ed here
+    int* range;          // fit mode, p-stable with one-byte elements: HashRange words; or null
     int n, d, L, k;
     int tables_per_group;  // G
     int key_words;         // NW
@@ -80,6 +81,7 @@ template <int FAMILY>
 __device__ __forceinline__ void pack_hash_values(const ProjectArgs& a, const int32_t* __restrict__ hbuf, int pitch,
                                                  int row0, int rows, int first_table, int tables_here, int threads) {
     const int NW = a.key_words;
+    HashRange range;
     for (int idx = threadIdx.x; idx < rows * tables_here; idx += threads) {
         int r = idx % rows, g = idx / rows;
         int row = row0 + r;
@@ -94,8 +96,11 @@ __device__ __forceinline__ void pack_hash_values(const ProjectArgs& a, const int
         if (FAMILY == CULSH_PSLSH) {
             if (a.ovf_rows) a.ovf_rows[item] = ovf ? 1 : 0;
             else if (ovf) atomicOr(a.d_error, DEV_ERR_NARROW_OVERFLOW);
+            if (a.range)
+                for (int j = 0; j < a.k; ++j) range.take(hbuf[r * pitch + g * a.k + j]);
         }
     }
+    if (FAMILY == CULSH_PSLSH && a.range) range.flush(a.range);
 }
 
 template <typename T, int FAMILY>
@@ -214,6 +219,7 @@ inline void launch_project_simt(const CtxPtr& c, cudaStream_t stream, int family
     ProjectArgs a{};
     a.X = X; a.P = P; a.bias = bias; a.keys = keys; a.ovf_rows = ovf_rows;
     a.d_error = c->d_error;
+    a.range = family == CULSH_PSLSH && ks.elem_bytes == 1 && !ovf_rows ? c->d_error + 2 : nullptr;
     a.n = n; a.d = d; a.L = L; a.k = k;
     a.tables_per_group = simt_tables_per_group(L, k);
     a.key_words = ks.key_words;

@@ -52,6 +52,7 @@ struct TcArgs {
     uint32_t* keys;
     uint8_t* ovf_rows;
     int* d_error;
+    int* range;                 // fit mode, p-stable with one-byte elements: HashRange words; or null
     unsigned long long* d_mma;  // [0] K-blocks issued, [1] of them with the low-part MMA (or null)
     const float* bias;
     int n, d, L, k;
@@ -194,7 +195,7 @@ struct KeyReg {
 // columns), as tcgen05.ld requires.
 template <int FAMILY, int KW>
 __device__ __forceinline__ bool epilogue_columns(const TcArgs& a, uint32_t taddr, int c_begin, int c_end,
-                                                 int first_table, int bias_base, int row, bool row_ok) {
+                                                 int first_table, int bias_base, int row, bool row_ok, HashRange& range) {
     const int k = a.k, NW = a.key_words;
     const int bits = FAMILY == CULSH_RPLSH ? 1 : 8 * a.elem_bytes;
     const int lim = a.elem_bytes == 1 ? 128 : (a.elem_bytes == 2 ? 32768 : 0);
@@ -219,6 +220,7 @@ __device__ __forceinline__ bool epilogue_columns(const TcArgs& a, uint32_t taddr
                 } else {
                     const int q = (int)floorf(__uint_as_float(r[j]) + a.bias[bias_base + col]);  // pslsh/hash.cuh:46
                     if (lim && (unsigned)(q + lim) >= (unsigned)(2 * lim)) ovf = true;
+                    if (row_ok) range.take(q);
                     const uint32_t uq = (uint32_t)q;
                     e = a.elem_bytes == 1 ? (uq & 0xFFu)
                         : a.elem_bytes == 2 ? (((uq & 0xFFu) << 8) | ((uq >> 8) & 0xFFu))
@@ -280,10 +282,11 @@ __device__ __forceinline__ bool epilogue_columns(const TcArgs& a, uint32_t taddr
 // bytes - no per-element bookkeeping or branches as in the general form.
 template <int K>
 __device__ __forceinline__ bool epilogue_pslsh_bytes(const TcArgs& a, uint32_t taddr, int c_begin, int c_end,
-                                                     int first_table, int bias_base, int row, bool row_ok) {
+                                                     int first_table, int bias_base, int row, bool row_ok, HashRange& range) {
     constexpr int PER_GROUP = 16 / K;
     constexpr int NW = K <= 4 ? 1 : K / 4;
     bool any_ovf = false;
+    HashRange mine;
     int tbl = first_table;
     int tables_left = (c_end - c_begin) / K;
     for (int g0 = c_begin; g0 < c_end; g0 += 16, tbl += PER_GROUP, tables_left -= PER_GROUP) {
@@ -303,6 +306,7 @@ __device__ __forceinline__ bool epilogue_pslsh_bytes(const TcArgs& a, uint32_t t
                     const int j = ti * K + e;
                     const int q = __float2int_rd(__uint_as_float(r[j]) + __ldg(bias + j));  // pslsh/hash.cuh:46
                     bad |= (uint32_t)(q + 128) >> 8;  // non-zero outside [-128, 127]
+                    mine.take(q);
                     const int pos = NW * 4 - K + e;    // byte position in the key, 0 = most significant
                     w[pos >> 2] |= ((uint32_t)q & 0xFFu) << (24 - 8 * (pos & 3));
                 }
@@ -318,6 +322,7 @@ __device__ __forceinline__ bool epilogue_pslsh_bytes(const TcArgs& a, uint32_t t
             }
         }
     }
+    if (row_ok) { range.take(mine.lo); range.take(mine.hi); }
     return any_ovf;
 }
 
@@ -547,6 +552,7 @@ project_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         uint32_t u = 0;
         bool live = true;
         bool any_ovf = false;
+        HashRange range;
         for (int tile = blockIdx.x; tile < a.n_tiles && live; tile += gridDim.x) {
             const int row = tile * TC_BM + quarter * 32 + lane;
             const bool row_ok = row < a.n;
@@ -564,13 +570,13 @@ project_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     bool o;
                     const bool byte_form = FAMILY == CULSH_PSLSH && a.elem_bytes == 1 && ((tb * k) & 15) == 0;
                     if (FAMILY == CULSH_RPLSH && NW == 1) { epilogue_rplsh_bits(a, taddr, tb * k, te * k, t0 + tb, row, row_ok); o = false; }
-                    else if (byte_form && k == 8) o = epilogue_pslsh_bytes<8>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok);
-                    else if (byte_form && k == 4) o = epilogue_pslsh_bytes<4>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok);
-                    else if (byte_form && k == 16) o = epilogue_pslsh_bytes<16>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok);
-                    else if (byte_form && k == 2) o = epilogue_pslsh_bytes<2>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok);
-                    else if (NW == 1) o = epilogue_columns<FAMILY, 1>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok);
-                    else if (NW == 2) o = epilogue_columns<FAMILY, 2>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok);
-                    else o = epilogue_columns<FAMILY, 0>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok);
+                    else if (byte_form && k == 8) o = epilogue_pslsh_bytes<8>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok, range);
+                    else if (byte_form && k == 4) o = epilogue_pslsh_bytes<4>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok, range);
+                    else if (byte_form && k == 16) o = epilogue_pslsh_bytes<16>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok, range);
+                    else if (byte_form && k == 2) o = epilogue_pslsh_bytes<2>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok, range);
+                    else if (NW == 1) o = epilogue_columns<FAMILY, 1>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok, range);
+                    else if (NW == 2) o = epilogue_columns<FAMILY, 2>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok, range);
+                    else o = epilogue_columns<FAMILY, 0>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok, range);
                     any_ovf |= o;
                 }
                 tc_fence_before();
@@ -579,6 +585,10 @@ project_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             }
         }
         if (any_ovf) atomicOr(a.d_error, DEV_ERR_NARROW_OVERFLOW);
+        if (FAMILY == CULSH_PSLSH && a.range) {
+            __syncwarp();
+            range.flush(a.range);
+        }
     }
 
     tc_fence_before();
@@ -830,6 +840,7 @@ project_ts_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         uint32_t u = 0;
         bool live = true;
         bool any_ovf = false;
+        HashRange range;
         for (int tile = blockIdx.x; tile < a.n_tiles && live; tile += gridDim.x) {
             const int row = tile * TC_BM + quarter * 32 + lane;
             const bool row_ok = row < a.n;
@@ -847,13 +858,13 @@ project_ts_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     bool o;
                     const bool byte_form = FAMILY == CULSH_PSLSH && a.elem_bytes == 1 && ((tb * k) & 15) == 0;
                     if (FAMILY == CULSH_RPLSH && NW == 1) { epilogue_rplsh_bits(a, taddr, tb * k, te * k, t0 + tb, row, row_ok); o = false; }
-                    else if (byte_form && k == 8) o = epilogue_pslsh_bytes<8>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok);
-                    else if (byte_form && k == 4) o = epilogue_pslsh_bytes<4>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok);
-                    else if (byte_form && k == 16) o = epilogue_pslsh_bytes<16>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok);
-                    else if (byte_form && k == 2) o = epilogue_pslsh_bytes<2>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok);
-                    else if (NW == 1) o = epilogue_columns<FAMILY, 1>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok);
-                    else if (NW == 2) o = epilogue_columns<FAMILY, 2>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok);
-                    else o = epilogue_columns<FAMILY, 0>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok);
+                    else if (byte_form && k == 8) o = epilogue_pslsh_bytes<8>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok, range);
+                    else if (byte_form && k == 4) o = epilogue_pslsh_bytes<4>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok, range);
+                    else if (byte_form && k == 16) o = epilogue_pslsh_bytes<16>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok, range);
+                    else if (byte_form && k == 2) o = epilogue_pslsh_bytes<2>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok, range);
+                    else if (NW == 1) o = epilogue_columns<FAMILY, 1>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok, range);
+                    else if (NW == 2) o = epilogue_columns<FAMILY, 2>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok, range);
+                    else o = epilogue_columns<FAMILY, 0>(a, taddr, tb * k, te * k, t0 + tb, t0 * k, row, row_ok, range);
                     any_ovf |= o;
                 }
                 tc_fence_before();
@@ -862,6 +873,10 @@ project_ts_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             }
         }
         if (any_ovf) atomicOr(a.d_error, DEV_ERR_NARROW_OVERFLOW);
+        if (FAMILY == CULSH_PSLSH && a.range) {
+            __syncwarp();
+            range.flush(a.range);
+        }
     }
 
     tc_fence_before();
@@ -1029,6 +1044,7 @@ inline bool launch_project_tc(const CtxPtr& c, cudaStream_t stream, int family, 
         return false;
     TcArgs a{};
     a.keys = keys; a.ovf_rows = ovf_rows; a.d_error = c->d_error; a.bias = bias;
+    a.range = family == CULSH_PSLSH && ks.elem_bytes == 1 && !ovf_rows ? c->d_error + 2 : nullptr;
     a.d_mma = c->d_mma;
     a.n = n; a.d = d; a.L = L; a.k = k;
     a.n_tiles = (int)ceil_div(n, TC_BM);

@@ -489,40 +489,6 @@ radix_key_gather_kernel(const uint32_t* __restrict__ keys, const uint32_t* __res
 }
 
 // ---------------------------------------------------------------------------------------
-// Range of the key bytes of p-stable keys with one byte per hash: out[0] = largest byte below
-// 128 (largest non-negative hash value, 0 if none), out[1] = smallest byte from 128 up (the
-// smallest negative value as an unsigned byte, 256 if none).  out must hold {0, 256} before.
-// ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
-key_byte_range_kernel(const uint32_t* __restrict__ keys, size_t n_words, uint32_t* __restrict__ out) {
-    uint32_t hi_pos = 0, lo_neg = 256;
-    auto take = [&](uint32_t w) {
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const uint32_t u = (w >> (8 * b)) & 0xFFu;
-            if (u < 128u) hi_pos = max(hi_pos, u); else lo_neg = min(lo_neg, u);
-        }
-    };
-    const size_t n4 = n_words / 4;  // the key array starts on a 16-byte boundary
-    const uint4* k4 = reinterpret_cast<const uint4*>(keys);
-    const size_t stride = (size_t)gridDim.x * blockDim.x, first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (size_t i = first; i < n4; i += stride) {
-        const uint4 v = k4[i];
-        take(v.x); take(v.y); take(v.z); take(v.w);
-    }
-    for (size_t i = 4 * n4 + first; i < n_words; i += stride) take(keys[i]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        hi_pos = max(hi_pos, __shfl_xor_sync(0xFFFFFFFFu, hi_pos, o));
-        lo_neg = min(lo_neg, __shfl_xor_sync(0xFFFFFFFFu, lo_neg, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(&out[0], hi_pos);
-        atomicMin(&out[1], lo_neg);
-    }
-}
-
-// ---------------------------------------------------------------------------------------
 // Host driver.  keys[0]/vals[0] hold the input (vals[0] is never read: the first pass
 // takes the row id from the position); after radix_sort_passes() passes the result is in
 // buffer radix_sort_final(passes, NW).  tile_hist must hold radix_sort_tile_words(n, L, NW) words.

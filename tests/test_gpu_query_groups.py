@@ -1,0 +1,49 @@
+"""Batches of a query share their launches as long as their lists are few, and the scans of a batch run in
+one CTA up to 32,768 queries: query counts at the edges of the scan's 8192-element steps and of that line, batch
+sizes that leave a rest, and lists of more than 2^25 entries, which are taken batch by batch, have to give
+what one batch gives.  P-stable fits keep the range of their hash values on the way: bytes at the edges of
+the compressed sort (32 levels) and of the byte itself, in each projection kernel."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _same(a, b):
+    for f in ("get_indices", "get_offsets", "get_counts"):
+        assert np.array_equal(getattr(a, f)(), getattr(b, f)())
+
+
+@pytest.mark.parametrize("nq,batch", [(8191, 1000), (8192, 8191), (8193, 64), (32_767, 32_766), (32_768, 5000), (32_769, 16_384)])
+def test_query_counts(nq, batch):
+    import culsh_b200 as culsh
+    rng = np.random.default_rng(nq)
+    X = rng.standard_normal((20_000, 16)).astype(np.float32)
+    Q = rng.standard_normal((nq, 16)).astype(np.float32)
+    m = culsh.RPLSH(6, 14, seed=2).fit(X)
+    _same(m.query(Q, batch_size=batch), m.query(Q))
+
+
+def test_long_lists_go_batch_by_batch():
+    import culsh_b200 as culsh
+    rng = np.random.default_rng(0)
+    X = rng.standard_normal((100_000, 8)).astype(np.float32)
+    m = culsh.RPLSH(4, 2, seed=2).fit(X)
+    Q = rng.standard_normal((501, 8)).astype(np.float32)  # about 4 x 25,000 entries each: 2^25.6
+    _same(m.query(Q, batch_size=100), m.query(Q))
+
+
+@pytest.mark.parametrize("dtype,d,k", [(np.float32, 8, 8), (np.float32, 8, 5), (np.float32, 7, 4), (np.float64, 8, 8)])
+@pytest.mark.parametrize("scale", [0.3, 3.0, 4.5, 12.0, 40.0])
+def test_hash_value_range(dtype, d, k, scale):
+    from culsh_b200 import _culsh_core as core_mod
+    n, L = 5000, 3
+    X = (scale * np.random.default_rng(d).standard_normal((n, d))).astype(dtype)
+    core = core_mod.PSLSHCore(L, k, 1, 3)
+    ix = (core.fit_float if dtype == np.float32 else core.fit_double)(X, n, d)
+    sig = core.hash(X, ix)  # [L][n][k] at full width
+    cand = ix.get_candidate_indices()
+    for t in range(L):
+        raw = np.ascontiguousarray(sig[t]).view(np.uint8).reshape(n, 4 * k)
+        order = np.lexsort(tuple(raw[:, j] for j in range(4 * k - 1, -1, -1)))
+        assert np.array_equal(cand[t * n:(t + 1) * n], order)
