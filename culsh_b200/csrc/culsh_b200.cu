@@ -503,8 +503,8 @@ struct SortBuffers {
         tile_hist.reserve(c, SL_STATUS, radix_sort_tile_words(n, L, ks.key_words));
     }
     // the last pass must write the row ids into vals_out
-    void set_passes(int passes, int key_words) {
-        final_buf = radix_sort_final(passes, key_words);
+    void set_final(int buf) {
+        final_buf = buf;
         vals[final_buf] = vals_out.p;
         vals[final_buf ^ 1] = vals_tmp.p;
     }
@@ -548,7 +548,7 @@ int build_index(culsh_index& ix, SortBuffers& sb, Scratch<uint32_t>* bounds, Sta
         }
     }
     const int passes = radix_sort_passes(ix.ks.key_bytes, compressed);
-    sb.set_passes(passes, NW);
+    sb.set_final(radix_sort_final(c, passes, n, L, NW, compressed));
     uint32_t* kp[2] = {sb.keys[0].p, sb.keys[1].p};
     uint32_t* vp[2] = {sb.vals[0], sb.vals[1]};
     int cur = radix_sort_tables(c, NW, kp, vp, n, L, ix.ks.key_bytes, sb.tile_hist.p, compressed, kc);

@@ -271,13 +271,28 @@ radix_chunk_base_kernel(uint32_t* __restrict__ chunk_tot, int n_chunks) {
 // ---------------------------------------------------------------------------------------
 // Pass step 3: stable scatter of one tile on byte `p`.
 //
-// Shared memory and the latency between its phases bound it, not HBM (8-byte items move at 3.2 TB/s of
+// Shared memory and the latency between its phases bound it, not HBM (8-byte items move at 3.9 TB/s of
 // the 6.5 a copy reaches).  Ranking costs a random shared-memory read and a write of the digits' last
 // lanes per 32 items; counting with atomics and a broadcast of their result took a shuffle and a second random read
 // in the reorder more, and words of lane bits set with atomicOr were slower where digits repeat.
-// Whole tiles have no bounds in the code.  480M items of 4 + 4 bytes: 2.66 -> 2.4 ms a pass; 200M packed
-// items of 8 bytes: first pass 1.59 -> 1.13, middle ones 1.26 -> 0.96.
+// Whole tiles have no bounds in the code.  480M items of 4 + 4 bytes: 2.66 -> 2.0 ms a pass; 200M packed
+// items of 8 bytes: first pass 1.59 -> 0.87, middle ones 1.26 -> 0.73, last 1.25 -> 0.90.
 // ---------------------------------------------------------------------------------------
+// Takes the lanes that differ from this one in the bit `mask` of d out of `lanes`.  Spelled out because the
+// scatter is bound by what it issues: with a ballot and a select in C++ 32M items of 4 + 4 bytes took 155 us a
+// pass, this way 128.
+__device__ __forceinline__ void keep_same_bit(uint32_t& lanes, uint32_t d, uint32_t mask) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b32 t, m;\n\t"
+        "and.b32 t, %1, %2;\n\t"
+        "setp.ne.b32 p, t, 0;\n\t"
+        "vote.sync.ballot.b32 m, p, 0xffffffff;\n\t"
+        "@!p not.b32 m, m;\n\t"
+        "and.b32 %0, %0, m;\n\t}"
+        : "+r"(lanes)
+        : "r"(d), "r"(mask));
+}
+
 // COMP: 0 plain keys; 1 first pass of a compressed sort (keys are compressed as they are
 // loaded); 2 its last pass (the original bytes are written back); 3 plain keys that nobody reads
 // after this pass (the last one over a word of a wide key): only the ids are written.
@@ -368,10 +383,7 @@ radix_scatter_kernel(const uint32_t* __restrict__ keys_in, const uint32_t* __res
             } else {
                 peers = FULL ? 0xFFFFFFFFu : __ballot_sync(0xFFFFFFFFu, ok);
 #pragma unroll
-                for (int b = 0; b < 8; ++b) {
-                    const uint32_t m = __ballot_sync(0xFFFFFFFFu, (d >> b) & 1u);
-                    peers &= ~(m ^ (uint32_t)((int)(d << (31 - b)) >> 31));
-                }
+                for (int b = 0; b < 8; ++b) keep_same_bit(peers, d, 1u << b);
             }
             pos[i] = bins[d] + __popc(peers & below);
             __syncwarp();
@@ -489,13 +501,198 @@ radix_key_gather_kernel(const uint32_t* __restrict__ keys, const uint32_t* __res
 }
 
 // ---------------------------------------------------------------------------------------
+// Short tables: one CTA sorts a whole table, every pass in shared memory.  A pass of the general form is
+// three launches, of which a table of a few thousand rows fills a few CTAs for 2 us each: what such a
+// sort costs are its 15 launches (48 and more for keys of four words) and the gaps between them.
+// 1,000 rows x 8 tables, five passes of packed items: 70 us of launches and gaps against 14 here; 10,000 x 16: 80
+// against 40.
+// Above 12,288 items (8,192 of two words and an id) a table no longer fits the registers of one CTA.
+// ---------------------------------------------------------------------------------------
+constexpr int RSS_THREADS = 1024;
+constexpr int RSS_WARPS = RSS_THREADS / 32;
+template <int NW, bool PACK>
+struct SmallSortCfg {
+    static constexpr int KW = NW >= 4 ? 1 : NW;  // key words an item carries (wide keys: the word being sorted)
+    static constexpr int IPT = KW == 1 || PACK ? 12 : 8;
+    static constexpr int MAX_ROWS = RSS_THREADS * IPT;
+    static constexpr size_t SMEM = sizeof(uint32_t) * ((size_t)MAX_ROWS * (KW + (PACK ? 0 : 1)) + RSS_WARPS * 256 + 4 * 256 + 256 + 8);
+};
+
+// COMP as a runtime flag: keys are compressed as they are loaded and restored as they are stored.
+template <int NW, bool PACK>
+__global__ void __launch_bounds__(RSS_THREADS, 1)
+radix_sort_small_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
+                        uint32_t* __restrict__ vals_out, int n, int passes, bool compressed, KeyComp kc) {
+    using Cfg = SmallSortCfg<NW, PACK>;
+    constexpr int KW = Cfg::KW, IPT = Cfg::IPT;
+    constexpr bool WORDS = NW >= 4;
+    extern __shared__ __align__(16) uint32_t smem[];
+    uint32_t* s_keys = smem;                                     // [MAX_ROWS][KW]
+    uint32_t* s_vals = s_keys + (size_t)Cfg::MAX_ROWS * KW;      // [MAX_ROWS], not packed
+    uint32_t* s_bins = s_vals + (PACK ? 0 : Cfg::MAX_ROWS);      // [RSS_WARPS][256]
+    uint32_t* s_part = s_bins + RSS_WARPS * 256;                 // [4][256]
+    uint32_t* s_start = s_part + 4 * 256;                        // [256]
+    uint32_t* s_warp = s_start + 256;                            // [8]
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const size_t base = (size_t)blockIdx.x * n;
+    const int steps = (n + RSS_THREADS - 1) / RSS_THREADS;  // at most IPT
+    const int first = warp * (32 * steps) + lane;           // a warp holds 32 * steps consecutive items
+    const uint32_t below = (1u << lane) - 1u;
+    uint32_t* bins = s_bins + warp * 256;
+    uint32_t key[IPT][KW], val[IPT], pos[IPT];
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) {
+        const int li = first + i * 32;
+#pragma unroll
+        for (int w = 0; w < KW; ++w) key[i][w] = 0;
+        val[i] = (uint32_t)li;
+        if (!WORDS && i < steps && li < n) {
+            load_key<KW>(keys_in + (base + li) * KW, key[i]);
+            if constexpr (!WORDS) {
+                if (compressed) comp_key<KW>(key[i], kc.sub);
+            }
+            if constexpr (PACK) {
+                key[i][0] = (key[i][0] << RS_PACK_ID_BITS) | (key[i][KW - 1] >> (32 - RS_PACK_ID_BITS));
+                key[i][KW - 1] = (key[i][KW - 1] << RS_PACK_ID_BITS) | (uint32_t)li;
+            }
+        }
+    }
+    for (int p = 0; p < passes; ++p) {
+        if (WORDS && (p & 3) == 0) {  // the next word of the key, from where the keys are
+#pragma unroll
+            for (int i = 0; i < IPT; ++i)
+                if (i < steps && first + i * 32 < n) key[i][0] = keys_in[(base + val[i]) * NW + (NW - 1 - (p >> 2))];
+        }
+        const int pd = PACK ? p + 3 : (WORDS ? (p & 3) : p);
+        const int dword = KW - 1 - (pd >> 2), dshift = 8 * (pd & 3);
+        auto digit = [&](const uint32_t* k) { return ((KW == 2 && dword == 1 ? k[KW - 1] : k[0]) >> dshift) & 0xFFu; };
+#pragma unroll
+        for (int i = 0; i < RSS_WARPS * 256 / 4 / RSS_THREADS; ++i)
+            reinterpret_cast<uint4*>(s_bins)[i * RSS_THREADS + tid] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) {
+            if (i < steps) {
+                const bool ok = first + i * 32 < n;
+                const uint32_t d = digit(key[i]);
+                uint32_t peers = __ballot_sync(0xFFFFFFFFu, ok);
+#pragma unroll
+                for (int b = 0; b < 8; ++b) keep_same_bit(peers, d, 1u << b);
+                pos[i] = bins[d] + __popc(peers & below);
+                __syncwarp();
+                if (ok && (peers >> lane) == 1u) bins[d] = pos[i] + 1u;
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+        // starts: a thread takes one bin and eight of the warps
+        const int b = tid & 255, q = tid >> 8;
+        uint32_t sum = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) sum += s_bins[(q * 8 + w) * 256 + b];
+        s_part[tid] = sum;
+        __syncthreads();
+        if (tid < 256) {
+            const uint32_t tot = s_part[tid] + s_part[256 + tid] + s_part[512 + tid] + s_part[768 + tid];
+            uint32_t inc = tot;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+                if (lane >= o) inc += x;
+            }
+            if (lane == 31) s_warp[warp] = inc;
+            s_start[tid] = inc - tot;
+        }
+        __syncthreads();
+        uint32_t run = s_start[b];
+        for (int w = 0; w < (b >> 5); ++w) run += s_warp[w];
+        for (int g = 0; g < q; ++g) run += s_part[g * 256 + b];
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            const uint32_t x = s_bins[(q * 8 + w) * 256 + b];
+            s_bins[(q * 8 + w) * 256 + b] = run;
+            run += x;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) {
+            if (i < steps && first + i * 32 < n) {
+                const uint32_t to = bins[digit(key[i])] + pos[i];
+                store_key<KW>(s_keys + (size_t)to * KW, key[i]);
+                if constexpr (!PACK) s_vals[to] = val[i];
+            }
+        }
+        __syncthreads();
+        if (p == passes - 1) break;
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) {
+            if (i < steps && first + i * 32 < n) {
+                load_key<KW>(s_keys + (size_t)(first + i * 32) * KW, key[i]);
+                if constexpr (!PACK) val[i] = s_vals[first + i * 32];
+            }
+        }
+    }
+    for (int at = tid; at < n; at += RSS_THREADS) {
+        uint32_t id;
+        if constexpr (WORDS) {
+            id = s_vals[at];
+            uint32_t kk[NW];
+            load_key<NW>(keys_in + (base + id) * NW, kk);
+            store_key<NW>(keys_out + (base + at) * NW, kk);
+        } else {
+            uint32_t kk[KW];
+            load_key<KW>(s_keys + (size_t)at * KW, kk);
+            if constexpr (PACK) {
+                id = kk[KW - 1] & ((1u << RS_PACK_ID_BITS) - 1u);
+                kk[KW - 1] = (kk[0] << (32 - RS_PACK_ID_BITS)) | (kk[KW - 1] >> RS_PACK_ID_BITS);
+                kk[0] >>= RS_PACK_ID_BITS;
+            } else {
+                id = s_vals[at];
+            }
+            if (compressed) decomp_key<KW>(kk, kc);
+            store_key<KW>(keys_out + (base + at) * KW, kk);
+        }
+        vals_out[base + at] = id;
+    }
+}
+
+// keys[0] -> keys[1], row ids to vals[1]
+template <int NW>
+inline int radix_sort_small(const CtxPtr& c, uint32_t* keys[2], uint32_t* vals[2], int n, int L, int passes,
+                            bool compressed, KeyComp kc) {
+    auto go = [&](auto kern, size_t smem) {
+        CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (c->profiling) cudaEventRecord(c->ev_pass[0], c->stream);
+        kern<<<(unsigned)L, RSS_THREADS, smem, c->stream>>>(keys[0], keys[1], vals[1], n, passes, compressed, kc);
+        KERNEL_CHECK();
+        if (c->profiling) cudaEventRecord(c->ev_pass[1], c->stream);
+    };
+    if constexpr (NW == 2) {
+        if (compressed) go(radix_sort_small_kernel<2, true>, SmallSortCfg<2, true>::SMEM);
+        else go(radix_sort_small_kernel<2, false>, SmallSortCfg<2, false>::SMEM);
+    } else {
+        go(radix_sort_small_kernel<NW, false>, SmallSortCfg<NW, false>::SMEM);
+    }
+    return 1;
+}
+
+// ---------------------------------------------------------------------------------------
 // Host driver.  keys[0]/vals[0] hold the input (vals[0] is never read: the first pass
 // takes the row id from the position); after radix_sort_passes() passes the result is in
 // buffer radix_sort_final(passes, NW).  tile_hist must hold radix_sort_tile_words(n, L, NW) words.
 // `compressed` (NW <= 2 only): sort the 5-bit-per-byte form of the keys, see the top of the file.
 // ---------------------------------------------------------------------------------------
 inline int radix_sort_passes(int KB, bool compressed) { return compressed ? (5 * KB + 7) / 8 : KB; }
-inline int radix_sort_final(int passes, int NW) { return NW >= 4 ? 1 : passes & 1; }
+// Tables that one CTA sorts, no more of them than there are SMs (CULSH_SORT_NO_PACK keeps the general form).
+inline bool radix_sort_is_small(const CtxPtr& c, int n, int L, int NW, bool compressed) {
+    const char* no_pack = getenv("CULSH_SORT_NO_PACK");
+    const int rows = NW == 2 && !compressed ? SmallSortCfg<2, false>::MAX_ROWS : SmallSortCfg<1, false>::MAX_ROWS;
+    return n <= rows && L <= c->sm_count && SmallSortCfg<2, true>::SMEM <= c->smem_optin && !(no_pack && atoi(no_pack) != 0);
+}
+inline int radix_sort_final(const CtxPtr& c, int passes, int n, int L, int NW, bool compressed) {
+    return NW >= 4 || radix_sort_is_small(c, n, L, NW, compressed) ? 1 : passes & 1;
+}
 
 // Pass step 2 on the host: tile histograms -> destination offsets.  Tables of many tiles leave the bases
 // of their chunks behind the tile histograms, [table][chunk][256].
@@ -623,6 +820,16 @@ inline size_t radix_sort_tile_words(int n, int L, int NW) {
 inline int radix_sort_tables(const CtxPtr& c, int NW, uint32_t* keys[2], uint32_t* vals[2], int n,
                              int L, int KB, uint32_t* tile_hist, bool compressed = false,
                              KeyComp kc = KeyComp{0u, 0u}) {
+    if (radix_sort_is_small(c, n, L, NW, compressed)) {
+        const int passes = radix_sort_passes(KB, compressed);
+        switch (NW) {
+            case 1: return radix_sort_small<1>(c, keys, vals, n, L, passes, compressed, kc);
+            case 2: return radix_sort_small<2>(c, keys, vals, n, L, passes, compressed, kc);
+            case 4: return radix_sort_small<4>(c, keys, vals, n, L, passes, compressed, kc);
+            case 8: return radix_sort_small<8>(c, keys, vals, n, L, passes, compressed, kc);
+            case 16: return radix_sort_small<16>(c, keys, vals, n, L, passes, compressed, kc);
+        }
+    }
     switch (NW) {
         case 1: return radix_sort_tables_nw<1>(c, keys, vals, n, L, KB, tile_hist, compressed, kc);
         case 2: return radix_sort_tables_nw<2>(c, keys, vals, n, L, KB, tile_hist, compressed, kc);
