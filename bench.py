@@ -649,6 +649,8 @@ def line_of(torch, args, wl, spec, world, m, peaks, tf32):
     sf, sq = stage["fit"][-1], stage["query"][-1]
     passes = max(1, sf["sort_passes"])
     items, kb = sf["n_items"], 4 * sf["key_words"]
+    # keys of four words and more: the last pass reads (word, row id) and writes the ids
+    item_bytes = 12.0 if sf["key_words"] >= 4 else (kb + 4) * 2.0
     roof = {}
     if spec["family"] == "minhash":
         nnz = m["nnz"]
@@ -672,7 +674,7 @@ def line_of(torch, args, wl, spec, world, m, peaks, tf32):
                                 "launch; peak = TF32 dense matmul measured in this run (8192^3) / 3 (3xTF32)",
                         "tf32_tflops_measured": tf32}
     if scatter_ms > 0:
-        roof["sort"] = {"bound": "hbm", "achieved": items * (kb + 4) * 2.0 / (scatter_ms * 1e-3) / 1e9,
+        roof["sort"] = {"bound": "hbm", "achieved": items * item_bytes / (scatter_ms * 1e-3) / 1e9,
                         "peak": peaks["hbm_gbs"], "unit": "GB/s", "kernel": "radix_scatter_kernel", "traffic": None,
                         "note": f"(key {kb} B + row id 4 B) read + written per item, one launch (the scatter of the "
                                 f"last of {passes} passes) timed with CUDA events; peak {peaks['source']}"}

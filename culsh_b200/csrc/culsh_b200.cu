@@ -3,6 +3,7 @@
 #include "host_feed.cuh"
 #include "index_build.cuh"
 #include "minhash.cuh"
+#include "project_f32.cuh"
 #include "project_f64.cuh"
 #include "project_simt.cuh"
 #include "project_tc.cuh"
@@ -347,12 +348,14 @@ void hash_dense(const culsh_index& ix, const KeySpec& ks, const T* X, int n, uin
         if (!tc) {
             if (c->projection_path == 2 && !allow_fallback)
                 fail(CULSH_ERR_UNSUPPORTED, "tensor-core projection path is not available for this shape");
-            if constexpr (std::is_same<T, double>::value) {
+            c->stats.hash_path = 0;
+            if constexpr (std::is_same<T, double>::value) {  // path 1: the CUDA cores
                 if (c->projection_path != 1 &&
-                    launch_project_f64(c, s, ix.family, Xd, P, bias, rows, ix.d, ix.L, ix.k, ks, keys, ovf_rows, off, n_total)) {
-                    c->stats.hash_path = 0;
+                    launch_project_f64(c, s, ix.family, Xd, P, bias, rows, ix.d, ix.L, ix.k, ks, keys, ovf_rows, off, n_total))
                     return;
-                }
+            } else {
+                if (launch_project_f32(c, s, ix.family, Xd, P, bias, rows, ix.d, ix.L, ix.k, ks, keys, ovf_rows, off, n_total))
+                    return;
             }
             launch_project_simt<T>(c, s, ix.family, Xd, P, bias, rows, ix.d, ix.L, ix.k, ks, keys,
                                    ovf_rows, off, n_total);

@@ -3,8 +3,9 @@
 // Replaces upstream's cublasSgemm/Dgemm + compute_signatures_kernel (rplsh/hash.cuh:24-48,
 // 93-129) and + bias_floor_reorder_kernel (pslsh/hash.cuh:26-47, 105-142).
 //
-// This is the exact-precision path (fp32 FMA for float inputs, fp64 FMA for double
-// inputs); the tcgen05 3xTF32 kernel in project_tc.cuh is the fast path for fp32.
+// Plain fp32 / fp64 FMA.  It takes tables of more than 128 hashes, and float64 rows when a caller asks for
+// the CUDA cores; project_f32.cuh and project_f64.cuh serve the other shapes that the tcgen05 3xTF32
+// kernels of project_tc.cuh cannot take.
 #pragma once
 
 #include "common.cuh"
@@ -65,8 +66,8 @@ __device__ __forceinline__ void assemble_key(const int32_t* __restrict__ hv, int
             for (int bb = 0; bb < 4; ++bb) {
                 int i = wi * 4 + bb - pad;
                 if (i >= 0) {
-                    uint32_t v = (uint32_t)hv[i / elem_bytes];
-                    uint32_t byte = (v >> (8 * (i % elem_bytes))) & 0xFFu;
+                    uint32_t v = (uint32_t)hv[i >> (elem_bytes >> 1)];  // 1, 2 or 4 bytes
+                    uint32_t byte = (v >> (8 * (i & (elem_bytes - 1)))) & 0xFFu;
                     w |= byte << (24 - 8 * bb);
                 }
             }
@@ -87,17 +88,41 @@ __device__ __forceinline__ void pack_hash_values(const ProjectArgs& a, const int
         int row = row0 + r;
         if (row >= a.n) continue;
         int t = first_table + g;
-        uint32_t w[16];
-        bool ovf;
-        assemble_key<FAMILY>(hbuf + r * pitch + g * a.k, a.k, NW, a.elem_bytes, w, ovf);
+        const int32_t* hv = hbuf + r * pitch + g * a.k;
         size_t item = (size_t)t * a.n_total + a.row_offset + row;
         uint32_t* dst = a.keys + item * NW;
-        for (int wi = 0; wi < NW; ++wi) dst[wi] = w[wi];
+        bool ovf = false;
+        if (NW <= 2) {
+            // The values of a table run through one 64-bit register: a loop over the bytes of the key, with a
+            // division for each, was most of the time for rows of few features.
+            const int bits = FAMILY == CULSH_RPLSH ? 1 : 8 * a.elem_bytes;
+            uint64_t acc = 0;
+            HashRange own;
+            for (int j = 0; j < a.k; ++j) {
+                const uint32_t v = (uint32_t)hv[j];
+                uint32_t e = v & 1u;
+                if (FAMILY == CULSH_PSLSH) {
+                    own.take((int)v);
+                    e = a.elem_bytes == 1 ? (v & 0xFFu) : a.elem_bytes == 2 ? (__byte_perm(v, 0, 0x0001) & 0xFFFFu) : __byte_perm(v, 0, 0x0123);
+                }
+                acc = (acc << bits) | e;
+            }
+            if (NW == 1) dst[0] = (uint32_t)acc;
+            else *reinterpret_cast<uint2*>(dst) = make_uint2((uint32_t)(acc >> 32), (uint32_t)acc);
+            if (FAMILY == CULSH_PSLSH) {
+                const int lim = a.elem_bytes == 1 ? 128 : 32768;
+                ovf = a.elem_bytes < 4 && (own.lo < -lim || own.hi >= lim);
+                range.take(own.lo);
+                range.take(own.hi);
+            }
+        } else {
+            uint32_t w[16];
+            assemble_key<FAMILY>(hv, a.k, NW, a.elem_bytes, w, ovf);
+            for (int wi = 0; wi < NW; ++wi) dst[wi] = w[wi];
+        }
         if (FAMILY == CULSH_PSLSH) {
             if (a.ovf_rows) a.ovf_rows[item] = ovf ? 1 : 0;
             else if (ovf) atomicOr(a.d_error, DEV_ERR_NARROW_OVERFLOW);
-            if (a.range)
-                for (int j = 0; j < a.k; ++j) range.take(hbuf[r * pitch + g * a.k + j]);
         }
     }
     if (FAMILY == CULSH_PSLSH && a.range) range.flush(a.range);
