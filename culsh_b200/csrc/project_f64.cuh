@@ -6,11 +6,12 @@
 // shared memory for every 32 FMA of a thread and waits for its loads once per 16 features; a matrix
 // instruction takes 32 FMA a lane from six words, and the tiles come through a ring of three
 // stages with cp.async (8 bytes each: rows of an odd number of features start on 8-byte
-// boundaries only).  A CTA takes 128 rows and up to 128 hash columns of whole tables, so that X is
-// read once per column group; the columns are spread evenly over the groups and, in steps of eight,
-// over the two halves of the warps, so that 224 columns are 2 x 112 and no column past the last
-// step of eight is computed.
-// 200,003 x 100 rows, 224 columns: 0.97 ms on the CUDA cores, 0.49 here (18 TFLOP/s).
+// boundaries only).  A CTA takes 64 rows and up to 128 hash columns of whole tables; two of them share an
+// SM, so that one packs its keys while the other multiplies (one CTA of 128 rows: 0.49 ms instead of
+// 0.46 below).  The columns are spread evenly over the groups and, in steps of eight, over
+// the two halves of the warps, so that 224 columns are 2 x 112 and no column past the last step of
+// eight is computed.
+// 200,003 x 100 rows, 224 columns: 0.97 ms on the CUDA cores, 0.46 here (20 TFLOP/s).
 #pragma once
 
 #include "common.cuh"
@@ -18,7 +19,7 @@
 
 namespace culsh_b200 {
 
-constexpr int PF_BM = 128;
+constexpr int PF_BM = 64;
 constexpr int PF_BN = 128;   // columns of a group at most
 constexpr int PF_BK = 16;    // features per stage
 constexpr int PF_PITCH = PF_BK + 4;  // 160-byte rows: the eight rows of a fragment fall on all banks
@@ -41,7 +42,7 @@ __device__ __forceinline__ void mma_f64(double (&c)[4], const double (&a)[4], co
 }
 
 template <int FAMILY>
-__global__ void __launch_bounds__(PF_THREADS, 1)
+__global__ void __launch_bounds__(PF_THREADS, 2)
 project_f64_kernel(ProjectArgs a) {
     extern __shared__ __align__(16) unsigned char pf_smem[];
     double* stages = reinterpret_cast<double*>(pf_smem);
@@ -84,17 +85,15 @@ project_f64_kernel(ProjectArgs a) {
     };
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
 
-    // warp tile: 32 rows and every second step of eight columns
-    const int wm = (warp >> 1) * 32, wn = warp & 1;
+    // warp tile: 16 rows and every second step of eight columns
+    const int wm = (warp >> 1) * 16, wn = warp & 1;
     const int g = lane >> 2, t = lane & 3;
     const int n_frag = (gc_valid + 7) / 8;
-    double acc[2][8][4];
+    double acc[8][4];
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
+    for (int j = 0; j < 8; ++j)
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[m][j][e] = 0.0;
+        for (int e = 0; e < 4; ++e) acc[j][e] = 0.0;
 
     load(0);
     commit();
@@ -109,23 +108,15 @@ project_f64_kernel(ProjectArgs a) {
         const double* ps = xs + (size_t)PF_BM * PF_PITCH;
 #pragma unroll
         for (int kk = 0; kk < PF_BK; kk += 8) {
-            double af[2][4];
-#pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                const double* x = xs + (wm + 16 * m + g) * PF_PITCH + kk + t;
-                af[m][0] = x[0];
-                af[m][1] = x[8 * PF_PITCH];
-                af[m][2] = x[4];
-                af[m][3] = x[8 * PF_PITCH + 4];
-            }
+            const double* x = xs + (wm + g) * PF_PITCH + kk + t;
+            const double af[4] = {x[0], x[8 * PF_PITCH], x[4], x[8 * PF_PITCH + 4]};
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int frag = 2 * j + wn;
                 if (frag < n_frag) {  // uniform
                     const double* p = ps + (frag * 8 + g) * PF_PITCH + kk + t;
                     const double bf[2] = {p[0], p[4]};
-                    mma_f64(acc[0][j], af[0], bf);
-                    mma_f64(acc[1][j], af[1], bf);
+                    mma_f64(acc[j], af, bf);
                 }
             }
         }
@@ -143,15 +134,13 @@ project_f64_kernel(ProjectArgs a) {
             if (c < gc_valid) {
                 const double bv = FAMILY == CULSH_PSLSH ? bias[col_base + c] : 0.0;
 #pragma unroll
-                for (int m = 0; m < 2; ++m)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const double v = acc[m][j][2 * h + e];
-                        const int32_t q = FAMILY == CULSH_RPLSH
-                                              ? (int32_t)((__float_as_uint((float)v) >> 31) ^ 1u)  // rplsh/hash.cuh:47
-                                              : static_cast<int32_t>(floor(v + bv));               // pslsh/hash.cuh:46
-                        hbuf[(wm + 16 * m + 8 * h + g) * pitch + c] = q;
-                    }
+                for (int h = 0; h < 2; ++h) {
+                    const double v = acc[j][2 * h + e];
+                    const int32_t q = FAMILY == CULSH_RPLSH
+                                          ? (int32_t)((__float_as_uint((float)v) >> 31) ^ 1u)  // rplsh/hash.cuh:47
+                                          : static_cast<int32_t>(floor(v + bv));               // pslsh/hash.cuh:46
+                    hbuf[(wm + 8 * h + g) * pitch + c] = q;
+                }
             }
         }
     }
