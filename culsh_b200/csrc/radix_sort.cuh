@@ -208,9 +208,10 @@ radix_tile_scan_kernel(uint32_t* __restrict__ tile_hist, int tiles_per_table) {
 // on its own (exclusive prefix over the chunk's tiles per digit, chunk totals on the side), a
 // second tiny launch turns the chunk totals into chunk bases (digit prefix + earlier chunks), and
 // the scatter adds the base of its chunk.  With one block per table the scan of a 10M-row table
-// (2441 tiles) ran on 48 SMs for 1.2 ms per pass.
-constexpr int RS_CHUNK_TILES = 256;
-constexpr int RS_CHUNK_MIN_TILES = 512;  // tables with fewer tiles keep the single-launch scan
+// (2441 tiles) ran on 48 SMs for 1.2 ms per pass; at 244 tiles x 32 tables a scan takes 7 us in chunks of
+// 64 tiles and 5 more for the bases, in place of 15 by one block per table.
+constexpr int RS_CHUNK_TILES = 64;
+constexpr int RS_CHUNK_MIN_TILES = 96;  // tables with fewer tiles keep the single-launch scan
 
 __global__ void __launch_bounds__(RS_SCAN_THREADS)
 radix_tile_scan_chunk_kernel(uint32_t* __restrict__ tile_hist, int tiles_per_table, int n_chunks,
@@ -925,33 +926,55 @@ scan_apply_kernel(const TIn* __restrict__ in, size_t n, const TOut* __restrict__
     }
 }
 
-// Short arrays: one CTA walks the array in steps of 8192 elements and carries the total along.  A query
-// batch scans two arrays of its size; three launches and the gaps between them cost 13 us whatever the
-// size, a step here about 2 (one query against a kept index: 159 -> 151 us, with one copy less to wait for).
+// Short arrays: one CTA walks the array in steps of 4096 elements and carries the total along.  Three
+// launches and the gaps between them cost 13 us whatever the size; a step takes about 1 as long as a warp's
+// accesses are 16 bytes a lane (with eight words a lane, one access each, it was 4: every access met
+// 16 lines).
 constexpr int SCAN_ONE_THREADS = 1024;
-constexpr int SCAN_ONE_STEP = SCAN_ONE_THREADS * SCAN_IPT;
-constexpr size_t SCAN_ONE_MAX = 4 * SCAN_ONE_STEP;
+constexpr int SCAN_ONE_IPT = 4;
+constexpr int SCAN_ONE_STEP = SCAN_ONE_THREADS * SCAN_ONE_IPT;
+constexpr size_t SCAN_ONE_MAX = 8 * SCAN_ONE_STEP;
 
-template <typename TIn, typename TOut>
+template <typename T>
+struct alignas(16) ScanVec {
+    T v[16 / sizeof(T)];
+};
+
+// in and out on 16-byte boundaries
+template <typename T>
 __global__ void __launch_bounds__(SCAN_ONE_THREADS)
-scan_one_kernel(const TIn* __restrict__ in, int n, TOut* __restrict__ out) {
-    __shared__ TOut s_warp[32];
-    TOut carry = 0;
+scan_one_kernel(const T* __restrict__ in, int n, T* __restrict__ out) {
+    constexpr int PER = 16 / sizeof(T), VECS = SCAN_ONE_IPT / PER;
+    __shared__ T s_warp[32];
+    T carry = 0;
     for (int base = 0; base < n; base += SCAN_ONE_STEP) {
-        const int first = base + threadIdx.x * SCAN_IPT;
-        TOut v[SCAN_IPT];
-        TOut sum = 0;
+        const int first = base + threadIdx.x * SCAN_ONE_IPT;
+        const bool whole = first + SCAN_ONE_IPT <= n;
+        ScanVec<T> v[VECS];
+        T sum = 0;
 #pragma unroll
-        for (int i = 0; i < SCAN_IPT; ++i) {
-            v[i] = first + i < n ? (TOut)in[first + i] : TOut(0);
-            sum += v[i];
+        for (int i = 0; i < VECS; ++i) {
+            if (whole) v[i] = reinterpret_cast<const ScanVec<T>*>(in + first)[i];
+#pragma unroll
+            for (int j = 0; j < PER; ++j) {
+                const int at = first + i * PER + j;
+                if (!whole) v[i].v[j] = at < n ? in[at] : T(0);
+                sum += v[i].v[j];
+            }
         }
-        TOut total;
-        TOut ex = block_exclusive_scan<TOut>(sum, s_warp, total) + carry;
+        T total;
+        T ex = block_exclusive_scan<T>(sum, s_warp, total) + carry;
 #pragma unroll
-        for (int i = 0; i < SCAN_IPT; ++i) {
-            if (first + i < n) out[first + i] = ex;
-            ex += v[i];
+        for (int i = 0; i < VECS; ++i) {
+#pragma unroll
+            for (int j = 0; j < PER; ++j) {
+                const T x = v[i].v[j];
+                v[i].v[j] = ex;
+                ex += x;
+                const int at = first + i * PER + j;
+                if (!whole && at < n) out[at] = v[i].v[j];
+            }
+            if (whole) reinterpret_cast<ScanVec<T>*>(out + first)[i] = v[i];
         }
         carry += total;
     }
@@ -965,10 +988,12 @@ inline void exclusive_scan(cudaStream_t s, const TIn* in, size_t n, TOut* out, T
         CU_CHECK(cudaMemsetAsync(out, 0, sizeof(TOut), s));
         return;
     }
-    if (n <= SCAN_ONE_MAX) {
-        scan_one_kernel<TIn, TOut><<<1, SCAN_ONE_THREADS, 0, s>>>(in, (int)n, out);
-        KERNEL_CHECK();
-        return;
+    if constexpr (std::is_same<TIn, TOut>::value) {
+        if (n <= SCAN_ONE_MAX && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+            scan_one_kernel<TOut><<<1, SCAN_ONE_THREADS, 0, s>>>(in, (int)n, out);
+            KERNEL_CHECK();
+            return;
+        }
     }
     size_t n_blocks = ceil_div(n, SCAN_TILE);
     scan_reduce_kernel<TIn, TOut><<<(unsigned)n_blocks, SCAN_THREADS, 0, s>>>(in, n, scratch);
