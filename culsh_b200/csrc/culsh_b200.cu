@@ -573,7 +573,7 @@ int build_index(culsh_index& ix, SortBuffers& sb, Scratch<uint32_t>* bounds, Sta
     if (err) return err;
     tr.lap("sort+count+scan+sync");
     ix.n_buckets = (int)B;
-    ix.bucket_keys.alloc(c, (size_t)B * NW);
+    if (!bounds) ix.bucket_keys.alloc(c, (size_t)B * NW);
     ix.bucket_offsets.alloc(c, (size_t)B + 1);
     ix.table_offsets.alloc(c, (size_t)L + 1);
     tr.lap("alloc bucket arrays");

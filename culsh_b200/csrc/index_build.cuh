@@ -110,10 +110,12 @@ bucket_write_kernel(const uint32_t* __restrict__ keys, int n, int L, int tiles_p
         // heads up to and including this item, minus one = bucket of the item
         const uint32_t bid = base_bucket + s_pref[local >> 5] + __popc(word & (0xFFFFFFFFu >> (31 - lane))) - 1u;
         if (head) {
-            const uint32_t* kp = keys + (tbase + li) * NW;
-            uint32_t kk[NW];
-            load_key<NW>(kp, kk);
-            store_key<NW>(bucket_keys + (size_t)bid * NW, kk);
+            if (bucket_keys) {  // null in a self-join, which looks nothing up
+                const uint32_t* kp = keys + (tbase + li) * NW;
+                uint32_t kk[NW];
+                load_key<NW>(kp, kk);
+                store_key<NW>(bucket_keys + (size_t)bid * NW, kk);
+            }
             bucket_offsets[bid] = (int32_t)(tbase + li);
         }
     }
