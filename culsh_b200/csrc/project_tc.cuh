@@ -913,7 +913,8 @@ inline int tc_kblk_choice() {
 //   10M x 256,   48 x 24                     24.8          29            22.7
 // One chunk: the 128-column form.  Several chunks: a unit of n_mma columns costs about
 // 40 + 1.3 * n_mma cycles per K step in every form (the tensor-memory form 9 % less), so the form
-// with the smaller chunks * (40 + 1.3 * n_mma) is taken, the shared-memory one on a tie.
+// with the smaller chunks * (40 + 1.3 * n_mma) is taken, the shared-memory one unless the other is 8 %
+// cheaper (24 x 18 at 96 features, 6 % cheaper by the model: 59.9 us in tensor memory, 55.2 shared).
 // CULSH_TC_VARIANT (read once per process) overrides: 0 = shared memory always, 1 = tensor memory /
 // 128 columns wherever it applies, 3 = tensor memory / 192 columns for shapes of several chunks
 // (the tests run every shape through each).
@@ -928,6 +929,9 @@ inline int tc_variant() {
 inline void tc_chunking(int L, int k, int bn, int& tables_per_chunk, int& n_chunks, int& n_mma) {
     tables_per_chunk = std::min(L, bn / k);
     n_chunks = (L + tables_per_chunk - 1) / tables_per_chunk;
+    // Evenly: a chunk of few tables costs as much as a full one.  22 x 13 hashes are two chunks of 144
+    // columns instead of 256 and 39 padded to 256; 24 x 18 two of 224 (100,003 x 96 rows: 56.4 -> 55.2 us).
+    tables_per_chunk = (L + n_chunks - 1) / n_chunks;
     n_mma = (tables_per_chunk * k + 15) / 16 * 16;
 }
 
@@ -947,7 +951,7 @@ inline bool tc_plan(int d, int L, int k, TcPlan& p) {
             const double cost_shared = c * (40.0 + 1.3 * m);
             tc_chunking(L, k, TS_BN_WIDE, t, c, m);
             const double cost_tensor = 0.91 * c * (40.0 + 1.3 * m);
-            if (cost_tensor < 0.97 * cost_shared) { ts = true; bn = TS_BN_WIDE; }
+            if (cost_tensor < 0.92 * cost_shared) { ts = true; bn = TS_BN_WIDE; }
         }
     }
     p.bn = bn;
