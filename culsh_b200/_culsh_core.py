@@ -441,6 +441,17 @@ class _CoreBase:
         _lib.check(self._h.lib.culsh_set_projection_path(self._h.ptr, int(path)))
 
 
+def mean_row_norm(X) -> float:
+    """Mean L2 norm of the rows of a C-contiguous 2-D float32 / float64 torch CUDA tensor."""
+    import torch
+    h = get_handle(X.device.index)
+    torch.cuda.current_stream(X.device).synchronize()  # the engine's stream does not wait for torch's
+    out = C.c_double()
+    _lib.check(h.lib.culsh_mean_row_norm(h.ptr, X.data_ptr(), int(X.shape[0]), int(X.shape[1]),
+                                         int(X.dtype == torch.float64), C.byref(out)))
+    return out.value
+
+
 def _batch(batch_size: Optional[int]) -> int:
     return -1 if batch_size is None else int(batch_size)
 

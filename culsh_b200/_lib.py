@@ -50,6 +50,7 @@ SIGNATURES = {
     "culsh_set_param_cache": [VP, I],
     "culsh_trim_scratch": [VP, U64],
     "culsh_set_projection_path": [VP, I],
+    "culsh_mean_row_norm": [VP, VP, I, I, I, C.POINTER(C.c_double)],
     "culsh_rplsh_fit_f32": [VP, VP, I, I, I, I, U64, PP],
     "culsh_rplsh_fit_f64": [VP, VP, I, I, I, I, U64, PP],
     "culsh_rplsh_query_f32": [VP, VP, I, VP, I, PP],

@@ -9,6 +9,7 @@
 #include "project_tc.cuh"
 #include "query.cuh"
 #include "radix_sort.cuh"
+#include "row_norm.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -1209,6 +1210,17 @@ int culsh_set_projection_path(culsh_handle* h, int path) {
         if (!h) fail(CULSH_ERR_INVALID, "null handle");
         if (path < 0 || path > 2) fail(CULSH_ERR_INVALID, "path must be 0, 1 or 2");
         h->ctx->projection_path = path;
+    });
+}
+
+int culsh_mean_row_norm(culsh_handle* h, const void* X, int n, int d, int is_double, double* mean_out) {
+    return guarded([&] {
+        if (!h || !X || !mean_out) fail(CULSH_ERR_INVALID, "null argument");
+        if (n <= 0 || d <= 0) fail(CULSH_ERR_INVALID, "n and d must be positive");
+        DeviceGuard g(h->ctx->device);
+        if (!is_device_pointer(X)) fail(CULSH_ERR_INVALID, "X must be device memory");
+        *mean_out = is_double ? mean_row_norm(h->ctx, static_cast<const double*>(X), n, d)
+                              : mean_row_norm(h->ctx, static_cast<const float*>(X), n, d);
     });
 }
 

@@ -1,0 +1,68 @@
+// Mean L2 norm of the rows of a matrix, from which a p-stable fit takes its default window
+// (pstable_lsh.py:191-223), in one launch and one wait.  At the few thousand rows it looks at nothing but
+// launches and waits counts: as a conversion to float64, a norm, a mean and a read of the result it
+// took three launches and two temporaries (self-join of 1,000 x 100 rows: 306 -> 296 us).
+#pragma once
+
+#include "common.cuh"
+
+namespace culsh_b200 {
+
+constexpr int RN_THREADS = 256;
+constexpr int RN_MAX_BLOCKS = 148;
+
+// A warp per row, sums in float64.  The last CTA to finish adds up the partial sums, in one order, so that
+// the result does not depend on which one that is.  `ticket` comes zeroed.
+template <typename T>
+__global__ void __launch_bounds__(RN_THREADS)
+mean_row_norm_kernel(const T* __restrict__ X, int n, int d, double* __restrict__ partial, unsigned* __restrict__ ticket,
+                     double* __restrict__ mean) {
+    __shared__ double s_sum[RN_THREADS / 32];
+    __shared__ bool s_last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int WARPS = RN_THREADS / 32;
+    double sum = 0.0;
+    for (int row = blockIdx.x * WARPS + warp; row < n; row += gridDim.x * WARPS) {
+        const T* x = X + (size_t)row * d;
+        double s = 0.0;
+        for (int i = lane; i < d; i += 32) {
+            const double v = (double)x[i];
+            s = fma(v, v, s);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+        sum += sqrt(s);
+    }
+    if (lane == 0) s_sum[warp] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int w = 0; w < WARPS; ++w) s += s_sum[w];
+        partial[blockIdx.x] = s;
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (s_last && warp == 0) {
+        __threadfence();
+        double s = 0.0;
+        for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(partial + b);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+        if (lane == 0) *mean = s / n;
+    }
+}
+
+template <typename T>
+inline double mean_row_norm(const CtxPtr& c, const T* X, int n, int d) {
+    const int blocks = (int)std::min<size_t>(ceil_div(n, RN_THREADS / 32), RN_MAX_BLOCKS);
+    Scratch<double> buf(c, SL_MISC2, RN_MAX_BLOCKS + 2);  // mean, ticket, partial sums
+    CU_CHECK(cudaMemsetAsync(buf.p, 0, 2 * sizeof(double), c->stream));
+    mean_row_norm_kernel<T><<<blocks, RN_THREADS, 0, c->stream>>>(X, n, d, buf.p + 2, reinterpret_cast<unsigned*>(buf.p + 1), buf.p);
+    KERNEL_CHECK();
+    double mean = 0.0;
+    read_words(c, buf.p, sizeof(double), &mean);
+    return mean;
+}
+
+}  // namespace culsh_b200

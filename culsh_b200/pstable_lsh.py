@@ -5,7 +5,7 @@ from typing import Literal, Optional, Union
 
 import numpy as np
 
-from ._culsh_core import Candidates, PSLSHCore, PSLSHIndex
+from ._culsh_core import Candidates, PSLSHCore, PSLSHIndex, mean_row_norm
 from .utils import ensure_engine_array, get_array_info, get_logger, is_device_array, resolve_seed
 
 
@@ -76,7 +76,10 @@ class PStableLSH:
             if type(X).__module__.startswith("torch"):
                 import torch
                 xs = X[torch.randperm(n, device=X.device)[:max_samples]] if n > max_samples else X
-                mean = float(torch.linalg.norm(xs.double(), dim=1).mean())
+                if xs.ndim == 2 and xs.numel() and xs.is_contiguous() and xs.dtype in (torch.float32, torch.float64):
+                    mean = mean_row_norm(xs)
+                else:
+                    mean = float(torch.linalg.norm(xs.double(), dim=1).mean())
             else:
                 import cupy as cp
                 xs = X[cp.random.choice(n, max_samples, replace=False)] if n > max_samples else X
