@@ -9,7 +9,6 @@
 #include <algorithm>
 #include <condition_variable>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -53,9 +52,10 @@ public:
         filled_.assign(n_, 0);
         const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
         const size_t want = std::min<size_t>({(size_t)FEED_MAX_THREADS, (size_t)std::max(1u, cores - 1), n_});
+        workers_.reserve(want);
         try {
             for (size_t i = 0; i < want; ++i) workers_.emplace_back([this] { work(); });
-        } catch (const std::system_error&) {  // fewer threads than asked for
+        } catch (...) {  // fewer threads than asked for; those that run have to be joined
         }
     }
     HostFeed(const HostFeed&) = delete;
