@@ -209,7 +209,7 @@ radix_tile_scan_kernel(uint32_t* __restrict__ tile_hist, int tiles_per_table) {
 // second tiny launch turns the chunk totals into chunk bases (digit prefix + earlier chunks), and
 // the scatter adds the base of its chunk.  With one block per table the scan of a 10M-row table
 // (2441 tiles) ran on 48 SMs for 1.2 ms per pass; at 244 tiles x 32 tables a scan takes 7 us in chunks of
-// 64 tiles and 5 more for the bases, in place of 15 by one block per table.
+// 64 tiles and 2 more for the bases, in place of 15 by one block per table.
 constexpr int RS_CHUNK_TILES = 64;
 constexpr int RS_CHUNK_MIN_TILES = 96;  // tables with fewer tiles keep the single-launch scan
 
