@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cstdlib>
+#include <functional>
 
 using namespace culsh_b200;
 
@@ -700,10 +701,19 @@ int chain_window_bits(int n_rows, int* n_win) {
     return (int)(ceil_div(ceil_div(n, wins), (size_t)4096) * 4096);
 }
 
+// Where the raw counts of a set of queries go.
+struct RawCounts {
+    uint64_t *cnt, *off;  // [n_q], [n_q + 1]
+    uint32_t *big_list, *mid_list, *counters;
+    int mid_max;
+};
+
+// `count`, if there is one, launches what finds the lists and counts them; they are in `bounds` else.
 // False, and nothing done, when there are more than raw_limit list entries.  On return the device
 // error word as it was behind the last kernel is in c->seen_error.
 bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool self_join, culsh_candidates& out,
-                        StageTimer& tm, uint64_t raw_limit = UINT64_MAX) {
+                        StageTimer& tm, uint64_t raw_limit = UINT64_MAX,
+                        const std::function<void(const RawCounts&)>& count = nullptr) {
     const CtxPtr& c = ix.ctx;
     cudaStream_t s = c->stream;
     const int L = ix.L, n_q = bounds.n_q;
@@ -722,12 +732,16 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
     const int wbits = bitmap_window_bits(c, ix.n);
     // with more rows than two bitmap windows, mid-sized candidate sets are sorted in shared memory
     const int mid_max = (size_t)ix.n > 2 * (size_t)wbits ? MID_MAX : 0;
-    CU_CHECK(cudaMemsetAsync(n_big, 0, 4 * sizeof(uint32_t), s));
     const uint32_t self_lists = self_join ? (uint32_t)L : 0u;
-    raw_count_kernel<<<(unsigned)ceil_div(n_q, 256), 256, 0, s>>>(bounds, n_q, L, self_join, raw_cnt.p, big_list.p,
-                                                                 mid_list, n_big, mid_max);
-    KERNEL_CHECK();
-    exclusive_scan<uint64_t, uint64_t>(s, raw_cnt.p, n_q, raw_off.p, scratch.p);
+    if (count) {
+        count(RawCounts{raw_cnt.p, raw_off.p, big_list.p, mid_list, n_big, mid_max});
+    } else {
+        CU_CHECK(cudaMemsetAsync(n_big, 0, 4 * sizeof(uint32_t), s));
+        raw_count_kernel<<<(unsigned)ceil_div(n_q, 256), 256, 0, s>>>(bounds, n_q, L, self_join, raw_cnt.p, big_list.p,
+                                                                     mid_list, n_big, mid_max);
+        KERNEL_CHECK();
+        exclusive_scan<uint64_t, uint64_t>(s, raw_cnt.p, n_q, raw_off.p, scratch.p);
+    }
     uint64_t raw_total = 0;
     uint32_t nc[3] = {0, 0, 0};
     CU_CHECK(cudaMemcpyAsync(c->pinned, raw_off.p + n_q, 3 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
@@ -907,11 +921,21 @@ bool query_batch(const culsh_index& ix, int n_q, HashFn&& hash_fn, culsh_candida
     tm.mark();
     hash_fn(ix.ks, qkeys.p, ovf.p);
     tm.mark();
-    CULSH_DISPATCH_NW(NW, (lookup_kernel<NW><<<(unsigned)ceil_div(pairs, 256), 256, 0, c->stream>>>(
-                              qkeys.p, ovf.p, n_q, ix.L, ix.bucket_keys.p, ix.bucket_offsets.p, ix.table_offsets.p, bounds.p)));
-    KERNEL_CHECK();
+    std::function<void(const RawCounts&)> count;
+    if (pairs <= LS_MAX_PAIRS) {
+        count = [&](const RawCounts& r) {
+            CULSH_DISPATCH_NW(NW, (lookup_count_kernel<NW><<<1, LS_THREADS, 0, c->stream>>>(
+                                      qkeys.p, ovf.p, n_q, ix.L, ix.bucket_keys.p, ix.bucket_offsets.p, ix.table_offsets.p, bounds.p,
+                                      r.cnt, r.off, r.big_list, r.mid_list, r.counters, r.mid_max)));
+            KERNEL_CHECK();
+        };
+    } else {
+        CULSH_DISPATCH_NW(NW, (lookup_kernel<NW><<<(unsigned)ceil_div(pairs, 256), 256, 0, c->stream>>>(
+                                  qkeys.p, ovf.p, n_q, ix.L, ix.bucket_keys.p, ix.bucket_offsets.p, ix.table_offsets.p, bounds.p)));
+        KERNEL_CHECK();
+    }
     tm.mark();
-    const bool done = query_from_matched(ix, query_bounds(bounds.p, n_q), false, out, tm, raw_limit);
+    const bool done = query_from_matched(ix, query_bounds(bounds.p, n_q), false, out, tm, raw_limit, count);
     c->stats.hash_ms += tm.between(0, 1);
     c->stats.lookup_ms += tm.between(1, 2);
     c->stats.gather_ms += tm.between(2, 3);
