@@ -121,12 +121,14 @@ inline KeySpec make_key_spec(int family, int k, int elem_bytes) {
 // Context behind a handle: device, stream, a pinned scratch block for small D2H reads,
 // staging buffers for host inputs, cached hash parameters.
 // ---------------------------------------------------------------------------------------
+// The generated numbers depend on L * k alone, but a set also holds the projection split for the tensor
+// cores, laid out in chunks of whole tables: sets of one L * k in another split must not be exchanged.
 struct ParamKey {
-    int family, H, d, window, is_double;
+    int family, L, k, d, window, is_double;
     uint64_t seed;
     bool operator<(const ParamKey& o) const {
-        return std::tie(family, H, d, window, is_double, seed) <
-               std::tie(o.family, o.H, o.d, o.window, o.is_double, o.seed);
+        return std::tie(family, L, k, d, window, is_double, seed) <
+               std::tie(o.family, o.L, o.k, o.d, o.window, o.is_double, o.seed);
     }
 };
 

@@ -26,7 +26,7 @@ struct culsh_handle {
 };
 
 // Hash parameters of an index; immutable once generated, so indexes built on one handle with
-// the same (family, shape, window, dtype, seed) share one set.
+// the same (family, L, k, d, window, dtype, seed) share one set.
 struct ParamSet {
     DevBuf<uint8_t> p0;       // projection (float/double [H][d]) | hash A (uint32 [H])
     DevBuf<uint8_t> p1;       // bias (float/double [H])          | hash B (uint32 [H])
@@ -251,7 +251,7 @@ void prepare_tc_split(culsh_index& ix);
 void generate_params(culsh_index& ix) {
     const CtxPtr& c = ix.ctx;
     c->last_params_ms = 0.f;
-    ParamKey key{ix.family, ix.L * ix.k, ix.family == CULSH_MINHASH ? 0 : ix.d, ix.window, ix.is_double, ix.seed};
+    ParamKey key{ix.family, ix.L, ix.k, ix.family == CULSH_MINHASH ? 0 : ix.d, ix.window, ix.is_double, ix.seed};
     if (c->param_cache_enabled) {
         auto it = c->param_cache.find(key);
         if (it != c->param_cache.end()) {
@@ -344,7 +344,7 @@ void hash_dense(const culsh_index& ix, const KeySpec& ks, const T* X, int n, uin
         bool tc = false;
         if (std::is_same<T, float>::value && c->projection_path != 1)
             tc = launch_project_tc(c, s, ix.family, reinterpret_cast<const float*>(Xd),
-                                   reinterpret_cast<const float*>(P), ix.params->p_split.p,
+                                   reinterpret_cast<const float*>(P), ix.params->p_split.p, ix.params->p_split.bytes(),
                                    reinterpret_cast<const float*>(bias), rows, ix.d, ix.L, ix.k, ks,
                                    keys, ovf_rows, off, n_total);
         if (!tc) {

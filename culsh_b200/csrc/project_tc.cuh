@@ -985,11 +985,13 @@ __global__ void split_projection_kernel(const float* __restrict__ P, int H, int 
     out[idx] = v;
 }
 
+inline size_t tc_split_bytes(const TcPlan& p) { return sizeof(float) * (size_t)p.n_chunks * 2 * p.n_mma * p.d_pad; }
+
 inline void prepare_project_tc(const CtxPtr& c, const float* P, int H, int d, int L, int k,
                                DevBuf<uint8_t>& out) {
     TcPlan p;
     if (c->projection_path == 1 || !tc_plan(d, L, k, p)) return;
-    size_t total = (size_t)p.n_chunks * 2 * p.n_mma * p.d_pad;
+    const size_t total = tc_split_bytes(p) / sizeof(float);
     out.alloc(c, total * sizeof(float));
     split_projection_kernel<<<(unsigned)ceil_div(total, 256), 256, 0, c->stream>>>(
         P, H, d, k, p.d_pad, p.tables_per_chunk, p.n_mma, p.n_chunks, reinterpret_cast<float*>(out.p));
@@ -1031,12 +1033,14 @@ inline bool make_map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64
 
 // Returns false when this shape / pointer cannot take the tensor-core path (caller falls back).
 inline bool launch_project_tc(const CtxPtr& c, cudaStream_t stream, int family, const float* X, const float* P,
-                              const uint8_t* p_split, const float* bias, int n, int d, int L, int k,
+                              const uint8_t* p_split, size_t split_bytes, const float* bias, int n, int d, int L, int k,
                               const KeySpec& ks, uint32_t* keys, uint8_t* ovf_rows, int row_offset,
                               int n_total) {
     (void)P;
     TcPlan p;
     if (!p_split || !tc_plan(d, L, k, p)) return false;
+    if (split_bytes != tc_split_bytes(p))  // the copies below are bounded by the plan, not by the buffer
+        fail(CULSH_ERR_INTERNAL, "projection split of %zu bytes does not belong to %d x %d hashes of %d features", split_bytes, L, k, d);
     if (ks.key_words > 8) return false;                       // key wider than the 256-bit packer
     if ((reinterpret_cast<uintptr_t>(X) & 15) != 0) return false;  // TMA base alignment
     if (n <= 0) return true;
