@@ -27,11 +27,11 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "project_plan.h"
 
 namespace culsh_b200 {
 
 constexpr int TC_BM = 128;          // rows per tile (MMA M)
-constexpr int TC_BN = 256;          // accumulator columns (max MMA N)
 constexpr int TC_TRANSFORM_THREADS = 128;
 constexpr int TC_EPI_WARPS = 8;     // two warps per TMEM lane quarter, each takes half of the tables
 constexpr int TC_EPI_THREADS = TC_EPI_WARPS * 32;
@@ -625,8 +625,6 @@ project_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 // split warps can take the K-blocks in turn (one group is enough: the issuing thread is the limit).  Roles, barriers, epilogue and abort protocol are those of the
 // kernel above; a work unit is (128-row tile, chunk of whole tables with <= 128 hash columns).
 // ------------------------------------------------------------------------------------------
-constexpr int TS_BN = 128;      // accumulator columns of the narrow form
-constexpr int TS_BN_WIDE = 192; // and of the wide form (shapes of several chunks)
 template <int KB, int BN>
 struct TsCfg {
     static constexpr int A_STAGES = (512 - 2 * BN) / (2 * KB);  // tensor-memory columns left for xh / xl
@@ -902,79 +900,6 @@ project_ts_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 // ------------------------------------------------------------------------------------------
 // Host side
 // ------------------------------------------------------------------------------------------
-struct TcPlan {
-    int kblk, d_pad, n_chunks, tables_per_chunk, n_mma, bn;
-    bool ts;
-};
-
-inline int tc_kblk_choice() {
-    static int v = [] {
-        const char* e = getenv("CULSH_TC_KBLK");
-        int k = e ? atoi(e) : 16;
-        return k == 32 ? 32 : 16;
-    }();
-    return v;
-}
-
-// Which kernel projects a shape.  Three forms: both operands in shared memory with chunks of
-// <= 256 hash columns (project_tc_kernel), X in tensor memory with chunks of <= 128 columns, or of
-// <= 192 columns (project_ts_kernel).  Measured on B200 (fit, ms):
-//                                        shared, 256   tensor, 128   tensor, 192
-//   12.5M x 96,  16 x 8  (one chunk)         2.31          1.85           -
-//   1M x 128,    32 x 16                     0.62          0.66          0.62
-//   10M x 256,   48 x 24                     24.8          29            22.7
-// One chunk: the 128-column form.  Several chunks: a unit of n_mma columns costs about
-// 40 + 1.3 * n_mma cycles per K step in every form (the tensor-memory form 9 % less), so the form
-// with the smaller chunks * (40 + 1.3 * n_mma) is taken, the shared-memory one unless the other is 8 %
-// cheaper (24 x 18 at 96 features, 6 % cheaper by the model: 59.9 us in tensor memory, 55.2 shared).
-// CULSH_TC_VARIANT (read once per process) overrides: 0 = shared memory always, 1 = tensor memory /
-// 128 columns wherever it applies, 3 = tensor memory / 192 columns for shapes of several chunks
-// (the tests run every shape through each).
-inline int tc_variant() {
-    static int v = [] {
-        const char* e = getenv("CULSH_TC_VARIANT");
-        return e && *e ? atoi(e) : 2;
-    }();
-    return v;
-}
-
-inline void tc_chunking(int L, int k, int bn, int& tables_per_chunk, int& n_chunks, int& n_mma) {
-    tables_per_chunk = std::min(L, bn / k);
-    n_chunks = (L + tables_per_chunk - 1) / tables_per_chunk;
-    // Evenly: a chunk of few tables costs as much as a full one.  22 x 13 hashes are two chunks of 144
-    // columns instead of 256 and 39 padded to 256; 24 x 18 two of 224 (100,003 x 96 rows: 56.4 -> 55.2 us).
-    tables_per_chunk = (L + n_chunks - 1) / n_chunks;
-    n_mma = (tables_per_chunk * k + 15) / 16 * 16;
-}
-
-inline bool tc_plan(int d, int L, int k, TcPlan& p) {
-    const int variant = tc_variant();
-    bool ts;
-    int bn;
-    if (variant == 0) { ts = false; bn = TC_BN; }
-    else if (variant == 1) { ts = k <= TS_BN; bn = ts ? TS_BN : TC_BN; }
-    else if (variant == 3) { ts = k <= TS_BN_WIDE; bn = ts ? (L * k > TS_BN ? TS_BN_WIDE : TS_BN) : TC_BN; }
-    else if (L * k <= TS_BN) { ts = true; bn = TS_BN; }
-    else {
-        ts = false; bn = TC_BN;
-        if (k <= TS_BN_WIDE && k <= TC_BN) {
-            int t, c, m;
-            tc_chunking(L, k, TC_BN, t, c, m);
-            const double cost_shared = c * (40.0 + 1.3 * m);
-            tc_chunking(L, k, TS_BN_WIDE, t, c, m);
-            const double cost_tensor = 0.91 * c * (40.0 + 1.3 * m);
-            if (cost_tensor < 0.92 * cost_shared) { ts = true; bn = TS_BN_WIDE; }
-        }
-    }
-    p.bn = bn;
-    if (k > bn || d % 4 != 0) return false;
-    p.ts = ts;
-    p.kblk = ts ? 32 : tc_kblk_choice();
-    p.d_pad = (d + p.kblk - 1) / p.kblk * p.kblk;
-    tc_chunking(L, k, bn, p.tables_per_chunk, p.n_chunks, p.n_mma);
-    return true;
-}
-
 // P_split layout: [chunk][hi | lo][n_mma rows][d_pad] fp32, zero where padded.
 __global__ void split_projection_kernel(const float* __restrict__ P, int H, int d, int k, int d_pad,
                                         int tables_per_chunk, int n_mma, int n_chunks, float* __restrict__ out) {
@@ -996,8 +921,6 @@ __global__ void split_projection_kernel(const float* __restrict__ P, int H, int 
     }
     out[idx] = v;
 }
-
-inline size_t tc_split_bytes(const TcPlan& p) { return sizeof(float) * (size_t)p.n_chunks * 2 * p.n_mma * p.d_pad; }
 
 inline void prepare_project_tc(const CtxPtr& c, const float* P, int H, int d, int L, int k,
                                DevBuf<uint8_t>& out) {
