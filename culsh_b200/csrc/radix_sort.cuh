@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "index_math.h"
 
 namespace culsh_b200 {
 
@@ -491,12 +492,12 @@ radix_key_gather_kernel(const uint32_t* __restrict__ keys, const uint32_t* __res
     constexpr int Q = NW / 4;  // 16-byte quarters of a key, one per thread
     const int t = blockIdx.x / tiles_per_table;
     const size_t base = (size_t)t * n;
-    const int q0 = (blockIdx.x - t * tiles_per_table) * (RS_THREADS * 8);
+    const int64_t q0 = tile_first(blockIdx.x - t * tiles_per_table, RS_THREADS * 8);
     const uint4* src = reinterpret_cast<const uint4*>(keys) + base * Q;
     uint4* dst = reinterpret_cast<uint4*>(out) + base * Q;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const int64_t q = (int64_t)q0 + i * RS_THREADS + threadIdx.x;
+        const int64_t q = q0 + i * RS_THREADS + threadIdx.x;
         if (q < (int64_t)n * Q) dst[q] = src[(size_t)vals[base + q / Q] * Q + q % Q];
     }
 }
