@@ -16,4 +16,10 @@ namespace culsh_b200 {
 // sixteen words has 2^31 quarters of a key.
 CULSH_HD int64_t tile_first(uint32_t tile, int per_tile) { return (int64_t)tile * per_tile; }
 
+// f(row) for the rows first, first + stride, ... below n.  Unsigned: the step past the last row may pass 2^31.
+template <typename F>
+CULSH_HD void walk_rows(uint32_t first, uint32_t stride, int n, F&& f) {
+    for (uint32_t row = first; row < (uint32_t)n; row += stride) f((int)row);
+}
+
 }  // namespace culsh_b200

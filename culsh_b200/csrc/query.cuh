@@ -88,8 +88,8 @@ __global__ void __launch_bounds__(256)
 raw_count_kernel(BoundsView bounds, int n_q, int L, bool self_join, uint64_t* __restrict__ raw_cnt,
                  uint32_t* __restrict__ big_list, uint32_t* __restrict__ mid_list, uint32_t* __restrict__ counters,
                  int mid_max) {
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n_q) return;
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;  // unsigned: the last CTA may reach past 2^31
+    if (q >= (uint32_t)n_q) return;
     uint32_t c = self_join ? 1u : 0u;  // at most n * L < 2^31
     int t = 0;
     for (; t + RC_BATCH <= L; t += RC_BATCH) {  // RC_BATCH loads in flight
@@ -120,8 +120,8 @@ raw_count_kernel(BoundsView bounds, int n_q, int L, bool self_join, uint64_t* __
     raw_cnt[q] = c;
     if (c > SMALL_MAX) {
         // the sort path gathers a self-join's lists with the own row in each
-        if (c + (self_join ? (uint32_t)L : 0u) <= (uint32_t)mid_max) mid_list[atomicAdd(&counters[1], 1u)] = (uint32_t)q;
-        else big_list[atomicAdd(&counters[0], 1u)] = (uint32_t)q;
+        if (c + (self_join ? (uint32_t)L : 0u) <= (uint32_t)mid_max) mid_list[atomicAdd(&counters[1], 1u)] = q;
+        else big_list[atomicAdd(&counters[0], 1u)] = q;
     } else if (c > SHORT_MAX) {
         atomicAdd(&counters[2], 1u);
     }
@@ -287,7 +287,8 @@ dedupe_small_kernel(BoundsView bounds, const int32_t* __restrict__ cand, const u
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n_q = bounds.n_q;
     int32_t* buf = s_buf[warp];
-    for (int q = blockIdx.x * SM_WARPS + warp; q < n_q; q += gridDim.x * SM_WARPS) {
+    for (uint32_t qu = blockIdx.x * SM_WARPS + warp; qu < (uint32_t)n_q; qu += gridDim.x * SM_WARPS) {
+        const int q = (int)qu;
         const uint64_t r64 = raw_cnt[q];
         if (r64 > CAP) continue;  // another launch owns it
         const int r = (int)r64;
@@ -1161,8 +1162,8 @@ dedupe_chained_rank_kernel(BoundsView bounds, const int32_t* __restrict__ cand, 
 // counts[q] = offsets[q + 1] - offsets[q]
 __global__ void counts_from_offsets_kernel(const uint64_t* __restrict__ offsets, int n_q,
                                            uint64_t* __restrict__ counts) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < n_q) counts[q] = offsets[q + 1] - offsets[q];
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < (uint32_t)n_q) counts[q] = offsets[q + 1] - offsets[q];
 }
 
 // ---------------------------------------------------------------------------------------

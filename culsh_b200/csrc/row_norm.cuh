@@ -5,6 +5,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "index_math.h"
 
 namespace culsh_b200 {
 
@@ -22,7 +23,7 @@ mean_row_norm_kernel(const T* __restrict__ X, int n, int d, double* __restrict__
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int WARPS = RN_THREADS / 32;
     double sum = 0.0;
-    for (int row = blockIdx.x * WARPS + warp; row < n; row += gridDim.x * WARPS) {
+    walk_rows(blockIdx.x * WARPS + warp, gridDim.x * WARPS, n, [&](int row) {
         const T* x = X + (size_t)row * d;
         double s = 0.0;
         for (int i = lane; i < d; i += 32) {
@@ -32,7 +33,7 @@ mean_row_norm_kernel(const T* __restrict__ X, int n, int d, double* __restrict__
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
         sum += sqrt(s);
-    }
+    });
     if (lane == 0) s_sum[warp] = sum;
     __syncthreads();
     if (threadIdx.x == 0) {

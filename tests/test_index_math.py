@@ -29,3 +29,32 @@ def test_key_gather_tiles(tmp_path):
     for (n, q), line in zip(cases, out):
         tiles = -(-n * q // 2048)
         assert [int(x) for x in line.split()] == [0, tiles // 2 * 2048, (tiles - 1) * 2048]
+
+
+ROWS = r"""
+#include "index_math.h"
+#include <cstdio>
+int main() {
+    long long first, stride, n;
+    while (std::scanf("%lld %lld %lld", &first, &stride, &n) == 3) {
+        long long seen = 0, sum = 0, bad = 0;
+        culsh_b200::walk_rows((uint32_t)first, (uint32_t)stride, (int)n, [&](int row) {
+            ++seen;
+            sum += row;
+            bad += row < 0 || row >= n;
+        });
+        std::printf("%lld %lld %lld\n", seen, sum, bad);
+    }
+}
+"""
+
+
+def test_row_walks_end(tmp_path):
+    """148 CTAs of 8 warps step by 1,184 rows: the last step of n = 2^31 - 1 rows ends beyond 2^31."""
+    top = (1 << 31) - 1
+    cases = [(0, 1, 0), (0, 1184, 1), (5, 1184, 5), (7, 1184, 10_000), (1183, 1184, top), (0, 1184, top),
+             (top - 1, 37_888, top), (top, 1184, top), (100, 37_888, top - 900)]
+    out = run_native(tmp_path, ROWS, "".join("%d %d %d\n" % c for c in cases)).split("\n")
+    for (first, stride, n), line in zip(cases, out):
+        rows = range(first, n, stride)
+        assert [int(x) for x in line.split()] == [len(rows), sum(rows), 0]
