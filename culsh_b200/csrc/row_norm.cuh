@@ -1,7 +1,8 @@
 // Mean L2 norm of the rows of a matrix, from which a p-stable fit takes its default window
 // (pstable_lsh.py:191-223), in one launch and one wait.  At the few thousand rows it looks at nothing but
 // launches and waits counts: as a conversion to float64, a norm, a mean and a read of the result it
-// took three launches and two temporaries (self-join of 1,000 x 100 rows: 306 -> 296 us).
+// takes three launches and two temporaries.  A warp takes a whole row, so that a few rows of very many columns
+// leave the chip idle; the caller in pstable_lsh.py says which rows come here, with both sides' times.
 #pragma once
 
 #include "common.cuh"
@@ -10,7 +11,8 @@
 namespace culsh_b200 {
 
 constexpr int RN_THREADS = 256;
-constexpr int RN_MAX_BLOCKS = 148;
+constexpr int RN_MAX_BLOCKS = 592;  // four CTAs an SM
+constexpr int RN_LOADS = 8;          // of a lane in flight
 
 // A warp per row, sums in float64.  The last CTA to finish adds up the partial sums, in one order, so that
 // the result does not depend on which one that is.  `ticket` comes zeroed.
@@ -26,10 +28,16 @@ mean_row_norm_kernel(const T* __restrict__ X, int n, int d, double* __restrict__
     walk_rows(blockIdx.x * WARPS + warp, gridDim.x * WARPS, n, [&](int row) {
         const T* x = X + (size_t)row * d;
         double s = 0.0;
-        for (int i = lane; i < d; i += 32) {
-            const double v = (double)x[i];
-            s = fma(v, v, s);
-        }
+        auto add = [&](int64_t i, bool whole) {
+            T v[RN_LOADS];
+#pragma unroll
+            for (int j = 0; j < RN_LOADS; ++j) v[j] = whole || i + 32 * j < d ? x[i + 32 * j] : T(0);
+#pragma unroll
+            for (int j = 0; j < RN_LOADS; ++j) s = fma((double)v[j], (double)v[j], s);
+        };
+        int64_t i = lane;
+        for (; i + 32 * (RN_LOADS - 1) < d; i += 32 * RN_LOADS) add(i, true);
+        if (i < d) add(i, false);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
         sum += sqrt(s);

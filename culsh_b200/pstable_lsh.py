@@ -9,6 +9,17 @@ from ._culsh_core import Candidates, PSLSHCore, PSLSHIndex, mean_row_norm
 from .utils import ensure_engine_array, get_array_info, get_logger, is_device_array, resolve_seed
 
 
+def _engine_takes_norms(xs) -> bool:
+    """Whether the engine's one-launch kernel or torch's norm gives the mean row norm.  The kernel saves the
+    conversion of float32 rows to float64, which counts from 256 columns on (10,000 x 256: 57 -> 46 us,
+    10,000 x 1,024: 91 -> 47), and two launches where a warp has one row (1,000 x 100: 41 -> 38); for
+    10,000 x 128 torch is as fast (42 against 45), for float64 rows, too (10,000 x 128: 36 against 41), and
+    for longer rows it spreads a row over more of the chip (50 x 200,000: 89 against 250)."""
+    import torch
+    n, d = xs.shape
+    return xs.dtype == torch.float32 and xs.is_contiguous() and n > 0 and 0 < d <= 4096 and (n <= 1024 or d >= 256)
+
+
 class PStableLSH:
     """h(x) = floor((x.p + b) / w) with Gaussian p: ``n_hash_tables`` tables of ``n_hashes``
     such values.  ``window_size`` is an integer bucket width, or "auto" to take
@@ -76,7 +87,7 @@ class PStableLSH:
             if type(X).__module__.startswith("torch"):
                 import torch
                 xs = X[torch.randperm(n, device=X.device)[:max_samples]] if n > max_samples else X
-                if xs.ndim == 2 and xs.numel() and xs.is_contiguous() and xs.dtype in (torch.float32, torch.float64):
+                if xs.ndim == 2 and _engine_takes_norms(xs):
                     mean = mean_row_norm(xs)
                 else:
                     mean = float(torch.linalg.norm(xs.double(), dim=1).mean())

@@ -1,5 +1,6 @@
-"""Mean row norm behind the default window: rows at the edges of a warp, of a CTA's eight rows and of the grid,
-against NumPy in float64 (two summation orders of at most 10,000 terms: 1e-12 relative)."""
+"""Mean row norm behind the default window: rows at the edges of a warp, of a CTA's eight rows and of the grid
+(592 CTAs), columns at the edges of a warp's load and of a lane's eight loads, against NumPy in float64 (two
+summation orders of at most 20,000 terms: 1e-12 relative); infinite and NaN values; and which rows take it."""
 import numpy as np
 import pytest
 
@@ -7,7 +8,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
-@pytest.mark.parametrize("n,d", [(1, 1), (7, 31), (8, 32), (9, 33), (1184, 5), (1185, 100), (10_000, 128), (3, 1000)])
+@pytest.mark.parametrize("n,d", [(1, 1), (7, 31), (8, 32), (9, 33), (1184, 5), (1185, 100), (10_000, 128), (3, 1000),
+                                 (4736, 223), (4737, 224), (5, 225), (5, 255), (6, 256), (7, 257), (2, 20_000)])
 def test_equals_numpy(n, d, dtype):
     import torch
     from culsh_b200._culsh_core import mean_row_norm
@@ -31,3 +33,31 @@ def test_window_of_a_side_stream_and_of_a_strided_view():
             Y = Y * 1.0
         Y = Y * 3.0
         assert PStableLSH._estimate_window_size(Y) == int(torch.linalg.norm(Y.double(), dim=1).mean())
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_values_that_are_not_finite(dtype):
+    import torch
+    from culsh_b200._culsh_core import mean_row_norm
+    X = np.ones((300, 33), dtype)
+    X[299, 32] = np.inf
+    assert mean_row_norm(torch.from_numpy(X).cuda()) == np.inf
+    X[0, 0] = np.nan
+    assert np.isnan(mean_row_norm(torch.from_numpy(X).cuda()))
+    X = np.full((4, 7), np.finfo(np.float32).max, dtype)  # the squares need float64
+    want = np.linalg.norm(X.astype(np.float64), axis=1).mean()
+    assert abs(mean_row_norm(torch.from_numpy(X).cuda()) - want) <= 1e-12 * want
+
+
+def test_which_rows_the_engine_takes(monkeypatch):
+    import torch
+    from culsh_b200 import PStableLSH, pstable_lsh
+    calls = []
+    monkeypatch.setattr(pstable_lsh, "mean_row_norm", lambda x: calls.append(x.shape) or 3.0)
+    f32, f64 = torch.float32, torch.float64
+    for rows, d, dtype, engine in [(1024, 63, f32, True), (1025, 63, f32, False), (1025, 255, f32, False), (1025, 256, f32, True),
+                                   (50, 4096, f32, True), (50, 4097, f32, False), (50, 63, f64, False), (2000, 511, f64, False)]:
+        X = torch.ones((rows, d), device="cuda", dtype=dtype)
+        calls.clear()
+        assert PStableLSH._estimate_window_size(X) == (3 if engine else int(np.sqrt(d)))
+        assert bool(calls) == engine
