@@ -1242,9 +1242,14 @@ int culsh_mean_row_norm(culsh_handle* h, const void* X, int n, int d, int is_dou
         if (!h || !X || !mean_out) fail(CULSH_ERR_INVALID, "null argument");
         if (n <= 0 || d <= 0) fail(CULSH_ERR_INVALID, "n and d must be positive");
         DeviceGuard g(h->ctx->device);
-        if (!is_device_pointer(X)) fail(CULSH_ERR_INVALID, "X must be device memory");
-        *mean_out = is_double ? mean_row_norm(h->ctx, static_cast<const double*>(X), n, d)
-                              : mean_row_norm(h->ctx, static_cast<const float*>(X), n, d);
+        // a CUDA tensor may also be a view of page-locked host memory
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, X) != cudaSuccess || at.type == cudaMemoryTypeUnregistered || !at.devicePointer) {
+            cudaGetLastError();
+            fail(CULSH_ERR_INVALID, "X must be memory that the device can read");
+        }
+        *mean_out = is_double ? mean_row_norm(h->ctx, static_cast<const double*>(at.devicePointer), n, d)
+                              : mean_row_norm(h->ctx, static_cast<const float*>(at.devicePointer), n, d);
     });
 }
 

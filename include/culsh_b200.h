@@ -103,9 +103,9 @@ int culsh_set_param_cache(culsh_handle* h, int enabled);
 int culsh_trim_scratch(culsh_handle* h, uint64_t keep_bytes);
 /* Force the projection path: 0 auto, 1 SIMT fp32/fp64 kernel, 2 tcgen05 3xTF32 kernel. */
 int culsh_set_projection_path(culsh_handle* h, int path);
-/* Mean L2 norm (float64) of the rows of a device matrix [n][d] of float32 / float64, the data side of
- * the default window of a p-stable fit (python/culsh/pstable_lsh.py:191-223).  Runs on the handle's
- * stream and waits for it. */
+/* Mean L2 norm (float64) of the rows of a matrix [n][d] of float32 / float64 in memory that the device can
+ * read, the data side of the default window of a p-stable fit (python/culsh/pstable_lsh.py:191-223).  Runs on
+ * the handle's stream and waits for it. */
 int culsh_mean_row_norm(culsh_handle* h, const void* X, int n, int d, int is_double, double* mean_out);
 
 /* ---- RPLSH: RPLSHCore, bindings.cu:25-116; rplsh/rplsh.cu:18-226 ---------------------- */

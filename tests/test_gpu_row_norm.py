@@ -61,3 +61,30 @@ def test_which_rows_the_engine_takes(monkeypatch):
         calls.clear()
         assert PStableLSH._estimate_window_size(X) == (3 if engine else int(np.sqrt(d)))
         assert bool(calls) == engine
+
+
+def test_cuda_view_of_pinned_memory():
+    """torch makes a CUDA tensor of a page-locked buffer that says it is device memory."""
+    import torch
+    from culsh_b200 import PStableLSH
+    from culsh_b200._culsh_core import mean_row_norm
+    host = torch.randn(300, 40).mul_(3.0).pin_memory()
+
+    class View:
+        __cuda_array_interface__ = {"shape": (300, 40), "typestr": "<f4", "data": (host.data_ptr(), False), "version": 3}
+
+    X = torch.as_tensor(View(), device="cuda")
+    if X.data_ptr() != host.data_ptr():
+        pytest.skip("this torch copies such a view")
+    want = float(torch.linalg.norm(host.double(), dim=1).mean())
+    assert abs(mean_row_norm(X) - want) <= 1e-12 * want
+    assert PStableLSH(4, 4, seed=1).fit(X).window_size == int(want)
+
+
+def test_pageable_memory_is_refused():
+    import ctypes
+    from culsh_b200 import _lib
+    from culsh_b200._culsh_core import get_handle
+    X, out = np.ones((4, 4), np.float32), ctypes.c_double()
+    h = get_handle()
+    assert h.lib.culsh_mean_row_norm(h.ptr, X.ctypes.data, 4, 4, 0, ctypes.byref(out)) != 0
