@@ -6,47 +6,18 @@
 #include <curand.h>
 #include <curand_kernel.h>
 
-#include <cstdarg>
 #include <cstdint>
-#include <cstdio>
 #include <cstring>
 #include <map>
 #include <memory>
-#include <stdexcept>
 #include <string>
 #include <tuple>
 #include <vector>
 
-#include "../../include/culsh_b200.h"
+#include "check.h"
+#include "host_feed.h"
 
 namespace culsh_b200 {
-
-// ---------------------------------------------------------------------------------------
-// Errors: host code throws Error, the C ABI catches it and returns the status code.
-// ---------------------------------------------------------------------------------------
-struct Error : public std::runtime_error {
-    int status;
-    Error(int s, const std::string& m) : std::runtime_error(m), status(s) {}
-};
-
-[[noreturn]] inline void fail(int status, const char* fmt, ...) {
-    char buf[512];
-    va_list ap;
-    va_start(ap, fmt);
-    vsnprintf(buf, sizeof(buf), fmt, ap);
-    va_end(ap);
-    throw Error(status, buf);
-}
-
-#define CU_CHECK(call)                                                                      \
-    do {                                                                                    \
-        cudaError_t e__ = (call);                                                           \
-        if (e__ != cudaSuccess)                                                             \
-            ::culsh_b200::fail(e__ == cudaErrorMemoryAllocation ? CULSH_ERR_ALLOC           \
-                                                                : CULSH_ERR_CUDA,           \
-                               "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e__),     \
-                               __FILE__, __LINE__);                                         \
-    } while (0)
 
 #define CURAND_CHECK(call)                                                                  \
     do {                                                                                    \
@@ -66,8 +37,6 @@ inline int& launch_counter() {
         ++::culsh_b200::launch_counter();  \
         CU_CHECK(cudaGetLastError());      \
     } while (0)
-
-inline size_t ceil_div(size_t a, size_t b) { return (a + b - 1) / b; }
 
 // ---------------------------------------------------------------------------------------
 // Key layout.  A signature of one (row, table) is held as NW 32-bit words, word 0 most
@@ -142,10 +111,6 @@ enum ScratchSlot {
     SL_SLICES, SL_BOUNDS, SL_COUNT
 };
 
-// Pinned ring that pageable host arrays go through on their way to the device.
-constexpr int FEED_SLOTS = 16;
-constexpr size_t FEED_PIECE = (size_t)2 << 20;
-
 struct Ctx {
     int device = 0;
     // hash parameters already generated on this handle (they depend only on the key): the
@@ -164,8 +129,7 @@ struct Ctx {
     cudaEvent_t copy_done[2] = {};
     cudaEvent_t chunk_free[2] = {};
     uint64_t* pinned = nullptr;       // 64 x u64 words of pinned host memory
-    void* feed_ring = nullptr;        // pinned ring for pageable host inputs (host_feed.cuh), made on first use
-    cudaEvent_t feed_free[FEED_SLOTS] = {};  // the last copy out of a slot
+    FeedRing feed_ring;               // for pageable host inputs, made on first use
     int* d_error = nullptr;           // device-side self-check word; [2], [3]: see HashRange
     int seen_error = 0;               // its value behind the last query
     unsigned long long* d_mma = nullptr;  // tensor-core projection: K-blocks issued / with the low-part MMA
@@ -195,8 +159,7 @@ struct Ctx {
         for (auto& q : slot_ptr) if (q) cudaFree(q);
         for (auto& b : big_free) cudaFree(b.p);
         if (pinned) cudaFreeHost(pinned);
-        for (auto& e : feed_free) if (e) cudaEventDestroy(e);
-        if (feed_ring) cudaFreeHost(feed_ring);
+        feed_ring.release();
         if (d_error) cudaFree(d_error);
         if (d_mma) cudaFree(d_mma);
         if (copy_stream) cudaStreamDestroy(copy_stream);

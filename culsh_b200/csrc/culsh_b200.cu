@@ -1,6 +1,5 @@
 // Host orchestration and the C ABI of the engine (see include/culsh_b200.h).
 #include "common.cuh"
-#include "host_feed.cuh"
 #include "index_build.cuh"
 #include "minhash.cuh"
 #include "project_f32.cuh"
@@ -381,7 +380,7 @@ void hash_dense(const culsh_index& ix, const KeySpec& ks, const T* X, int n, uin
     CU_CHECK(cudaEventRecord(c->chunk_free[0], c->stream));
     CU_CHECK(cudaEventRecord(c->chunk_free[1], c->stream));
     int slot = 0;
-    HostFeed feed(c, X, (size_t)n * row_bytes);
+    HostFeed feed(c->feed_ring, c->device, c->copy_stream, X, (size_t)n * row_bytes);
     for (size_t r0 = 0; r0 < (size_t)n; r0 += chunk_rows, slot ^= 1) {
         const int rows = (int)std::min(chunk_rows, (size_t)n - r0);
         CU_CHECK(cudaStreamWaitEvent(c->copy_stream, c->chunk_free[slot], 0));
@@ -438,7 +437,8 @@ void hash_csr(const culsh_index& ix, const KeySpec& ks, const int32_t* indices, 
         int slot = 0;
         // entries in front of row 0 (indptr[0] > 0) belong to no row
         const int64_t first = indptr[0];
-        HostFeed feed(c, indices ? indices + first : nullptr, sizeof(int32_t) * (size_t)std::max<int64_t>(nnz - first, 0));
+        HostFeed feed(c->feed_ring, c->device, c->copy_stream, indices ? indices + first : nullptr,
+                      sizeof(int32_t) * (size_t)std::max<int64_t>(nnz - first, 0));
         for (size_t i = 0; i + 1 < cuts.size(); ++i, slot ^= 1) {
             const int r0 = cuts[i], rows = cuts[i + 1] - r0;
             const int64_t e0 = indptr[r0], cnt = indptr[r0 + rows] - e0;
@@ -1206,10 +1206,7 @@ int culsh_trim_scratch(culsh_handle* h, uint64_t keep_bytes) {
         DeviceGuard g(c->device);
         CU_CHECK(cudaStreamSynchronize(c->stream));
         CU_CHECK(cudaStreamSynchronize(c->copy_stream));
-        if (c->feed_ring && FEED_SLOTS * FEED_PIECE > keep_bytes) {
-            CU_CHECK(cudaFreeHost(c->feed_ring));
-            c->feed_ring = nullptr;
-        }
+        if (FEED_SLOTS * FEED_PIECE > keep_bytes) c->feed_ring.release();
         for (int i = 0; i < SL_COUNT; ++i) {
             if (c->slot_ptr[i] && c->slot_cap[i] > keep_bytes) {
                 CU_CHECK(cudaFree(c->slot_ptr[i]));

@@ -8,13 +8,53 @@
 
 #include <algorithm>
 #include <condition_variable>
+#include <cstdint>
+#include <cstring>
 #include <mutex>
 #include <thread>
 #include <vector>
 
-#include "common.cuh"
+#include "check.h"
 
 namespace culsh_b200 {
+
+constexpr int FEED_SLOTS = 16;
+constexpr size_t FEED_PIECE = (size_t)2 << 20;
+
+// The pinned ring of a handle.
+struct FeedRing {
+    uint8_t* mem = nullptr;                // FEED_SLOTS pieces
+    cudaEvent_t sent[FEED_SLOTS] = {};     // the last copy out of a slot
+
+    // False, and nothing is held, when the memory or an event cannot be had.
+    bool make() {
+        if (mem) return true;
+        bool ok = true;
+        for (auto& e : sent) {
+            if (ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+                e = nullptr;
+                ok = false;
+            }
+        }
+        void* p = nullptr;
+        ok = ok && cudaMallocHost(&p, FEED_SLOTS * FEED_PIECE) == cudaSuccess;
+        if (ok) {
+            mem = static_cast<uint8_t*>(p);
+        } else {
+            cudaGetLastError();
+            release();
+        }
+        return ok;
+    }
+    void release() {
+        for (auto& e : sent) {
+            if (e) cudaEventDestroy(e);
+            e = nullptr;
+        }
+        if (mem) cudaFreeHost(mem);
+        mem = nullptr;
+    }
+};
 
 // True for memory the driver does not know: a copy from it is staged.
 inline bool is_pageable_pointer(const void* p) {
@@ -34,18 +74,9 @@ class HostFeed {
 public:
     // Nothing runs (active() is false) when the source is small or not pageable, when the pinned ring
     // cannot be had or no thread starts: the caller copies straight from the source then.
-    HostFeed(const CtxPtr& ctx, const void* src, size_t total_bytes) : c_(ctx) {
-        if (total_bytes < FEED_MIN_BYTES || !is_pageable_pointer(src)) return;
-        if (!c_->feed_ring) {
-            if (cudaMallocHost(&c_->feed_ring, FEED_SLOTS * FEED_PIECE) != cudaSuccess) {
-                cudaGetLastError();
-                c_->feed_ring = nullptr;
-                return;
-            }
-            for (auto& e : c_->feed_free)
-                if (!e) CU_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        }
-        ring_ = static_cast<uint8_t*>(c_->feed_ring);
+    HostFeed(FeedRing& ring, int device, cudaStream_t copy_stream, const void* src, size_t total_bytes)
+        : ring_(ring), device_(device), stream_(copy_stream) {
+        if (total_bytes < FEED_MIN_BYTES || !is_pageable_pointer(src) || !ring_.make()) return;
         src_ = static_cast<const uint8_t*>(src);
         bytes_ = total_bytes;
         n_ = ceil_div(total_bytes, FEED_PIECE);
@@ -83,9 +114,9 @@ public:
                 cv_.wait(g, [&] { return filled_[piece] != 0; });
                 if (failed_ != cudaSuccess) fail(CULSH_ERR_CUDA, "host feed: %s", cudaGetErrorString(failed_));
             }
-            CU_CHECK(cudaMemcpyAsync(out, ring_ + (piece % FEED_SLOTS) * FEED_PIECE + at, part, cudaMemcpyHostToDevice, c_->copy_stream));
+            CU_CHECK(cudaMemcpyAsync(out, ring_.mem + (piece % FEED_SLOTS) * FEED_PIECE + at, part, cudaMemcpyHostToDevice, stream_));
             if (at + part == FEED_PIECE || begin + part == bytes_) {  // the piece has been sent whole
-                CU_CHECK(cudaEventRecord(c_->feed_free[piece % FEED_SLOTS], c_->copy_stream));
+                CU_CHECK(cudaEventRecord(ring_.sent[piece % FEED_SLOTS], stream_));
                 {
                     std::lock_guard<std::mutex> g(m_);
                     sent_ = piece + 1;
@@ -100,7 +131,7 @@ public:
 
 private:
     void work() {
-        cudaError_t e = cudaSetDevice(c_->device);
+        cudaError_t e = cudaSetDevice(device_);
         while (true) {
             size_t i;
             {
@@ -111,9 +142,9 @@ private:
                 if (stop_) return;
             }
             // ... and has left it (a piece of an earlier call may still be on its way, too)
-            if (e == cudaSuccess) e = cudaEventSynchronize(c_->feed_free[i % FEED_SLOTS]);
+            if (e == cudaSuccess) e = cudaEventSynchronize(ring_.sent[i % FEED_SLOTS]);
             if (e == cudaSuccess)
-                std::memcpy(ring_ + (i % FEED_SLOTS) * FEED_PIECE, src_ + i * FEED_PIECE, std::min(FEED_PIECE, bytes_ - i * FEED_PIECE));
+                std::memcpy(ring_.mem + (i % FEED_SLOTS) * FEED_PIECE, src_ + i * FEED_PIECE, std::min(FEED_PIECE, bytes_ - i * FEED_PIECE));
             {
                 std::lock_guard<std::mutex> g(m_);
                 if (e != cudaSuccess) failed_ = e;
@@ -123,8 +154,9 @@ private:
         }
     }
 
-    const CtxPtr& c_;
-    uint8_t* ring_ = nullptr;
+    FeedRing& ring_;
+    const int device_;
+    const cudaStream_t stream_;
     const uint8_t* src_ = nullptr;
     size_t bytes_ = 0, n_ = 0;
     std::mutex m_;
