@@ -3,7 +3,7 @@
 // NumPy program holds, a fifth of what the link takes.  Here a few threads of the call copy pieces of
 // the source into a ring of pinned memory kept by the handle, and the calling thread issues the
 // device copies in order as the pieces become ready.
-// 400,000 x 128 float32 rows (205 MB): the copies take 17.9 ms from pageable memory, 6.0 this way (34 GB/s).
+// A fit of 256 MB of float32 rows: 23.6 ms from pageable memory, 6.7 this way; 64 MB: 4.0 and 2.1.
 #pragma once
 
 #include <algorithm>
@@ -18,17 +18,33 @@
 
 namespace culsh_b200 {
 
-constexpr int FEED_SLOTS = 16;
+// 8 pieces of 2 MB.  A ring of 16 and 8 threads were no faster for 256 MB and more (6.9 ms against 6.6 - 6.8, 1 GB
+// 22.9 against 23.2), slower for less (32 MB 2.0 against 1.4, 64 MB 2.7 against 2.1), and 32 MB take twice
+// as long to page-lock.
+constexpr int FEED_SLOTS = 8;
 constexpr size_t FEED_PIECE = (size_t)2 << 20;
+// Four threads read as fast as the link takes it until the source is far beyond the caches (1 GB: 24.6 ms with
+// four, 23.2 with six; 64 MB: 2.1 and 2.5).
+inline size_t feed_threads(size_t bytes) { return bytes < ((size_t)256 << 20) ? 4 : 6; }
+// Below this the driver's own staging is as fast, because the threads have to start (16 MB: 0.94 ms direct, 1.1
+// through the ring; 24 MB: 1.35 and 1.3; 32 MB: 1.74 and 1.4).
+constexpr size_t FEED_MIN_BYTES = (size_t)32 << 20;
+// The ring takes about 10 ms to make, what 160 MB gain by it: a handle makes it when it has been given so
+// much, so that a program of one or two small fits does not pay for it.
+constexpr size_t FEED_RING_AFTER = (size_t)160 << 20;
 
 // The pinned ring of a handle.
 struct FeedRing {
     uint8_t* mem = nullptr;                // FEED_SLOTS pieces
+    size_t seen = 0;                       // bytes of sources that could have used it
     cudaEvent_t sent[FEED_SLOTS] = {};     // the last copy out of a slot
 
-    // False, and nothing is held, when the memory or an event cannot be had.
-    bool make() {
+    // False, and nothing is held, before the handle has been given FEED_RING_AFTER bytes, these included,
+    // or when the memory or an event cannot be had.
+    bool make(size_t bytes) {
         if (mem) return true;
+        seen += std::min(bytes, FEED_RING_AFTER);
+        if (seen < FEED_RING_AFTER) return false;
         bool ok = true;
         for (auto& e : sent) {
             if (ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
@@ -53,6 +69,7 @@ struct FeedRing {
         }
         if (mem) cudaFreeHost(mem);
         mem = nullptr;
+        seen = 0;
     }
 };
 
@@ -66,23 +83,19 @@ inline bool is_pageable_pointer(const void* p) {
     return a.type == cudaMemoryTypeUnregistered;
 }
 
-// Below this the driver's own staging is over before the threads are up.
-constexpr size_t FEED_MIN_BYTES = (size_t)8 << 20;
-constexpr int FEED_MAX_THREADS = 8;
-
 class HostFeed {
 public:
-    // Nothing runs (active() is false) when the source is small or not pageable, when the pinned ring
-    // cannot be had or no thread starts: the caller copies straight from the source then.
+    // Nothing runs (active() is false) when the source is small or not pageable, when there is no pinned ring
+    // yet or it cannot be had, or when no thread starts: the caller copies straight from the source then.
     HostFeed(FeedRing& ring, int device, cudaStream_t copy_stream, const void* src, size_t total_bytes)
         : ring_(ring), device_(device), stream_(copy_stream) {
-        if (total_bytes < FEED_MIN_BYTES || !is_pageable_pointer(src) || !ring_.make()) return;
+        if (total_bytes < FEED_MIN_BYTES || !is_pageable_pointer(src) || !ring_.make(total_bytes)) return;
         src_ = static_cast<const uint8_t*>(src);
         bytes_ = total_bytes;
         n_ = ceil_div(total_bytes, FEED_PIECE);
         filled_.assign(n_, 0);
         const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
-        const size_t want = std::min<size_t>({(size_t)FEED_MAX_THREADS, (size_t)std::max(1u, cores - 1), n_});
+        const size_t want = std::min<size_t>({feed_threads(total_bytes), (size_t)std::max(1u, cores - 1), n_});
         workers_.reserve(want);
         try {
             for (size_t i = 0; i < want; ++i) workers_.emplace_back([this] { work(); });

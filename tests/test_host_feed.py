@@ -138,7 +138,14 @@ int main() {
     bool same = false;
     {
         FeedRing ring;
-        EXPECT(send(ring, big - 1, big, same) == 0);
+        // no ring before the handle has been given FEED_RING_AFTER bytes, and one at once for that many
+        EXPECT(send(ring, big - 1, big, same) == 0 && ring.seen == 0);
+        for (size_t given = big; given < FEED_RING_AFTER; given += big)
+            EXPECT(send(ring, big, big, same) == 0 && !ring.mem && live_events == 0 && live_blocks == 0);
+        EXPECT(send(ring, big, big, same) == 1 && same);
+        ring.release();
+        EXPECT(send(ring, big, big, same) == 0);
+        EXPECT(send(ring, FEED_RING_AFTER, big, same) == 1 && same);
         const size_t sizes[] = {big, big + 1, big + FEED_PIECE - 1, 3 * big + 12345, FEED_SLOTS * FEED_PIECE * 2 + big + 1};
         const size_t chunks[] = {big, FEED_PIECE, FEED_PIECE * 3 / 2 + 7, (size_t)1 << 30};
         for (size_t n : sizes)
@@ -152,16 +159,20 @@ int main() {
         EXPECT(live_events == 0 && live_blocks == 0);
         for (int n : {0, 1, FEED_SLOTS - 1}) {
             fail_event_after = n;
+            ring.seen = FEED_RING_AFTER;
             EXPECT(send(ring, big, big, same) == 0);
             EXPECT(!ring.mem && live_events == 0 && live_blocks == 0);
             fail_event_after = -1;
+            ring.seen = FEED_RING_AFTER;
             EXPECT(send(ring, 2 * big, big, same) == 1 && same);
             ring.release();
         }
         fail_memory = true;
+        ring.seen = FEED_RING_AFTER;
         EXPECT(send(ring, big, big, same) == 0);
         EXPECT(!ring.mem && live_events == 0 && live_blocks == 0);
         fail_memory = false;
+        ring.seen = FEED_RING_AFTER;
         EXPECT(send(ring, big, big, same) == 1 && same);
         // no thread, and one only
         fail_thread_after = 0;
