@@ -6,6 +6,7 @@
 #include "project_f64.cuh"
 #include "project_simt.cuh"
 #include "project_tc.cuh"
+#include "query_groups.h"
 #include "query.cuh"
 #include "radix_sort.cuh"
 #include "row_norm.cuh"
@@ -985,6 +986,19 @@ void empty_result(const CtxPtr& c, culsh_candidates& out) {
     CU_CHECK(cudaStreamSynchronize(c->stream));
 }
 
+// Scratch slots of more than keep_bytes go back to the device.
+void release_scratch(const CtxPtr& c, uint64_t keep_bytes) {
+    CU_CHECK(cudaStreamSynchronize(c->stream));
+    CU_CHECK(cudaStreamSynchronize(c->copy_stream));
+    for (int i = 0; i < SL_COUNT; ++i) {
+        if (c->slot_ptr[i] && c->slot_cap[i] > keep_bytes) {
+            CU_CHECK(cudaFree(c->slot_ptr[i]));
+            c->slot_ptr[i] = nullptr;
+            c->slot_cap[i] = 0;
+        }
+    }
+}
+
 // -----------------------------------------------------------------------------------------
 // Family front ends
 // -----------------------------------------------------------------------------------------
@@ -1044,9 +1058,6 @@ void fit_query_dense(culsh_handle* h, int family, const T* X, int n, int d, int 
     *out = res.release();
 }
 
-constexpr int64_t GROUP_PAIRS = (int64_t)4 << 20;  // lists of a group of batches: 32 MB of bounds
-constexpr uint64_t GROUP_IDS = (uint64_t)32 << 20; // and their entries: 128 MB
-
 template <typename T>
 void query_dense(culsh_handle* h, int family, const T* Q, int n_q, const culsh_index* ix,
                  int batch_size, culsh_candidates** out) {
@@ -1081,30 +1092,15 @@ void query_dense(culsh_handle* h, int family, const T* Q, int n_q, const culsh_i
     if (batch_size <= 0 || batch_size >= n_q) {  // rplsh.cu:190-192
         run(Q, n_q, *res);
     } else {
-        // A batch bounds the temporaries.  Batches that are far below what is worth bounding share their
-        // launches and waits: as many whole ones as GROUP_PAIRS lists hold, unless their lists turn out
-        // to have more than GROUP_IDS entries, or memory is short; then each goes by itself.  100,003
-        // queries in batches of 10,000 (24 tables, 1.7 M ids a batch): 1.94 -> 0.56 ms.
         std::vector<std::unique_ptr<culsh_candidates>> parts;
-        const int most = (int)std::min<int64_t>(n_q, std::max<int64_t>(1, GROUP_PAIRS / ix->L / batch_size) * batch_size);
-        int step = std::max(most, batch_size);
-        for (int s0 = 0; s0 < n_q;) {
-            const int nb = std::min(step, n_q - s0);
+        const int group = query_group(n_q, batch_size, ix->L, ix->ks.key_words);
+        run_query_groups(n_q, batch_size, group, [&](int s0, int nb, uint64_t raw_limit) {
             auto part = std::make_unique<culsh_candidates>();
-            bool done = false;
-            try {
-                done = run(Q + (size_t)s0 * ix->d, nb, *part, nb > batch_size ? GROUP_IDS : UINT64_MAX);
-            } catch (const Error& e) {
-                if (e.status != CULSH_ERR_ALLOC || nb <= batch_size) throw;
-            }
-            if (!done) {
-                step = batch_size;
-                continue;
-            }
+            if (!run(Q + (size_t)s0 * ix->d, nb, *part, raw_limit)) return false;
             check_error_word(read_error_word(c));
             parts.push_back(std::move(part));
-            s0 += nb;
-        }
+            return true;
+        }, [&] { release_scratch(c, 0); });
         if (parts.size() == 1) res = std::move(parts[0]);
         else concat_candidates(c, parts, *res);
     }
@@ -1207,13 +1203,7 @@ int culsh_trim_scratch(culsh_handle* h, uint64_t keep_bytes) {
         CU_CHECK(cudaStreamSynchronize(c->stream));
         CU_CHECK(cudaStreamSynchronize(c->copy_stream));
         if (FEED_SLOTS * FEED_PIECE > keep_bytes) c->feed_ring.release();
-        for (int i = 0; i < SL_COUNT; ++i) {
-            if (c->slot_ptr[i] && c->slot_cap[i] > keep_bytes) {
-                CU_CHECK(cudaFree(c->slot_ptr[i]));
-                c->slot_ptr[i] = nullptr;
-                c->slot_cap[i] = 0;
-            }
-        }
+        release_scratch(c, keep_bytes);
         for (auto it = c->big_free.begin(); it != c->big_free.end();) {
             if (it->cap > keep_bytes) {
                 c->big_free_bytes -= it->cap;
