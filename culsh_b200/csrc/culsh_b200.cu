@@ -752,7 +752,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
     const uint32_t nb = nc[0], nm = nc[1];
     tr.lap("count+scan+sync");
     if (raw_total > raw_limit) return false;
-    auto finish = [&] {  // the last wait of a call brings the error word along
+    auto finish = [&] {  // the wait at the end brings the error word along
         CU_CHECK(cudaMemcpyAsync(c->pinned + 8, c->d_error, sizeof(int), cudaMemcpyDeviceToHost, s));
         CU_CHECK(cudaStreamSynchronize(s));
         std::memcpy(&c->seen_error, c->pinned + 8, sizeof(int));
@@ -1089,12 +1089,15 @@ void query_dense(culsh_handle* h, int family, const T* Q, int n_q, const culsh_i
             hash_dense<T>(*ix, ks, Qb, nb, keys, ovf, nb, 0);
         }, dst, raw_limit);
     };
-    if (batch_size <= 0 || batch_size >= n_q) {  // rplsh.cu:190-192
+    const bool whole = batch_size <= 0 || batch_size >= n_q;  // rplsh.cu:190-192
+    if (whole && !query_is_wide(n_q, ix->L)) {
         run(Q, n_q, *res);
     } else {
         std::vector<std::unique_ptr<culsh_candidates>> parts;
-        const int group = query_group(n_q, batch_size, ix->L, ix->ks.key_words);
-        run_query_groups(n_q, batch_size, group, [&](int s0, int nb, uint64_t raw_limit) {
+        if (whole) batch_size = n_q - n_q / 2;
+        const int group = whole ? n_q : query_group(n_q, batch_size, ix->L, ix->ks.key_words);
+        const uint64_t most = whole ? UINT64_MAX : GROUP_IDS;
+        run_query_groups(n_q, batch_size, group, most, [&](int s0, int nb, uint64_t raw_limit) {
             auto part = std::make_unique<culsh_candidates>();
             if (!run(Q + (size_t)s0 * ix->d, nb, *part, raw_limit)) return false;
             check_error_word(read_error_word(c));
@@ -1328,10 +1331,26 @@ int culsh_minhash_query(culsh_handle* h, const int32_t* indices, const int32_t* 
         if ((uint64_t)n_q * ix->L >= (1ull << 31))
             fail(CULSH_ERR_UNSUPPORTED, "n_queries * n_hash_tables must be below 2^31");
         reset_error_word(c);
-        query_batch(*ix, n_q, [&](const KeySpec& ks, uint32_t* keys, uint8_t*) {
-            hash_csr(*ix, ks, indices, indptr, n_q, keys, n_q, 0);
-        }, *res);
-        check_error_word(read_error_word(c));
+        auto run = [&](int s0, int nb, culsh_candidates& dst, uint64_t raw_limit) {
+            return query_batch(*ix, nb, [&](const KeySpec& ks, uint32_t* keys, uint8_t*) {
+                hash_csr(*ix, ks, indices, indptr + s0, nb, keys, nb, 0);
+            }, dst, raw_limit);
+        };
+        if (!query_is_wide(n_q, ix->L)) {
+            run(0, n_q, *res, UINT64_MAX);
+            check_error_word(read_error_word(c));
+        } else {
+            std::vector<std::unique_ptr<culsh_candidates>> parts;
+            run_query_groups(n_q, n_q - n_q / 2, n_q, UINT64_MAX, [&](int s0, int nb, uint64_t raw_limit) {
+                auto part = std::make_unique<culsh_candidates>();
+                if (!run(s0, nb, *part, raw_limit)) return false;
+                check_error_word(read_error_word(c));
+                parts.push_back(std::move(part));
+                return true;
+            }, [&] { release_scratch(c, 0); });
+            if (parts.size() == 1) res = std::move(parts[0]);
+            else concat_candidates(c, parts, *res);
+        }
         *out = res.release();
     });
 }

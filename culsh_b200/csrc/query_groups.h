@@ -20,16 +20,20 @@ inline int query_group(int n_q, int batch, int L, int key_words) {
     return (int)std::min<int64_t>(n_q, std::max<int64_t>(1, lists / L / batch) * batch);
 }
 
+// A query of more (table, query) pairs than this that asks for no batches holds 8 bytes a pair for its lists, 8.6 to
+// 17 GB; when there is no memory for that it goes in two halves.
+inline bool query_is_wide(int n_q, int L) { return (uint64_t)n_q * (uint64_t)L > ((uint64_t)1 << 30); }
+
 // Calls run(first query, queries, most list entries) until n_q are done, `group` at a time; when that is more than
-// a batch and run gives it up (false) or finds no memory (CULSH_ERR_ALLOC, after which release() is called),
-// these and all that follow go batch by batch.
+// a batch and run gives it up (false; most entries: `group_ids`) or finds no memory (CULSH_ERR_ALLOC, after which
+// release() is called), these and all that follow go batch by batch.
 template <typename Run, typename Release>
-inline void run_query_groups(int n_q, int batch, int group, Run&& run, Release&& release) {
+inline void run_query_groups(int n_q, int batch, int group, uint64_t group_ids, Run&& run, Release&& release) {
     for (int64_t s0 = 0; s0 < n_q;) {
         const int nb = (int)std::min<int64_t>(group, n_q - s0);
         bool done = false;
         try {
-            done = run((int)s0, nb, nb > batch ? GROUP_IDS : UINT64_MAX);
+            done = run((int)s0, nb, nb > batch ? group_ids : UINT64_MAX);
         } catch (const Error& e) {
             if (e.status != CULSH_ERR_ALLOC || nb <= batch) throw;
             release();

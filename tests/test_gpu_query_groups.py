@@ -47,3 +47,31 @@ def test_hash_value_range(dtype, d, k, scale):
         raw = np.ascontiguousarray(sig[t]).view(np.uint8).reshape(n, 4 * k)
         order = np.lexsort(tuple(raw[:, j] for j in range(4 * k - 1, -1, -1)))
         assert np.array_equal(cand[t * n:(t + 1) * n], order)
+
+
+def test_more_pairs_than_fit_30_bits():
+    """A query without batches above 2^30 (table, query) pairs, against the same one in batches."""
+    import torch
+    import culsh_b200 as culsh
+    from culsh_b200._culsh_core import MinHashCore
+    n, L, nq = 2000, 1024, (1 << 20) + 3
+    g = torch.Generator("cuda").manual_seed(3)
+    X = torch.randn(n, 8, device="cuda", generator=g)
+    Q = torch.randn(nq, 8, device="cuda", generator=g)
+    Q[::1000] = X[:1049]
+    m = culsh.RPLSH(L, 30, seed=2).fit(X)
+    whole, parts = m.query(Q), m.query(Q, batch_size=300_000)
+    for f in ("get_indices", "get_offsets"):
+        assert torch.equal(getattr(whole, f)(as_torch=True).view(torch.int32), getattr(parts, f)(as_torch=True).view(torch.int32))
+    assert whole.n_total_candidates >= 1049
+    del whole, parts, m, Q
+    ids = torch.randint(0, 1 << 28, (2 * nq,), device="cuda", generator=g, dtype=torch.int32)
+    ptr = (2 * torch.arange(nq + 1, device="cuda")).to(torch.int32)
+    core = MinHashCore(L, 2, 5)
+    ix = core.fit(ids[:2 * n], ptr[:n + 1].contiguous(), n, 1 << 28)
+    c = core.query(ids, ptr, nq, ix)
+    off = c.get_offsets()
+    few = core.query(ids[:2 * n], ptr[:n + 1].contiguous(), n, ix)
+    assert np.array_equal(off[:n + 1], few.get_offsets())
+    assert np.array_equal(c.get_indices()[:int(off[n])], few.get_indices())
+    core.trim_scratch(0)

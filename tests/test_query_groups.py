@@ -25,7 +25,7 @@ int main() {
         std::printf("%d", group);
         int released = 0;
         try {
-            run_query_groups(n_q, batch, group, [&](int s0, int nb, uint64_t limit) {
+            run_query_groups(n_q, batch, group, GROUP_IDS, [&](int s0, int nb, uint64_t limit) {
                 const bool hit = s0 + nb > at && (nb > batch || fail_how >= 3);
                 if ((nb > batch) != (limit == GROUP_IDS)) fail(CULSH_ERR_INTERNAL, "limit");
                 if (hit && fail_how == 1) return false;
@@ -80,3 +80,40 @@ def test_what_a_group_cannot_do_goes_batch_by_batch(tmp_path):
     assert sum(nb for _, nb in parts) == 1 << 20 and late.endswith("released 1")
     assert "error" in other and not _parts(other) and other.endswith("released 0")
     assert "error" in every and not _parts(every) and every.endswith("released 1")
+
+
+WIDE = r"""
+#include "query_groups.h"
+#include <cstdio>
+using namespace culsh_b200;
+extern "C" const char* cudaGetErrorString(cudaError_t) { return ""; }
+int main() {
+    int n_q, L, memory;
+    while (std::scanf("%d %d %d", &n_q, &L, &memory) == 3) {
+        std::printf("%d", query_is_wide(n_q, L) ? 1 : 0);
+        try {
+            run_query_groups(n_q, n_q - n_q / 2, n_q, UINT64_MAX, [&](int s0, int nb, uint64_t limit) {
+                if (limit != UINT64_MAX) fail(CULSH_ERR_INTERNAL, "limit");
+                if (nb > memory) fail(CULSH_ERR_ALLOC, "none left");
+                std::printf(" %d:%d", s0, nb);
+                return true;
+            }, [] {});
+        } catch (const Error& e) {
+            std::printf(" error %d", e.status);
+        }
+        std::printf("\n");
+    }
+}
+"""
+
+
+def test_a_wide_query_goes_in_halves_when_memory_is_short(tmp_path):
+    top = (1 << 31) - 1
+    cases = [(1 << 20, 1024, top), ((1 << 20) + 1, 1024, top), ((1 << 20) + 1, 1024, 1 << 20), (top, 1, 1 << 30), (top, 1, 5)]
+    out = run_native(tmp_path, WIDE, "".join("%d %d %d\n" % c for c in cases), flags=["-I", CUDA]).strip().split("\n")
+    assert [int(line.split()[0]) for line in out] == [0, 1, 1, 1, 1]
+    half = ((1 << 20) + 2) // 2
+    assert _parts(out[1]) == [(0, (1 << 20) + 1)]
+    assert _parts(out[2]) == [(0, half), (half, half - 1)]
+    assert _parts(out[3]) == [(0, 1 << 30), (1 << 30, (1 << 30) - 1)]
+    assert "error" in out[4] and not _parts(out[4])
