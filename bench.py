@@ -649,8 +649,14 @@ def line_of(torch, args, wl, spec, world, m, peaks, tf32):
     sf, sq = stage["fit"][-1], stage["query"][-1]
     passes = max(1, sf["sort_passes"])
     items, kb = sf["n_items"], 4 * sf["key_words"]
-    # keys of four words and more: the last pass reads (word, row id) and writes the ids
-    item_bytes = 12.0 if sf["key_words"] >= 4 else (kb + 4) * 2.0
+    # keys of four words and more: the last pass reads (word, row id) and writes the ids; short tables: one launch
+    # reads the keys and writes keys and ids
+    short = n <= (8192 if sf["key_words"] == 2 and passes > 5 else 12_288)
+    wide = sf["key_words"] >= 4
+    item_bytes = 2.0 * kb + 4.0 if short else (12.0 if wide else (kb + 4) * 2.0)
+    item_note = (f"key {kb} B read, key and row id written per item, one launch for all passes" if short else
+                 "key word and row id read, row id written per item, one launch" if wide else
+                 f"(key {kb} B + row id 4 B) read + written per item, one launch")
     roof = {}
     if spec["family"] == "minhash":
         nnz = m["nnz"]
@@ -675,9 +681,10 @@ def line_of(torch, args, wl, spec, world, m, peaks, tf32):
                         "tf32_tflops_measured": tf32}
     if scatter_ms > 0:
         roof["sort"] = {"bound": "hbm", "achieved": items * item_bytes / (scatter_ms * 1e-3) / 1e9,
-                        "peak": peaks["hbm_gbs"], "unit": "GB/s", "kernel": "radix_scatter_kernel", "traffic": None,
-                        "note": f"(key {kb} B + row id 4 B) read + written per item, one launch (the scatter of the "
-                                f"last of {passes} passes) timed with CUDA events; peak {peaks['source']}"}
+                        "peak": peaks["hbm_gbs"], "unit": "GB/s", "traffic": None,
+                        "kernel": "radix_sort_small_kernel" if short else "radix_scatter_kernel",
+                        "note": item_note + ("" if short else f" (the scatter of the last of {passes} passes)") +
+                                f", timed with CUDA events; peak {peaks['source']}"}
     dedupe_ms = mean("dedupe_ms", "query")
     if dedupe_ms > 0:
         roof["gather"] = {"bound": "hbm", "peak": peaks["hbm_gbs"], "unit": "GB/s", "traffic": None,

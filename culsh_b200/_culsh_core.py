@@ -420,7 +420,7 @@ class _CoreBase:
 
     def set_param_cache(self, enabled: bool):
         """False: every fit generates its hash parameters again (upstream's behaviour) instead
-        of reusing the set this handle made for the same (family, shape, seed)."""
+        of reusing the set this handle made for the same (family, tables, hashes, features, window, dtype, seed)."""
         _lib.check(self._h.lib.culsh_set_param_cache(self._h.ptr, int(bool(enabled))))
 
     def query_keys(self, keys_ptr: int, n_queries: int, index) -> Candidates:

@@ -68,8 +68,8 @@ lookup_kernel(const uint32_t* __restrict__ qkeys, const uint8_t* __restrict__ q_
 // the queries of 513 - 1024 ids of a 12.5M-row shard took a CTA each on the sort path: 0.77 -> 0.50 ms
 // per 10k queries, the 10M-row self-join, all below 512, is unchanged)
 constexpr int SMALL_MAX = 1024;
-// ... and by its short form (4 ids per lane: 512 bytes of shared memory and 40 registers, so that all
-// of an SM's warp slots are filled; the long form runs at half of that)
+// ... and by its short form (4 ids per lane: 512 bytes of shared memory a warp and 40 registers, so that 48 of an
+// SM's 64 warp slots are filled; the long form, 64 registers, fills 32)
 constexpr int SHORT_MAX = 128;
 
 // rows of a packed list other than the query's own
@@ -129,7 +129,9 @@ raw_count_kernel(BoundsView bounds, int n_q, int L, bool self_join, uint64_t* __
 
 // Few (table, query) pairs: lookup, raw counts, their scan and the counters in one CTA and one launch
 // in place of five (memset, lookup, count, scan; one query against 32 tables, the whole call: 153 -> 143 us).  Every
-// search is a chain of about twenty dependent reads, so the CTA should not have to go round more than twice.
+// search is a chain of about twenty dependent reads, so the CTA should not have to go round more than twice: at
+// 2,048 and 2,049 pairs the two ways are within 7 us of one another (1M rows 104 here and 97 - 100 there, 10M
+// 135 - 143 and 130 - 141), with fewer this one is the faster.
 constexpr int LS_THREADS = 1024;
 constexpr size_t LS_MAX_PAIRS = 2 * LS_THREADS;
 template <int NW>

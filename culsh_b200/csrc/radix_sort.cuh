@@ -280,7 +280,8 @@ radix_chunk_base_kernel(uint32_t* __restrict__ chunk_tot, int n_chunks) {
 // Whole tiles have no bounds in the code.  480M items of 4 + 4 bytes: 2.66 -> 2.0 ms a pass; 200M packed
 // items of 8 bytes: first pass 1.59 -> 0.87, middle ones 1.26 -> 0.73, last 1.25 -> 0.90.
 // ---------------------------------------------------------------------------------------
-// Takes the lanes that differ from this one in the bit `mask` of d out of `lanes`.  Spelled out because the
+// Takes the lanes that differ from this one in the bit `mask` of d out of `lanes`: the step of CUB's MatchAny
+// (cub/util_ptx.cuh: test, ballot, complement where the bit is clear, and).  Spelled out because the
 // scatter is bound by what it issues: with a ballot and a select in C++ 32M items of 4 + 4 bytes took 155 us a
 // pass, this way 128.
 __device__ __forceinline__ void keep_same_bit(uint32_t& lanes, uint32_t d, uint32_t mask) {
@@ -507,7 +508,8 @@ radix_key_gather_kernel(const uint32_t* __restrict__ keys, const uint32_t* __res
 // three launches, of which a table of a few thousand rows fills a few CTAs for 2 us each: what such a
 // sort costs are its 15 launches (48 and more for keys of four words) and the gaps between them.
 // 1,000 rows x 8 tables, five passes of packed items: 70 us of launches and gaps against 14 here; 10,000 x 16: 80
-// against 40.
+// against 40.  At the line it is still the faster one for every key and number of tables: 12,288 rows, one table, two
+// byte passes 42 and 27, 64 passes of sixteen-word keys 1,101 and 602 (148 tables: 7,419 and 706).
 // Above 12,288 items (8,192 of two words and an id) a table no longer fits the registers of one CTA.
 // ---------------------------------------------------------------------------------------
 constexpr int RSS_THREADS = 1024;
@@ -783,10 +785,9 @@ inline int radix_sort_words(const CtxPtr& c, uint32_t* keys[2], uint32_t* vals[2
     const TileScan scan{s, L, tiles_per_table, tile_hist};
     uint32_t* words[2] = {keys[1], keys[1] + (size_t)n * L};
     auto k_first = radix_scatter_kernel<1, true, 0>;
-    auto k_first_last = radix_scatter_kernel<1, true, 3>;
     auto k_next = radix_scatter_kernel<1, false, 0>;
     auto k_last = radix_scatter_kernel<1, false, 3>;
-    for (auto k : {k_first, k_first_last, k_next, k_last})
+    for (auto k : {k_first, k_next, k_last})
         CU_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM));
     // the ids alternate between the two arrays so that the last pass writes vals[1]
     auto ids_of = [&](int pass) { return vals[((KB - 1 - pass) & 1) ? 0 : 1]; };
@@ -802,7 +803,7 @@ inline int radix_sort_words(const CtxPtr& c, uint32_t* keys[2], uint32_t* vals[2
         KERNEL_CHECK();
         scan.run();
         if (p == KB - 1 && c->profiling) cudaEventRecord(c->ev_pass[0], s);
-        auto kern = p == 0 ? (word_end ? k_first_last : k_first) : (word_end ? k_last : k_next);
+        auto kern = p == 0 ? k_first : (word_end ? k_last : k_next);  // a key has nine bytes at least
         kern<<<(unsigned)total_tiles, RS_THREADS, Cfg::SMEM, s>>>(w_in, ids, words[(p & 1) ^ 1], ids_of(p), n, tiles_per_table, p & 3,
                                                                KeyComp{0u, 0u}, tile_hist, scan.chunk_base(), scan.n_chunks());
         KERNEL_CHECK();

@@ -92,7 +92,7 @@ int culsh_get_stats(const culsh_handle* h, culsh_stats* out);
 /* 1 = time stages with CUDA events (adds a few event records per call). Default 0. */
 int culsh_set_profiling(culsh_handle* h, int enabled);
 /* 1 (default) = hash parameters generated on this handle are kept and reused by later fits
- * with the same (family, shape, window, dtype, seed); 0 = every fit generates them again,
+ * with the same (family, tables, hashes, features, window, dtype, seed); 0 = every fit generates them again,
  * as upstream does (rplsh/hash.cuh:59-78, pslsh/hash.cuh:60-89, minhash/hash.cuh:42-54). */
 int culsh_set_param_cache(culsh_handle* h, int enabled);
 /* Temporaries live in per-handle device buffers that only grow (after a 10M-row self-join:
@@ -101,7 +101,7 @@ int culsh_set_param_cache(culsh_handle* h, int enabled);
  * a buffer allocates it again.  No upstream counterpart (upstream allocates and frees its
  * temporaries inside every call, core/fit.cuh:160-252, core/query.cuh:290-478). */
 int culsh_trim_scratch(culsh_handle* h, uint64_t keep_bytes);
-/* Force the projection path: 0 auto, 1 SIMT fp32/fp64 kernel, 2 tcgen05 3xTF32 kernel. */
+/* Force the projection path: 0 auto, 1 the CUDA cores (fp32 / fp64 multiply-adds), 2 tcgen05 3xTF32 kernel. */
 int culsh_set_projection_path(culsh_handle* h, int path);
 /* Mean L2 norm (float64) of the rows of a matrix [n][d] of float32 / float64 in memory that the device can
  * read, the data side of the default window of a p-stable fit (python/culsh/pstable_lsh.py:191-223).  Runs on
