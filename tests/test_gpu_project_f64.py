@@ -1,5 +1,5 @@
 """float64 projection on the matrix instructions: rows, features and hash columns on both sides of the
-128-row tile, the 16-feature stage, the 8-column step and the 128-column group, against the CUDA-core
+64-row tile, the 16-feature stage, the 8-column step and the 128-column group, against the CUDA-core
 kernel (projection path 1).  Both round in float64: a sign or floor may differ only where the sum lies
 within d * 2^-52 * sum|x p| of the boundary, which for standard normals and a few million values
 happens with a probability below 1e-6, so the signatures are compared whole."""
@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("family", ["rplsh", "pslsh"])
-@pytest.mark.parametrize("n,d,L,k", [(1, 1, 2, 1), (127, 15, 2, 4), (128, 16, 1, 8), (129, 17, 3, 6), (300, 32, 16, 8),
+@pytest.mark.parametrize("n,d,L,k", [(1, 1, 2, 1), (63, 14, 2, 4), (64, 30, 3, 5), (65, 31, 2, 16), (127, 15, 2, 4), (128, 16, 1, 8), (129, 17, 3, 6), (300, 32, 16, 8),
                                      (300, 33, 17, 8), (513, 50, 2, 9), (260, 100, 16, 14), (200, 7, 2, 15), (64, 256, 130, 1)])
 def test_equals_cuda_core_projection(family, n, d, L, k):
     from culsh_b200 import _culsh_core as core_mod

@@ -1,7 +1,7 @@
 """Batches of a query share their launches as long as their lists are few, and the scans of a batch run in
-one CTA up to 32,768 queries: query counts at the edges of the scan's 8192-element steps and of that line, batch
+one CTA up to 32,768 queries: query counts at the edges of the scan's 4096-element steps and of that line, batch
 sizes that leave a rest, and lists of more than 2^25 entries, which are taken batch by batch, have to give
-what one batch gives.  P-stable fits keep the range of their hash values on the way: bytes at the edges of
+what one batch gives (tests/test_query_groups.py has the way back when memory is short).  P-stable fits keep the range of their hash values on the way: bytes at the edges of
 the compressed sort (32 levels) and of the byte itself, in each projection kernel."""
 import numpy as np
 import pytest
@@ -14,7 +14,7 @@ def _same(a, b):
         assert np.array_equal(getattr(a, f)(), getattr(b, f)())
 
 
-@pytest.mark.parametrize("nq,batch", [(8191, 1000), (8192, 8191), (8193, 64), (32_767, 32_766), (32_768, 5000), (32_769, 16_384)])
+@pytest.mark.parametrize("nq,batch", [(4095, 1000), (4096, 4095), (4097, 64), (8191, 1000), (8192, 8191), (8193, 64), (32_767, 32_766), (32_768, 5000), (32_769, 16_384)])
 def test_query_counts(nq, batch):
     import culsh_b200 as culsh
     rng = np.random.default_rng(nq)

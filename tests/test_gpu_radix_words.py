@@ -1,7 +1,9 @@
-"""Keys of four words and more are sorted word by word: row counts on both sides of the 4096-item tile
-and of the 512 tiles from which tile offsets are scanned in chunks, key lengths that end inside a word (16 to 64
-bytes), and collections where the rows agree in the leading, the trailing or all hashes, so that
-the order depends on every word and equal keys keep their row order."""
+"""Keys of four words and more are sorted word by word, tables of more than 12,288 rows and, with the one-CTA sort
+switched off, shorter ones: row counts on both sides of the 4096-item tile, of the 96 tiles from which tile offsets
+are scanned in chunks, and of whole chunks of 64 tiles, key lengths that end inside a word (16 to 64
+bytes, 8-word keys among them), and collections where the rows agree in the leading, the trailing or all hashes, so that
+the order depends on every word and equal keys keep their row order.  The chunked scan of one- and
+two-word keys (tiles of 4096 and 3072) is checked at the same counts of tiles."""
 import numpy as np
 import pytest
 
@@ -10,9 +12,16 @@ from oracle import oracle
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,k", [(1, 3), (31, 16), (4095, 3), (4096, 4), (4097, 5), (8193, 8), (12_289, 9), (20_000, 16), (2_097_153, 3)])
-def test_index_equals_oracle_order(n, k):
+TILE = 4096
+
+
+@pytest.mark.parametrize("n,k", [(1, 3), (31, 16), (4095, 3), (4096, 4), (4097, 5), (8193, 8), (12_289, 9), (12_289, 5), (20_000, 16),
+                                 (20_000, 8), (95 * TILE, 5), (95 * TILE + 1, 3), (96 * TILE + 1, 8), (128 * TILE, 3),
+                                 (128 * TILE + 1, 4), (2_097_153, 3)])
+def test_index_equals_oracle_order(n, k, monkeypatch):
     from culsh_b200 import _culsh_core as core_mod
+    if n <= 12_288:
+        monkeypatch.setenv("CULSH_SORT_NO_PACK", "1")
     rng = np.random.default_rng(n)
     L = 2
     # row r of block b has b's set of ids with a few of the positions changed: many equal hashes
@@ -39,3 +48,21 @@ def test_index_equals_oracle_order(n, k):
         assert np.array_equal(off[tab[t]:tab[t + 1]], t * n + np.flatnonzero(head))
     want = oracle.minhash_signatures(indices[:600], indptr[:min(n, 100) + 1], ix.get_hash_a(), ix.get_hash_b())
     assert np.array_equal(sig[:, :min(n, 100)].transpose(1, 0, 2).reshape(-1, L * k), want)
+
+
+@pytest.mark.parametrize("k,tile", [(16, 4096), (40, 3072)])
+@pytest.mark.parametrize("tiles,extra", [(95, 0), (95, 1), (96, 0), (96, 1), (128, 0), (128, 1), (192, -1)])
+def test_scan_of_many_tiles(k, tile, tiles, extra):
+    """Sign keys of one and two words: the index against a stable sort of the signatures on the host."""
+    from culsh_b200 import _culsh_core as core_mod
+    n, d, L = tiles * tile + extra, 8, 2
+    rng = np.random.default_rng(n)
+    base = rng.standard_normal((n // 3 + 1, d)).astype(np.float32)  # every row about three times
+    X = base[rng.integers(0, len(base), n)]
+    core = core_mod.RPLSHCore(L, k, 5)
+    ix = core.fit_float(X, n, d)
+    sig = core.hash(X, ix)  # [L][n][k] bytes
+    cand = ix.get_candidate_indices()
+    for t in range(L):
+        key = (sig[t].astype(np.uint64) << np.arange(k - 1, -1, -1, dtype=np.uint64)).sum(axis=1, dtype=np.uint64)
+        assert np.array_equal(cand[t * n:(t + 1) * n], np.argsort(key, kind="stable"))
