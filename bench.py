@@ -454,7 +454,6 @@ def config_of(wl, spec):
 # a workload or size without a capture reports null.
 NCU_TRAFFIC = {
     ("c2", 1_000_000): {
-        "gather": 273_526_528 + 677_084_416,   # profiles/dedupe_chained_rank_kernel_c2_1M.md
         "sort": 264_078_336 + 203_595_776,     # profiles/radix_scatter_kernel_c2_1M.md (second pass)
         "hash": 512_630_784 + 113_564_928,     # profiles/project_tc_kernel_c2_1M.md
     },
@@ -689,7 +688,7 @@ def line_of(torch, args, wl, spec, world, m, peaks, tf32):
     if dedupe_ms > 0:
         roof["gather"] = {"bound": "hbm", "peak": peaks["hbm_gbs"], "unit": "GB/s", "traffic": None,
                           "achieved": 4.0 * (sq["raw_candidates"] + sq["unique_candidates"]) / (dedupe_ms * 1e-3) / 1e9,
-                          "kernel": "dedupe kernel of the gather (chained rank / bitmap / warp path)",
+                          "kernel": "dedupe kernel of the gather (window / bitmap form)",
                           "note": "4 B per raw candidate id read + 4 B per unique id written, over the CUDA-event "
                                   f"time of the dedupe launch alone; peak {peaks['source']}"}
     for key, r in roof.items():

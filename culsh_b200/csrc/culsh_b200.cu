@@ -678,24 +678,24 @@ int bitmap_window_bits(const CtxPtr& c, int n_rows) {
     return (int)std::min(want, cap);
 }
 
-// Tuning knobs of the chained kernel, read from the environment at every call (tests vary them):
-//   CULSH_CHAIN_BITS    rows per window (default 344,064: bitmap and prefixes of three CTAs fit
-//                       one SM); the row range is cut into the fewest such windows, each a
-//                       multiple of 4096 rows
-//   CULSH_CHAIN_STAGE   ids staged in shared memory per copy-out chunk; 0 (default) = no stage,
-//                       every id is stored straight at its CSR position (measured on 1M rows x
-//                       10k queries: 1.22 ms against 1.29 ms with a 5120-id stage and the 253,952-row
-//                       windows that then fit)
+// Tuning knobs of the window kernel, read from the environment at every call (tests vary them):
+//   CULSH_CHAIN_BITS    rows per window at most (default WINDOW_ROWS); the row range is cut into the fewest such
+//                       windows, each a multiple of 4096 rows
 //   CULSH_CHAIN_THREADS threads per CTA: 256, 384 (default) or 512
-//   CULSH_CHAIN_LOADS   loads in flight per lane in the list walks: 4, 8 or 16 (default)
+//   CULSH_CHAIN_LOADS   loads in flight per lane in the list walk: 4, 8 (default) or 16
 //   CULSH_CHAIN_SLICES  0 = CTAs search their list slices themselves (default 1: precomputed)
-constexpr int CHAIN_MAX_WINDOWS = 8;
+//   CULSH_COMPACT_BOUNCE ids of the buffer through which a result is brought together inside its raw array
+//                       (default 0: only if there is no memory for a second array)
+constexpr int MAX_WINDOWS = 8;
+// 43 KB of bitmap: five CTAs of 384 threads share an SM (1M rows: three windows 820 us, four of 254,000 rows 889, two of 504,000
+// 909; 2M rows of sparser sets 670, 740, 750)
+constexpr long WINDOW_ROWS = 344064;
 inline long env_long(const char* name, long dflt) {
     const char* e = getenv(name);
     return e && *e ? atol(e) : dflt;
 }
-int chain_window_bits(int n_rows, int* n_win) {
-    const size_t cap_bits = std::max<size_t>(4096, (size_t)env_long("CULSH_CHAIN_BITS", 344064) / 4096 * 4096);
+int window_bits(int n_rows, int* n_win) {
+    const size_t cap_bits = std::max<size_t>(4096, (size_t)env_long("CULSH_CHAIN_BITS", WINDOW_ROWS) / 4096 * 4096);
     const size_t n = (size_t)std::max(n_rows, 1);
     const size_t wins = ceil_div(n, cap_bits);
     *n_win = (int)std::min<size_t>(wins, 1u << 20);
@@ -708,6 +708,29 @@ struct RawCounts {
     uint32_t *big_list, *mid_list, *counters;
     int mid_max;
 };
+
+// The result inside its raw array, when there is no memory for a second one: what a run of queries has goes
+// through a buffer to where it belongs, at or before where it was and before what the next run has.
+template <typename Compact>
+void compact_in_place(const CtxPtr& c, culsh_candidates& out, DevBuf<int32_t>& raw_ids, uint64_t bounce, Compact&& compact) {
+    const int n_q = out.n_queries;
+    std::vector<uint64_t> off((size_t)n_q + 1);
+    CU_CHECK(cudaMemcpyAsync(off.data(), out.offsets.p, sizeof(uint64_t) * off.size(), cudaMemcpyDeviceToHost, c->stream));
+    CU_CHECK(cudaStreamSynchronize(c->stream));
+    uint64_t most = 0;
+    for (int q = 0; q < n_q; ++q) most = std::max(most, off[(size_t)q + 1] - off[q]);
+    const uint64_t cap = std::max(bounce ? bounce : (uint64_t)(BIG_BLOCK_MIN / sizeof(int32_t)), most);
+    DevBuf<int32_t> buf(c, cap);
+    for (int q0 = 0; q0 < n_q;) {
+        const int q1 = (int)(std::upper_bound(off.begin() + q0 + 1, off.end(), off[q0] + cap) - off.begin()) - 1;
+        if (off[q1] > off[q0]) {
+            compact(q0, q1, off[q0], buf.p);
+            CU_CHECK(cudaMemcpyAsync(raw_ids.p + off[q0], buf.p, sizeof(int32_t) * (off[q1] - off[q0]), cudaMemcpyDeviceToDevice, c->stream));
+        }
+        q0 = q1;
+    }
+    out.indices = std::move(raw_ids);
+}
 
 // `count`, if there is one, launches what finds the lists and counts them; they are in `bounds` else.
 // False, and nothing done, when there are more than raw_limit list entries.  On return the device
@@ -733,7 +756,6 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
     const int wbits = bitmap_window_bits(c, ix.n);
     // with more rows than two bitmap windows, mid-sized candidate sets are sorted in shared memory
     const int mid_max = (size_t)ix.n > 2 * (size_t)wbits ? MID_MAX : 0;
-    const uint32_t self_lists = self_join ? (uint32_t)L : 0u;
     if (count) {
         count(RawCounts{raw_cnt.p, raw_off.p, big_list.p, mid_list, n_big, mid_max});
     } else {
@@ -771,22 +793,25 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         finish();
         return true;
     }
-    // Single pass (ids emitted at their final CSR position, no compaction) when most queries have
-    // large candidate sets and the row range is a few chain windows; otherwise scratch + compaction.
+    // Large sets: a CTA for each (query, window of the rows) where that is a few windows, else one for each query.
     int n_win = 1;
-    const int cbits = chain_window_bits(ix.n, &n_win);
-    const long stage_env = env_long("CULSH_CHAIN_STAGE", 0);
-    const int stage_ids = stage_env == 0 ? 0 : (int)std::min<long>(40960, std::max<long>(256, stage_env));
-    const bool chained = n_win <= CHAIN_MAX_WINDOWS && L <= CW_MAX_L && (size_t)nb * 2 >= (size_t)n_q &&
-                         (uint64_t)n_q * (uint64_t)n_win < (1ull << 31) &&
-                         chain_window_smem_bytes(cbits, stage_ids) + 1024 <= c->smem_optin;
+    const int cbits = window_bits(ix.n, &n_win);
+    const bool windows = nb && n_win <= MAX_WINDOWS && L <= CW_MAX_L && (uint64_t)nb * (uint64_t)n_win < (1ull << 31) &&
+                         window_smem_bytes(cbits) + 1024 <= c->smem_optin;
     const uint32_t n_other = (uint32_t)n_q - nb - nm;  // queries on the warp path (incl. empty ones)
-    // Scratch copy of the ids of the queries that do not take the chained kernel (warp / sort
-    // paths write it, indexed by raw offsets); the chained kernel reads it only for those, so a
-    // query set that is all large sets (the 1M-row benchmark: 743 MB) needs none.
+    // The ids of a query land in its raw span first.  A large such array is a block of the result's kind: it goes
+    // back when the call is done, and takes the result's place when there is no memory for both.
     Scratch<int32_t> tmp;
-    if (!(chained && n_other == 0 && nm == 0)) tmp.reserve(c, SL_TMP, raw_total);
+    DevBuf<int32_t> raw_ids;
+    if (windows && raw_total * sizeof(int32_t) >= BIG_BLOCK_MIN) {
+        raw_ids.alloc(c, raw_total);
+        tmp.p = raw_ids.p;
+        tmp.n = raw_total;
+    } else {
+        tmp.reserve(c, SL_TMP, raw_total);
+    }
     tr.lap("alloc tmp");
+    if (windows && n_win > 1) CU_CHECK(cudaMemsetAsync(out.counts.p, 0, out.counts.bytes(), s));  // the windows add up in it
     if (n_other) {
         // Short lists in a form that fits twice as many warps on an SM, the rest in a second launch; a
         // set that one launch takes in a wave or two is not worth a second one.
@@ -808,94 +833,93 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
                                                        id_bytes, tmp.p, out.counts.p);
         KERNEL_CHECK();
     }
-    if (chained) {
-        out.indices.alloc(c, raw_total);  // capacity: the unique total is not known yet
-        const size_t n_tk = (size_t)n_q * n_win;
-        Scratch<unsigned long long> status(c, SL_CHAIN, n_tk + 1);
-        uint32_t* ticket = reinterpret_cast<uint32_t*>(status.p + n_tk);
-        CU_CHECK(cudaMemsetAsync(status.p, 0, sizeof(unsigned long long) * (n_tk + 1), s));
+    const size_t n_pieces = (size_t)nb * n_win;
+    Scratch<uint2> pieces;
+    if (windows) {
+        pieces.reserve(c, SL_CHAIN, n_pieces);
         // list slices per window, precomputed when the table is small enough (<= 256 MB)
         Scratch<int2> slices;
-        if (env_long("CULSH_CHAIN_SLICES", 1) && n_win > 1 && n_tk * (size_t)L <= ((size_t)32 << 20)) {
-            slices.reserve(c, SL_SLICES, n_tk * (size_t)L);
-            slice_lists_kernel<<<(unsigned)ceil_div(n_tk * (size_t)L, 256), 256, 0, s>>>(
-                bounds, ix.cand.p, raw_cnt.p, n_q, L, cbits, n_win, mid_max, self_lists, slices.p);
+        if (env_long("CULSH_CHAIN_SLICES", 1) && n_win > 1 && n_pieces * (size_t)L <= ((size_t)32 << 20)) {
+            slices.reserve(c, SL_SLICES, n_pieces * (size_t)L);
+            slice_lists_kernel<<<(unsigned)ceil_div(n_pieces * (size_t)L, 256), 256, 0, s>>>(
+                big_list.p, bounds, ix.cand.p, (int)nb, L, cbits, n_win, slices.p);
             KERNEL_CHECK();
         }
         auto launch = [&](auto nt_tag, auto mk_tag) {
             constexpr int NT = decltype(nt_tag)::value;
             constexpr int MK = decltype(mk_tag)::value;
-            const size_t smem = chain_window_smem_bytes(cbits, stage_ids);
-            CU_CHECK(cudaFuncSetAttribute(dedupe_chained_rank_kernel<NT, MK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            CU_CHECK(cudaFuncSetAttribute(dedupe_chained_rank_kernel<NT, MK>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-            dedupe_chained_rank_kernel<NT, MK><<<(unsigned)n_tk, NT, smem, s>>>(
-                bounds, ix.cand.p, raw_cnt.p, raw_off.p, n_q, L, ix.n, cbits, n_win, stage_ids, mid_max, self_lists,
-                slices.p, tmp.p, status.p, ticket, out.indices.p, out.counts.p, out.offsets.p, c->d_error);
+            const size_t smem = window_smem_bytes(cbits);
+            auto kern = dedupe_window_kernel<NT, MK>;
+            CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+            kern<<<(unsigned)n_pieces, NT, smem, s>>>(big_list.p, bounds, ix.cand.p, raw_off.p, L, ix.n, cbits, n_win, self_join,
+                                                      slices.p, tmp.p, pieces.p, reinterpret_cast<unsigned long long*>(out.counts.p));
+            KERNEL_CHECK();
         };
         const long cw_threads = env_long("CULSH_CHAIN_THREADS", 384);
-        const long cw_mk = env_long("CULSH_CHAIN_LOADS", 16);
+        const long cw_mk = env_long("CULSH_CHAIN_LOADS", 8);
         if (c->profiling) cudaEventRecord(c->ev_dedupe[0], s);
         auto with_loads = [&](auto nt_tag) {
             if (cw_mk == 4) launch(nt_tag, std::integral_constant<int, 4>{});
-            else if (cw_mk == 8) launch(nt_tag, std::integral_constant<int, 8>{});
-            else launch(nt_tag, std::integral_constant<int, 16>{});
+            else if (cw_mk == 16) launch(nt_tag, std::integral_constant<int, 16>{});
+            else launch(nt_tag, std::integral_constant<int, 8>{});
         };
         if (cw_threads == 512) with_loads(std::integral_constant<int, 512>{});
         else if (cw_threads == 256) with_loads(std::integral_constant<int, 256>{});
         else with_loads(std::integral_constant<int, 384>{});
+        if (c->profiling) { cudaEventRecord(c->ev_dedupe[1], s); dedupe_timed = true; }
+    } else if (nb) {
+        size_t smem = bitmap_smem_bytes(wbits);
+        CU_CHECK(cudaFuncSetAttribute(dedupe_bitmap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (c->profiling) cudaEventRecord(c->ev_dedupe[0], s);
+        dedupe_bitmap_kernel<<<nb, BM_THREADS, smem, s>>>(big_list.p, bounds, ix.cand.p, raw_off.p,
+                                                          L, ix.n, wbits, tmp.p, out.counts.p);
         KERNEL_CHECK();
         if (c->profiling) { cudaEventRecord(c->ev_dedupe[1], s); dedupe_timed = true; }
-        if (n_win > 1) {
-            counts_from_offsets_kernel<<<(unsigned)ceil_div(n_q, 256), 256, 0, s>>>(out.offsets.p, n_q, out.counts.p);
+    }
+    exclusive_scan<uint64_t, uint64_t>(s, out.counts.p, n_q, out.offsets.p, scratch.p);
+    uint64_t total = 0;
+    read_words(c, out.offsets.p + n_q, sizeof(uint64_t), &total);
+    tr.lap("dedupe+scan+sync");
+    out.total = total;
+    c->stats.unique_candidates += total;
+    // ids of the queries [q_lo, q_hi) from their raw spans to dst[offsets - first]
+    auto compact = [&](int q_lo, int q_hi, uint64_t first, int32_t* dst) {
+        const int count = q_hi - q_lo;
+        if (n_other) {
+            const int per = count >= (1 << 17) ? 32 : CS_ROWS;  // from here on full warps still fill the chip
+            const size_t blocks = std::min<size_t>(ceil_div(ceil_div((size_t)count, per) * 32, 256), (size_t)c->sm_count * 32);
+            compact_small_kernel<<<(unsigned)blocks, 256, 0, s>>>(tmp.p, raw_cnt.p + q_lo, raw_off.p + q_lo, out.counts.p + q_lo,
+                                                                 out.offsets.p + q_lo, count, per, first, dst);
             KERNEL_CHECK();
         }
-        uint64_t total = 0;
-        read_words(c, out.offsets.p + n_q, sizeof(uint64_t), &total);
-        tr.lap("chained dedupe+sync");
-        out.total = total;
-        c->stats.unique_candidates += total;
-        if (total == 0) {
-            out.indices.release();
-        } else if (total * 4 < raw_total * 3) {  // much smaller than the capacity: keep an exact copy
-            DevBuf<int32_t> exact(c, total);
-            CU_CHECK(cudaMemcpyAsync(exact.p, out.indices.p, sizeof(int32_t) * total, cudaMemcpyDeviceToDevice, s));
-            out.indices = std::move(exact);
-        }
-    } else {
-        if (nb) {
-            size_t smem = bitmap_smem_bytes(wbits);
-            CU_CHECK(cudaFuncSetAttribute(dedupe_bitmap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            if (c->profiling) cudaEventRecord(c->ev_dedupe[0], s);
-            dedupe_bitmap_kernel<<<nb, BM_THREADS, smem, s>>>(big_list.p, bounds, ix.cand.p, raw_off.p,
-                                                              L, ix.n, wbits, tmp.p, out.counts.p);
+        if (windows) {
+            compact_windows_kernel<<<(unsigned)n_pieces, 256, 0, s>>>(big_list.p, tmp.p, raw_off.p, pieces.p, out.offsets.p, n_win,
+                                                                     (uint32_t)q_lo, (uint32_t)q_hi, first, dst);
             KERNEL_CHECK();
-            if (c->profiling) { cudaEventRecord(c->ev_dedupe[1], s); dedupe_timed = true; }
         }
-        exclusive_scan<uint64_t, uint64_t>(s, out.counts.p, n_q, out.offsets.p, scratch.p);
-        uint64_t total = 0;
-        read_words(c, out.offsets.p + n_q, sizeof(uint64_t), &total);
-        tr.lap("dedupe+scan+sync");
-        out.total = total;
-        c->stats.unique_candidates += total;
-        if (total) {
-            out.indices.alloc(c, total);
-            tr.lap("alloc indices");
-            const int per = n_q >= (1 << 17) ? 32 : CS_ROWS;  // from here on full warps still fill the chip
-            const size_t blocks = std::min<size_t>(ceil_div(ceil_div((size_t)n_q, per) * 32, 256), (size_t)c->sm_count * 32);
-            compact_small_kernel<<<(unsigned)blocks, 256, 0, s>>>(tmp.p, raw_cnt.p, raw_off.p, out.counts.p,
-                                                                 out.offsets.p, n_q, per, out.indices.p);
+        auto copy_list = [&](const uint32_t* list, uint32_t n_list) {
+            compact_big_kernel<<<n_list, 256, 0, s>>>(list, tmp.p, raw_off.p, out.counts.p, out.offsets.p,
+                                                      (uint32_t)q_lo, (uint32_t)q_hi, first, dst);
             KERNEL_CHECK();
-            if (nb) {
-                compact_big_kernel<<<nb, 256, 0, s>>>(big_list.p, tmp.p, raw_off.p, out.counts.p,
-                                                      out.offsets.p, out.indices.p);
-                KERNEL_CHECK();
-            }
-            if (nm) {
-                compact_big_kernel<<<nm, 256, 0, s>>>(mid_list, tmp.p, raw_off.p, out.counts.p,
-                                                      out.offsets.p, out.indices.p);
-                KERNEL_CHECK();
+        };
+        if (nb && !windows) copy_list(big_list.p, nb);
+        if (nm) copy_list(mid_list, nm);
+    };
+    if (total) {
+        const long bounce_env = env_long("CULSH_COMPACT_BOUNCE", 0);
+        bool second = !(raw_ids.p && bounce_env > 0);
+        if (second) {
+            try {
+                out.indices.alloc(c, total);
+            } catch (const Error& e) {
+                if (e.status != CULSH_ERR_ALLOC || !raw_ids.p) throw;
+                second = false;
             }
         }
+        tr.lap("alloc indices");
+        if (second) compact(0, n_q, 0, out.indices.p);
+        else compact_in_place(c, out, raw_ids, (uint64_t)std::max(bounce_env, 0l), compact);
     }
     tm.mark();
     finish();

@@ -4,7 +4,7 @@
 // candidates, runs a 32-bit segmented radix sort over them, flags/reduces/scans and
 // compacts (about 15 passes over `raw` ints); here each query's bucket lists are merged
 // on chip - a shared-memory bitmap over row ids for large candidate sets, a warp-level
-// sort for small ones - and each list is read once and its unique ids written once.
+// sort for small ones - and each list is read once, its unique ids written to the query's raw span and copied from there.
 #pragma once
 
 #include "common.cuh"
@@ -175,11 +175,6 @@ lookup_count_kernel(const uint32_t* __restrict__ qkeys, const uint8_t* __restric
     __syncthreads();
     if (tid == 0) raw_off[n_q] = carry;
     if (tid < 3) counters[tid] = s_counters[tid];
-}
-
-// A query is on the bitmap / chained path when neither the warp nor the sort path takes it.
-__device__ __forceinline__ bool is_big(uint64_t raw, int mid_max, uint32_t self_lists) {
-    return raw > (uint64_t)SMALL_MAX && raw + self_lists > (uint64_t)mid_max;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -713,101 +708,25 @@ dedupe_bitmap_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds,
 }
 
 // ---------------------------------------------------------------------------------------
-// Chained single-pass dedupe for query sets dominated by large candidate sets: CTAs take
-// (query, window) tickets from an atomic counter IN CSR ORDER, so a CTA only ever waits on CTAs
-// that started before it.  After counting its unique ids a CTA publishes the count, obtains the
-// sum over all earlier tickets from a chained look-back over `status` (a warp reads 32
-// predecessors per round), and writes its sorted ids straight at their final CSR position - no
-// scratch copy, no compaction pass.  Queries that took the warp / sort paths have their count
-// and ids in `tmp` already; their first ticket joins the chain with that count and copies the
-// ids, their other tickets publish zero.
-// status word: bits 62-63 flag (0 empty, 1 own count, 2 inclusive prefix), low 62 bits value.
-// Every wait is bounded; on expiry DEV_ERR_LOOKBACK_TIMEOUT is recorded and the CTA goes on.
-// ---------------------------------------------------------------------------------------
-constexpr unsigned long long CH_FLAG_AGG = 1ull << 62;
-constexpr unsigned long long CH_FLAG_INC = 2ull << 62;
-constexpr unsigned long long CH_VAL_MASK = (1ull << 62) - 1;
-constexpr int CH_SPIN_LIMIT = 1 << 22;
-
-__device__ __forceinline__ unsigned long long ld_volatile_u64(const unsigned long long* p) {
-    return *reinterpret_cast<const volatile unsigned long long*>(p);
-}
-
-// Executed by warp 0 of the CTA that owns ticket q; returns the exclusive prefix.
-// `publish` stores this query's own count first (done once); with `blocking` false the walk
-// gives up (returns false, nothing published) as soon as a needed predecessor is missing.
-__device__ __forceinline__ bool chain_exclusive_prefix(unsigned long long* status, int q,
-                                                       unsigned long long own, int lane, int* d_error,
-                                                       bool publish, bool blocking, unsigned long long& excl_out) {
-    unsigned long long* mine = status + q;
-    excl_out = 0ull;
-    if (q == 0) {
-        if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(mine) = CH_FLAG_INC | own;
-        return true;
-    }
-    if (publish && lane == 0) *reinterpret_cast<volatile unsigned long long*>(mine) = CH_FLAG_AGG | own;
-    unsigned long long excl = 0;
-    int j = q - 1;
-    bool done = false;
-    while (!done) {
-        const int idx = j - lane;
-        unsigned long long s = idx >= 0 ? ld_volatile_u64(status + idx) : CH_FLAG_INC;  // before query 0: prefix 0
-        int spins = 0;
-        while (__any_sync(0xFFFFFFFFu, (s >> 62) == 0)) {  // someone in the window has not published yet
-            if (!blocking) {
-                // usable only if a prefix sits nearer than the first missing entry
-                const uint32_t miss = __ballot_sync(0xFFFFFFFFu, (s >> 62) == 0);
-                const uint32_t inc = __ballot_sync(0xFFFFFFFFu, (s >> 62) == 2);
-                if (inc && (__ffs(inc) < __ffs(miss))) break;
-                return false;
-            }
-            if (++spins > CH_SPIN_LIMIT) {
-                if (lane == 0) atomicOr(d_error, DEV_ERR_LOOKBACK_TIMEOUT);
-                s |= CH_FLAG_INC;  // give up: treat as a prefix so that the walk ends
-                break;
-            }
-            if (spins > 16) __nanosleep(64);
-            if ((s >> 62) == 0) s = ld_volatile_u64(status + idx);
-        }
-        const uint32_t inc_mask = __ballot_sync(0xFFFFFFFFu, (s >> 62) == 2);
-        const int stop = inc_mask ? __ffs(inc_mask) - 1 : 32;  // nearest predecessor holding a prefix
-        unsigned long long v = lane <= stop ? (s & CH_VAL_MASK) : 0ull;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-        excl += v;
-        done = inc_mask != 0;
-        j -= 32;
-    }
-    if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(mine) = CH_FLAG_INC | ((excl + own) & CH_VAL_MASK);
-    excl_out = excl;
-    return true;
-}
-
-// ---------------------------------------------------------------------------------------
-// Rank form of the chained kernel.  The row range is cut into n_win windows of window_bits rows
-// and one CTA handles one (query, window) pair, tickets in (query, window) order - the order of
-// the ids in the CSR.  A CTA
-//   1. narrows every bucket list (ascending row ids) to its window with a 32-way warp search,
-//   2. marks the ids of those slices in a shared-memory bitmap,
-//   3. scans the bitmap once: pop-count prefix per 32-bit word (16 bits, inside blocks of 512
-//      rows), a base per block and the number of unique ids, which it publishes to the chain,
-//   4. goes over the ids a second time (from registers when a warp's share fits one batch, else
-//      from L2): the rank of an id among the unique ids of the window is base[block] +
-//      prefix[word] + popc(bits below it), so the id is dropped at stage[rank] in shared memory -
-//      duplicates write the same value to the same slot,
-//   5. resolves its exclusive prefix from the chain and copies the staged ids, now sorted and
-//      unique, to their final CSR position with coalesced stores.
-// Work is proportional to the candidates (two walks) plus one pass over the window, there is no
-// per-bit emission loop and no scratch copy; windows of 32 KB let several CTAs share an SM so the
-// dependent loads of one overlap the work of the others.  A window with more unique ids than the
-// stage holds repeats steps 4-5 per stage-sized chunk of ranks.
+// Window form of the block path: the row range is cut into n_win windows and a CTA takes one
+// (query, window) pair.  It
+//   1. takes the slices of the query's ascending bucket lists that fall into its window,
+//   2. marks their ids in a shared-memory bitmap,
+//   3. counts the bits,
+//   4. writes the ids of the set bits, ascending, to the place of its slices inside the query's raw span of `tmp` -
+//      what is known beforehand, so that no CTA waits for another one.
+// compact_windows_kernel brings the pieces together once the counts of all queries are known.
+//
+// The instructions bound it, not the 8 bytes an id moves (issue slots 89 % taken, the pipe of pop-counts and bit searches 55):
+// 10,000 queries of 20,500 entries over a million rows take 823 us and 218 more for the pieces.  Tickets that chained their
+// counts and wrote to the final place waited for one another as long as they worked (1,140 us); ids kept in registers,
+// ranked by the bits before them and put in order in shared memory have fewer instructions, but random reads of shared
+// memory instead, and fewer CTAs fit an SM (890 to 1,400 us).
 // ---------------------------------------------------------------------------------------
 constexpr int CW_MAX_L = 256;    // lists per query kept in shared memory (<= threads per CTA)
 
-inline size_t chain_window_smem_bytes(int window_bits, int stage_ids) {
-    // bitmap (1 bit per row) + 16-bit prefix per 32-bit word + 32-bit base per 512 rows + stage + lists
-    return (size_t)window_bits / 8 + (size_t)window_bits / 16 + (size_t)window_bits / 128 +
-           (size_t)stage_ids * sizeof(int32_t) + (3 * CW_MAX_L + 1) * sizeof(int);
+inline size_t window_smem_bytes(int window_bits) {
+    return (size_t)window_bits / 8 + (3 * CW_MAX_L + 1) * sizeof(int);  // bitmap, lists
 }
 
 // First position p in [lo, hi) with a[p] >= target (hi if there is none).  Called by a full warp.
@@ -874,25 +793,23 @@ struct ListWalk {
     }
 };
 
-// Slice of every bucket list that falls into every window: slices[(q * n_win + w) * L + t] =
-// [a, b) in cand.  One thread per (query, list, window) finds the window's lower boundary with a
+// Slice of every bucket list that falls into every window: slices[(b * n_win + w) * L + t] =
+// [a, z) in cand for the query big_list[b].  One thread per (query, list, window) finds the window's lower boundary with a
 // binary search and writes it as the start of its own slice and the end of the previous one;
 // with a million independent searches in flight the dependent loads cost nothing, whereas
-// inside the chained kernel they would sit on the critical path of every CTA.
+// inside the window kernel they would sit on the critical path of every CTA.
 __global__ void __launch_bounds__(256)
-slice_lists_kernel(BoundsView bounds, const int32_t* __restrict__ cand,
-                   const uint64_t* __restrict__ raw_cnt, int n_q, int L, int window_bits, int n_win, int mid_max,
-                   uint32_t self_lists, int2* __restrict__ slices) {
+slice_lists_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds, const int32_t* __restrict__ cand, int n_big, int L,
+                   int window_bits, int n_win, int2* __restrict__ slices) {
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (size_t)n_q * L * n_win) return;
+    if (idx >= (size_t)n_big * L * n_win) return;
     const int w = (int)(idx % n_win);
-    const size_t pair = idx / n_win;  // q * L + t
-    const int q = (int)(pair / L), t = (int)(pair - (size_t)q * L);
-    if (!is_big(raw_cnt[q], mid_max, self_lists)) return;
-    const int2 be = bounds.get(t, q);
+    const size_t pair = idx / n_win;  // b * L + t
+    const int b = (int)(pair / L), t = (int)(pair - (size_t)b * L);
+    const int2 be = bounds.get(t, (int)big_list[b]);
     const int lo = be.x, we = be.y;
     int* flat = reinterpret_cast<int*>(slices);
-    const size_t mine = (((size_t)q * n_win + w) * L + t) * 2;
+    const size_t mine = (((size_t)b * n_win + w) * L + t) * 2;
     int a = lo;
     if (w > 0) {
         const long long bound = (long long)w * window_bits;
@@ -903,287 +820,193 @@ slice_lists_kernel(BoundsView bounds, const int32_t* __restrict__ cand,
     if (w == n_win - 1) flat[mine + 1] = we;
 }
 
+// pieces[b * n_win + w]: x = where the piece starts inside the query's raw span, y = its ids
 template <int NT, int MK>
 __global__ void __launch_bounds__(NT)
-dedupe_chained_rank_kernel(BoundsView bounds, const int32_t* __restrict__ cand, const uint64_t* __restrict__ raw_cnt,
-                           const uint64_t* __restrict__ raw_off, int n_q, int L, int n_rows, int window_bits,
-                           int n_win, int stage_ids, int mid_max, uint32_t self_lists, const int2* __restrict__ slices /* or null */,
-                           const int32_t* __restrict__ tmp,
-                           unsigned long long* __restrict__ status, uint32_t* __restrict__ ticket,
-                           int32_t* __restrict__ out_indices, uint64_t* __restrict__ counts,
-                           uint64_t* __restrict__ offsets, int* __restrict__ d_error) {
+dedupe_window_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds, const int32_t* __restrict__ cand,
+                     const uint64_t* __restrict__ raw_off, int L, int n_rows, int window_bits, int n_win, bool self_join,
+                     const int2* __restrict__ slices /* or null */, int32_t* __restrict__ tmp, uint2* __restrict__ pieces,
+                     unsigned long long* __restrict__ uniq_cnt) {
     constexpr int NWARP = NT / 32;
     extern __shared__ __align__(16) uint32_t s_dyn[];
-    const int n32 = window_bits / 32;      // a multiple of 128
-    const int n_blocks = n32 / 16;         // blocks of 512 rows
-    uint32_t* bm32 = s_dyn;                                                    // [n32] bitmap
-    uint16_t* pre16 = reinterpret_cast<uint16_t*>(bm32 + n32);                // [n32] set bits before the word, inside its block
-    uint32_t* base32 = reinterpret_cast<uint32_t*>(pre16 + n32);              // [n_blocks] set bits before the block
-    int32_t* stage = reinterpret_cast<int32_t*>(base32 + n_blocks);          // [stage_ids]
-    int* s_lo = reinterpret_cast<int*>(stage + stage_ids);                    // [L] slice start in cand
-    int* s_we = s_lo + CW_MAX_L;                                               // [L] slice end
-    int* s_pre = s_we + CW_MAX_L;                                              // [L + 1] prefix of slice lengths
+    const int n32 = window_bits / 32;                        // a multiple of 128
+    uint32_t* bm32 = s_dyn;                                  // [n32] bitmap
+    int* s_lo = reinterpret_cast<int*>(bm32 + n32);          // [L] slice start in cand
+    int* s_we = s_lo + CW_MAX_L;                             // [L] slice end
+    int* s_pre = s_we + CW_MAX_L;                            // [L + 1] prefix of slice lengths
     __shared__ uint32_t s_wtot[NWARP];
-    __shared__ unsigned long long s_excl;
-    __shared__ int s_tk;
+    __shared__ uint32_t s_wskip[NWARP];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) s_tk = (int)atomicAdd(ticket, 1u);
-    __syncthreads();
-    const int tk = s_tk;
-    const long long n_tk = (long long)n_q * n_win;
-    if (tk >= n_tk) return;
-    const int q = tk / n_win, w = tk - q * n_win;
-    const bool last_ticket = tk == n_tk - 1;
-    const bool big = is_big(raw_cnt[q], mid_max, self_lists);
-
-    if (!big) {  // count and ids are in tmp already: window 0 joins the chain with them and copies
-        if (w > 0 && !last_ticket) {
-            if (tid == 0) *reinterpret_cast<volatile unsigned long long*>(status + tk) = CH_FLAG_AGG;
-            return;
-        }
-        const unsigned long long c = w == 0 ? counts[q] : 0ull;
-        if (warp == 0) {
-            unsigned long long e;
-            chain_exclusive_prefix(status, tk, c, lane, d_error, true, true, e);
-            if (lane == 0) s_excl = e;
-        }
-        __syncthreads();
-        const unsigned long long excl = s_excl;
-        const int32_t* src = tmp + raw_off[q];
-        for (unsigned long long i = tid; i < c; i += NT) out_indices[excl + i] = src[i];
-        if (tid == 0) {
-            if (w == 0) offsets[q] = excl;
-            if (last_ticket) offsets[n_q] = excl + c;
-        }
-        return;
-    }
-
+    const int slot = blockIdx.x / n_win, w = blockIdx.x - slot * n_win;
+    const int q = (int)big_list[slot];
     const int win_lo = w * window_bits;
     const int win_hi = min(n_rows, win_lo + window_bits);
-    // ---- 1. clear, list bounds, slices ----
-    {
-        uint4* b4 = reinterpret_cast<uint4*>(s_dyn);
-        for (int i = tid; i < n32 / 4; i += NT) b4[i] = make_uint4(0, 0, 0, 0);
-    }
+    // ---- 1. clear, slices, their prefix and the raw ids of the windows before this one ----
+    int first = 0;  // of this thread's whole list
+    int2 mine = make_int2(0, 0);
     if (slices) {
         if (tid < L) {
-            const int2 sl = slices[(size_t)tk * L + tid];
-            s_lo[tid] = sl.x; s_we[tid] = sl.y;
+            mine = slices[(size_t)blockIdx.x * L + tid];
+            first = slices[(size_t)slot * n_win * L + tid].x;
         }
-    } else {
-        if (tid < L) {
-            const int2 be = bounds.get(tid, q);
-            s_lo[tid] = be.x; s_we[tid] = be.y;
-        }
-        if (n_win > 1) {
-            __syncthreads();
-            for (int t = warp; t < L; t += NWARP) {
-                const int lo = s_lo[t], we = s_we[t];
-                if (lo >= we) continue;
-                int a = lo, b = we;
-                if (w > 0) a = warp_lower_bound(cand, lo, we, win_lo, lane);
-                if (w < n_win - 1) b = warp_lower_bound(cand, a, we, win_hi, lane);
-                if (lane == 0) { s_lo[t] = a; s_we[t] = b; }
-            }
-        }
+    } else if (tid < L) {
+        mine = bounds.get(tid, q);
+        first = mine.x;
     }
-    __syncthreads();
+    {
+        uint4* b4 = reinterpret_cast<uint4*>(bm32);
+        for (int i = tid; i < n32 / 4; i += NT) b4[i] = make_uint4(0, 0, 0, 0);
+    }
+    if (!slices && n_win > 1) {
+        if (tid < L) { s_lo[tid] = mine.x; s_we[tid] = mine.y; }
+        __syncthreads();
+        for (int t = warp; t < L; t += NWARP) {
+            const int lo = s_lo[t], we = s_we[t];
+            if (lo >= we) continue;
+            int a = lo, b = we;
+            if (w > 0) a = warp_lower_bound(cand, lo, we, win_lo, lane);
+            if (w < n_win - 1) b = warp_lower_bound(cand, a, we, win_hi, lane);
+            if (lane == 0) { s_lo[t] = a; s_we[t] = b; }
+        }
+        __syncthreads();
+        if (tid < L) mine = make_int2(s_lo[tid], s_we[tid]);
+    }
+    // A self-join's raw count takes the own row off every list and adds it once, and so does the place of a piece:
+    // a list with ids before this window has the own row among them if that lies there.
+    const bool own_before = self_join && q < win_lo;
+    uint32_t skip = (uint32_t)(mine.x - first);
+    if (own_before && skip) --skip;
     {   // exclusive prefix of the slice lengths (L <= NT)
-        const int len = tid < L ? s_we[tid] - s_lo[tid] : 0;
+        const int len = mine.y - mine.x;
         int inc = len;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
             if (lane >= o) inc += x;
         }
-        if (lane == 31) s_wtot[warp] = (uint32_t)inc;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) skip += __shfl_xor_sync(0xFFFFFFFFu, skip, o);
+        if (lane == 31) { s_wtot[warp] = (uint32_t)inc; s_wskip[warp] = skip; }
+        if (tid < L) s_lo[tid] = mine.x;
         __syncthreads();
         int base = 0;
         for (int i = 0; i < warp; ++i) base += (int)s_wtot[i];
         if (tid < L) s_pre[tid] = base + inc - len;
         if (tid == L - 1) s_pre[L] = base + inc;
+        skip = own_before ? 1u : 0u;
+        for (int i = 0; i < (L + 31) / 32; ++i) skip += s_wskip[i];
     }
     __syncthreads();
-    // ---- 2. mark.  A stretch that fits one batch keeps its ids in registers for step 4. ----
-    ListWalk<NT, MK> wk;
-    wk.init(s_lo, s_pre, L);
-    const bool single = wk.per_warp <= 32 * MK;  // same for every warp
-    int32_t v[MK];
-    auto mark = [&](int32_t x) {
-        const uint32_t id = (uint32_t)(x - win_lo);
-        atomicOr(&bm32[id >> 5], 1u << (id & 31));
-    };
-    if (single) {
-        wk.load(cand, s_lo, s_pre, wk.w_begin + lane, v);
-#pragma unroll
-        for (int j = 0; j < MK; ++j)
-            if (v[j] >= 0) mark(v[j]);
-    } else {
+    // ---- 2. mark ----
+    {
+        ListWalk<NT, MK> wk;
+        wk.init(s_lo, s_pre, L);
+        int32_t v[MK];
         for (int e0 = wk.w_begin + lane; e0 - lane < wk.w_end; e0 += 32 * MK) {
             wk.load(cand, s_lo, s_pre, e0, v);
 #pragma unroll
-            for (int j = 0; j < MK; ++j)
-                if (v[j] >= 0) mark(v[j]);
-        }
-    }
-    __syncthreads();
-    // ---- 3. pop-count prefixes.  A warp takes 128 words at a time, a lane four of them; four
-    // lanes make a block of 512 rows: 16-bit prefixes inside the block, block totals on the side,
-    // then one scan over the block totals. ----
-    {
-        const uint4* bm4 = reinterpret_cast<const uint4*>(bm32);
-        uint2* pre2 = reinterpret_cast<uint2*>(pre16);
-        for (int g = warp; g < n32 / 128; g += NWARP) {
-            const uint4 x = bm4[g * 32 + lane];
-            const uint32_t c0 = __popc(x.x), c1 = __popc(x.y), c2 = __popc(x.z), c3 = __popc(x.w);
-            const uint32_t sum = c0 + c1 + c2 + c3;
-            uint32_t inc = sum;
-            uint32_t up = __shfl_up_sync(0xFFFFFFFFu, inc, 1);
-            if ((lane & 3) >= 1) inc += up;
-            up = __shfl_up_sync(0xFFFFFFFFu, inc, 2);
-            if ((lane & 3) >= 2) inc += up;
-            const uint32_t p0 = inc - sum, p1 = p0 + c0, p2 = p1 + c1, p3 = p2 + c2;  // each <= 512
-            pre2[g * 32 + lane] = make_uint2(p0 | (p1 << 16), p2 | (p3 << 16));
-            if ((lane & 3) == 3) base32[g * 8 + (lane >> 2)] = inc;  // block total, turned into a base below
-        }
-    }
-    __syncthreads();
-    const int per_thread = (n_blocks + NT - 1) / NT;
-    const int b_begin = min(n_blocks, tid * per_thread), b_end = min(n_blocks, b_begin + per_thread);
-    uint32_t mine = 0;
-    for (int i = b_begin; i < b_end; ++i) mine += base32[i];
-    uint32_t inc = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-        if (lane >= o) inc += x;
-    }
-    if (lane == 31) s_wtot[warp] = inc;  // safe: every thread passed a barrier after its last read
-    __syncthreads();
-    uint32_t run = inc - mine, wtotal = 0;
-    for (int i = 0; i < NWARP; ++i) {
-        const uint32_t x = s_wtot[i];
-        if (i < warp) run += x;
-        wtotal += x;
-    }
-    for (int i = b_begin; i < b_end; ++i) {
-        const uint32_t x = base32[i];
-        base32[i] = run;
-        run += x;
-    }
-    // publish the count now; the prefix is resolved after the first chunk has been ranked
-    if (tid == 0 && tk > 0) *reinterpret_cast<volatile unsigned long long*>(status + tk) = CH_FLAG_AGG | wtotal;
-    __syncthreads();
-    // ---- 4 + 5. rank, stage, copy out ----
-    unsigned long long excl = 0;
-    if (stage_ids == 0) {
-        // Direct form (no stage): ranks are computed while warp 0 walks the chain, then every id
-        // is stored at out[excl + rank]; the ~20 KB target span of a window merges in L2.
-        auto rank_of = [&](int32_t x) -> uint32_t {
-            const uint32_t id = (uint32_t)(x - win_lo);
-            const uint32_t word = id >> 5;
-            const uint32_t below = bm32[word] & ((1u << (id & 31)) - 1u);
-            return base32[id >> 9] + (uint32_t)pre16[word] + (uint32_t)__popc(below);
-        };
-        uint32_t rk[MK];
-        if (single && warp != 0) {
-#pragma unroll
-            for (int j = 0; j < MK; ++j) rk[j] = v[j] >= 0 ? rank_of(v[j]) : 0u;
-        }
-        if (warp == 0) {
-            unsigned long long e;
-            chain_exclusive_prefix(status, tk, (unsigned long long)wtotal, lane, d_error, false, true, e);
-            if (lane == 0) s_excl = e;
-            if (single) {
-#pragma unroll
-                for (int j = 0; j < MK; ++j) rk[j] = v[j] >= 0 ? rank_of(v[j]) : 0u;
-            }
-        }
-        __syncthreads();
-        excl = s_excl;
-        int32_t* dst = out_indices + excl;
-        if (single) {
-#pragma unroll
-            for (int j = 0; j < MK; ++j)
-                if (v[j] >= 0) dst[rk[j]] = v[j];
-        } else {
-            wk.init(s_lo, s_pre, L);
-            for (int e0 = wk.w_begin + lane; e0 - lane < wk.w_end; e0 += 32 * MK) {
-                wk.load(cand, s_lo, s_pre, e0, v);
-#pragma unroll
-                for (int j = 0; j < MK; ++j)
-                    if (v[j] >= 0) dst[rank_of(v[j])] = v[j];
-            }
-        }
-    } else
-    for (uint32_t chunk_lo = 0; chunk_lo == 0 || chunk_lo < wtotal; chunk_lo += (uint32_t)stage_ids) {
-        auto rank = [&](int32_t x) {
-            const uint32_t id = (uint32_t)(x - win_lo);
-            const uint32_t word = id >> 5;
-            const uint32_t below = bm32[word] & ((1u << (id & 31)) - 1u);
-            const uint32_t r = base32[id >> 9] + (uint32_t)pre16[word] + (uint32_t)__popc(below) - chunk_lo;
-            if (r < (uint32_t)stage_ids) stage[r] = x;
-        };
-        if (wtotal > 0) {
-            if (single) {
-#pragma unroll
-                for (int j = 0; j < MK; ++j)
-                    if (v[j] >= 0) rank(v[j]);
-            } else {
-                wk.init(s_lo, s_pre, L);
-                for (int e0 = wk.w_begin + lane; e0 - lane < wk.w_end; e0 += 32 * MK) {
-                    wk.load(cand, s_lo, s_pre, e0, v);
-#pragma unroll
-                    for (int j = 0; j < MK; ++j)
-                        if (v[j] >= 0) rank(v[j]);
+            for (int j = 0; j < MK; ++j) {
+                if (v[j] >= 0) {
+                    const uint32_t id = (uint32_t)(v[j] - win_lo);
+                    atomicOr(&bm32[id >> 5], 1u << (id & 31));
                 }
             }
         }
-        if (chunk_lo == 0) {
-            if (warp == 0) {
-                unsigned long long e;
-                chain_exclusive_prefix(status, tk, (unsigned long long)wtotal, lane, d_error, false, true, e);
-                if (lane == 0) s_excl = e;
-            }
-        }
-        __syncthreads();
-        excl = s_excl;
-        const uint32_t n_chunk = min((uint32_t)stage_ids, wtotal - chunk_lo);
-        int32_t* dst = out_indices + excl + chunk_lo;
-        for (uint32_t i = tid; i < n_chunk; i += NT) dst[i] = stage[i];
-        if (chunk_lo + (uint32_t)stage_ids < wtotal) __syncthreads();  // stage is reused by the next chunk
+    }
+    __syncthreads();
+    // ---- 3. count.  The bitmap in groups of 128 words, one uint4 a lane; a warp owns a stretch of groups. ----
+    const uint4* bm4 = reinterpret_cast<const uint4*>(bm32);
+    const int groups = n32 / 128, per_warp = (groups + NWARP - 1) / NWARP;
+    const int g_begin = min(groups, warp * per_warp), g_end = min(groups, g_begin + per_warp);
+    uint32_t sum = 0;
+    for (int g = g_begin; g < g_end; ++g) {
+        const uint4 x = bm4[g * 32 + lane];
+        sum += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    if (lane == 0) s_wtot[warp] = sum;
+    __syncthreads();
+    uint32_t at = 0, total = 0;
+    for (int i = 0; i < NWARP; ++i) {
+        const uint32_t x = s_wtot[i];
+        if (i < warp) at += x;
+        total += x;
     }
     if (tid == 0) {
-        if (w == 0) offsets[q] = excl;
-        if (n_win == 1) counts[q] = wtotal;
-        if (last_ticket) offsets[n_q] = excl + wtotal;
+        pieces[blockIdx.x] = make_uint2(skip, total);
+        if (n_win == 1) uniq_cnt[q] = total;
+        else if (total) atomicAdd(&uniq_cnt[q], (unsigned long long)total);
     }
-}
-
-// counts[q] = offsets[q + 1] - offsets[q]
-__global__ void counts_from_offsets_kernel(const uint64_t* __restrict__ offsets, int n_q,
-                                           uint64_t* __restrict__ counts) {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < (uint32_t)n_q) counts[q] = offsets[q + 1] - offsets[q];
+    // ---- 4. emit ----
+    int32_t* out = tmp + raw_off[q] + skip + at;
+    for (int g = g_begin; g < g_end; ++g) {
+        const uint4 x = bm4[g * 32 + lane];
+        const uint32_t wv[4] = {x.x, x.y, x.z, x.w};
+        const uint32_t c = __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+        uint32_t inc = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        int32_t* dst = out + (inc - c);
+        const int32_t id0 = win_lo + (g * 128 + lane * 4) * 32;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            uint32_t bits = wv[j];
+            while (bits) {
+                *dst++ = id0 + j * 32 + (__ffs(bits) - 1);
+                bits &= bits - 1;
+            }
+        }
+        out += __shfl_sync(0xFFFFFFFFu, inc, 31);
+    }
 }
 
 // ---------------------------------------------------------------------------------------
 // Compaction of the per-query segments from their raw offsets to their final offsets.
 // ---------------------------------------------------------------------------------------
-// Queries of big_list: a whole block copies the segment.
+// Queries of big_list in [q_lo, q_hi): a whole block copies the segment, to out[offsets[q] - first ...].
 __global__ void __launch_bounds__(256)
 compact_big_kernel(const uint32_t* __restrict__ big_list, const int32_t* __restrict__ tmp,
                    const uint64_t* __restrict__ raw_off, const uint64_t* __restrict__ uniq_cnt,
-                   const uint64_t* __restrict__ offsets, int32_t* __restrict__ out) {
-    const int q = (int)big_list[blockIdx.x];
+                   const uint64_t* __restrict__ offsets, uint32_t q_lo, uint32_t q_hi, uint64_t first, int32_t* __restrict__ out) {
+    const uint32_t q = big_list[blockIdx.x];
+    if (q < q_lo || q >= q_hi) return;
     const uint64_t c = uniq_cnt[q];
     const int32_t* src = tmp + raw_off[q];
-    int32_t* dst = out + offsets[q];
+    int32_t* dst = out + (offsets[q] - first);
     for (uint64_t i = threadIdx.x; i < c; i += blockDim.x) dst[i] = src[i];
 }
 
-// Small queries only (big ones are copied by compact_big_kernel).  A warp takes `per` <= 32 queries
+// The pieces of the queries that went through dedupe_window_kernel, a CTA per (query, window): queries [q_lo, q_hi), to
+// out[offsets[q] - first ...].  Bound by the 8 bytes an id moves.
+constexpr int CWN_LOADS = 8;
+__global__ void __launch_bounds__(256)
+compact_windows_kernel(const uint32_t* __restrict__ big_list, const int32_t* __restrict__ tmp, const uint64_t* __restrict__ raw_off,
+                       const uint2* __restrict__ pieces, const uint64_t* __restrict__ offsets, int n_win, uint32_t q_lo, uint32_t q_hi,
+                       uint64_t first, int32_t* __restrict__ out) {
+    const int slot = blockIdx.x / n_win, w = blockIdx.x - slot * n_win;
+    const uint32_t q = big_list[slot];
+    if (q < q_lo || q >= q_hi) return;
+    uint64_t to = offsets[q] - first;
+    for (int i = 0; i < w; ++i) to += pieces[slot * (size_t)n_win + i].y;
+    const uint2 p = pieces[blockIdx.x];
+    const int32_t* src = tmp + raw_off[q] + p.x;
+    int32_t* dst = out + to;
+    for (uint32_t i0 = threadIdx.x; i0 < p.y; i0 += 256 * CWN_LOADS) {
+        int32_t v[CWN_LOADS];
+#pragma unroll
+        for (int j = 0; j < CWN_LOADS; ++j) v[j] = i0 + 256 * j < p.y ? src[i0 + 256 * j] : 0;
+#pragma unroll
+        for (int j = 0; j < CWN_LOADS; ++j)
+            if (i0 + 256 * j < p.y) dst[i0 + 256 * j] = v[j];
+    }
+}
+
+// Small queries only (big ones are copied by the two kernels above).  A warp takes `per` <= 32 queries
 // (few for a small set, which would leave the chip idle otherwise), reads
 // their descriptors with one coalesced load each and copies CS_ROWS segments at a time, two words
 // per lane each, so that 2 * CS_ROWS independent loads are in flight; one segment after another
@@ -1192,7 +1015,7 @@ constexpr int CS_ROWS = 4;
 __global__ void __launch_bounds__(256)
 compact_small_kernel(const int32_t* __restrict__ tmp, const uint64_t* __restrict__ raw_cnt,
                      const uint64_t* __restrict__ raw_off, const uint64_t* __restrict__ uniq_cnt,
-                     const uint64_t* __restrict__ offsets, int n_q, int per, int32_t* __restrict__ out) {
+                     const uint64_t* __restrict__ offsets, int n_q, int per, uint64_t first, int32_t* __restrict__ out) {
     const int lane = threadIdx.x & 31;
     const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const size_t n_warps = ((size_t)gridDim.x * blockDim.x) >> 5;
@@ -1203,7 +1026,7 @@ compact_small_kernel(const int32_t* __restrict__ tmp, const uint64_t* __restrict
         if (lane < per && q < (size_t)n_q && raw_cnt[q] <= SMALL_MAX) {
             cnt = (int)uniq_cnt[q];
             from = raw_off[q];
-            to = offsets[q];
+            to = offsets[q] - first;
         }
         for (int i = 0; i < per; i += CS_ROWS) {
             const int32_t* src[CS_ROWS];
