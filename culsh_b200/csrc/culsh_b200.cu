@@ -955,9 +955,8 @@ bool query_batch(const culsh_index& ix, int n_q, HashFn&& hash_fn, culsh_candida
             KERNEL_CHECK();
         };
     } else {
-        CULSH_DISPATCH_NW(NW, (lookup_kernel<NW><<<(unsigned)ceil_div(pairs, 256), 256, 0, c->stream>>>(
-                                  qkeys.p, ovf.p, n_q, ix.L, ix.bucket_keys.p, ix.bucket_offsets.p, ix.table_offsets.p, bounds.p)));
-        KERNEL_CHECK();
+        CULSH_DISPATCH_NW(NW, launch_lookup<NW>(c, qkeys.p, ovf.p, n_q, ix.L, ix.bucket_keys.p, ix.bucket_offsets.p,
+                                                ix.table_offsets.p, bounds.p));
     }
     tm.mark();
     const bool done = query_from_matched(ix, query_bounds(bounds.p, n_q), false, out, tm, raw_limit, count);
@@ -1487,9 +1486,8 @@ int culsh_index_query_keys(culsh_handle* h, const culsh_index* ix, const uint32_
         StageTimer tm(c);
         Scratch<int2> bounds(c, SL_BOUNDS, pairs);
         tm.mark();
-        CULSH_DISPATCH_NW(NW, (lookup_kernel<NW><<<(unsigned)ceil_div(pairs, 256), 256, 0, c->stream>>>(
-                                  keys, nullptr, n_q, ix->L, ix->bucket_keys.p, ix->bucket_offsets.p, ix->table_offsets.p, bounds.p)));
-        KERNEL_CHECK();
+        CULSH_DISPATCH_NW(NW, launch_lookup<NW>(c, keys, nullptr, n_q, ix->L, ix->bucket_keys.p, ix->bucket_offsets.p,
+                                                ix->table_offsets.p, bounds.p));
         tm.mark();
         query_from_matched(*ix, query_bounds(bounds.p, n_q), false, *res, tm);
         c->stats.lookup_ms = tm.between(0, 1);
