@@ -13,6 +13,7 @@
 namespace culsh_b200 {
 
 constexpr uint32_t MINHASH_PRIME = 4294967291u;  // minhash/hash.cuh:17
+constexpr int MH_STEPS = 4;  // pairs of ids a turn of the loop
 constexpr int MH_THREADS = 256;
 constexpr int MH_MAX_PER_LANE = 8;               // hashes per lane per sweep (H <= 256 in one sweep)
 
@@ -57,12 +58,30 @@ __device__ __forceinline__ uint32_t hash_plus5_any(uint32_t a, uint32_t c, uint6
     return t < lo ? t + 5u : t;
 }
 
+// Column ids below 2^20: a*c + b5 + 2^52 is below 2^53, so that one double-precision multiply-add gives it exactly, the low
+// word of x in the low word of the result and the high word of x behind the constant exponent in the other.  The double
+// pipe, which nothing else here uses, takes a warp's multiply-add in two cycles, the integer one a wide one in eight.  What
+// is left - a 32-bit multiply-add for the fold, an add, its carry, and half of a three-way minimum - is bound by
+// issue.  2M sets of 20 to 200 ids into 128 hash functions (with the 10,000 queries): 7,730 -> 6,610 us, 100,003 sets 414 -> 364; two steps a turn of the loop instead of four 6,740 and 372.
+constexpr uint32_t MH_DOUBLE_COL = 1u << 20;
+constexpr double MH_2_52 = 4503599627370496.0;
+constexpr uint32_t MH_2_52_HI = 0x43300000u;
+__device__ __forceinline__ double mh_id(uint32_t c) { return __hiloint2double((int)MH_2_52_HI, (int)c) - MH_2_52; }
+// b52 = b + 5 + 2^52
+__device__ __forceinline__ uint32_t hash_plus5_double(double a, double c, double b52) {
+    const double x = __fma_rn(a, c, b52);
+    const uint32_t five_hi = 5u * (uint32_t)__double2hiint(x) - 5u * MH_2_52_HI;
+    uint32_t t, wrapped;
+    asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, 0, 0;" : "=r"(t), "=r"(wrapped) : "r"((uint32_t)__double2loint(x)), "r"(five_hi));
+    return t + 5u * wrapped;
+}
+
 // keys: [L][n_total][NW] with NW = round_key_words(4k); word j (right-aligned) = bswap32(min).
 // PL = hash functions per lane per sweep; a sweep covers 32*PL consecutive hash functions and
 // H > 256 takes several sweeps.  Slots past H hold a = b = 0, evaluate to 0 and are never stored,
 // so the inner loop carries no predicate.
 template <int PL>
-__global__ void __launch_bounds__(MH_THREADS)
+__global__ void __launch_bounds__(MH_THREADS, PL <= 4 ? 3 : 2)
 minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ indptr,
                const uint32_t* __restrict__ A, const uint32_t* __restrict__ B, int n_rows,
                int L, int k, int NW, uint32_t* __restrict__ keys, int n_total, int row_offset) {
@@ -75,18 +94,39 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
     for (int row = warp; row < n_rows; row += n_warps) {
         const int start = indptr[row], end = indptr[row + 1];
         for (int h0 = 0; h0 < H; h0 += 32 * PL) {
-            uint32_t a[PL], m[PL];
-            uint64_t b[PL];
+            uint32_t m[PL];
+            double ad[PL], bd[PL];
 #pragma unroll
             for (int i = 0; i < PL; ++i) {
                 int h = h0 + i * 32 + lane;
-                a[i] = h < H ? A[h] : 0u;
-                b[i] = h < H ? (uint64_t)B[h] + 5ull : 5ull;
+                ad[i] = h < H ? (double)A[h] : 0.0;
+                bd[i] = (h < H ? (double)B[h] : 0.0) + 5.0 + MH_2_52;
                 m[i] = 0xFFFFFFFFu;
             }
+            // the integer forms take their parameters from the doubles: these are all the loop has registers for
+            auto a_of = [&](int i) { return __double2uint_rz(ad[i]); };
+            auto b5_of = [&](int i) { return (uint64_t)(bd[i] - MH_2_52); };
             for (int base = start; base < end; base += 32) {
                 const int mine = base + lane < end ? indices[base + lane] : 0;
                 const int cnt = min(32, end - base);
+                if (!__any_sync(0xFFFFFFFFu, (uint32_t)mine >= MH_DOUBLE_COL)) {
+#pragma unroll MH_STEPS
+                    for (int s = 0; s < cnt; s += 2) {  // the last id of an odd number twice
+                        const double c0 = mh_id((uint32_t)__shfl_sync(0xFFFFFFFFu, mine, s));
+                        const double c1 = mh_id((uint32_t)__shfl_sync(0xFFFFFFFFu, mine, min(s + 1, cnt - 1)));
+#pragma unroll
+                        for (int i = 0; i < PL; ++i)
+                            m[i] = __vimin3_u32(m[i], hash_plus5_double(ad[i], c0, bd[i]), hash_plus5_double(ad[i], c1, bd[i]));
+                    }
+                    continue;
+                }
+                uint32_t a[PL];
+                uint64_t b[PL];
+#pragma unroll
+                for (int i = 0; i < PL; ++i) {
+                    a[i] = a_of(i);
+                    b[i] = b5_of(i);
+                }
                 if (__any_sync(0xFFFFFFFFu, (uint32_t)mine >= MH_FAST_COL)) {
 #pragma unroll 4
                     for (int s = 0; s < cnt; ++s) {
@@ -108,7 +148,7 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
                 if (m[i] < 5u) {
                     uint32_t exact = 0xFFFFFFFFu;
                     for (int e = start; e < end; ++e)
-                        exact = min(exact, hash_mod_prime(a[i], (uint32_t)indices[e], b[i] - 5ull));
+                        exact = min(exact, hash_mod_prime(a_of(i), (uint32_t)indices[e], b5_of(i) - 5ull));
                     m[i] = exact;
                 } else if (end > start) {
                     m[i] -= 5u;
