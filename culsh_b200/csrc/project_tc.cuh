@@ -128,13 +128,15 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
-__device__ __forceinline__ void tc_mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+// a and b: low words of the operands' descriptors, which share the high one.
+__device__ __forceinline__ void tc_mma_tf32(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t desc_hi, uint32_t idesc,
                                             uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+        "mov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(desc_hi)
         : "memory");
 }
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t* r) {
@@ -150,17 +152,54 @@ __device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sy
 
 // Shared-memory matrix descriptor of a K-major tile whose rows are one swizzle span wide
 // (KBLK fp32 = 128 B or 64 B): 8-row groups follow each other every 8 * span bytes.
+// The address is in the low word, in 16-byte units, the rest in the high one.
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t saddr) { return (saddr & 0x3FFFFu) >> 4; }
 template <int KBLK>
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
-    constexpr uint64_t SBO = (8u * KBLK * 4u) >> 4;
-    constexpr uint64_t LAYOUT = KBLK == 32 ? 2ull /*SWIZZLE_128B*/ : 4ull /*SWIZZLE_64B*/;
-    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (SBO << 32) | (1ull << 46) | (LAYOUT << 61);
+__host__ __device__ constexpr uint32_t smem_desc_hi() {
+    return ((8u * KBLK * 4u) >> 4) | (1u << 14) | ((KBLK == 32 ? 2u /*SWIZZLE_128B*/ : 4u /*SWIZZLE_64B*/) << 29);
 }
 
 // kind::tf32, fp32 accumulate, both operands K-major: c_format=F32 (bit 4), a/b format TF32 (=2)
 __device__ __forceinline__ uint32_t make_idesc_tf32(int M, int N) {
     return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
+
+// What the issuing thread knows of its ring.  It is the serial resource of both kernels: an MMA of N columns keeps the
+// tensor pipe busy for N / 2 cycles, and what the thread does between the MMAs of two K-blocks - waits, whose
+// answer alone takes a few dozen cycles, addresses, the commit - is hidden only as far as the few MMAs that the pipe
+// takes in advance.  So stages are counted, not divided, descriptors are one add away from one another, and the
+// barriers and the flag of the next stage are asked for behind most of the MMAs of this one, late enough to have come and
+// early enough for the answer.  1M x 128 rows and 10,000 queries into 512 columns 546 -> 521 us, 10M x 256 into 1,152 22.2 -> 21.5 ms.
+template <int STAGES>
+struct IssueRing {
+    uint32_t s = 0, parity = 0;
+    bool known = false;  // the stage is ready, as asked for before
+    int flag = 0;
+    __device__ __forceinline__ void ask_next(uint64_t* full, uint64_t* ready, volatile int* lo_flag) {
+        const uint32_t n = s + 1 == STAGES ? 0u : s + 1, p = s + 1 == STAGES ? parity ^ 1u : parity;
+        const bool r = mbar_test_wait(&ready[n], p), f = mbar_test_wait(&full[n], p);
+        flag = lo_flag[n];  // meaningful only when both phases have completed
+        known = r && f;
+    }
+    // Waits for the stage and says whether its low part has anything in it; `live` false: the CTA is aborting.
+    __device__ __forceinline__ int take(uint64_t* full, uint64_t* ready, volatile int* lo_flag, volatile int* abort_flag, int* d_error,
+                                        bool& live) {
+        if (!known) {
+            live = mbar_wait(&ready[s], parity, abort_flag, d_error) && mbar_wait(&full[s], parity, abort_flag, d_error);
+            if (!live) return 0;
+            flag = lo_flag[s];
+        }
+        tc_fence_after();
+        lo_flag[s] = 0;
+        return flag;
+    }
+    __device__ __forceinline__ void advance() {
+        if (++s == STAGES) {
+            s = 0;
+            parity ^= 1u;
+        }
+    }
+};
 
 // 256-bit shift register that receives the key bytes / bits of one table, first element most
 // significant; after k elements it holds the right-aligned key (w[0] most significant).
@@ -464,10 +503,11 @@ project_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
             const uint32_t idesc = make_idesc_tf32(TC_BM, a.n_mma);
-            uint32_t it = 0, u = 0;
-            unsigned long long n_kb = 0, n_lo = 0;
-            bool pre_ok = false;
-            int pre_flag = 0;
+            constexpr uint32_t HI = smem_desc_hi<KBLK>();
+            constexpr uint32_t X16 = Cfg::X_BYTES / 16, P16 = Cfg::P_BYTES / 16, STAGE16 = Cfg::STAGE_BYTES / 16;
+            const uint32_t desc0 = smem_desc_lo(smem_u32(xh(0)));
+            IssueRing<STAGES> ring;
+            uint32_t u = 0, n_kb = 0, n_lo = 0;
             bool live = true;
             for (int tile = blockIdx.x; tile < a.n_tiles && live; tile += gridDim.x) {
                 for (int c = 0; c < n_units_per_tile && live; ++c, ++u) {
@@ -476,47 +516,29 @@ project_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     if (!mbar_wait(&acc_empty[ab], aph ^ 1, s_abort, a.d_error)) { live = false; break; }
                     tc_fence_after();
                     const uint32_t d_tmem = tmem_base + (uint32_t)(ab * TC_BN);
-                    for (int kb = 0; kb < a.n_kblocks; ++kb, ++it) {
-                        const int s = it % STAGES;
-                        const uint32_t phs = (it / STAGES) & 1;
-                        // The issuing thread is the serial resource of the kernel (a wait that succeeds
-                        // at once still costs ~100 cycles), so the barriers and the flag of the next
-                        // stage are probed before this stage's MMAs are issued and the answer is used
-                        // one iteration later.
-                        if (!pre_ok && (!mbar_wait(&full[s], phs, s_abort, a.d_error) ||
-                                        !mbar_wait(&ready[s], phs, s_abort, a.d_error))) { live = false; break; }
-                        tc_fence_after();
-                        const int use_lo = pre_ok ? pre_flag : s_lo_flag[s];
-                        s_lo_flag[s] = 0;
-                        {
-                            const int s1 = (it + 1) % STAGES;
-                            const uint32_t ph1 = ((it + 1) / STAGES) & 1;
-                            const bool f = mbar_test_wait(&full[s1], ph1);
-                            const bool r = mbar_test_wait(&ready[s1], ph1);
-                            pre_flag = s_lo_flag[s1];  // meaningful only when both phases have completed
-                            pre_ok = f && r;
-                        }
-                        ++n_kb;
-                        n_lo += use_lo ? 1u : 0u;
-                        const uint64_t dxh = make_smem_desc<KBLK>(smem_u32(xh(s)));
-                        const uint64_t dxl = make_smem_desc<KBLK>(smem_u32(xl(s)));
-                        const uint64_t dph = make_smem_desc<KBLK>(smem_u32(ph(s)));
-                        const uint64_t dpl = make_smem_desc<KBLK>(smem_u32(pl(s)));
+                    for (int kb = 0; kb < a.n_kblocks; ++kb) {
+                        const int use_lo = ring.take(full, ready, s_lo_flag, s_abort, a.d_error, live);
+                        if (!live) break;
+                        const uint32_t xh_d = desc0 + ring.s * STAGE16, xl_d = xh_d + X16, ph_d = xh_d + 2 * X16, pl_d = ph_d + P16;
 #pragma unroll
                         for (int ks = 0; ks < KBLK / 8; ++ks) {
-                            const uint64_t adv = (uint64_t)(ks * 2);  // 32 bytes per K step, in 16-byte units
-                            tc_mma_tf32(d_tmem, dxh + adv, dpl + adv, idesc, (kb | ks) != 0);
-                            if (use_lo) tc_mma_tf32(d_tmem, dxl + adv, dph + adv, idesc, 1u);
-                            tc_mma_tf32(d_tmem, dxh + adv, dph + adv, idesc, 1u);
+                            const uint32_t adv = (uint32_t)(ks * 2);  // 32 bytes per K step, in 16-byte units
+                            tc_mma_tf32(d_tmem, xh_d + adv, pl_d + adv, HI, idesc, (kb | ks) != 0);
+                            if (use_lo) tc_mma_tf32(d_tmem, xl_d + adv, ph_d + adv, HI, idesc, 1u);
+                            if (ks == KBLK / 8 - 1) ring.ask_next(full, ready, s_lo_flag);
+                            tc_mma_tf32(d_tmem, xh_d + adv, ph_d + adv, HI, idesc, 1u);
                         }
-                        tc_commit(&empty[s]);  // stage reusable once these MMAs have read it
+                        tc_commit(&empty[ring.s]);  // stage reusable once these MMAs have read it
+                        ++n_kb;
+                        n_lo += use_lo ? 1u : 0u;
+                        ring.advance();
                     }
                     if (live) tc_commit(&acc_full[ab]);
                 }
             }
             if (a.d_mma) {
-                atomicAdd(a.d_mma, n_kb);
-                atomicAdd(a.d_mma + 1, n_lo);
+                atomicAdd(a.d_mma, (unsigned long long)n_kb);
+                atomicAdd(a.d_mma + 1, (unsigned long long)n_lo);
             }
         }
     } else if (warp < 6) {
@@ -636,13 +658,14 @@ struct TsCfg {
     static_assert(A_STAGES >= 2 && STAGES >= A_STAGES, "ring sizes");
 };
 
-__device__ __forceinline__ void tc_mma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+__device__ __forceinline__ void tc_mma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b, uint32_t desc_hi, uint32_t idesc,
                                                uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+        "mov.b64 db, {%2, %5};\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], db, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "r"(b), "r"(idesc), "r"(accumulate), "r"(desc_hi)
         : "memory");
 }
 __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t* r) {
@@ -731,10 +754,12 @@ project_ts_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
             const uint32_t idesc = make_idesc_tf32(TC_BM, a.n_mma);
-            uint32_t it = 0, u = 0;
-            unsigned long long n_kb = 0, n_lo = 0;
-            bool pre_ok = false;
-            int pre_flag = 0;
+            constexpr uint32_t HI = smem_desc_hi<TS_KBLK>();
+            constexpr uint32_t P16 = Cfg::P_BYTES / 16, STAGE16 = Cfg::STAGE_BYTES / 16;
+            const uint32_t desc0 = smem_desc_lo(smem_u32(ph(0)));
+            IssueRing<STAGES> ring;
+            uint32_t as = 0;  // A stage
+            uint32_t u = 0, n_kb = 0, n_lo = 0;
             bool live = true;
             for (int tile = blockIdx.x; tile < a.n_tiles && live; tile += gridDim.x) {
                 for (int c = 0; c < n_units_per_tile && live; ++c, ++u) {
@@ -743,45 +768,33 @@ project_ts_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     if (!mbar_wait(&acc_empty[ab], aph ^ 1, s_abort, a.d_error)) { live = false; break; }
                     tc_fence_after();
                     const uint32_t d_tmem = tmem_base + (uint32_t)(ab * BN);
-                    for (int kb = 0; kb < a.n_kblocks; ++kb, ++it) {
-                        const int s = it % STAGES;
-                        const uint32_t phs = (it / STAGES) & 1;
-                        // next stage's barriers and flag are probed early, as in project_tc_kernel
-                        if (!pre_ok && (!mbar_wait(&full[s], phs, s_abort, a.d_error) ||
-                                        !mbar_wait(&ready[s], phs, s_abort, a.d_error))) { live = false; break; }
-                        tc_fence_after();
-                        const int use_lo = pre_ok ? pre_flag : s_lo_flag[s];
-                        s_lo_flag[s] = 0;
-                        {
-                            const int s1 = (it + 1) % STAGES;
-                            const uint32_t ph1 = ((it + 1) / STAGES) & 1;
-                            const bool f = mbar_test_wait(&full[s1], ph1);
-                            const bool r = mbar_test_wait(&ready[s1], ph1);
-                            pre_flag = s_lo_flag[s1];  // meaningful only when both phases have completed
-                            pre_ok = f && r;
-                        }
-                        ++n_kb;
-                        n_lo += use_lo ? 1u : 0u;
-                        const uint32_t axh = tmem_base + (uint32_t)(TS_A_COL0 + (int)(it % A_STAGES) * 2 * TS_KBLK);
+                    for (int kb = 0; kb < a.n_kblocks; ++kb) {
+                        const int use_lo = ring.take(full, ready, s_lo_flag, s_abort, a.d_error, live);
+                        if (!live) break;
+                        const uint32_t axh = tmem_base + (uint32_t)TS_A_COL0 + as * (uint32_t)(2 * TS_KBLK);
                         const uint32_t axl = axh + (uint32_t)TS_KBLK;
-                        const uint64_t dph = make_smem_desc<TS_KBLK>(smem_u32(ph(s)));
-                        const uint64_t dpl = make_smem_desc<TS_KBLK>(smem_u32(pl(s)));
+                        const uint32_t ph_d = desc0 + ring.s * STAGE16, pl_d = ph_d + P16;
 #pragma unroll
                         for (int ks = 0; ks < TS_KBLK / 8; ++ks) {
-                            const uint64_t adv = (uint64_t)(ks * 2);  // 32 bytes per K step, in 16-byte units
+                            const uint32_t adv = (uint32_t)(ks * 2);  // 32 bytes per K step, in 16-byte units
                             const uint32_t acol = (uint32_t)(ks * 8);  // 8 tf32 values = 8 columns per K step
-                            tc_mma_tf32_ts(d_tmem, axh + acol, dpl + adv, idesc, (kb | ks) != 0);
-                            if (use_lo) tc_mma_tf32_ts(d_tmem, axl + acol, dph + adv, idesc, 1u);
-                            tc_mma_tf32_ts(d_tmem, axh + acol, dph + adv, idesc, 1u);
+                            tc_mma_tf32_ts(d_tmem, axh + acol, pl_d + adv, HI, idesc, (kb | ks) != 0);
+                            if (use_lo) tc_mma_tf32_ts(d_tmem, axl + acol, ph_d + adv, HI, idesc, 1u);
+                            if (ks == TS_KBLK / 8 - 1) ring.ask_next(full, ready, s_lo_flag);
+                            tc_mma_tf32_ts(d_tmem, axh + acol, ph_d + adv, HI, idesc, 1u);
                         }
-                        tc_commit(&empty[s]);  // shared-memory stage and A stage reusable once these MMAs are done
+                        tc_commit(&empty[ring.s]);  // shared-memory stage and A stage reusable once these MMAs are done
+                        ++n_kb;
+                        n_lo += use_lo ? 1u : 0u;
+                        ring.advance();
+                        if (++as == (uint32_t)A_STAGES) as = 0;
                     }
                     if (live) tc_commit(&acc_full[ab]);
                 }
             }
             if (a.d_mma) {
-                atomicAdd(a.d_mma, n_kb);
-                atomicAdd(a.d_mma + 1, n_lo);
+                atomicAdd(a.d_mma, (unsigned long long)n_kb);
+                atomicAdd(a.d_mma + 1, (unsigned long long)n_lo);
             }
         }
     } else if (warp < 2 + 4 * G) {
