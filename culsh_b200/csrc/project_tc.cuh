@@ -59,6 +59,7 @@ struct TcArgs {
     int n_tiles, n_chunks, tables_per_chunk, n_mma, n_kblocks;
     int key_words, elem_bytes, family;
     int row_offset, n_total;
+    bool spread;                // a CTA for each unit: few tiles
 };
 
 // ------------------------------------------------------------------------------------------
@@ -556,7 +557,9 @@ project_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     tc_fence_after();
     const uint32_t tmem_base = *s_tmem;
 
-    const int n_units_per_tile = a.n_chunks;
+    // all chunks of every gridDim.x-th tile, or one chunk of one tile
+    const int tile_begin = a.spread ? blockIdx.x / a.n_chunks : blockIdx.x;
+    const int c_begin = a.spread ? blockIdx.x - tile_begin * a.n_chunks : 0, c_end = a.spread ? c_begin + 1 : a.n_chunks;
     const uint32_t stage_tx = (uint32_t)(Cfg::X_BYTES + 2 * a.n_mma * KBLK * 4);
 
     if (warp == 0) {
@@ -564,8 +567,8 @@ project_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         if (lane == 0) {
             uint32_t it = 0;
             bool live = true;
-            for (int tile = blockIdx.x; tile < a.n_tiles && live; tile += gridDim.x) {
-                for (int c = 0; c < n_units_per_tile && live; ++c) {
+            for (int tile = tile_begin; tile < a.n_tiles && live; tile += gridDim.x) {
+                for (int c = c_begin; c < c_end && live; ++c) {
                     for (int kb = 0; kb < a.n_kblocks; ++kb, ++it) {
                         const int s = it % STAGES;
                         const uint32_t phs = (it / STAGES) & 1;
@@ -588,8 +591,8 @@ project_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             IssueRing<STAGES> ring;
             uint32_t u = 0, n_kb = 0, n_lo = 0;
             bool live = true;
-            for (int tile = blockIdx.x; tile < a.n_tiles && live; tile += gridDim.x) {
-                for (int c = 0; c < n_units_per_tile && live; ++c, ++u) {
+            for (int tile = tile_begin; tile < a.n_tiles && live; tile += gridDim.x) {
+                for (int c = c_begin; c < c_end && live; ++c, ++u) {
                     const int ab = u & 1;
                     const uint32_t aph = (u >> 1) & 1;
                     if (!mbar_wait(&acc_empty[ab], aph ^ 1, s_abort, a.d_error)) { live = false; break; }
@@ -625,8 +628,8 @@ project_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         const int tt = threadIdx.x - 64;  // 0..127
         uint32_t it = 0;
         bool live = true;
-        for (int tile = blockIdx.x; tile < a.n_tiles && live; tile += gridDim.x) {
-            for (int c = 0; c < n_units_per_tile && live; ++c) {
+        for (int tile = tile_begin; tile < a.n_tiles && live; tile += gridDim.x) {
+            for (int c = c_begin; c < c_end && live; ++c) {
                 for (int kb = 0; kb < a.n_kblocks; ++kb, ++it) {
                     const int s = it % STAGES;
                     const uint32_t phs = (it / STAGES) & 1;
@@ -666,10 +669,10 @@ project_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         bool live = true;
         bool any_ovf = false;
         HashRange range;
-        for (int tile = blockIdx.x; tile < a.n_tiles && live; tile += gridDim.x) {
+        for (int tile = tile_begin; tile < a.n_tiles && live; tile += gridDim.x) {
             const int row = tile * TC_BM + quarter * 32 + lane;
             const bool row_ok = row < a.n;
-            for (int c = 0; c < n_units_per_tile && live; ++c, ++u) {
+            for (int c = c_begin; c < c_end && live; ++c, ++u) {
                 const int ab = u & 1;
                 const uint32_t aph = (u >> 1) & 1;
                 if (!mbar_wait(&acc_full[ab], aph, s_abort, a.d_error)) { live = false; break; }
@@ -807,7 +810,9 @@ project_ts_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     tc_fence_after();
     const uint32_t tmem_base = *s_tmem;
 
-    const int n_units_per_tile = a.n_chunks;
+    // all chunks of every gridDim.x-th tile, or one chunk of one tile
+    const int tile_begin = a.spread ? blockIdx.x / a.n_chunks : blockIdx.x;
+    const int c_begin = a.spread ? blockIdx.x - tile_begin * a.n_chunks : 0, c_end = a.spread ? c_begin + 1 : a.n_chunks;
     const uint32_t stage_tx = (uint32_t)(TS_X_BYTES + 2 * a.n_mma * TS_KBLK * 4);
 
     if (warp == 0) {
@@ -815,8 +820,8 @@ project_ts_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         if (lane == 0) {
             uint32_t it = 0;
             bool live = true;
-            for (int tile = blockIdx.x; tile < a.n_tiles && live; tile += gridDim.x) {
-                for (int c = 0; c < n_units_per_tile && live; ++c) {
+            for (int tile = tile_begin; tile < a.n_tiles && live; tile += gridDim.x) {
+                for (int c = c_begin; c < c_end && live; ++c) {
                     for (int kb = 0; kb < a.n_kblocks; ++kb, ++it) {
                         const int s = it % STAGES;
                         const uint32_t phs = (it / STAGES) & 1;
@@ -840,8 +845,8 @@ project_ts_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             uint32_t as = 0;  // A stage
             uint32_t u = 0, n_kb = 0, n_lo = 0;
             bool live = true;
-            for (int tile = blockIdx.x; tile < a.n_tiles && live; tile += gridDim.x) {
-                for (int c = 0; c < n_units_per_tile && live; ++c, ++u) {
+            for (int tile = tile_begin; tile < a.n_tiles && live; tile += gridDim.x) {
+                for (int c = c_begin; c < c_end && live; ++c, ++u) {
                     const int ab = u & 1;
                     const uint32_t aph = (u >> 1) & 1;
                     if (!mbar_wait(&acc_empty[ab], aph ^ 1, s_abort, a.d_error)) { live = false; break; }
@@ -887,8 +892,8 @@ project_ts_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         const int sw = KB == 32 ? (r & 7) : ((r >> 1) & 3);
         uint32_t it = 0;
         bool live = true;
-        for (int tile = blockIdx.x; tile < a.n_tiles && live; tile += gridDim.x) {
-            for (int c = 0; c < n_units_per_tile && live; ++c) {
+        for (int tile = tile_begin; tile < a.n_tiles && live; tile += gridDim.x) {
+            for (int c = c_begin; c < c_end && live; ++c) {
                 for (int kb = 0; kb < a.n_kblocks; ++kb, ++it) {
                     if ((int)(it % G) != grp) continue;
                     const int s = it % STAGES;
@@ -943,10 +948,10 @@ project_ts_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         bool live = true;
         bool any_ovf = false;
         HashRange range;
-        for (int tile = blockIdx.x; tile < a.n_tiles && live; tile += gridDim.x) {
+        for (int tile = tile_begin; tile < a.n_tiles && live; tile += gridDim.x) {
             const int row = tile * TC_BM + quarter * 32 + lane;
             const bool row_ok = row < a.n;
-            for (int c = 0; c < n_units_per_tile && live; ++c, ++u) {
+            for (int c = c_begin; c < c_end && live; ++c, ++u) {
                 const int ab = u & 1;
                 const uint32_t aph = (u >> 1) & 1;
                 if (!mbar_wait(&acc_full[ab], aph, s_abort, a.d_error)) { live = false; break; }
@@ -1087,7 +1092,9 @@ inline bool launch_project_tc(const CtxPtr& c, cudaStream_t stream, int family, 
     a.n_kblocks = p.d_pad / p.kblk;
     a.key_words = ks.key_words; a.elem_bytes = ks.elem_bytes; a.family = family;
     a.row_offset = row_offset; a.n_total = n_total;
-    int grid = std::min(a.n_tiles, c->sm_count);
+    // Few rows: the chunks of a tile go to CTAs of their own (one query, 512 columns of 128 features: 14.0 -> 9.9 us).
+    a.spread = (int64_t)a.n_tiles * a.n_chunks <= c->sm_count;
+    const int grid = a.spread ? a.n_tiles * a.n_chunks : std::min(a.n_tiles, c->sm_count);
     if (p.ts) {
         auto go = [&](auto kern, int smem_bytes) -> bool {
             if ((size_t)smem_bytes > c->smem_optin) return false;
