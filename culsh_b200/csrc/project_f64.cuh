@@ -145,7 +145,7 @@ project_f64_kernel(ProjectArgs a) {
         }
     }
     __syncthreads();
-    pack_hash_values<FAMILY>(a, hbuf, pitch, row0, PF_BM, group * G, gc_valid / a.k, PF_THREADS);
+    pack_hash_values<FAMILY>(a, RowMajorHashes{hbuf, pitch}, row0, PF_BM, group * G, gc_valid / a.k, PF_THREADS);
 }
 
 // Tables of at most 128 hashes (a group holds whole tables); the caller takes the CUDA-core kernel else.

@@ -35,9 +35,16 @@ struct ProjectArgs {
     int n_total;           // rows of the whole key array (table stride)
 };
 
-// Assemble the packed key of one (row, table) from k int32 hash values in shared memory.
-template <int FAMILY>
-__device__ __forceinline__ void assemble_key(const int32_t* __restrict__ hv, int k, int NW,
+// Hash values of a tile in shared memory.
+struct RowMajorHashes {
+    const int32_t* v;  // [row][pitch]
+    int pitch;
+    __device__ __forceinline__ int32_t operator()(int row, int col) const { return v[row * pitch + col]; }
+};
+
+// Assemble the packed key of one (row, table) from k int32 hash values: hv(j) is hash j.
+template <int FAMILY, typename HashOf>
+__device__ __forceinline__ void assemble_key(HashOf&& hv, int k, int NW,
                                              int elem_bytes, uint32_t* __restrict__ out,
                                              bool& overflow) {
     overflow = false;
@@ -47,7 +54,7 @@ __device__ __forceinline__ void assemble_key(const int32_t* __restrict__ hv, int
             uint32_t w = 0;
             for (int b = 0; b < 32; ++b) {
                 int pos = lo + b;
-                if (pos < k) w |= (uint32_t)(hv[k - 1 - pos] & 1) << b;
+                if (pos < k) w |= (uint32_t)(hv(k - 1 - pos) & 1) << b;
             }
             out[wi] = w;
         }
@@ -57,7 +64,7 @@ __device__ __forceinline__ void assemble_key(const int32_t* __restrict__ hv, int
         if (elem_bytes < 4) {
             const int lim = elem_bytes == 1 ? 128 : 32768;
             for (int j = 0; j < k; ++j) {
-                int v = hv[j];
+                int v = hv(j);
                 if (v < -lim || v >= lim) overflow = true;
             }
         }
@@ -66,7 +73,7 @@ __device__ __forceinline__ void assemble_key(const int32_t* __restrict__ hv, int
             for (int bb = 0; bb < 4; ++bb) {
                 int i = wi * 4 + bb - pad;
                 if (i >= 0) {
-                    uint32_t v = (uint32_t)hv[i >> (elem_bytes >> 1)];  // 1, 2 or 4 bytes
+                    uint32_t v = (uint32_t)hv(i >> (elem_bytes >> 1));  // 1, 2 or 4 bytes
                     uint32_t byte = (v >> (8 * (i & (elem_bytes - 1)))) & 0xFFu;
                     w |= byte << (24 - 8 * bb);
                 }
@@ -78,8 +85,8 @@ __device__ __forceinline__ void assemble_key(const int32_t* __restrict__ hv, int
 
 // Pack and store the hash values of `rows` rows and `tables_here` tables in shared memory: consecutive
 // threads -> consecutive rows of one table.
-template <int FAMILY>
-__device__ __forceinline__ void pack_hash_values(const ProjectArgs& a, const int32_t* __restrict__ hbuf, int pitch,
+template <int FAMILY, typename Hashes>
+__device__ __forceinline__ void pack_hash_values(const ProjectArgs& a, const Hashes& hashes,
                                                  int row0, int rows, int first_table, int tables_here, int threads) {
     const int NW = a.key_words;
     HashRange range;
@@ -88,7 +95,7 @@ __device__ __forceinline__ void pack_hash_values(const ProjectArgs& a, const int
         int row = row0 + r;
         if (row >= a.n) continue;
         int t = first_table + g;
-        const int32_t* hv = hbuf + r * pitch + g * a.k;
+        auto hv = [&](int j) { return hashes(r, g * a.k + j); };
         size_t item = (size_t)t * a.n_total + a.row_offset + row;
         uint32_t* dst = a.keys + item * NW;
         bool ovf = false;
@@ -99,7 +106,7 @@ __device__ __forceinline__ void pack_hash_values(const ProjectArgs& a, const int
             uint64_t acc = 0;
             HashRange own;
             for (int j = 0; j < a.k; ++j) {
-                const uint32_t v = (uint32_t)hv[j];
+                const uint32_t v = (uint32_t)hv(j);
                 uint32_t e = v & 1u;
                 if (FAMILY == CULSH_PSLSH) {
                     own.take((int)v);
@@ -219,7 +226,7 @@ project_simt_kernel(ProjectArgs a) {
     }
     __syncthreads();
 
-    pack_hash_values<FAMILY>(a, hbuf, pitch, row0, PS_BM, group * G, gc_valid / a.k, PS_THREADS);
+    pack_hash_values<FAMILY>(a, RowMajorHashes{hbuf, pitch}, row0, PS_BM, group * G, gc_valid / a.k, PS_THREADS);
 }
 
 inline int simt_tables_per_group(int L, int k) {
