@@ -9,9 +9,13 @@
 // boundaries only).  A CTA takes 64 rows and up to 128 hash columns of whole tables; two of them share an
 // SM, so that one packs its keys while the other multiplies (one CTA of 128 rows: 0.49 ms instead of
 // 0.46 below).  The columns are spread evenly over the groups and, in steps of eight, over
-// the two halves of the warps, so that 224 columns are 2 x 112 and no column past the last step of
-// eight is computed.
-// 200,003 x 100 rows, 224 columns: 0.97 ms on the CUDA cores, 0.46 here (20 TFLOP/s).
+// the two halves of the warps, so that 224 columns are 2 x 112; the number of steps is a template argument, without
+// which every instruction stood behind a branch of its own.  Steps of eight features past d are left out.
+//
+// A row of a hundred features is over in seven stages of a microsecond, and what surrounds them weighs as much: a CTA
+// stays for many row blocks of its group of columns and, for sign bits, fetches the first stages of the next block before
+// it packs the keys of this one.  The bits of a step of eight columns are one byte a row, made from ballots.
+// 200,003 x 100 rows, 224 columns: 0.97 ms on the CUDA cores, with one block of rows a CTA and a branch before every instruction 0.46 (with 2,001 queries), now 0.367.
 #pragma once
 
 #include "common.cuh"
@@ -26,8 +30,11 @@ constexpr int PF_PITCH = PF_BK + 4;  // 160-byte rows: the eight rows of a fragm
 constexpr int PF_STAGES = 3;
 constexpr int PF_THREADS = 256;
 constexpr size_t PF_STAGE = (size_t)(PF_BM + PF_BN) * PF_PITCH;  // doubles
-constexpr size_t PF_SMEM = PF_STAGES * PF_STAGE * sizeof(double);
-static_assert(PF_SMEM >= sizeof(int32_t) * PF_BM * (PF_BN + 1), "the hash values take the place of the stages");
+constexpr int PF_BITS = PF_BN / 8 + 4;  // bytes of a row's sign bits, and a word that the last one's neighbour is read from
+constexpr size_t PF_STAGES_BYTES = PF_STAGES * PF_STAGE * sizeof(double);
+constexpr size_t PF_SMEM = PF_STAGES_BYTES + PF_BM * PF_BITS;
+static_assert(PF_STAGES_BYTES >= sizeof(int32_t) * PF_BM * (PF_BN + 1), "p-stable hash values take the place of the stages");
+static_assert(2 * (PF_SMEM + 1024) <= 227 * 1024, "two CTAs an SM");
 
 __device__ __forceinline__ void cp_async8(void* dst, const void* src, bool valid) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
@@ -41,12 +48,40 @@ __device__ __forceinline__ void mma_f64(double (&c)[4], const double (&a)[4], co
         : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-template <int FAMILY>
+// bit t of n to bit 6 - 2 t
+__device__ __forceinline__ uint32_t spread_nibble(uint32_t n) {
+    return ((n & 1u) << 6) | ((n & 2u) << 3) | (n & 4u) | ((n & 8u) >> 3);
+}
+
+// Keys of the tables of a block of rows from their bits in shared memory, hash 0 in the top bit of byte 0 of its row.
+__device__ __forceinline__ void pack_sign_bits(const ProjectArgs& a, const uint32_t* __restrict__ bits, int row0, int first_table, int tables_here) {
+    const int NW = a.key_words;
+    for (int idx = threadIdx.x; idx < PF_BM * tables_here; idx += PF_THREADS) {
+        const int r = idx % PF_BM, g = idx / PF_BM, row = row0 + r;
+        if (row >= a.n) continue;
+        const uint32_t* line = bits + r * (PF_BITS / 4);
+        uint32_t* dst = a.keys + ((size_t)(first_table + g) * a.n_total + a.row_offset + row) * NW;
+        for (int w = 0; w < NW; ++w) {
+            const int end = a.k - 32 * (NW - 1 - w), len = min(32, end);  // the word's bits of the table: [end - len, end)
+            uint32_t v = 0;
+            if (end > 0) {
+                const int at = g * a.k + end - len;
+                const uint32_t hi = __byte_perm(line[at >> 5], 0, 0x0123), lo = __byte_perm(line[(at >> 5) + 1], 0, 0x0123);
+                v = __funnelshift_l(lo, hi, at & 31) >> (32 - len);
+            }
+            dst[w] = v;
+        }
+    }
+}
+
+template <int FAMILY, int NF>  // NF: steps of eight columns of a warp
 __global__ void __launch_bounds__(PF_THREADS, 2)
 project_f64_kernel(ProjectArgs a) {
+    constexpr bool BITS = FAMILY == CULSH_RPLSH;
     extern __shared__ __align__(16) unsigned char pf_smem[];
     double* stages = reinterpret_cast<double*>(pf_smem);
-    int32_t* hbuf = reinterpret_cast<int32_t*>(pf_smem);  // after the last stage: [PF_BM][GC | 1]
+    int32_t* hbuf = reinterpret_cast<int32_t*>(pf_smem);  // p-stable, after the last stage: [PF_BM][GC | 1]
+    unsigned char* bits = pf_smem + PF_STAGES_BYTES;      // sign bits: [PF_BM][PF_BITS]
 
     const double* __restrict__ X = static_cast<const double*>(a.X);
     const double* __restrict__ P = static_cast<const double*>(a.P);
@@ -56,7 +91,7 @@ project_f64_kernel(ProjectArgs a) {
     const int G = a.tables_per_group;
     const int n_groups = (a.L + G - 1) / G;
     const int group = blockIdx.x % n_groups;  // fastest: the groups of one row block share X in L2
-    const int row0 = (blockIdx.x / n_groups) * PF_BM;
+    const int n_blocks = (a.n + PF_BM - 1) / PF_BM, block_step = gridDim.x / n_groups;  // the grid is a multiple of the groups
     const int GC = G * a.k;
     const int col_base = group * GC;
     const int gc_valid = min(GC, a.L * a.k - col_base);
@@ -65,87 +100,111 @@ project_f64_kernel(ProjectArgs a) {
     // a thread copies feature tid % 16 of rows (columns) tid / 16, + 16, ...; rows and columns past the
     // end and features past d are zero
     const int lf = tid & 15, lr = tid >> 4;
-    auto load = [&](int step) {
-        double* xs = stages + (size_t)(step % PF_STAGES) * PF_STAGE;
+    auto load = [&](int block, int step, int slot) {
+        double* xs = stages + (size_t)slot * PF_STAGE;
         double* ps = xs + (size_t)PF_BM * PF_PITCH;
-        const int f = step * PF_BK + lf;
+        const int f = step * PF_BK + lf, row0 = block * PF_BM;
         const bool f_ok = f < a.d;
 #pragma unroll
         for (int i = 0; i < PF_BM / 16; ++i) {
             const int r = lr + 16 * i;
-            const bool ok = f_ok && row0 + r < a.n;
+            const bool ok = f_ok && r < a.n - row0;
             cp_async8(xs + r * PF_PITCH + lf, ok ? X + (size_t)(row0 + r) * a.d + f : X, ok);
         }
 #pragma unroll
-        for (int i = 0; i < PF_BN / 16; ++i) {
+        for (int i = 0; i < NF; ++i) {  // 16 * NF columns are multiplied
             const int c = lr + 16 * i;
             const bool ok = f_ok && c < gc_valid;
             cp_async8(ps + c * PF_PITCH + lf, ok ? P + (size_t)(col_base + c) * a.d + f : P, ok);
         }
     };
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+    auto next_slot = [](int slot) { return slot + 1 == PF_STAGES ? 0 : slot + 1; };
+    int slot = 0;  // of the step that is multiplied; the two after it are in flight
+    auto begin = [&](int block) {
+        load(block, 0, slot);
+        commit();
+        if (n_steps > 1) load(block, 1, next_slot(slot));
+        commit();
+    };
 
     // warp tile: 16 rows and every second step of eight columns
     const int wm = (warp >> 1) * 16, wn = warp & 1;
     const int g = lane >> 2, t = lane & 3;
-    const int n_frag = (gc_valid + 7) / 8;
-    double acc[8][4];
+    int block = blockIdx.x / n_groups;
+    if (block < n_blocks) begin(block);
+    for (; block < n_blocks; block += block_step) {
+        double acc[NF][4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+        for (int j = 0; j < NF; ++j)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[j][e] = 0.0;
-
-    load(0);
-    commit();
-    if (n_steps > 1) load(1);
-    commit();
-    for (int step = 0; step < n_steps; ++step) {
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();  // the stage has landed for every thread, and the one that is refilled now has been read
-        if (step + 2 < n_steps) load(step + 2);
-        commit();
-        const double* xs = stages + (size_t)(step % PF_STAGES) * PF_STAGE;
-        const double* ps = xs + (size_t)PF_BM * PF_PITCH;
+            for (int e = 0; e < 4; ++e) acc[j][e] = 0.0;
+        for (int step = 0; step < n_steps; ++step) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();  // the stage has landed for every thread, and the one that is refilled now has been read
+            if (step + 2 < n_steps) load(block, step + 2, next_slot(next_slot(slot)));
+            commit();
+            const double* xs = stages + (size_t)slot * PF_STAGE + (wm + g) * PF_PITCH + t;
+            const double* ps = stages + (size_t)slot * PF_STAGE + (size_t)(PF_BM + wn * 8 + g) * PF_PITCH + t;
 #pragma unroll
-        for (int kk = 0; kk < PF_BK; kk += 8) {
-            const double* x = xs + (wm + g) * PF_PITCH + kk + t;
-            const double af[4] = {x[0], x[8 * PF_PITCH], x[4], x[8 * PF_PITCH + 4]};
+            for (int kk = 0; kk < PF_BK; kk += 8) {
+                if (kk == 0 || a.d - step * PF_BK > kk) {  // uniform
+                    const double af[4] = {xs[kk], xs[8 * PF_PITCH + kk], xs[kk + 4], xs[8 * PF_PITCH + kk + 4]};
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int frag = 2 * j + wn;
-                if (frag < n_frag) {  // uniform
-                    const double* p = ps + (frag * 8 + g) * PF_PITCH + kk + t;
-                    const double bf[2] = {p[0], p[4]};
-                    mma_f64(acc[j], af, bf);
+                    for (int j = 0; j < NF; ++j) {
+                        const double bf[2] = {ps[16 * j * PF_PITCH + kk], ps[16 * j * PF_PITCH + kk + 4]};
+                        mma_f64(acc[j], af, bf);
+                    }
                 }
             }
+            slot = next_slot(slot);
+        }
+        const int left = a.d % PF_BK;
+        if (left > 0 && left <= 8) {  // what the step left out would have added: a sum of -0 becomes +0
+#pragma unroll
+            for (int j = 0; j < NF; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[j][e] += 0.0;
+        }
+        // The two stages after the last one read are free: nothing was loaded into them, and every thread is past
+        // the step before the last.  So is the last one behind the barrier below.
+        if constexpr (BITS) {
+            if (block + block_step < n_blocks) begin(block + block_step);
+#pragma unroll
+            for (int j = 0; j < NF; ++j) {
+                uint32_t b[4];  // rows g, columns 2 t and 2 t + 1; the same of rows g + 8
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    b[e] = __ballot_sync(0xFFFFFFFFu, (__float_as_uint((float)acc[j][e]) >> 31) == 0);  // rplsh/hash.cuh:47
+                const int sh = 4 * (lane & 7);
+                const uint32_t even = ((lane & 8 ? b[2] : b[0]) >> sh) & 15u, odd = ((lane & 8 ? b[3] : b[1]) >> sh) & 15u;
+                if (lane < 16) bits[(wm + lane) * PF_BITS + 2 * j + wn] = (unsigned char)((spread_nibble(even) << 1) | spread_nibble(odd));
+            }
+            __syncthreads();
+            pack_sign_bits(a, reinterpret_cast<const uint32_t*>(bits), block * PF_BM, group * G, gc_valid / a.k);
+        } else {
+            __syncthreads();
+            const int pitch = GC | 1;  // odd: the packing threads read one column of many rows
+#pragma unroll
+            for (int j = 0; j < NF; ++j) {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int c = (2 * j + wn) * 8 + 2 * t + e;
+                    if (c < gc_valid) {
+                        const double bv = bias[col_base + c];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            hbuf[(wm + 8 * h + g) * pitch + c] = static_cast<int32_t>(floor(acc[j][2 * h + e] + bv));  // pslsh/hash.cuh:46
+                    }
+                }
+            }
+            __syncthreads();
+            pack_hash_values<FAMILY>(a, RowMajorHashes{hbuf, pitch}, block * PF_BM, PF_BM, group * G, gc_valid / a.k, PF_THREADS);
+            __syncthreads();
+            if (block + block_step < n_blocks) begin(block + block_step);
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-
-    const int pitch = GC | 1;  // odd: the packing threads read one column of many rows
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int c0 = (2 * j + wn) * 8 + 2 * t;
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int c = c0 + e;
-            if (c < gc_valid) {
-                const double bv = FAMILY == CULSH_PSLSH ? bias[col_base + c] : 0.0;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const double v = acc[j][2 * h + e];
-                    const int32_t q = FAMILY == CULSH_RPLSH
-                                          ? (int32_t)((__float_as_uint((float)v) >> 31) ^ 1u)  // rplsh/hash.cuh:47
-                                          : static_cast<int32_t>(floor(v + bv));               // pslsh/hash.cuh:46
-                    hbuf[(wm + 8 * h + g) * pitch + c] = q;
-                }
-            }
-        }
-    }
-    __syncthreads();
-    pack_hash_values<FAMILY>(a, RowMajorHashes{hbuf, pitch}, row0, PF_BM, group * G, gc_valid / a.k, PF_THREADS);
 }
 
 // Tables of at most 128 hashes (a group holds whole tables); the caller takes the CUDA-core kernel else.
@@ -166,11 +225,25 @@ inline bool launch_project_f64(const CtxPtr& c, cudaStream_t stream, int family,
     a.elem_bytes = ks.elem_bytes;
     a.row_offset = row_offset;
     a.n_total = n_total;
-    const dim3 grid((unsigned)(ceil_div(L, a.tables_per_group) * ceil_div(n, PF_BM)));
-    auto kern = family == CULSH_RPLSH ? project_f64_kernel<CULSH_RPLSH> : project_f64_kernel<CULSH_PSLSH>;
-    CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM));
-    kern<<<grid, PF_THREADS, PF_SMEM, stream>>>(a);
-    KERNEL_CHECK();
+    // a whole number of CTAs for each group, two an SM where there is work for them
+    const size_t n_groups = ceil_div(L, a.tables_per_group), per_group = std::max<size_t>(1, 2 * (size_t)c->sm_count / n_groups);
+    const dim3 grid((unsigned)(n_groups * std::min<size_t>(ceil_div(n, PF_BM), per_group)));
+    auto go = [&](auto kern) {
+        CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM));
+        kern<<<grid, PF_THREADS, PF_SMEM, stream>>>(a);
+        KERNEL_CHECK();
+    };
+    auto with_steps = [&](auto nf) {
+        constexpr int NF = decltype(nf)::value;
+        if (family == CULSH_RPLSH) go(project_f64_kernel<CULSH_RPLSH, NF>);
+        else go(project_f64_kernel<CULSH_PSLSH, NF>);
+    };
+    const int steps = (int)ceil_div(a.tables_per_group * k, 16);  // of a warp
+    if (steps <= 2) with_steps(std::integral_constant<int, 2>{});
+    else if (steps <= 4) with_steps(std::integral_constant<int, 4>{});
+    else if (steps <= 6) with_steps(std::integral_constant<int, 6>{});
+    else if (steps == 7) with_steps(std::integral_constant<int, 7>{});
+    else with_steps(std::integral_constant<int, 8>{});
     return true;
 }
 
