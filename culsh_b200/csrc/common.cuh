@@ -111,6 +111,9 @@ enum ScratchSlot {
     SL_SLICES, SL_BOUNDS, SL_COUNT
 };
 
+// Where kernels leave what the host reads behind its next wait: words of Ctx::pinned, a total and up to eight 32-bit words.
+enum HostSlot { HS_BUCKETS = 32, HS_RAW = 40, HS_UNIQUE = 48 };
+
 struct Ctx {
     int device = 0;
     // hash parameters already generated on this handle (they depend only on the key): the
@@ -128,7 +131,7 @@ struct Ctx {
     cudaEvent_t ev_dedupe[2] = {};    // around the window / bitmap dedupe launch of the last query batch
     cudaEvent_t copy_done[2] = {};
     cudaEvent_t chunk_free[2] = {};
-    uint64_t* pinned = nullptr;       // 64 x u64 words of pinned host memory
+    uint64_t* pinned = nullptr;       // 64 x u64 words of pinned host memory: read_words' first, see HostSlot
     FeedRing feed_ring;               // for pageable host inputs, made on first use
     int* d_error = nullptr;           // device-side self-check word; [2], [3]: see HashRange
     int seen_error = 0;               // its value behind the last query
@@ -329,9 +332,9 @@ inline void copy_out(const CtxPtr& c, void* dst, const void* src_dev, size_t byt
     CU_CHECK(cudaStreamSynchronize(c->stream));
 }
 
-// Read up to 64 u64 words from device memory through the pinned scratch block.
+// Read up to 32 u64 words from device memory through the pinned scratch block.
 inline void read_words(const CtxPtr& c, const void* src_dev, size_t bytes, void* host_out) {
-    if (bytes > 64 * sizeof(uint64_t)) fail(CULSH_ERR_INTERNAL, "read_words: too large");
+    if (bytes > HS_BUCKETS * sizeof(uint64_t)) fail(CULSH_ERR_INTERNAL, "read_words: too large");
     CU_CHECK(cudaMemcpyAsync(c->pinned, src_dev, bytes, cudaMemcpyDeviceToHost, c->stream));
     CU_CHECK(cudaStreamSynchronize(c->stream));
     std::memcpy(host_out, c->pinned, bytes);

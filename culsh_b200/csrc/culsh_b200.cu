@@ -516,6 +516,13 @@ struct SortBuffers {
     }
 };
 
+// A total, `n` words of the device and the self-check word, left by a kernel in a slot of the pinned block.
+HostWords host_words(const CtxPtr& c, HostSlot slot, const uint32_t* words, int n) {
+    return HostWords{c->pinned + slot, reinterpret_cast<uint32_t*>(c->pinned + slot + 1), words,
+                     reinterpret_cast<const uint32_t*>(c->d_error), n, 1};
+}
+const uint32_t* slot_words(const CtxPtr& c, HostSlot slot) { return reinterpret_cast<const uint32_t*>(c->pinned + slot + 1); }
+
 // Lists of a self-join from the finished buckets.  Cleared and filled a few tables at a time: the
 // strips are still in the L2 when the scattered words arrive, so that no half-written sector has
 // to be read back from memory.
@@ -532,6 +539,9 @@ void fill_self_bounds(const culsh_index& ix, const int32_t* cand, const uint32_t
     }
 }
 
+// Bucket arrays that are made before the number of buckets is known, at most.
+constexpr size_t BUCKETS_AHEAD = (size_t)4 << 20;
+
 // Sort + bucket construction.  On return ix holds cand/bucket arrays; a self-join's `bounds` hold
 // the list of every (table, row).  Returns the device error word read at the one
 // host synchronisation of the build.
@@ -539,53 +549,81 @@ int build_index(culsh_index& ix, SortBuffers& sb, Scratch<uint32_t>* bounds, Sta
     const CtxPtr& c = ix.ctx;
     const int n = ix.n, L = ix.L, NW = ix.ks.key_words;
     HostTrace tr;
-    // compressed sort (5 bits per hash) when the hash values span at most 32 levels
-    bool compressed = false;
-    KeyComp kc{0u, 0u};
-    if (SortBuffers::may_compress(ix.ks) && !getenv("CULSH_SORT_PLAIN_KEYS")) {
-        int w[4] = {0, 0, 0, 0};
-        read_words(c, c->d_error, sizeof(w), w);
-        if (w[0]) return w[0];  // values that do not fit a byte: no need to sort them
-        const uint32_t n_pos = (uint32_t)w[3] + 1, n_neg = (uint32_t)-w[2];
-        if (n_pos + n_neg <= 32 && radix_sort_passes(ix.ks.key_bytes, true) < ix.ks.key_bytes) {
-            compressed = true;
-            kc.n_pos = n_pos;
-            kc.sub = n_neg ? 256u - n_neg - n_pos : 0u;
-        }
-    }
-    const int passes = radix_sort_passes(ix.ks.key_bytes, compressed);
-    sb.set_final(radix_sort_final(c, passes, n, L, NW, compressed));
-    uint32_t* kp[2] = {sb.keys[0].p, sb.keys[1].p};
-    uint32_t* vp[2] = {sb.vals[0], sb.vals[1]};
-    int cur = radix_sort_tables(c, NW, kp, vp, n, L, ix.ks.key_bytes, sb.tile_hist.p, compressed, kc);
-    tm.mark();
     const int tpt = (int)ceil_div(n, IB_TILE);
     const size_t n_tiles = (size_t)tpt * L;
     Scratch<uint32_t> tile_heads(c, SL_TILE_HEADS, n_tiles), tile_base(c, SL_TILE_BASE, n_tiles + 1),
         scratch(c, SL_SCAN, scan_scratch_elems(n_tiles) * 2);
-    CULSH_DISPATCH_NW(NW, launch_bucket_count<NW>(c->stream, kp[cur], n, L, tile_heads.p));
-    exclusive_scan<uint32_t, uint32_t>(c->stream, tile_heads.p, n_tiles, tile_base.p, scratch.p);
-    // the one host round trip of the build: bucket total + self-check word
-    uint32_t B = 0;
-    int err = 0;
-    CU_CHECK(cudaMemcpyAsync(c->pinned, tile_base.p + n_tiles, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
-    CU_CHECK(cudaMemcpyAsync(c->pinned + 1, c->d_error, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CU_CHECK(cudaStreamSynchronize(c->stream));
-    std::memcpy(&B, c->pinned, sizeof(uint32_t));
-    std::memcpy(&err, c->pinned + 1, sizeof(int));
-    if (err) return err;
-    tr.lap("sort+count+scan+sync");
-    ix.n_buckets = (int)B;
-    if (!bounds) ix.bucket_keys.alloc(c, (size_t)B * NW);
-    ix.bucket_offsets.alloc(c, (size_t)B + 1);
-    ix.table_offsets.alloc(c, (size_t)L + 1);
-    tr.lap("alloc bucket arrays");
-    CULSH_DISPATCH_NW(NW, launch_bucket_write<NW>(c->stream, kp[cur], n, L, tile_base.p, ix.bucket_keys.p,
-                                                  ix.bucket_offsets.p, ix.table_offsets.p));
-    if (bounds) {
-        bounds->reserve(c, SL_BOUNDS, (size_t)n * L);
-        fill_self_bounds(ix, reinterpret_cast<const int32_t*>(vp[cur]), tile_base.p, true, bounds->p);
+    uint32_t* kp[2] = {sb.keys[0].p, sb.keys[1].p};
+    // compressed sort (5 bits per hash) when the hash values span at most 32 levels
+    const bool may_compress = SortBuffers::may_compress(ix.ks) && !getenv("CULSH_SORT_PLAIN_KEYS") &&
+                              radix_sort_passes(ix.ks.key_bytes, true) < ix.ks.key_bytes;
+    bool compressed = false;
+    KeyComp kc{0u, 0u};
+    // Small tables and indexes do not wait for what the device finds out on the way: the sort looks at the range
+    // of the values itself, and the bucket arrays are made for as many buckets as there are items (1,000 rows x 8
+    // tables: two waits less of seven in a self-join).
+    const int* check = nullptr;
+    if (may_compress && radix_sort_is_small(c, n, L, NW, true)) {
+        compressed = true;
+        check = c->d_error;
+    } else if (may_compress) {
+        int w[4] = {0, 0, 0, 0};
+        read_words(c, c->d_error, sizeof(w), w);
+        if (w[0]) return w[0];  // values that do not fit a byte: no need to sort them
+        compressed = key_comp_of(w[0], w[2], w[3], kc);
     }
+    const bool ahead = (size_t)n * L * (NW + 1) * sizeof(uint32_t) <= BUCKETS_AHEAD;
+    uint32_t B = 0;
+    int cur = 0, passes = 0;
+    while (true) {
+        passes = radix_sort_passes(ix.ks.key_bytes, compressed);
+        sb.set_final(radix_sort_final(c, passes, n, L, NW, compressed));
+        uint32_t* vp[2] = {sb.vals[0], sb.vals[1]};
+        cur = radix_sort_tables(c, NW, kp, vp, n, L, ix.ks.key_bytes, sb.tile_hist.p, compressed, kc, check);
+        tm.mark();
+        CULSH_DISPATCH_NW(NW, launch_bucket_count<NW>(c->stream, kp[cur], n, L, tile_heads.p));
+        exclusive_scan<uint32_t, uint32_t>(c->stream, tile_heads.p, n_tiles, tile_base.p, scratch.p,
+                                           host_words(c, HS_BUCKETS, reinterpret_cast<const uint32_t*>(c->d_error) + 2, 2));
+        // the one host round trip of the build: bucket total, range and self-check word
+        const uint32_t* words = slot_words(c, HS_BUCKETS);
+        auto wait = [&] {
+            CU_CHECK(cudaStreamSynchronize(c->stream));
+            B = (uint32_t)c->pinned[HS_BUCKETS];
+            tr.lap("sort+count+scan+sync");
+        };
+        // the values span too much for what the sort was to look at itself: once more, as they are
+        auto again = [&] {
+            if (!check || key_comp_of((int)words[2], (int)words[0], (int)words[1], kc)) return false;
+            check = nullptr;
+            compressed = false;
+            tm.next = 2;
+            return true;
+        };
+        if (!ahead) {
+            wait();
+            if (words[2]) return (int)words[2];
+            if (again()) continue;
+        } else {
+            B = (uint32_t)((size_t)n * L);
+        }
+        if (!bounds) ix.bucket_keys.alloc(c, (size_t)B * NW);
+        ix.bucket_offsets.alloc(c, (size_t)B + 1);
+        ix.table_offsets.alloc(c, (size_t)L + 1);
+        tr.lap("alloc bucket arrays");
+        CULSH_DISPATCH_NW(NW, launch_bucket_write<NW>(c->stream, kp[cur], n, L, tile_base.p, ix.bucket_keys.p,
+                                                      ix.bucket_offsets.p, ix.table_offsets.p));
+        if (bounds) {
+            bounds->reserve(c, SL_BOUNDS, (size_t)n * L);
+            fill_self_bounds(ix, reinterpret_cast<const int32_t*>(vp[cur]), tile_base.p, true, bounds->p);
+        }
+        if (!ahead) break;
+        wait();
+        if (words[2]) return (int)words[2];
+        ix.bucket_keys.n = bounds ? 0 : (size_t)B * NW;
+        ix.bucket_offsets.n = (size_t)B + 1;
+        if (!again()) break;
+    }
+    ix.n_buckets = (int)B;
     // the sorted row ids are the candidate array: adopt the buffer
     static_assert(sizeof(int32_t) == sizeof(uint32_t), "");
     if (cur != sb.final_buf) fail(CULSH_ERR_INTERNAL, "radix sort ended in the scratch buffer");
@@ -707,7 +745,16 @@ struct RawCounts {
     uint64_t *cnt, *off;  // [n_q], [n_q + 1]
     uint32_t *big_list, *mid_list, *counters;
     int mid_max;
+    uint64_t* uniq;       // [n_q], 0 for those in the lists
+    HostWords host;
 };
+
+// Sets of up to this many queries do not wait for their counts: what usually comes next is launched behind the count, for
+// up to AHEAD_IDS ids, and done again if the counts ask for something else (one query against
+// an index of a million rows: 144 -> 124 us, with the waits and copies that went).
+constexpr int AHEAD_QUERIES = 4096;
+constexpr size_t AHEAD_IDS = (size_t)1 << 20;
+constexpr int AHEAD_PIECES = 64;  // CTAs of the window kernel that may turn out to have nothing to do
 
 // The result inside its raw array, when there is no memory for a second one: what a run of queries has goes
 // through a buffer to where it belongs, at or before where it was and before what the next run has.
@@ -734,7 +781,7 @@ void compact_in_place(const CtxPtr& c, culsh_candidates& out, DevBuf<int32_t>& r
 
 // `count`, if there is one, launches what finds the lists and counts them; they are in `bounds` else.
 // False, and nothing done, when there are more than raw_limit list entries.  On return the device
-// error word as it was behind the last kernel is in c->seen_error.
+// error word as it was behind the last kernel that may report there is in c->seen_error.
 bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool self_join, culsh_candidates& out,
                         StageTimer& tm, uint64_t raw_limit = UINT64_MAX,
                         const std::function<void(const RawCounts&)>& count = nullptr) {
@@ -747,7 +794,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
     out.n_queries = n_q;
     out.counts.alloc(c, (size_t)n_q);
     out.offsets.alloc(c, (size_t)n_q + 1);
-    // offsets, their total and three counters next to one another: one copy brings both to the host
+    // offsets, their total and three counters next to one another
     Scratch<uint64_t> raw_cnt(c, SL_RAW_CNT, n_q), raw_off(c, SL_RAW_OFF, (size_t)n_q + 3),
         scratch(c, SL_SCAN, scan_scratch_elems(n_q));
     Scratch<uint32_t> big_list(c, SL_BIG_LIST, 2 * (size_t)n_q);
@@ -756,29 +803,77 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
     const int wbits = bitmap_window_bits(c, ix.n);
     // with more rows than two bitmap windows, mid-sized candidate sets are sorted in shared memory
     const int mid_max = (size_t)ix.n > 2 * (size_t)wbits ? MID_MAX : 0;
+    const HostWords host_raw = host_words(c, HS_RAW, n_big, 3);
     if (count) {
-        count(RawCounts{raw_cnt.p, raw_off.p, big_list.p, mid_list, n_big, mid_max});
+        count(RawCounts{raw_cnt.p, raw_off.p, big_list.p, mid_list, n_big, mid_max, out.counts.p, host_raw});
     } else {
         CU_CHECK(cudaMemsetAsync(n_big, 0, 4 * sizeof(uint32_t), s));
         raw_count_kernel<<<(unsigned)ceil_div(n_q, 256), 256, 0, s>>>(bounds, n_q, L, self_join, raw_cnt.p, big_list.p,
-                                                                     mid_list, n_big, mid_max);
+                                                                     mid_list, n_big, mid_max, out.counts.p);
         KERNEL_CHECK();
-        exclusive_scan<uint64_t, uint64_t>(s, raw_cnt.p, n_q, raw_off.p, scratch.p);
+        exclusive_scan<uint64_t, uint64_t>(s, raw_cnt.p, n_q, raw_off.p, scratch.p, host_raw);
     }
-    uint64_t raw_total = 0;
-    uint32_t nc[3] = {0, 0, 0};
-    CU_CHECK(cudaMemcpyAsync(c->pinned, raw_off.p + n_q, 3 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+    // Large sets: a CTA for each (query, window of the rows) where that is a few windows, else one for each query.
+    int n_win = 1;
+    const int cbits = window_bits(ix.n, &n_win);
+    const bool may_window = n_win <= MAX_WINDOWS && L <= CW_MAX_L && window_smem_bytes(cbits) + 1024 <= c->smem_optin;
+    Scratch<int32_t> tmp;
+    DevBuf<int32_t> raw_ids;
+    Scratch<uint2> pieces;
+    Scratch<int2> slices;
+    auto launch_small = [&](auto kernel, int above, uint64_t room) {
+        const size_t blocks = std::min<size_t>(ceil_div(n_q, SM_WARPS), (size_t)c->sm_count * 32);
+        kernel<<<(unsigned)blocks, SM_THREADS, 0, s>>>(bounds, ix.cand.p, raw_cnt.p, raw_off.p, L, above, room, tmp.p, out.counts.p);
+        KERNEL_CHECK();
+    };
+    auto launch_windows = [&](size_t n_ctas, const uint32_t* n_slots, uint64_t room) {
+        auto launch = [&](auto nt_tag, auto mk_tag) {
+            constexpr int NT = decltype(nt_tag)::value;
+            constexpr int MK = decltype(mk_tag)::value;
+            const size_t smem = window_smem_bytes(cbits);
+            auto kern = dedupe_window_kernel<NT, MK>;
+            CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+            kern<<<(unsigned)n_ctas, NT, smem, s>>>(big_list.p, bounds, ix.cand.p, raw_off.p, L, ix.n, cbits, n_win, self_join,
+                                                    slices.p, n_slots, room, tmp.p, pieces.p,
+                                                    reinterpret_cast<unsigned long long*>(out.counts.p));
+            KERNEL_CHECK();
+        };
+        const long cw_threads = env_long("CULSH_CHAIN_THREADS", 384);
+        const long cw_mk = env_long("CULSH_CHAIN_LOADS", 8);
+        auto with_loads = [&](auto nt_tag) {
+            if (cw_mk == 4) launch(nt_tag, std::integral_constant<int, 4>{});
+            else if (cw_mk == 16) launch(nt_tag, std::integral_constant<int, 16>{});
+            else launch(nt_tag, std::integral_constant<int, 8>{});
+        };
+        if (cw_threads == 512) with_loads(std::integral_constant<int, 512>{});
+        else if (cw_threads == 256) with_loads(std::integral_constant<int, 256>{});
+        else with_loads(std::integral_constant<int, 384>{});
+    };
+    auto scan_unique = [&] {
+        exclusive_scan<uint64_t, uint64_t>(s, out.counts.p, n_q, out.offsets.p, scratch.p, host_words(c, HS_UNIQUE, nullptr, 0));
+    };
+    // A self-join's rows for the windows need their lists in another form, the sort path its number of queries.
+    const bool ahead = n_q <= AHEAD_QUERIES;
+    const bool ahead_windows = ahead && may_window && !self_join && mid_max == 0 && (size_t)n_q * n_win <= AHEAD_PIECES;
+    uint64_t room = 0;
+    if (ahead) {
+        tmp.reserve(c, SL_TMP, AHEAD_IDS);
+        room = c->slot_cap[SL_TMP] / sizeof(int32_t);
+        launch_small(self_join ? dedupe_small_kernel<SMALL_MAX, true> : dedupe_small_kernel<SMALL_MAX, false>, 0, room);
+        if (ahead_windows) {
+            pieces.reserve(c, SL_CHAIN, (size_t)n_q * n_win);
+            launch_windows((size_t)n_q * n_win, n_big, room);
+        }
+        scan_unique();
+    }
     CU_CHECK(cudaStreamSynchronize(s));
-    std::memcpy(&raw_total, c->pinned, sizeof(uint64_t));
-    std::memcpy(nc, c->pinned + 1, sizeof(nc));
-    const uint32_t nb = nc[0], nm = nc[1];
+    const uint64_t raw_total = c->pinned[HS_RAW];
+    const uint32_t nb = slot_words(c, HS_RAW)[0], nm = slot_words(c, HS_RAW)[1], n_long = slot_words(c, HS_RAW)[2];
+    c->seen_error = (int)slot_words(c, HS_RAW)[3];  // what follows has no waits that could run out
     tr.lap("count+scan+sync");
     if (raw_total > raw_limit) return false;
-    auto finish = [&] {  // the wait at the end brings the error word along
-        CU_CHECK(cudaMemcpyAsync(c->pinned + 8, c->d_error, sizeof(int), cudaMemcpyDeviceToHost, s));
-        CU_CHECK(cudaStreamSynchronize(s));
-        std::memcpy(&c->seen_error, c->pinned + 8, sizeof(int));
-    };
+    const bool done = ahead && raw_total <= room && nm == 0 && (nb == 0 || ahead_windows);
     // The bitmap and sort paths walk lists: a self-join with rows for them takes its pairs as lists too
     // (the tile bases of the build are still in their slot).
     if (self_join && (nb || nm))
@@ -790,96 +885,66 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         CU_CHECK(cudaMemsetAsync(out.counts.p, 0, out.counts.bytes(), s));
         CU_CHECK(cudaMemsetAsync(out.offsets.p, 0, out.offsets.bytes(), s));
         out.total = 0;
-        finish();
+        CU_CHECK(cudaStreamSynchronize(s));
         return true;
     }
-    // Large sets: a CTA for each (query, window of the rows) where that is a few windows, else one for each query.
-    int n_win = 1;
-    const int cbits = window_bits(ix.n, &n_win);
-    const bool windows = nb && n_win <= MAX_WINDOWS && L <= CW_MAX_L && (uint64_t)nb * (uint64_t)n_win < (1ull << 31) &&
-                         window_smem_bytes(cbits) + 1024 <= c->smem_optin;
-    const uint32_t n_other = (uint32_t)n_q - nb - nm;  // queries on the warp path (incl. empty ones)
-    // The ids of a query land in its raw span first.  A large such array is a block of the result's kind: it goes
-    // back when the call is done, and takes the result's place when there is no memory for both.
-    Scratch<int32_t> tmp;
-    DevBuf<int32_t> raw_ids;
-    if (windows && raw_total * sizeof(int32_t) >= BIG_BLOCK_MIN) {
-        raw_ids.alloc(c, raw_total);
-        tmp.p = raw_ids.p;
-        tmp.n = raw_total;
-    } else {
-        tmp.reserve(c, SL_TMP, raw_total);
-    }
-    tr.lap("alloc tmp");
-    if (windows && n_win > 1) CU_CHECK(cudaMemsetAsync(out.counts.p, 0, out.counts.bytes(), s));  // the windows add up in it
-    if (n_other) {
-        // Short lists in a form that fits twice as many warps on an SM, the rest in a second launch; a
-        // set that one launch takes in a wave or two is not worth a second one.
-        const size_t blocks = std::min<size_t>(ceil_div(n_q, SM_WARPS), (size_t)c->sm_count * 32);
-        auto launch = [&](auto kernel, int above) {
-            kernel<<<(unsigned)blocks, SM_THREADS, 0, s>>>(bounds, ix.cand.p, raw_cnt.p, raw_off.p, L, above, tmp.p, out.counts.p);
-            KERNEL_CHECK();
-        };
-        const bool both = nc[2] && n_q < (1 << 15);
-        if (n_other > nc[2] && !both) launch(self_join ? dedupe_small_kernel<SHORT_MAX, true> : dedupe_small_kernel<SHORT_MAX, false>, 0);
-        if (nc[2]) launch(self_join ? dedupe_small_kernel<SMALL_MAX, true> : dedupe_small_kernel<SMALL_MAX, false>, both ? 0 : SHORT_MAX);
-    }
-    if (nm) {
-        int id_bytes = 1;
-        while (id_bytes < 4 && ((uint64_t)ix.n - 1) >> (8 * id_bytes)) ++id_bytes;
-        size_t smem = sort_path_smem_bytes();
-        CU_CHECK(cudaFuncSetAttribute(dedupe_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        dedupe_sort_kernel<<<nm, MS_THREADS, smem, s>>>(mid_list, bounds, ix.cand.p, raw_off.p, L,
-                                                       id_bytes, tmp.p, out.counts.p);
-        KERNEL_CHECK();
-    }
+    const bool windows = nb && may_window && (uint64_t)nb * (uint64_t)n_win < (1ull << 31);
     const size_t n_pieces = (size_t)nb * n_win;
-    Scratch<uint2> pieces;
-    if (windows) {
-        pieces.reserve(c, SL_CHAIN, n_pieces);
-        // list slices per window, precomputed when the table is small enough (<= 256 MB)
-        Scratch<int2> slices;
-        if (env_long("CULSH_CHAIN_SLICES", 1) && n_win > 1 && n_pieces * (size_t)L <= ((size_t)32 << 20)) {
-            slices.reserve(c, SL_SLICES, n_pieces * (size_t)L);
-            slice_lists_kernel<<<(unsigned)ceil_div(n_pieces * (size_t)L, 256), 256, 0, s>>>(
-                big_list.p, bounds, ix.cand.p, (int)nb, L, cbits, n_win, slices.p);
+    const uint32_t n_other = (uint32_t)n_q - nb - nm;  // queries on the warp path (incl. empty ones)
+    if (!done) {
+        // The ids of a query land in its raw span first.  A large such array is a block of the result's kind: it goes
+        // back when the call is done, and takes the result's place when there is no memory for both.
+        if (windows && raw_total * sizeof(int32_t) >= BIG_BLOCK_MIN) {
+            raw_ids.alloc(c, raw_total);
+            tmp.p = raw_ids.p;
+            tmp.n = raw_total;
+        } else {
+            tmp.reserve(c, SL_TMP, raw_total);
+        }
+        tr.lap("alloc tmp");
+        if (n_other) {
+            // Short lists in a form that fits twice as many warps on an SM, the rest in a second launch; a
+            // set that one launch takes in a wave or two is not worth a second one.
+            const bool both = n_long && n_q < (1 << 15);
+            if (n_other > n_long && !both)
+                launch_small(self_join ? dedupe_small_kernel<SHORT_MAX, true> : dedupe_small_kernel<SHORT_MAX, false>, 0, UINT64_MAX);
+            if (n_long)
+                launch_small(self_join ? dedupe_small_kernel<SMALL_MAX, true> : dedupe_small_kernel<SMALL_MAX, false>, both ? 0 : SHORT_MAX, UINT64_MAX);
+        }
+        if (nm) {
+            int id_bytes = 1;
+            while (id_bytes < 4 && ((uint64_t)ix.n - 1) >> (8 * id_bytes)) ++id_bytes;
+            size_t smem = sort_path_smem_bytes();
+            CU_CHECK(cudaFuncSetAttribute(dedupe_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            dedupe_sort_kernel<<<nm, MS_THREADS, smem, s>>>(mid_list, bounds, ix.cand.p, raw_off.p, L,
+                                                           id_bytes, tmp.p, out.counts.p);
             KERNEL_CHECK();
         }
-        auto launch = [&](auto nt_tag, auto mk_tag) {
-            constexpr int NT = decltype(nt_tag)::value;
-            constexpr int MK = decltype(mk_tag)::value;
-            const size_t smem = window_smem_bytes(cbits);
-            auto kern = dedupe_window_kernel<NT, MK>;
-            CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-            kern<<<(unsigned)n_pieces, NT, smem, s>>>(big_list.p, bounds, ix.cand.p, raw_off.p, L, ix.n, cbits, n_win, self_join,
-                                                      slices.p, tmp.p, pieces.p, reinterpret_cast<unsigned long long*>(out.counts.p));
+        if (windows) {
+            pieces.reserve(c, SL_CHAIN, n_pieces);
+            // list slices per window, precomputed when the table is small enough (<= 256 MB)
+            if (env_long("CULSH_CHAIN_SLICES", 1) && n_win > 1 && n_pieces * (size_t)L <= ((size_t)32 << 20)) {
+                slices.reserve(c, SL_SLICES, n_pieces * (size_t)L);
+                slice_lists_kernel<<<(unsigned)ceil_div(n_pieces * (size_t)L, 256), 256, 0, s>>>(
+                    big_list.p, bounds, ix.cand.p, (int)nb, L, cbits, n_win, slices.p);
+                KERNEL_CHECK();
+            }
+            if (c->profiling) cudaEventRecord(c->ev_dedupe[0], s);
+            launch_windows(n_pieces, nullptr, UINT64_MAX);
+            if (c->profiling) { cudaEventRecord(c->ev_dedupe[1], s); dedupe_timed = true; }
+        } else if (nb) {
+            size_t smem = bitmap_smem_bytes(wbits);
+            CU_CHECK(cudaFuncSetAttribute(dedupe_bitmap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            if (c->profiling) cudaEventRecord(c->ev_dedupe[0], s);
+            dedupe_bitmap_kernel<<<nb, BM_THREADS, smem, s>>>(big_list.p, bounds, ix.cand.p, raw_off.p,
+                                                              L, ix.n, wbits, tmp.p, out.counts.p);
             KERNEL_CHECK();
-        };
-        const long cw_threads = env_long("CULSH_CHAIN_THREADS", 384);
-        const long cw_mk = env_long("CULSH_CHAIN_LOADS", 8);
-        if (c->profiling) cudaEventRecord(c->ev_dedupe[0], s);
-        auto with_loads = [&](auto nt_tag) {
-            if (cw_mk == 4) launch(nt_tag, std::integral_constant<int, 4>{});
-            else if (cw_mk == 16) launch(nt_tag, std::integral_constant<int, 16>{});
-            else launch(nt_tag, std::integral_constant<int, 8>{});
-        };
-        if (cw_threads == 512) with_loads(std::integral_constant<int, 512>{});
-        else if (cw_threads == 256) with_loads(std::integral_constant<int, 256>{});
-        else with_loads(std::integral_constant<int, 384>{});
-        if (c->profiling) { cudaEventRecord(c->ev_dedupe[1], s); dedupe_timed = true; }
-    } else if (nb) {
-        size_t smem = bitmap_smem_bytes(wbits);
-        CU_CHECK(cudaFuncSetAttribute(dedupe_bitmap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (c->profiling) cudaEventRecord(c->ev_dedupe[0], s);
-        dedupe_bitmap_kernel<<<nb, BM_THREADS, smem, s>>>(big_list.p, bounds, ix.cand.p, raw_off.p,
-                                                          L, ix.n, wbits, tmp.p, out.counts.p);
-        KERNEL_CHECK();
-        if (c->profiling) { cudaEventRecord(c->ev_dedupe[1], s); dedupe_timed = true; }
+            if (c->profiling) { cudaEventRecord(c->ev_dedupe[1], s); dedupe_timed = true; }
+        }
+        scan_unique();
+        CU_CHECK(cudaStreamSynchronize(s));
     }
-    exclusive_scan<uint64_t, uint64_t>(s, out.counts.p, n_q, out.offsets.p, scratch.p);
-    uint64_t total = 0;
-    read_words(c, out.offsets.p + n_q, sizeof(uint64_t), &total);
+    const uint64_t total = c->pinned[HS_UNIQUE];
     tr.lap("dedupe+scan+sync");
     out.total = total;
     c->stats.unique_candidates += total;
@@ -922,7 +987,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         else compact_in_place(c, out, raw_ids, (uint64_t)std::max(bounce_env, 0l), compact);
     }
     tm.mark();
-    finish();
+    CU_CHECK(cudaStreamSynchronize(s));
     if (dedupe_timed) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, c->ev_dedupe[0], c->ev_dedupe[1]);
@@ -951,7 +1016,7 @@ bool query_batch(const culsh_index& ix, int n_q, HashFn&& hash_fn, culsh_candida
         count = [&](const RawCounts& r) {
             CULSH_DISPATCH_NW(NW, (lookup_count_kernel<NW><<<1, LS_THREADS, 0, c->stream>>>(
                                       qkeys.p, ovf.p, n_q, ix.L, ix.bucket_keys.p, ix.bucket_offsets.p, ix.table_offsets.p, bounds.p,
-                                      r.cnt, r.off, r.big_list, r.mid_list, r.counters, r.mid_max)));
+                                      r.cnt, r.off, r.big_list, r.mid_list, r.counters, r.mid_max, r.uniq, r.host)));
             KERNEL_CHECK();
         };
     } else {

@@ -139,7 +139,7 @@ constexpr int RC_BATCH = 8;
 __global__ void __launch_bounds__(256)
 raw_count_kernel(BoundsView bounds, int n_q, int L, bool self_join, uint64_t* __restrict__ raw_cnt,
                  uint32_t* __restrict__ big_list, uint32_t* __restrict__ mid_list, uint32_t* __restrict__ counters,
-                 int mid_max) {
+                 int mid_max, uint64_t* __restrict__ uniq_cnt) {
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;  // unsigned: the last CTA may reach past 2^31
     if (q >= (uint32_t)n_q) return;
     uint32_t c = self_join ? 1u : 0u;  // at most n * L < 2^31
@@ -171,6 +171,7 @@ raw_count_kernel(BoundsView bounds, int n_q, int L, bool self_join, uint64_t* __
     }
     raw_cnt[q] = c;
     if (c > SMALL_MAX) {
+        uniq_cnt[q] = 0;  // its windows add up in it
         // the sort path gathers a self-join's lists with the own row in each
         if (c + (self_join ? (uint32_t)L : 0u) <= (uint32_t)mid_max) mid_list[atomicAdd(&counters[1], 1u)] = q;
         else big_list[atomicAdd(&counters[0], 1u)] = q;
@@ -192,7 +193,7 @@ lookup_count_kernel(const uint32_t* __restrict__ qkeys, const uint8_t* __restric
                     const uint32_t* __restrict__ bucket_keys, const int32_t* __restrict__ bucket_offsets,
                     const int32_t* __restrict__ table_offsets, int2* __restrict__ bounds, uint64_t* __restrict__ raw_cnt,
                     uint64_t* __restrict__ raw_off, uint32_t* __restrict__ big_list, uint32_t* __restrict__ mid_list,
-                    uint32_t* __restrict__ counters, int mid_max) {
+                    uint32_t* __restrict__ counters, int mid_max, uint64_t* __restrict__ uniq_cnt, HostWords host) {
     __shared__ uint32_t s_cnt[LS_MAX_PAIRS];  // at most as many queries as pairs
     __shared__ uint32_t s_counters[3];
     __shared__ uint64_t s_warp[32];
@@ -216,6 +217,7 @@ lookup_count_kernel(const uint32_t* __restrict__ qkeys, const uint8_t* __restric
             raw_cnt[q] = c;
             raw_off[q] = carry + ex;
             if (c > SMALL_MAX) {
+                uniq_cnt[q] = 0;
                 if (c <= (uint32_t)mid_max) mid_list[atomicAdd(&s_counters[1], 1u)] = (uint32_t)q;
                 else big_list[atomicAdd(&s_counters[0], 1u)] = (uint32_t)q;
             } else if (c > SHORT_MAX) {
@@ -227,6 +229,8 @@ lookup_count_kernel(const uint32_t* __restrict__ qkeys, const uint8_t* __restric
     __syncthreads();
     if (tid == 0) raw_off[n_q] = carry;
     if (tid < 3) counters[tid] = s_counters[tid];
+    __syncwarp();
+    if (tid < 32) host.write(carry);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -337,11 +341,12 @@ struct WarpLists {
     int32_t dst[64];   // and goes to buf[dst + p]
 };
 
-// Takes the queries with `above` < raw <= CAP (and with `above` = 0 the empty ones).
+// Takes the queries with `above` < raw <= CAP (and with `above` = 0 the empty ones).  Nothing is done when all of them
+// together have more than `room` ids: a launch whose counts the host has not seen says how many `tmp` holds.
 template <int CAP, bool SELF>
 __global__ void __launch_bounds__(SM_THREADS, CAP == SHORT_MAX ? 6 : 4)
 dedupe_small_kernel(BoundsView bounds, const int32_t* __restrict__ cand, const uint64_t* __restrict__ raw_cnt,
-                    const uint64_t* __restrict__ raw_off, int L, int above, int32_t* __restrict__ tmp,
+                    const uint64_t* __restrict__ raw_off, int L, int above, uint64_t room, int32_t* __restrict__ tmp,
                     uint64_t* __restrict__ uniq_cnt) {
     __shared__ int32_t s_buf[SM_WARPS][CAP];
     __shared__ WarpLists s_lists[SELF ? 1 : SM_WARPS];
@@ -349,6 +354,7 @@ dedupe_small_kernel(BoundsView bounds, const int32_t* __restrict__ cand, const u
     const int n_q = bounds.n_q;
     int32_t* buf = s_buf[warp];
     WarpLists& wl = s_lists[SELF ? 0 : warp];
+    if (raw_off[n_q] > room) return;
     for (uint32_t qu = blockIdx.x * SM_WARPS + warp; qu < (uint32_t)n_q; qu += gridDim.x * SM_WARPS) {
         const int q = (int)qu;
         const uint64_t r64 = raw_cnt[q];
@@ -928,13 +934,14 @@ slice_lists_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds, con
     if (w == n_win - 1) flat[mine + 1] = we;
 }
 
-// pieces[b * n_win + w]: x = where the piece starts inside the query's raw span, y = its ids
+// pieces[b * n_win + w]: x = where the piece starts inside the query's raw span, y = its ids.  A launch whose counts the
+// host has not seen covers all queries: n_big says how many there are to do, and `room` is as in dedupe_small_kernel.
 template <int NT, int MK>
 __global__ void __launch_bounds__(NT)
 dedupe_window_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds, const int32_t* __restrict__ cand,
                      const uint64_t* __restrict__ raw_off, int L, int n_rows, int window_bits, int n_win, bool self_join,
-                     const int2* __restrict__ slices /* or null */, int32_t* __restrict__ tmp, uint2* __restrict__ pieces,
-                     unsigned long long* __restrict__ uniq_cnt) {
+                     const int2* __restrict__ slices /* or null */, const uint32_t* __restrict__ n_big /* or null: all */, uint64_t room,
+                     int32_t* __restrict__ tmp, uint2* __restrict__ pieces, unsigned long long* __restrict__ uniq_cnt) {
     constexpr int NWARP = NT / 32;
     extern __shared__ __align__(16) uint32_t s_dyn[];
     const int n32 = window_bits / 32;                        // a multiple of 128
@@ -947,6 +954,7 @@ dedupe_window_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds, c
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int slot = blockIdx.x / n_win, w = blockIdx.x - slot * n_win;
+    if (n_big && (slot >= (int)*n_big || raw_off[bounds.n_q] > room)) return;
     const int q = (int)big_list[slot];
     const int win_lo = w * window_bits;
     const int win_hi = min(n_rows, win_lo + window_bits);

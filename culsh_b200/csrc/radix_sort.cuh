@@ -85,6 +85,15 @@ struct KeyComp {
     uint32_t n_pos;  // ranks below n_pos are non-negative values
 };
 
+// From the self-check word and the range behind it (see HashRange): whether the values span at most 32 levels.
+__host__ __device__ inline bool key_comp_of(int err, int lo, int hi, KeyComp& kc) {
+    const uint32_t n_pos = (uint32_t)hi + 1, n_neg = (uint32_t)-lo;
+    if (err || n_pos + n_neg > 32) return false;
+    kc.n_pos = n_pos;
+    kc.sub = n_neg ? 256u - n_neg - n_pos : 0u;
+    return true;
+}
+
 __device__ __forceinline__ uint32_t comp_word(uint32_t w, uint32_t sub) {  // 4 bytes -> 20 bits
     const uint32_t neg = (w >> 7) & 0x01010101u;
     uint32_t c = w - neg * sub;                                   // four ranks, one per byte
@@ -522,11 +531,13 @@ struct SmallSortCfg {
     static constexpr size_t SMEM = sizeof(uint32_t) * ((size_t)MAX_ROWS * (KW + (PACK ? 0 : 1)) + RSS_WARPS * 256 + 4 * 256 + 256 + 8);
 };
 
-// COMP as a runtime flag: keys are compressed as they are loaded and restored as they are stored.
+// COMP as a runtime flag: keys are compressed as they are loaded and restored as they are stored.  With
+// `check` (the self-check word and the range) the kernel finds out itself whether they can be, which the host would have to
+// wait for; where they cannot the items go through in row order, and the host, which sees that later, sorts again.
 template <int NW, bool PACK>
 __global__ void __launch_bounds__(RSS_THREADS, 1)
 radix_sort_small_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
-                        uint32_t* __restrict__ vals_out, int n, int passes, bool compressed, KeyComp kc) {
+                        uint32_t* __restrict__ vals_out, int n, int passes, bool compressed, KeyComp kc, const int* __restrict__ check) {
     using Cfg = SmallSortCfg<NW, PACK>;
     constexpr int KW = Cfg::KW, IPT = Cfg::IPT;
     constexpr bool WORDS = NW >= 4;
@@ -544,6 +555,17 @@ radix_sort_small_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restri
     const int first = warp * (32 * steps) + lane;           // a warp holds 32 * steps consecutive items
     const uint32_t below = (1u << lane) - 1u;
     uint32_t* bins = s_bins + warp * 256;
+    if constexpr (!WORDS) {
+        if (check && !key_comp_of(check[0], check[2], check[3], kc)) {
+            for (int at = tid; at < n; at += RSS_THREADS) {
+                uint32_t kk[KW];
+                load_key<KW>(keys_in + (base + at) * KW, kk);
+                store_key<KW>(keys_out + (base + at) * KW, kk);
+                vals_out[base + at] = (uint32_t)at;
+            }
+            return;
+        }
+    }
     uint32_t key[IPT][KW], val[IPT], pos[IPT];
 #pragma unroll
     for (int i = 0; i < IPT; ++i) {
@@ -664,11 +686,11 @@ radix_sort_small_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restri
 // keys[0] -> keys[1], row ids to vals[1]
 template <int NW>
 inline int radix_sort_small(const CtxPtr& c, uint32_t* keys[2], uint32_t* vals[2], int n, int L, int passes,
-                            bool compressed, KeyComp kc) {
+                            bool compressed, KeyComp kc, const int* check) {
     auto go = [&](auto kern, size_t smem) {
         CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (c->profiling) cudaEventRecord(c->ev_pass[0], c->stream);
-        kern<<<(unsigned)L, RSS_THREADS, smem, c->stream>>>(keys[0], keys[1], vals[1], n, passes, compressed, kc);
+        kern<<<(unsigned)L, RSS_THREADS, smem, c->stream>>>(keys[0], keys[1], vals[1], n, passes, compressed, kc, check);
         KERNEL_CHECK();
         if (c->profiling) cudaEventRecord(c->ev_pass[1], c->stream);
     };
@@ -822,15 +844,15 @@ inline size_t radix_sort_tile_words(int n, int L, int NW) {
 
 inline int radix_sort_tables(const CtxPtr& c, int NW, uint32_t* keys[2], uint32_t* vals[2], int n,
                              int L, int KB, uint32_t* tile_hist, bool compressed = false,
-                             KeyComp kc = KeyComp{0u, 0u}) {
+                             KeyComp kc = KeyComp{0u, 0u}, const int* check = nullptr) {
     if (radix_sort_is_small(c, n, L, NW, compressed)) {
         const int passes = radix_sort_passes(KB, compressed);
         switch (NW) {
-            case 1: return radix_sort_small<1>(c, keys, vals, n, L, passes, compressed, kc);
-            case 2: return radix_sort_small<2>(c, keys, vals, n, L, passes, compressed, kc);
-            case 4: return radix_sort_small<4>(c, keys, vals, n, L, passes, compressed, kc);
-            case 8: return radix_sort_small<8>(c, keys, vals, n, L, passes, compressed, kc);
-            case 16: return radix_sort_small<16>(c, keys, vals, n, L, passes, compressed, kc);
+            case 1: return radix_sort_small<1>(c, keys, vals, n, L, passes, compressed, kc, check);
+            case 2: return radix_sort_small<2>(c, keys, vals, n, L, passes, compressed, kc, check);
+            case 4: return radix_sort_small<4>(c, keys, vals, n, L, passes, compressed, kc, check);
+            case 8: return radix_sort_small<8>(c, keys, vals, n, L, passes, compressed, kc, check);
+            case 16: return radix_sort_small<16>(c, keys, vals, n, L, passes, compressed, kc, check);
         }
     }
     switch (NW) {
@@ -888,9 +910,26 @@ scan_reduce_kernel(const TIn* __restrict__ in, size_t n, TOut* __restrict__ bloc
     if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
 }
 
+// What a scan leaves in page-locked host memory besides its result: its total and a few 32-bit words from elsewhere.  The
+// host reads them behind its next wait; as a copy of its own each of them cost 3 us on the device and as much
+// in between.
+struct HostWords {
+    uint64_t* total;       // or null: nothing
+    uint32_t* words;       // [n_a + n_b]
+    const uint32_t *a, *b;
+    int n_a, n_b;
+    __device__ __forceinline__ void write(uint64_t t) const {  // by one warp
+        if (!total) return;
+        const int i = threadIdx.x & 31;
+        if (i == 0) *total = t;
+        if (i < n_a) words[i] = a[i];
+        else if (i < n_a + n_b) words[i] = b[i - n_a];
+    }
+};
+
 template <typename TOut>
 __global__ void __launch_bounds__(1024)
-scan_block_sums_kernel(TOut* __restrict__ block_sums, size_t n_blocks, TOut* __restrict__ total_out) {
+scan_block_sums_kernel(TOut* __restrict__ block_sums, size_t n_blocks, TOut* __restrict__ total_out, HostWords host) {
     __shared__ TOut s_warp[32];
     TOut carry = 0;
     for (size_t base = 0; base < n_blocks; base += 1024) {
@@ -902,6 +941,7 @@ scan_block_sums_kernel(TOut* __restrict__ block_sums, size_t n_blocks, TOut* __r
         carry += total;
     }
     if (threadIdx.x == 0 && total_out) *total_out = carry;
+    if (threadIdx.x < 32) host.write((uint64_t)carry);
 }
 
 template <typename TIn, typename TOut>
@@ -945,7 +985,7 @@ struct alignas(16) ScanVec {
 // in and out on 16-byte boundaries
 template <typename T>
 __global__ void __launch_bounds__(SCAN_ONE_THREADS)
-scan_one_kernel(const T* __restrict__ in, int n, T* __restrict__ out) {
+scan_one_kernel(const T* __restrict__ in, int n, T* __restrict__ out, HostWords host) {
     constexpr int PER = 16 / sizeof(T), VECS = SCAN_ONE_IPT / PER;
     __shared__ T s_warp[32];
     T carry = 0;
@@ -981,18 +1021,19 @@ scan_one_kernel(const T* __restrict__ in, int n, T* __restrict__ out) {
         carry += total;
     }
     if (threadIdx.x == 0) out[n] = carry;
+    if (threadIdx.x < 32) host.write((uint64_t)carry);
 }
 
-// scratch must hold ceil(n / SCAN_TILE) TOut elements.  out[n] receives the total.
+// scratch must hold ceil(n / SCAN_TILE) TOut elements.  out[n] receives the total.  `host` needs n > 0.
 template <typename TIn, typename TOut>
-inline void exclusive_scan(cudaStream_t s, const TIn* in, size_t n, TOut* out, TOut* scratch) {
+inline void exclusive_scan(cudaStream_t s, const TIn* in, size_t n, TOut* out, TOut* scratch, const HostWords& host = HostWords{}) {
     if (n == 0) {
         CU_CHECK(cudaMemsetAsync(out, 0, sizeof(TOut), s));
         return;
     }
     if constexpr (std::is_same<TIn, TOut>::value) {
         if (n <= SCAN_ONE_MAX && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
-            scan_one_kernel<TOut><<<1, SCAN_ONE_THREADS, 0, s>>>(in, (int)n, out);
+            scan_one_kernel<TOut><<<1, SCAN_ONE_THREADS, 0, s>>>(in, (int)n, out, host);
             KERNEL_CHECK();
             return;
         }
@@ -1000,7 +1041,7 @@ inline void exclusive_scan(cudaStream_t s, const TIn* in, size_t n, TOut* out, T
     size_t n_blocks = ceil_div(n, SCAN_TILE);
     scan_reduce_kernel<TIn, TOut><<<(unsigned)n_blocks, SCAN_THREADS, 0, s>>>(in, n, scratch);
     KERNEL_CHECK();
-    scan_block_sums_kernel<TOut><<<1, 1024, 0, s>>>(scratch, n_blocks, out + n);
+    scan_block_sums_kernel<TOut><<<1, 1024, 0, s>>>(scratch, n_blocks, out + n, host);
     KERNEL_CHECK();
     scan_apply_kernel<TIn, TOut><<<(unsigned)n_blocks, SCAN_THREADS, 0, s>>>(in, n, scratch, out);
     KERNEL_CHECK();

@@ -1,0 +1,59 @@
+"""Small fits and small sets of queries go on before the host has seen their counts, and what was launched is done again
+where the counts ask for something else: hash values that span more than the compressed sort takes, in tables
+that one CTA sorts (bucket arrays below and above the 4 MB that are made beforehand); sets of up to 4,096 queries with more
+ids than fit, with sets for the windows, and on an index with a sort path; each against the same queries in a
+larger set."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _same(a, b):
+    for f in ("get_indices", "get_offsets", "get_counts"):
+        assert np.array_equal(getattr(a, f)(), getattr(b, f)())
+
+
+@pytest.mark.parametrize("n,L", [(1, 2), (5, 8), (1000, 8), (8192, 3), (12_288, 40), (12_288, 2)])
+@pytest.mark.parametrize("scale", [0.2, 2.0, 4.4, 9.0, 200.0])
+def test_p_stable_spans(n, L, scale):
+    import culsh_b200 as culsh
+    from culsh_b200 import _culsh_core as core_mod
+    rng = np.random.default_rng(n)
+    d, k = 8, 8
+    base = (scale * rng.standard_normal((n // 3 + 1, d))).astype(np.float32)
+    X = base[rng.integers(0, len(base), n)]
+    core = core_mod.PSLSHCore(L, k, 1, 3)
+    ix = core.fit_float(X, n, d)
+    sig = core.hash(X, ix)
+    cand, tab, off = ix.get_candidate_indices(), ix.get_table_bucket_offsets(), ix.get_bucket_candidate_offsets()
+    keys = ix.get_bucket_signatures().reshape(ix.n_total_buckets, -1)
+    assert len(off) == ix.n_total_buckets + 1 and off[-1] == n * L
+    for t in range(L):
+        raw = np.ascontiguousarray(sig[t]).view(np.uint8).reshape(n, 4 * k)
+        order = np.lexsort(tuple(raw[:, j] for j in range(4 * k - 1, -1, -1)))
+        assert np.array_equal(cand[t * n:(t + 1) * n], order)
+        srt = raw[order]
+        head = np.concatenate([[True], (srt[1:] != srt[:-1]).any(axis=1)])
+        assert np.array_equal(keys[tab[t]:tab[t + 1]], srt[head])
+    lsh = culsh.PStableLSH(L, k, window_size=1, seed=3)
+    _same(lsh.fit_query(X), lsh.fit(X).query(X))
+
+
+@pytest.mark.parametrize("n,L,k", [(60_000, 4, 2), (60_000, 4, 6), (60_000, 12, 12), (2_400_000, 4, 12)])
+def test_queries_equal_those_of_a_larger_set(n, L, k):
+    import culsh_b200 as culsh
+    rng = np.random.default_rng(k)
+    X = rng.standard_normal((n, 6)).astype(np.float32)
+    Q = np.concatenate([X[:2000], rng.standard_normal((2200, 6)), 1e4 * np.eye(6)]).astype(np.float32)
+    if k == 2:
+        Q = np.concatenate([Q[:30], Q[4195:]])
+    m = culsh.RPLSH(L, k, seed=6).fit(X)
+    big = np.concatenate([Q, Q[:max(1, 4200 - len(Q))]]) if k != 2 else Q
+    whole = m.query(big)
+    off, ids = whole.get_offsets().astype(np.int64), whole.get_indices()
+    for a, b in [(0, 1), (0, 2), (3, 40), (0, 3000), (100, 4196), (len(Q) - 6, len(Q))]:
+        a, b = min(a, len(Q) - 1), min(b, len(Q))
+        part = m.query(Q[a:b])
+        assert np.array_equal(part.get_offsets().astype(np.int64), off[a:b + 1] - off[a])
+        assert np.array_equal(part.get_indices(), ids[off[a]:off[b]])
