@@ -105,7 +105,7 @@ struct ParamKey {
 // lives as long as the handle, so steady-state calls allocate nothing for temporaries and
 // the stream-ordered pool only ever sees the (repeating) sizes of results.
 enum ScratchSlot {
-    SL_STAGE0, SL_STAGE1, SL_CSR_INDPTR, SL_CSR_INDICES, SL_KEYS0, SL_KEYS1, SL_VALS, SL_GHIST,
+    SL_STAGE0, SL_STAGE1, SL_CSR_INDPTR, SL_CSR_INDICES, SL_KEYS0, SL_KEYS1, SL_VALS, SL_HEADS,
     SL_STATUS, SL_COUNTER, SL_TILE_HEADS, SL_TILE_BASE, SL_SCAN, SL_RAW_CNT, SL_RAW_OFF,
     SL_BIG_LIST, SL_TMP, SL_QKEYS, SL_QOVF, SL_MISC0, SL_MISC1, SL_MISC2, SL_CHAIN,
     SL_SLICES, SL_BOUNDS, SL_COUNT

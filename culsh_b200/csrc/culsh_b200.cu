@@ -551,7 +551,7 @@ int build_index(culsh_index& ix, SortBuffers& sb, Scratch<uint32_t>* bounds, Sta
     HostTrace tr;
     const int tpt = (int)ceil_div(n, IB_TILE);
     const size_t n_tiles = (size_t)tpt * L;
-    Scratch<uint32_t> tile_heads(c, SL_TILE_HEADS, n_tiles), tile_base(c, SL_TILE_BASE, n_tiles + 1),
+    Scratch<uint32_t> tile_heads(c, SL_TILE_HEADS, n_tiles), tile_base(c, SL_TILE_BASE, n_tiles + 1), heads(c, SL_HEADS, n_tiles * IB_WORDS),
         scratch(c, SL_SCAN, scan_scratch_elems(n_tiles) * 2);
     uint32_t* kp[2] = {sb.keys[0].p, sb.keys[1].p};
     // compressed sort (5 bits per hash) when the hash values span at most 32 levels
@@ -581,7 +581,7 @@ int build_index(culsh_index& ix, SortBuffers& sb, Scratch<uint32_t>* bounds, Sta
         uint32_t* vp[2] = {sb.vals[0], sb.vals[1]};
         cur = radix_sort_tables(c, NW, kp, vp, n, L, ix.ks.key_bytes, sb.tile_hist.p, compressed, kc, check);
         tm.mark();
-        CULSH_DISPATCH_NW(NW, launch_bucket_count<NW>(c->stream, kp[cur], n, L, tile_heads.p));
+        CULSH_DISPATCH_NW(NW, launch_bucket_count<NW>(c->stream, kp[cur], n, L, tile_heads.p, heads.p));
         exclusive_scan<uint32_t, uint32_t>(c->stream, tile_heads.p, n_tiles, tile_base.p, scratch.p,
                                            host_words(c, HS_BUCKETS, reinterpret_cast<const uint32_t*>(c->d_error) + 2, 2));
         // the one host round trip of the build: bucket total, range and self-check word
@@ -610,7 +610,7 @@ int build_index(culsh_index& ix, SortBuffers& sb, Scratch<uint32_t>* bounds, Sta
         ix.bucket_offsets.alloc(c, (size_t)B + 1);
         ix.table_offsets.alloc(c, (size_t)L + 1);
         tr.lap("alloc bucket arrays");
-        CULSH_DISPATCH_NW(NW, launch_bucket_write<NW>(c->stream, kp[cur], n, L, tile_base.p, ix.bucket_keys.p,
+        CULSH_DISPATCH_NW(NW, launch_bucket_write<NW>(c->stream, kp[cur], n, L, tile_base.p, heads.p, ix.bucket_keys.p,
                                                       ix.bucket_offsets.p, ix.table_offsets.p));
         if (bounds) {
             bounds->reserve(c, SL_BOUNDS, (size_t)n * L);
