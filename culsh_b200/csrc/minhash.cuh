@@ -61,12 +61,20 @@ __device__ __forceinline__ uint32_t hash_plus5_any(uint32_t a, uint32_t c, uint6
 // Column ids below 2^20: a*c + b5 + 2^52 is below 2^53, so that one double-precision multiply-add gives it exactly, the low
 // word of x in the low word of the result and the high word of x behind the constant exponent in the other.  The double
 // pipe, which nothing else here uses, takes a warp's multiply-add in two cycles, the integer one a wide one in eight.  What
-// is left - a 32-bit multiply-add for the fold, an add, its carry, and half of a three-way minimum - is bound by
-// issue.  2M sets of 20 to 200 ids into 128 hash functions (with the 10,000 queries): 7,730 -> 6,610 us, 100,003 sets 414 -> 364; two steps a turn of the loop instead of four 6,740 and 372.
+// is left is bound by issue.
+//
+// Ids below 2^16 leave the wrap of the fold out, which takes the evaluation to three instructions (the multiply-add, the fold,
+// an add with the minimum in one): x_hi is at most the id + 1, so a fold that wraps comes out below MH_AGAIN, and a
+// minimum at or above that is right.  One below it, rare as long as the row is short (about 8e-5 for each id), is evaluated again in
+// full by the whole warp.  A step of 32 ids is sorted into those below and above through shared memory, as the doubles that
+// all lanes then read.  2M sets of 20 to 200 ids into 128 hash functions (with the 10,000 queries): 7,730 us in the integer form,
+// 6,630 with the wrap for all, now 4,870 (two pairs of ids a turn 4,900, the line at 2^14 4,940); 100,003 sets 414, 367 and 278.
 constexpr uint32_t MH_DOUBLE_COL = 1u << 20;
 constexpr double MH_2_52 = 4503599627370496.0;
 constexpr uint32_t MH_2_52_HI = 0x43300000u;
-__device__ __forceinline__ double mh_id(uint32_t c) { return __hiloint2double((int)MH_2_52_HI, (int)c) - MH_2_52; }
+constexpr uint32_t MH_SHORT_COL = 1u << 16;
+constexpr uint32_t MH_AGAIN = 5u * (MH_SHORT_COL + 1u);
+constexpr int MH_SHORT_ROW = 1024;  // ids of a row: at the line a twelfth of the minima is evaluated again
 // b52 = b + 5 + 2^52
 __device__ __forceinline__ uint32_t hash_plus5_double(double a, double c, double b52) {
     const double x = __fma_rn(a, c, b52);
@@ -74,6 +82,10 @@ __device__ __forceinline__ uint32_t hash_plus5_double(double a, double c, double
     uint32_t t, wrapped;
     asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, 0, 0;" : "=r"(t), "=r"(wrapped) : "r"((uint32_t)__double2loint(x)), "r"(five_hi));
     return t + 5u * wrapped;
+}
+__device__ __forceinline__ uint32_t min_plus5_short(uint32_t m, double a, double c, double b52) {
+    const double x = __fma_rn(a, c, b52);
+    return __viaddmin_u32(5u * (uint32_t)__double2hiint(x) + (uint32_t)__double2loint(x), 0u - 5u * MH_2_52_HI, m);
 }
 
 // keys: [L][n_total][NW] with NW = round_key_words(4k); word j (right-aligned) = bswap32(min).
@@ -90,9 +102,14 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
     const int n_warps = gridDim.x * (MH_THREADS / 32);
     const int H = L * k;
     const int pad_words = NW - k;  // leading zero words when 4k is not 4, 8, 16 or 32 bytes
+    __shared__ __align__(16) double s_ids[MH_THREADS / 32][2][34];
+    double* const ids_short = s_ids[threadIdx.x >> 5][0];
+    double* const ids_long = s_ids[threadIdx.x >> 5][1];
+    const uint32_t below = (1u << lane) - 1u;
 
     for (int row = warp; row < n_rows; row += n_warps) {
         const int start = indptr[row], end = indptr[row + 1];
+        const uint32_t short_col = end - start <= MH_SHORT_ROW ? MH_SHORT_COL : 0u;
         for (int h0 = 0; h0 < H; h0 += 32 * PL) {
             uint32_t m[PL];
             double ad[PL], bd[PL];
@@ -110,14 +127,30 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
                 const int mine = base + lane < end ? indices[base + lane] : 0;
                 const int cnt = min(32, end - base);
                 if (!__any_sync(0xFFFFFFFFu, (uint32_t)mine >= MH_DOUBLE_COL)) {
+                    // the two lists, the last id of an odd number twice
+                    const bool have = lane < cnt, is_short = have && (uint32_t)mine < short_col;
+                    const uint32_t m_short = __ballot_sync(0xFFFFFFFFu, is_short), m_long = __ballot_sync(0xFFFFFFFFu, have && !is_short);
+                    const int n_short = __popc(m_short), n_long = __popc(m_long);
+                    if (have) {
+                        double* const list = is_short ? ids_short : ids_long;
+                        const int at = __popc((is_short ? m_short : m_long) & below);
+                        list[at] = (double)mine;
+                        if (at + 1 == (is_short ? n_short : n_long)) list[at + 1] = (double)mine;
+                    }
+                    __syncwarp();
 #pragma unroll MH_STEPS
-                    for (int s = 0; s < cnt; s += 2) {  // the last id of an odd number twice
-                        const double c0 = mh_id((uint32_t)__shfl_sync(0xFFFFFFFFu, mine, s));
-                        const double c1 = mh_id((uint32_t)__shfl_sync(0xFFFFFFFFu, mine, min(s + 1, cnt - 1)));
+                    for (int s = 0; s < n_short; s += 2) {
+                        const double2 c = *reinterpret_cast<const double2*>(ids_short + s);
+#pragma unroll
+                        for (int i = 0; i < PL; ++i) m[i] = min_plus5_short(min_plus5_short(m[i], ad[i], c.x, bd[i]), ad[i], c.y, bd[i]);
+                    }
+                    for (int s = 0; s < n_long; s += 2) {
+                        const double2 c = *reinterpret_cast<const double2*>(ids_long + s);
 #pragma unroll
                         for (int i = 0; i < PL; ++i)
-                            m[i] = __vimin3_u32(m[i], hash_plus5_double(ad[i], c0, bd[i]), hash_plus5_double(ad[i], c1, bd[i]));
+                            m[i] = __vimin3_u32(m[i], hash_plus5_double(ad[i], c.x, bd[i]), hash_plus5_double(ad[i], c.y, bd[i]));
                     }
+                    __syncwarp();
                     continue;
                 }
                 uint32_t a[PL];
@@ -145,14 +178,18 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
             }
 #pragma unroll
             for (int i = 0; i < PL; ++i) {
-                if (m[i] < 5u) {
+                uint32_t again = __ballot_sync(0xFFFFFFFFu, h0 + i * 32 + lane < H && m[i] < (short_col ? MH_AGAIN : 5u));
+                while (again) {
+                    const int src = __ffs(again) - 1;
+                    again &= again - 1u;
+                    const uint32_t a = __shfl_sync(0xFFFFFFFFu, a_of(i), src);
+                    const uint32_t b = __shfl_sync(0xFFFFFFFFu, (uint32_t)(b5_of(i) - 5ull), src);
                     uint32_t exact = 0xFFFFFFFFu;
-                    for (int e = start; e < end; ++e)
-                        exact = min(exact, hash_mod_prime(a_of(i), (uint32_t)indices[e], b5_of(i) - 5ull));
-                    m[i] = exact;
-                } else if (end > start) {
-                    m[i] -= 5u;
+                    for (int e = start + lane; e < end; e += 32) exact = min(exact, hash_mod_prime(a, (uint32_t)indices[e], b));
+                    exact = __reduce_min_sync(0xFFFFFFFFu, exact);
+                    if (lane == src) m[i] = exact + 5u;
                 }
+                if (end > start) m[i] -= 5u;
             }
 #pragma unroll
             for (int i = 0; i < PL; ++i) {
