@@ -2,6 +2,7 @@
 // buffers and the key layout description.
 #pragma once
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <curand.h>
 #include <curand_kernel.h>
@@ -367,5 +368,23 @@ enum DeviceErrorBits : int {
     DEV_ERR_MBAR_TIMEOUT = 4,      // a bounded mbarrier wait ran out (tensor-core projection)
     DEV_ERR_RANGE = 8              // an index outside its array was skipped
 };
+
+// A launch in clusters of `ctas` CTAs each; `grid` is a multiple of that.
+template <typename... P, typename... A>
+inline void launch_cluster(cudaStream_t stream, void (*kern)(P...), unsigned grid, unsigned ctas, unsigned threads, size_t smem, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = ctas;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = ctas > 1 ? 1 : 0;  // an ordinary launch starts 2 us earlier
+    CU_CHECK(cudaLaunchKernelEx(&cfg, kern, args...));
+    KERNEL_CHECK();
+}
 
 }  // namespace culsh_b200

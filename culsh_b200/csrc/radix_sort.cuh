@@ -683,10 +683,233 @@ radix_sort_small_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restri
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// The same with a cluster of CTAs for each table, while all tables' clusters find room at once: a CTA holds
+// one stretch of the order, its digit totals go to all CTAs of the cluster, and an item is stored right into the shared
+// memory of the CTA that holds its new place.  Two cluster barriers a pass keep the CTAs in step: totals are read after the first
+// and items stored, which the second makes visible; what a barrier follows was read into registers before it.  What
+// bounds it are the barriers and a warp's chain of steps.  Packed items, five passes: 10,000 rows x 16 tables with four CTAs 40 -> 25 us,
+// 12,000 x 8 with eight 47 -> 21; 20,000 x 8, before in 15 launches, 81 -> 27, keys of four words in 49 289 -> 99.
+// ---------------------------------------------------------------------------------------
+constexpr int RSC_THREADS = 512;
+constexpr int RSC_WARPS = RSC_THREADS / 32;
+constexpr int RSC_MAX_CTAS = 8;  // the portable limit
+template <int NW, bool PACK>
+struct ClusterSortCfg {
+    static constexpr int KW = SmallSortCfg<NW, PACK>::KW;
+    static constexpr int IPT = SmallSortCfg<NW, PACK>::IPT;
+    static constexpr int CTA_ROWS = RSC_THREADS * IPT;
+    static constexpr size_t SMEM = sizeof(uint32_t) * ((size_t)CTA_ROWS * (KW + (PACK ? 0 : 1)) + RSC_WARPS * 256 + RSC_MAX_CTAS * 256 +
+                                                       2 * 256 + 256 + 8);
+};
+
+template <int NW, bool PACK>
+__global__ void __launch_bounds__(RSC_THREADS, 1)
+radix_sort_cluster_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
+                          uint32_t* __restrict__ vals_out, int n, int cta_rows, uint32_t cta_rows_inv, int passes, bool compressed,
+                          KeyComp kc, const int* __restrict__ check) {
+    using Cfg = ClusterSortCfg<NW, PACK>;
+    constexpr int KW = Cfg::KW, IPT = Cfg::IPT;
+    constexpr bool WORDS = NW >= 4;
+    extern __shared__ __align__(16) uint32_t smem[];
+    uint32_t* s_keys = smem;                                  // [CTA_ROWS][KW]
+    uint32_t* s_vals = s_keys + (size_t)Cfg::CTA_ROWS * KW;   // [CTA_ROWS], not packed
+    uint32_t* s_bins = s_vals + (PACK ? 0 : Cfg::CTA_ROWS);   // [RSC_WARPS][256]
+    uint32_t* s_total = s_bins + RSC_WARPS * 256;             // [RSC_MAX_CTAS][256] of every CTA
+    uint32_t* s_half = s_total + RSC_MAX_CTAS * 256;          // [2][256] of each half of the warps
+    uint32_t* s_start = s_half + 2 * 256;                     // [256]
+    uint32_t* s_warp = s_start + 256;                         // [8]
+
+    auto cluster = cooperative_groups::this_cluster();
+    const int ctas = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row0 = rank * cta_rows;  // place in the table
+    const int count = max(0, min(cta_rows, n - row0));
+    const size_t base = (size_t)(blockIdx.x / ctas) * n;
+    const int steps = (cta_rows + RSC_THREADS - 1) / RSC_THREADS;  // at most IPT
+    const int first = warp * (32 * steps) + lane;                 // a warp holds 32 * steps consecutive items
+    const uint32_t below = (1u << lane) - 1u;
+    uint32_t* bins = s_bins + warp * 256;
+    if constexpr (!WORDS) {
+        if (check && !key_comp_of(check[0], check[2], check[3], kc)) {  // every CTA of the cluster finds the same
+            for (int at = tid; at < count; at += RSC_THREADS) {
+                uint32_t kk[KW];
+                load_key<KW>(keys_in + (base + row0 + at) * KW, kk);
+                store_key<KW>(keys_out + (base + row0 + at) * KW, kk);
+                vals_out[base + row0 + at] = (uint32_t)(row0 + at);
+            }
+            return;
+        }
+    }
+    uint32_t key[IPT][KW], val[IPT], pos[IPT];
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) {
+        const int li = first + i * 32;
+#pragma unroll
+        for (int w = 0; w < KW; ++w) key[i][w] = 0;
+        val[i] = (uint32_t)(row0 + li);
+        if (!WORDS && i < steps && li < count) {
+            load_key<KW>(keys_in + (base + row0 + li) * KW, key[i]);
+            if constexpr (!WORDS) {
+                if (compressed) comp_key<KW>(key[i], kc.sub);
+            }
+            if constexpr (PACK) {
+                key[i][0] = (key[i][0] << RS_PACK_ID_BITS) | (key[i][KW - 1] >> (32 - RS_PACK_ID_BITS));
+                key[i][KW - 1] = (key[i][KW - 1] << RS_PACK_ID_BITS) | (uint32_t)(row0 + li);
+            }
+        }
+    }
+    cluster.sync();  // all of them run: their shared memory may be written
+    for (int p = 0; p < passes; ++p) {
+        if (WORDS && (p & 3) == 0) {  // the next word of the key, from where the keys are
+#pragma unroll
+            for (int i = 0; i < IPT; ++i)
+                if (i < steps && first + i * 32 < count) key[i][0] = keys_in[(base + val[i]) * NW + (NW - 1 - (p >> 2))];
+        }
+        const int pd = PACK ? p + 3 : (WORDS ? (p & 3) : p);
+        const int dword = KW - 1 - (pd >> 2), dshift = 8 * (pd & 3);
+        auto digit = [&](const uint32_t* k) { return ((KW == 2 && dword == 1 ? k[KW - 1] : k[0]) >> dshift) & 0xFFu; };
+#pragma unroll
+        for (int i = 0; i < RSC_WARPS * 256 / 4 / RSC_THREADS; ++i)
+            reinterpret_cast<uint4*>(s_bins)[i * RSC_THREADS + tid] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) {
+            if (i < steps) {
+                const bool ok = first + i * 32 < count;
+                const uint32_t d = digit(key[i]);
+                uint32_t peers = __ballot_sync(0xFFFFFFFFu, ok);
+#pragma unroll
+                for (int b = 0; b < 8; ++b) keep_same_bit(peers, d, 1u << b);
+                pos[i] = bins[d] + __popc(peers & below);
+                __syncwarp();
+                if (ok && (peers >> lane) == 1u) bins[d] = pos[i] + 1u;
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+        // totals of this CTA to all: a thread takes one bin and half of the warps, then half of the CTAs
+        const int b = tid & 255, q = tid >> 8;
+        uint32_t sum = 0;
+#pragma unroll
+        for (int w = 0; w < RSC_WARPS / 2; ++w) sum += s_bins[(q * (RSC_WARPS / 2) + w) * 256 + b];
+        s_half[tid] = sum;
+        __syncthreads();
+        for (int r = q; r < ctas; r += 2) *cluster.map_shared_rank(s_total + rank * 256 + b, r) = s_half[b] + s_half[256 + b];
+        cluster.sync();
+        if (tid < 256) {
+            uint32_t tot = 0, before = 0;
+            for (int r = 0; r < ctas; ++r) {
+                const uint32_t x = s_total[r * 256 + tid];
+                before += r < rank ? x : 0u;
+                tot += x;
+            }
+            uint32_t inc = tot;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+                if (lane >= o) inc += x;
+            }
+            if (lane == 31) s_warp[warp] = inc;
+            s_start[tid] = inc - tot + before;
+        }
+        __syncthreads();
+        uint32_t run = s_start[b] + (q ? s_half[b] : 0u);
+        for (int w = 0; w < (b >> 5); ++w) run += s_warp[w];
+#pragma unroll
+        for (int w = 0; w < RSC_WARPS / 2; ++w) {
+            const uint32_t x = s_bins[(q * (RSC_WARPS / 2) + w) * 256 + b];
+            s_bins[(q * (RSC_WARPS / 2) + w) * 256 + b] = run;
+            run += x;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) {
+            if (i < steps && first + i * 32 < count) {
+                const uint32_t to = bins[digit(key[i])] + pos[i];
+                const uint32_t owner = __umulhi(to, cta_rows_inv), at = to - owner * (uint32_t)cta_rows;
+                store_key<KW>(cluster.map_shared_rank(s_keys + (size_t)at * KW, owner), key[i]);
+                if constexpr (!PACK) *cluster.map_shared_rank(s_vals + at, owner) = val[i];
+            }
+        }
+        cluster.sync();
+        if (p == passes - 1) break;
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) {
+            if (i < steps && first + i * 32 < count) {
+                load_key<KW>(s_keys + (size_t)(first + i * 32) * KW, key[i]);
+                if constexpr (!PACK) val[i] = s_vals[first + i * 32];
+            }
+        }
+    }
+    const size_t out = base + row0;
+    for (int at = tid; at < count; at += RSC_THREADS) {
+        uint32_t id;
+        if constexpr (WORDS) {
+            id = s_vals[at];
+            uint32_t kk[NW];
+            load_key<NW>(keys_in + (base + id) * NW, kk);
+            store_key<NW>(keys_out + (out + at) * NW, kk);
+        } else {
+            uint32_t kk[KW];
+            load_key<KW>(s_keys + (size_t)at * KW, kk);
+            if constexpr (PACK) {
+                id = kk[KW - 1] & ((1u << RS_PACK_ID_BITS) - 1u);
+                kk[KW - 1] = (kk[0] << (32 - RS_PACK_ID_BITS)) | (kk[KW - 1] >> RS_PACK_ID_BITS);
+                kk[0] >>= RS_PACK_ID_BITS;
+            } else {
+                id = s_vals[at];
+            }
+            if (compressed) decomp_key<KW>(kk, kc);
+            store_key<KW>(keys_out + (out + at) * KW, kk);
+        }
+        vals_out[out + at] = id;
+    }
+}
+
+// CTAs that sort a table: 0 when it is not short.  All tables' clusters are to run at once, each CTA on an SM of its own:
+// eight CTAs as long as they are three quarters of the SMs (a GPC holds whole clusters only: 16 of eight CTAs
+// went in two turns), four up to eight ninths.  A cluster costs 3 us to start and two barriers a pass, which few rows do not
+// earn: from 2,048 rows on it pays with packed items (2,000 x 16: 16.9 -> 15.6 us), without from 4,096 with eight
+// CTAs (4,000 x 8 in two passes 9.7 -> 9.5, sixteen 63 -> 58) and from 8,192 with four (8,000 x 32: 13.7 -> 14.1 and 99 -> 88,
+// 4,000 x 32: 9.7 -> 10.7 and 63 -> 66).  Clusters of two were slower without packed items at every size.
+inline int radix_sort_short_ctas(const CtxPtr& c, int n, int L, int NW, bool compressed) {
+    // CULSH_SORT_NO_PACK keeps the general form
+    const char* no_pack = getenv("CULSH_SORT_NO_PACK");
+    if ((no_pack && atoi(no_pack) != 0) || SmallSortCfg<2, true>::SMEM > c->smem_optin) return 0;
+    const bool packed = NW == 2 && compressed;
+    const int ipt = NW == 2 && !compressed ? SmallSortCfg<2, false>::IPT : SmallSortCfg<1, false>::IPT;
+    const int rows = (n + 31) / 32 * 32;  // CTAs hold whole warps of rows
+    const int64_t sms = c->sm_count;
+    if (L * 8ll * 4 <= sms * 3 && n >= (packed ? 2048 : 4096) && rows <= 8 * RSC_THREADS * ipt) return 8;
+    if (L * 4ll * 9 <= sms * 8 && n >= (packed ? 2048 : 8192) && rows <= 4 * RSC_THREADS * ipt) return 4;
+    return n <= RSS_THREADS * ipt && L <= sms ? 1 : 0;
+}
+
 // keys[0] -> keys[1], row ids to vals[1]
+template <int NW, bool PACK>
+inline void launch_sort_cluster(const CtxPtr& c, int ctas, uint32_t* keys[2], uint32_t* vals[2], int n, int L, int passes,
+                                bool compressed, KeyComp kc, const int* check) {
+    constexpr size_t smem = ClusterSortCfg<NW, PACK>::SMEM;
+    auto kern = radix_sort_cluster_kernel<NW, PACK>;
+    CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int cta_rows = (int)ceil_div(ceil_div((size_t)n, (size_t)ctas), 32) * 32;
+    const uint32_t inv = 0xFFFFFFFFu / (uint32_t)cta_rows + 1u;  // exact below 2^16 rows of a table
+    launch_cluster(c->stream, kern, (unsigned)(L * ctas), (unsigned)ctas, RSC_THREADS, smem, (const uint32_t*)keys[0], keys[1], vals[1], n, cta_rows, inv,
+                   passes, compressed, kc, check);
+}
+
 template <int NW>
 inline int radix_sort_small(const CtxPtr& c, uint32_t* keys[2], uint32_t* vals[2], int n, int L, int passes,
                             bool compressed, KeyComp kc, const int* check) {
+    const int ctas = radix_sort_short_ctas(c, n, L, NW, compressed);
+    if (ctas > 1) {
+        if (c->profiling) cudaEventRecord(c->ev_pass[0], c->stream);
+        if (NW == 2 && compressed) launch_sort_cluster<NW, NW == 2>(c, ctas, keys, vals, n, L, passes, compressed, kc, check);
+        else launch_sort_cluster<NW, false>(c, ctas, keys, vals, n, L, passes, compressed, kc, check);
+        if (c->profiling) cudaEventRecord(c->ev_pass[1], c->stream);
+        return 1;
+    }
     auto go = [&](auto kern, size_t smem) {
         CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (c->profiling) cudaEventRecord(c->ev_pass[0], c->stream);
@@ -710,11 +933,8 @@ inline int radix_sort_small(const CtxPtr& c, uint32_t* keys[2], uint32_t* vals[2
 // `compressed` (NW <= 2 only): sort the 5-bit-per-byte form of the keys, see the top of the file.
 // ---------------------------------------------------------------------------------------
 inline int radix_sort_passes(int KB, bool compressed) { return compressed ? (5 * KB + 7) / 8 : KB; }
-// Tables that one CTA sorts, no more of them than there are SMs (CULSH_SORT_NO_PACK keeps the general form).
 inline bool radix_sort_is_small(const CtxPtr& c, int n, int L, int NW, bool compressed) {
-    const char* no_pack = getenv("CULSH_SORT_NO_PACK");
-    const int rows = NW == 2 && !compressed ? SmallSortCfg<2, false>::MAX_ROWS : SmallSortCfg<1, false>::MAX_ROWS;
-    return n <= rows && L <= c->sm_count && SmallSortCfg<2, true>::SMEM <= c->smem_optin && !(no_pack && atoi(no_pack) != 0);
+    return radix_sort_short_ctas(c, n, L, NW, compressed) > 0;
 }
 inline int radix_sort_final(const CtxPtr& c, int passes, int n, int L, int NW, bool compressed) {
     return NW >= 4 || radix_sort_is_small(c, n, L, NW, compressed) ? 1 : passes & 1;
