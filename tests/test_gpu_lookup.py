@@ -18,8 +18,8 @@ def test_against_the_host(k, values):
     ids = np.repeat(rng.permutation(1 << 20)[:2 * values:2], copies)[rng.permutation(n)].astype(np.int32)
     core = core_mod.MinHashCore(L, k, 3)
     ix = core.fit(ids, np.arange(n + 1, dtype=np.int32), n, 1 << 20)
-    nq = 300  # 2,700 pairs: beyond what one CTA looks up
-    q = np.concatenate([rng.choice(ids, 150), rng.integers(0, 1 << 20, 150)]).astype(np.int32)
+    nq = 1000  # 9,000 pairs: beyond what is looked up and counted in one launch
+    q = np.concatenate([rng.choice(ids, 500), rng.integers(0, 1 << 20, 500)]).astype(np.int32)
     got = core.query(q, np.arange(nq + 1, dtype=np.int32), nq, ix)
     sx, sq = core.hash(ids, np.arange(n + 1, dtype=np.int32), n, ix), core.hash(q, np.arange(nq + 1, dtype=np.int32), nq, ix)
     off, cand = got.get_offsets().astype(np.int64), got.get_indices()
