@@ -14,7 +14,13 @@ namespace culsh_b200 {
 
 constexpr uint32_t MINHASH_PRIME = 4294967291u;  // minhash/hash.cuh:17
 constexpr int MH_STEPS = 4;  // pairs of ids a turn of the loop
-constexpr int MH_THREADS = 256;
+// A warp is a CTA of its own: rows differ in length tenfold, and with eight warps a CTA held its place until the longest of their
+// rows was over.
+constexpr int MH_THREADS = 32;
+// Rows of a warp: many for what it sets up once, few for the last warps to end together, but no fewer warps than
+// MH_WARPS of an SM, eight turns (2M sets: 4 rows 4,525 us, 16 4,450, 64 4,497; 100,003: 4 rows 248, 16 269, 64 288).
+constexpr int MH_ROWS = 16;
+constexpr int MH_WARPS = 192;
 constexpr int MH_MAX_PER_LANE = 8;               // hashes per lane per sweep (H <= 256 in one sweep)
 
 __device__ __forceinline__ uint64_t mad_wide_u32(uint32_t a, uint32_t b, uint64_t c) {
@@ -93,38 +99,54 @@ __device__ __forceinline__ uint32_t min_plus5_short(uint32_t m, double a, double
 // H > 256 takes several sweeps.  Slots past H hold a = b = 0, evaluate to 0 and are never stored,
 // so the inner loop carries no predicate.
 template <int PL>
-__global__ void __launch_bounds__(MH_THREADS, PL <= 4 ? 3 : 2)
+__global__ void __launch_bounds__(MH_THREADS, PL <= 4 ? 24 : 16)
 minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ indptr,
                const uint32_t* __restrict__ A, const uint32_t* __restrict__ B, int n_rows,
                int L, int k, int NW, uint32_t* __restrict__ keys, int n_total, int row_offset) {
     const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * (MH_THREADS / 32)) + (threadIdx.x >> 5);
-    const int n_warps = gridDim.x * (MH_THREADS / 32);
     const int H = L * k;
     const int pad_words = NW - k;  // leading zero words when 4k is not 4, 8, 16 or 32 bytes
-    __shared__ __align__(16) double s_ids[MH_THREADS / 32][2][34];
-    double* const ids_short = s_ids[threadIdx.x >> 5][0];
-    double* const ids_long = s_ids[threadIdx.x >> 5][1];
+    __shared__ __align__(16) double ids_short[34], ids_long[34];
     const uint32_t below = (1u << lane) - 1u;
+    double ad[PL], bd[PL];
+    auto load_params = [&](int h0) {
+#pragma unroll
+        for (int i = 0; i < PL; ++i) {
+            const int h = h0 + i * 32 + lane;
+            ad[i] = h < H ? (double)A[h] : 0.0;
+            bd[i] = (h < H ? (double)B[h] : 0.0) + 5.0 + MH_2_52;
+        }
+    };
+    // the integer forms take their parameters from the doubles: these are all the loop has registers for
+    auto a_of = [&](int i) { return __double2uint_rz(ad[i]); };
+    auto b5_of = [&](int i) { return (uint64_t)(bd[i] - MH_2_52); };
+    load_params(0);
 
-    for (int row = warp; row < n_rows; row += n_warps) {
-        const int start = indptr[row], end = indptr[row + 1];
+    // the ids of a step are fetched a step ahead, the bounds of a row a row ahead
+    int start = 0, end = 0;
+    if (blockIdx.x < n_rows) {
+        start = indptr[blockIdx.x];
+        end = indptr[blockIdx.x + 1];
+    }
+    int ahead = start + lane < end ? indices[start + lane] : 0;
+    int next_start, next_end;
+    for (int row = blockIdx.x; row < n_rows; row += gridDim.x, start = next_start, end = next_end) {
+        const bool more = n_rows - row > (int)gridDim.x;
+        next_start = more ? indptr[row + gridDim.x] : 0;
+        next_end = more ? indptr[row + gridDim.x + 1] : 0;
         const uint32_t short_col = end - start <= MH_SHORT_ROW ? MH_SHORT_COL : 0u;
         for (int h0 = 0; h0 < H; h0 += 32 * PL) {
+            const bool last = h0 + 32 * PL >= H;
+            if (H > 32 * PL) load_params(h0);
             uint32_t m[PL];
-            double ad[PL], bd[PL];
 #pragma unroll
-            for (int i = 0; i < PL; ++i) {
-                int h = h0 + i * 32 + lane;
-                ad[i] = h < H ? (double)A[h] : 0.0;
-                bd[i] = (h < H ? (double)B[h] : 0.0) + 5.0 + MH_2_52;
-                m[i] = 0xFFFFFFFFu;
-            }
-            // the integer forms take their parameters from the doubles: these are all the loop has registers for
-            auto a_of = [&](int i) { return __double2uint_rz(ad[i]); };
-            auto b5_of = [&](int i) { return (uint64_t)(bd[i] - MH_2_52); };
+            for (int i = 0; i < PL; ++i) m[i] = 0xFFFFFFFFu;
             for (int base = start; base < end; base += 32) {
-                const int mine = base + lane < end ? indices[base + lane] : 0;
+                const int mine = ahead;
+                // the next step's, then the row's first again for another sweep, or the next row's
+                const bool inside = base + 32 < end;
+                const int at = (inside ? base + 32 : last ? next_start : start) + lane;
+                ahead = at < (inside || !last ? end : next_end) ? indices[at] : 0;
                 const int cnt = min(32, end - base);
                 if (!__any_sync(0xFFFFFFFFu, (uint32_t)mine >= MH_DOUBLE_COL)) {
                     // the two lists, the last id of an odd number twice
@@ -201,6 +223,7 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
                 }
             }
         }
+        if (end <= start) ahead = next_start + lane < next_end ? indices[next_start + lane] : 0;
         if (pad_words > 0) {
             for (int idx = lane; idx < L * pad_words; idx += 32) {
                 int t = idx / pad_words, j = idx - t * pad_words;
@@ -216,10 +239,7 @@ inline void launch_minhash(const CtxPtr& c, cudaStream_t stream, const int32_t* 
                            int L, int k, const KeySpec& ks, uint32_t* keys, int n_total,
                            int row_offset) {
     if (n_rows == 0) return;
-    int warps_per_block = MH_THREADS / 32;
-    size_t blocks = ceil_div((size_t)n_rows, warps_per_block);
-    size_t cap = (size_t)c->sm_count * 32;
-    if (blocks > cap) blocks = cap;
+    const size_t blocks = std::min<size_t>(n_rows, std::max<size_t>(ceil_div((size_t)n_rows, MH_ROWS), (size_t)c->sm_count * MH_WARPS));
     const int H = L * k;
     const int sweeps = (int)ceil_div(H, 32 * MH_MAX_PER_LANE);
     const int per_lane = (int)ceil_div(H, 32 * sweeps);  // 1..MH_MAX_PER_LANE
