@@ -4,7 +4,7 @@
 //
 // One warp per row.  Lanes own hash functions (lane, lane+32, ...), so every lane is busy
 // however short the row is and no cross-lane reduction is needed; the row's column ids
-// are loaded 32 at a time (coalesced) and broadcast with shuffles.  The modulus is
+// are loaded 32 at a time (coalesced) and reach all lanes through shared memory or shuffles.  The modulus is
 // folded with 2^32 = 5 (mod p) instead of a 64-bit division.
 #pragma once
 
@@ -74,7 +74,7 @@ __device__ __forceinline__ uint32_t hash_plus5_any(uint32_t a, uint32_t c, uint6
 // minimum at or above that is right.  One below it, rare as long as the row is short (about 8e-5 for each id), is evaluated again in
 // full by the whole warp.  A step of 32 ids is sorted into those below and above through shared memory, as the doubles that
 // all lanes then read.  2M sets of 20 to 200 ids into 128 hash functions (with the 10,000 queries): 7,730 us in the integer form,
-// 6,630 with the wrap for all, now 4,870 (two pairs of ids a turn 4,900, the line at 2^14 4,940); 100,003 sets 414, 367 and 278.
+// 6,630 with the wrap for all, 4,870 without (two pairs of ids a turn 4,900, the line at 2^14 4,940); 100,003 sets 414, 367 and 278.
 constexpr uint32_t MH_DOUBLE_COL = 1u << 20;
 constexpr double MH_2_52 = 4503599627370496.0;
 constexpr uint32_t MH_2_52_HI = 0x43300000u;
