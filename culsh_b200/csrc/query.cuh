@@ -238,8 +238,7 @@ lookup_count_kernel(const uint32_t* __restrict__ qkeys, const uint8_t* __restric
     __syncthreads();
     if (tid == 0) raw_off[n_q] = carry;
     if (tid < 3) counters[tid] = s_counters[tid];
-    __syncwarp();
-    if (tid < 32) host.write(carry);
+    if (tid < 32) host.write(carry, s_counters);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -1141,11 +1141,13 @@ struct HostWords {
     uint32_t* words;       // [n_a + n_b]
     const uint32_t *a, *b;
     int n_a, n_b;
-    __device__ __forceinline__ void write(uint64_t t) const {  // by one warp
+    __device__ __forceinline__ void write(uint64_t t) const { write(t, a); }
+    // By one warp.  `from` in place of a: a kernel that makes these words itself writes the array that a is, through another pointer.
+    __device__ __forceinline__ void write(uint64_t t, const uint32_t* from) const {
         if (!total) return;
         const int i = threadIdx.x & 31;
         if (i == 0) *total = t;
-        if (i < n_a) words[i] = a[i];
+        if (i < n_a) words[i] = from[i];
         else if (i < n_a + n_b) words[i] = b[i - n_a];
     }
 };
