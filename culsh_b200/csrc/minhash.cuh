@@ -9,6 +9,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "index_math.h"
 
 namespace culsh_b200 {
 
@@ -130,7 +131,7 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
     }
     int ahead = start + lane < end ? indices[start + lane] : 0;
     int next_start, next_end;
-    for (int row = blockIdx.x; row < n_rows; row += gridDim.x, start = next_start, end = next_end) {
+    walk_rows(blockIdx.x, gridDim.x, n_rows, [&](int row) {
         const bool more = n_rows - row > (int)gridDim.x;
         next_start = more ? indptr[row + gridDim.x] : 0;
         next_end = more ? indptr[row + gridDim.x + 1] : 0;
@@ -231,7 +232,9 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
                 keys[item * NW + j] = 0u;
             }
         }
-    }
+        start = next_start;
+        end = next_end;
+    });
 }
 
 inline void launch_minhash(const CtxPtr& c, cudaStream_t stream, const int32_t* indices,

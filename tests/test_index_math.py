@@ -50,10 +50,12 @@ int main() {
 
 
 def test_row_walks_end(tmp_path):
-    """148 CTAs of 8 warps step by 1,184 rows: the last step of n = 2^31 - 1 rows ends beyond 2^31."""
+    """148 CTAs of 8 warps step by 1,184 rows: the last step of n = 2^31 - 1 rows ends beyond 2^31.  MinHash, with up to 16 rows
+    a warp, steps by a sixteenth of the rows."""
     top = (1 << 31) - 1
     cases = [(0, 1, 0), (0, 1184, 1), (5, 1184, 5), (7, 1184, 10_000), (1183, 1184, top), (0, 1184, top),
-             (top - 1, 37_888, top), (top, 1184, top), (100, 37_888, top - 900)]
+             (top - 1, 37_888, top), (top, 1184, top), (100, 37_888, top - 900),
+             (0, -(-top // 16), top), (-(-top // 16) - 1, -(-top // 16), top), (126_250_000, 126_250_001, 2_020_000_016), (5, top, top)]
     out = run_native(tmp_path, ROWS, "".join("%d %d %d\n" % c for c in cases)).split("\n")
     for (first, stride, n), line in zip(cases, out):
         rows = range(first, n, stride)

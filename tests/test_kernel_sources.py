@@ -29,3 +29,10 @@ def test_host_words_are_not_read_through_a_second_pointer():
     assert "HostWords host" in params and re.search(r"__restrict__\s+counters\b", params)
     calls = re.findall(r"host\.write\(([^;]*)\);", body)
     assert calls and all(c.split(",")[1:] == [" s_counters"] for c in calls)
+
+
+def test_rows_are_not_counted_up_in_signed_steps():
+    """A step of a whole grid past the last of n < 2^31 rows may pass 2^31: rows are gone through by walk_rows, which counts unsigned
+    (tests/test_index_math.py), or by an unsigned loop."""
+    assert not [(f, m) for f, t in _sources().items()
+                for m in re.findall(r"for \((?:int|int32_t) (?:row|q)\b[^;]*;[^;]*;[^)]*\+=[^)]*(?:gridDim|n_warps)[^)]*\)", t)]
