@@ -863,7 +863,9 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         launch_small(self_join ? dedupe_small_kernel<SMALL_MAX, true> : dedupe_small_kernel<SMALL_MAX, false>, 0, room);
         if (ahead_windows) {
             pieces.reserve(c, SL_CHAIN, (size_t)n_q * n_win);
+            if (c->profiling) cudaEventRecord(c->ev_dedupe[0], s);
             launch_windows((size_t)n_q * n_win, n_big, room);
+            if (c->profiling) cudaEventRecord(c->ev_dedupe[1], s);
         }
         scan_unique();
     }
@@ -874,6 +876,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
     tr.lap("count+scan+sync");
     if (raw_total > raw_limit) return false;
     const bool done = ahead && raw_total <= room && nm == 0 && (nb == 0 || ahead_windows);
+    dedupe_timed = done && nb && c->profiling;
     // The bitmap and sort paths walk lists: a self-join with rows for them takes its pairs as lists too
     // (the tile bases of the build are still in their slot).
     if (self_join && (nb || nm))

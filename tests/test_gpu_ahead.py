@@ -57,3 +57,19 @@ def test_queries_equal_those_of_a_larger_set(n, L, k):
         part = m.query(Q[a:b])
         assert np.array_equal(part.get_offsets().astype(np.int64), off[a:b + 1] - off[a])
         assert np.array_equal(part.get_indices(), ids[off[a]:off[b]])
+
+
+def test_windows_launched_ahead_are_timed():
+    from culsh_b200 import _culsh_core as core_mod
+    rng = np.random.default_rng(4)
+    n, d = 60_000, 6
+    X = rng.standard_normal((n, d)).astype(np.float32)
+    core = core_mod.RPLSHCore(4, 2, 6)
+    core.set_profiling(True)
+    try:
+        ix = core.fit_float(X, n, d)
+        for nq in (1, 30, 200):  # the last is too many for windows before the counts are known
+            assert core.query_float(X[:nq], nq, ix).n_total_candidates > 1024 * nq
+            assert core.last_stats()["dedupe_ms"] > 0
+    finally:
+        core.set_profiling(False)
