@@ -650,7 +650,8 @@ def line_of(torch, args, wl, spec, world, m, peaks, tf32):
     items, kb = sf["n_items"], 4 * sf["key_words"]
     # keys of four words and more: the last pass reads (word, row id) and writes the ids; short tables: one launch
     # reads the keys and writes keys and ids
-    short = n <= (8192 if sf["key_words"] == 2 and passes > 5 else 12_288)
+    ctas = sf["sort_ctas"]
+    short = ctas > 0
     wide = sf["key_words"] >= 4
     item_bytes = 2.0 * kb + 4.0 if short else (12.0 if wide else (kb + 4) * 2.0)
     item_note = (f"key {kb} B read, key and row id written per item, one launch for all passes" if short else
@@ -681,7 +682,8 @@ def line_of(torch, args, wl, spec, world, m, peaks, tf32):
     if scatter_ms > 0:
         roof["sort"] = {"bound": "hbm", "achieved": items * item_bytes / (scatter_ms * 1e-3) / 1e9,
                         "peak": peaks["hbm_gbs"], "unit": "GB/s", "traffic": None,
-                        "kernel": "radix_sort_small_kernel" if short else "radix_scatter_kernel",
+                        "kernel": ("radix_sort_cluster_kernel" if ctas > 1 else "radix_sort_small_kernel" if short else
+                                   "radix_scatter_kernel"),
                         "note": item_note + ("" if short else f" (the scatter of the last of {passes} passes)") +
                                 f", timed with CUDA events; peak {peaks['source']}"}
     dedupe_ms = mean("dedupe_ms", "query")
@@ -697,7 +699,7 @@ def line_of(torch, args, wl, spec, world, m, peaks, tf32):
         r["traffic"] = traffic
         r["traffic_note"] = ("ncu DRAM bytes of one launch of this size (profiles/)" if traffic is not None
                              else "no ncu capture of a launch of this size")
-    shares = {"hash": hash_ms if "hash" in roof else 0.0, "sort": scatter_ms * passes if "sort" in roof else 0.0,
+    shares = {"hash": hash_ms if "hash" in roof else 0.0, "sort": scatter_ms * (1 if short else passes) if "sort" in roof else 0.0,
               "gather": dedupe_ms if "gather" in roof else 0.0}
     dominant = roof[max(shares, key=shares.get)] if roof else None
     t_dev = m["t_dev"]

@@ -32,7 +32,7 @@ class Stats(C.Structure):
         ("n_items", C.c_uint64), ("n_buckets", C.c_uint64), ("raw_candidates", C.c_uint64),
         ("unique_candidates", C.c_uint64),
         ("sort_passes", C.c_int32), ("key_words", C.c_int32), ("elem_bytes", C.c_int32),
-        ("hash_path", C.c_int32), ("launches", C.c_int32), ("reserved1", C.c_int32),
+        ("hash_path", C.c_int32), ("launches", C.c_int32), ("sort_ctas", C.c_int32),
     ]
 
 

@@ -639,6 +639,7 @@ int build_index(culsh_index& ix, SortBuffers& sb, Scratch<uint32_t>* bounds, Sta
     c->stats.n_items = (uint64_t)n * L;
     c->stats.n_buckets = B;
     c->stats.sort_passes = passes;
+    c->stats.sort_ctas = radix_sort_short_ctas(c, n, L, NW, compressed);
     c->stats.key_words = NW;
     c->stats.elem_bytes = ix.ks.elem_bytes;
     return 0;

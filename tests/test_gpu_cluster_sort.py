@@ -46,3 +46,11 @@ def test_wide_keys(n, L, k):
     core = core_mod.MinHashCore(L, k, 7)
     ix = core.fit(indices, indptr, n, 400)
     _check(ix, core.hash(indices, indptr, n, ix), n, L)
+
+
+@pytest.mark.parametrize("n,L,ctas", [(1000, 8, 1), (10_000, 13, 8), (24_576, 32, 4), (49_152, 13, 8), (49_153, 13, 0)])
+def test_stats_name_the_form(n, L, ctas):
+    from culsh_b200 import _culsh_core as core_mod
+    core = core_mod.RPLSHCore(L, 12, 1)
+    core.fit_float(np.random.default_rng(n).standard_normal((n, 8)).astype(np.float32), n, 8)
+    assert core.last_stats()["sort_ctas"] == ctas
