@@ -690,9 +690,10 @@ def line_of(torch, args, wl, spec, world, m, peaks, tf32):
     if dedupe_ms > 0:
         roof["gather"] = {"bound": "hbm", "peak": peaks["hbm_gbs"], "unit": "GB/s", "traffic": None,
                           "achieved": 4.0 * (sq["raw_candidates"] + sq["unique_candidates"]) / (dedupe_ms * 1e-3) / 1e9,
-                          "kernel": "dedupe kernel of the gather (window / bitmap form)",
-                          "note": "4 B per raw candidate id read + 4 B per unique id written, over the CUDA-event "
-                                  f"time of the dedupe launch alone; peak {peaks['source']}"}
+                          "kernel": "dedupe_window_kernel and compact_windows_kernel (or the bitmap form)",
+                          "note": "4 B per raw candidate id read + 4 B per unique id written, over the CUDA-event time "
+                                  "of the dedupe launch, which writes the ids to the sets' raw spans, and of the copy "
+                                  f"that brings them to the result; peak {peaks['source']}"}
     for key, r in roof.items():
         r["frac"] = r["achieved"] / r["peak"]
         traffic = NCU_TRAFFIC.get((wl, n), {}).get(key)

@@ -129,7 +129,7 @@ struct Ctx {
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t ev[8] = {};
     cudaEvent_t ev_pass[2] = {};      // around the scatter launch of the last radix pass
-    cudaEvent_t ev_dedupe[2] = {};    // around the window / bitmap dedupe launch of the last query batch
+    cudaEvent_t ev_dedupe[4] = {};    // around the window / bitmap dedupe launch of the last query batch and around its copy to the result
     cudaEvent_t copy_done[2] = {};
     cudaEvent_t chunk_free[2] = {};
     uint64_t* pinned = nullptr;       // 64 x u64 words of pinned host memory: read_words' first, see HostSlot

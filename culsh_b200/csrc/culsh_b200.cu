@@ -987,8 +987,10 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
             }
         }
         tr.lap("alloc indices");
+        if (dedupe_timed) cudaEventRecord(c->ev_dedupe[2], s);
         if (second) compact(0, n_q, 0, out.indices.p);
         else compact_in_place(c, out, raw_ids, (uint64_t)std::max(bounce_env, 0l), compact);
+        if (dedupe_timed) cudaEventRecord(c->ev_dedupe[3], s);
     }
     tm.mark();
     CU_CHECK(cudaStreamSynchronize(s));
@@ -996,6 +998,10 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         float ms = 0.f;
         cudaEventElapsedTime(&ms, c->ev_dedupe[0], c->ev_dedupe[1]);
         c->stats.dedupe_ms += ms;
+        if (total) {
+            cudaEventElapsedTime(&ms, c->ev_dedupe[2], c->ev_dedupe[3]);
+            c->stats.dedupe_ms += ms;
+        }
     }
     tr.lap("compact+sync");
     return true;

@@ -73,7 +73,8 @@ typedef struct culsh_index_meta {
 typedef struct culsh_stats {
     float hash_ms, sort_ms, build_ms, lookup_ms, gather_ms, total_ms;
     float scatter_ms; /* the scatter launch of the last radix pass alone */
-    float dedupe_ms;  /* the dedupe launch (window or bitmap kernel) of the query batches alone */
+    float dedupe_ms;  /* large sets of the query batches: the dedupe launch (window or bitmap kernel) and the copy of all
+                         ids to the result */
     float params_ms;  /* fit: host wall time of the hash-parameter generation (0 on a cache hit) */
     float hash_lo_fraction; /* tensor-core projection with profiling on: share of the K-blocks whose rows had
                                a non-zero low part, i.e. that issued three MMAs instead of two */
