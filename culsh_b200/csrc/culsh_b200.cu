@@ -751,8 +751,8 @@ struct RawCounts {
 };
 
 // Sets of up to this many queries do not wait for their counts: what usually comes next is launched behind the count, for
-// up to AHEAD_IDS ids, and done again if the counts ask for something else (one query against
-// an index of a million rows: 144 -> 124 us, with the waits and copies that went).
+// up to AHEAD_IDS ids or as many as earlier calls have made room for, and done again if the counts ask for something else
+// (one query against an index of a million rows: 144 -> 124 us, with the waits and copies that went).
 constexpr int AHEAD_QUERIES = 4096;
 constexpr size_t AHEAD_IDS = (size_t)1 << 20;
 constexpr int AHEAD_PIECES = 64;  // CTAs of the window kernel that may turn out to have nothing to do
@@ -876,7 +876,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
     c->seen_error = (int)slot_words(c, HS_RAW)[3];  // what follows has no waits that could run out
     tr.lap("count+scan+sync");
     if (raw_total > raw_limit) return false;
-    const bool done = ahead && raw_total <= room && nm == 0 && (nb == 0 || ahead_windows);
+    const bool fits = ahead && raw_total <= room, done = fits && nm == 0 && (nb == 0 || ahead_windows);
     dedupe_timed = done && nb && c->profiling;
     // The bitmap and sort paths walk lists: a self-join with rows for them takes its pairs as lists too
     // (the tile bases of the build are still in their slot).
@@ -898,7 +898,8 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
     if (!done) {
         // The ids of a query land in its raw span first.  A large such array is a block of the result's kind: it goes
         // back when the call is done, and takes the result's place when there is no memory for both.
-        if (windows && raw_total * sizeof(int32_t) >= BIG_BLOCK_MIN) {
+        const bool block = windows && raw_total * sizeof(int32_t) >= BIG_BLOCK_MIN;
+        if (block) {
             raw_ids.alloc(c, raw_total);
             tmp.p = raw_ids.p;
             tmp.n = raw_total;
@@ -906,7 +907,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
             tmp.reserve(c, SL_TMP, raw_total);
         }
         tr.lap("alloc tmp");
-        if (n_other) {
+        if (n_other && (block || !fits)) {  // else they were written ahead, to where they stay
             // Short lists in a form that fits twice as many warps on an SM, the rest in a second launch; a
             // set that one launch takes in a wave or two is not worth a second one.
             const bool both = n_long && n_q < (1 << 15);

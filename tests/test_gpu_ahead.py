@@ -73,3 +73,29 @@ def test_windows_launched_ahead_are_timed():
             assert core.last_stats()["dedupe_ms"] > 0
     finally:
         core.set_profiling(False)
+
+
+def test_small_sets_are_gathered_once():
+    """Next to sets for the windows that wait for their counts, the small ones that were gathered ahead stay as they are."""
+    from culsh_b200 import _culsh_core as core_mod
+    rng = np.random.default_rng(5)
+    n, d = 60_000, 6
+    X = rng.standard_normal((n, d)).astype(np.float32)
+    X[:3000] = X[0]
+    core = core_mod.RPLSHCore(4, 16, 6)
+    ix = core.fit_float(X, n, d)
+    few = np.ascontiguousarray(X[10_000:10_100])
+    mixed = few.copy()
+    mixed[::10] = X[0]
+    small = core.query_float(few, 100, ix)
+    launches = core.last_stats()["launches"]
+    assert int(small.get_counts().max()) < 512
+    got = core.query_float(mixed, 100, ix)
+    # the windows, the second scan of the counts and the copy of the pieces
+    assert core.last_stats()["launches"] == launches + 3
+    counts = got.get_counts()
+    assert (counts[::10] >= 3000).all()
+    for q in (1, 10, 55):
+        one = core.query_float(mixed[q:q + 1], 1, ix)
+        off = got.get_offsets()
+        assert np.array_equal(one.get_indices(), got.get_indices()[int(off[q]):int(off[q + 1])])
