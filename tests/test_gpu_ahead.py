@@ -79,7 +79,7 @@ def test_small_sets_are_gathered_once():
     """Next to sets for the windows that wait for their counts, the small ones that were gathered ahead stay as they are."""
     from culsh_b200 import _culsh_core as core_mod
     rng = np.random.default_rng(5)
-    n, d = 60_000, 6
+    n, d = 60_000, 32
     X = rng.standard_normal((n, d)).astype(np.float32)
     X[:3000] = X[0]
     core = core_mod.RPLSHCore(4, 16, 6)
@@ -89,7 +89,7 @@ def test_small_sets_are_gathered_once():
     mixed[::10] = X[0]
     small = core.query_float(few, 100, ix)
     launches = core.last_stats()["launches"]
-    assert int(small.get_counts().max()) < 512
+    assert int(small.get_counts().max()) < 256
     got = core.query_float(mixed, 100, ix)
     # the windows, the second scan of the counts and the copy of the pieces
     assert core.last_stats()["launches"] == launches + 3
