@@ -22,4 +22,7 @@ CULSH_HD void walk_rows(uint32_t first, uint32_t stride, int n, F&& f) {
     for (uint32_t row = first; row < (uint32_t)n; row += stride) f((int)row);
 }
 
+// Blocks of `per` rows in n.  Unsigned: n + per - 1 may pass 2^31.
+CULSH_HD int row_blocks(int n, int per) { return (int)(((uint32_t)n + (uint32_t)per - 1u) / (uint32_t)per); }
+
 }  // namespace culsh_b200

@@ -18,6 +18,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "index_math.h"
 #include "project_simt.cuh"
 
 namespace culsh_b200 {
@@ -69,7 +70,7 @@ project_f32_kernel(ProjectArgs a) {
     const int G = a.tables_per_group;
     const int n_groups = (a.L + G - 1) / G;
     const int group = blockIdx.x % n_groups;  // fastest: the groups of one row block share X in L2
-    const int n_blocks = (a.n + PG_BM - 1) / PG_BM, block_step = gridDim.x / n_groups;  // the grid is a multiple of the groups
+    const int n_blocks = row_blocks(a.n, PG_BM), block_step = gridDim.x / n_groups;  // the grid is a multiple of the groups
     const int GC = G * a.k;
     const int col_base = group * GC;
     const int gc_valid = min(GC, a.L * a.k - col_base);

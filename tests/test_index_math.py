@@ -60,3 +60,21 @@ def test_row_walks_end(tmp_path):
     for (first, stride, n), line in zip(cases, out):
         rows = range(first, n, stride)
         assert [int(x) for x in line.split()] == [len(rows), sum(rows), 0]
+
+
+BLOCKS = r"""
+#include "index_math.h"
+#include <cstdio>
+int main() {
+    long long n, per;
+    while (std::scanf("%lld %lld", &n, &per) == 2) std::printf("%d\n", culsh_b200::row_blocks((int)n, (int)per));
+}
+"""
+
+
+def test_blocks_of_rows(tmp_path):
+    """Blocks of 64 and 128 rows, up to n = 2^31 - 1 (queries and rows that are only hashed may be as many)."""
+    top = (1 << 31) - 1
+    cases = [(n, per) for per in (64, 128) for n in (1, per - 1, per, per + 1, 10 * per, top - per, top - per + 1, top - 1, top)]
+    out = run_native(tmp_path, BLOCKS, "".join("%d %d\n" % c for c in cases)).split("\n")
+    assert [int(x) for x in out[:len(cases)]] == [-(-n // per) for n, per in cases]

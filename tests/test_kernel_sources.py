@@ -31,6 +31,12 @@ def test_host_words_are_not_read_through_a_second_pointer():
     assert calls and all(c.split(",")[1:] == [" s_counters"] for c in calls)
 
 
+def test_blocks_of_rows_are_not_rounded_up_by_a_sum():
+    """n + per - 1 passes 2^31 for the largest n: kernels count blocks of rows by row_blocks (tests/test_index_math.py)."""
+    assert not [(f, n) for f, t in _sources().items() for n, _, body in _kernels(t)
+                if re.search(r"\(a\.n \+ \w+ - 1\) / ", body)]
+
+
 def test_rows_are_not_counted_up_in_signed_steps():
     """A step of a whole grid past the last of n < 2^31 rows may pass 2^31: rows are gone through by walk_rows, which counts unsigned
     (tests/test_index_math.py), or by an unsigned loop."""
