@@ -12,9 +12,9 @@
 // the two halves of the warps, so that 224 columns are 2 x 112; the number of steps is a template argument, without
 // which every instruction stood behind a branch of its own.  Steps of eight features past d are left out.
 //
-// A row of a hundred features is over in seven stages of a microsecond, and what surrounds them weighs as much: a CTA
-// stays for many row blocks of its group of columns and, for sign bits, fetches the first stages of the next block before
-// it packs the keys of this one.  The bits of a step of eight columns are one byte a row, made from ballots.
+// A row of a few dozen features is over in two or three stages of a microsecond, and what surrounds them weighs as much: a CTA
+// then stays for many row blocks of its group of columns (see launch_project_f64) and, for sign bits, fetches the first stages of
+// the next block before it packs the keys of this one.  The bits of a step of eight columns are one byte a row, made from ballots.
 // 200,003 x 100 rows, 224 columns: 0.97 ms on the CUDA cores, with one block of rows a CTA and a branch before every instruction 0.46 (with 2,001 queries), now 0.367.
 #pragma once
 
@@ -226,9 +226,18 @@ inline bool launch_project_f64(const CtxPtr& c, cudaStream_t stream, int family,
     a.elem_bytes = ks.elem_bytes;
     a.row_offset = row_offset;
     a.n_total = n_total;
-    // a whole number of CTAs for each group, two an SM where there is work for them
-    const size_t n_groups = ceil_div(L, a.tables_per_group), per_group = std::max<size_t>(1, 2 * (size_t)c->sm_count / n_groups);
-    const dim3 grid((unsigned)(n_groups * std::min<size_t>(ceil_div(n, PF_BM), per_group)));
+    // Rows of few features, and few rows: a whole number of CTAs for each group that stay for all of its blocks, two an SM, where that
+    // many groups leave no more than a tenth of the places empty.  Else a CTA for each block and group: from four stages on
+    // (from five on with up to 32 columns, p-stable 64) it is the faster one, as packing and multiplying of the CTAs of an SM spread
+    // in time.  200,003 rows, staying and not: 17 features x 128 columns 69 and 74 us, 33 x 128 97 and 95 (p-stable 115 and 119), 50 x
+    // 128 137 and 120, 98 x 224 355 and 342, 201 x 1,008 2,963 and 2,760, p-stable 98 x 128 243 and 218; 17 x 16 27 and 31, 50 x 32
+    // 45 and 48, 66 x 32 55 and 55; 20,000 x 100 x 128 33.5 and 35.3.
+    const int steps = (int)ceil_div(a.tables_per_group * k, 16);  // of eight columns, of a warp
+    const size_t n_groups = ceil_div(L, a.tables_per_group), n_blocks = row_blocks(n, PF_BM), places = 2 * (size_t)c->sm_count;
+    const int stay_stages = steps <= (family == CULSH_PSLSH ? 4 : 2) ? 4 : 3;
+    const bool stay = ((int)ceil_div(d, PF_BK) <= stay_stages || n_blocks * n_groups <= 2 * places) &&
+                      places / n_groups * n_groups * 10 >= places * 9;
+    const dim3 grid((unsigned)(n_groups * (stay ? std::min<size_t>(n_blocks, places / n_groups) : n_blocks)));
     auto go = [&](auto kern) {
         CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM));
         kern<<<grid, PF_THREADS, PF_SMEM, stream>>>(a);
@@ -239,7 +248,9 @@ inline bool launch_project_f64(const CtxPtr& c, cudaStream_t stream, int family,
         if (family == CULSH_RPLSH) go(project_f64_kernel<CULSH_RPLSH, NF>);
         else go(project_f64_kernel<CULSH_PSLSH, NF>);
     };
-    const int steps = (int)ceil_div(a.tables_per_group * k, 16);  // of a warp
+    // Forms of every second number of steps, and 7, which two groups of 112 columns take; the others round up to columns of
+    // zeros.  That is still faster than a branch before every step, which left these out: 100 features x 80 columns in 6 steps for 5
+    // 160 us in place of 225, x 48 in 4 for 3 116 in place of 216, x 16 in 2 for 1 72 in place of 207.
     if (steps <= 2) with_steps(std::integral_constant<int, 2>{});
     else if (steps <= 4) with_steps(std::integral_constant<int, 4>{});
     else if (steps <= 6) with_steps(std::integral_constant<int, 6>{});
