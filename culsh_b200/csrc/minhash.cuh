@@ -100,7 +100,7 @@ __device__ __forceinline__ uint32_t min_plus5_short(uint32_t m, double a, double
 // H > 256 takes several sweeps.  Slots past H hold a = b = 0, evaluate to 0 and are never stored,
 // so the inner loop carries no predicate.
 template <int PL>
-__global__ void __launch_bounds__(MH_THREADS, PL <= 4 ? 24 : 16)
+__global__ void __launch_bounds__(MH_THREADS, PL <= 4 ? 24 : 18)
 minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ indptr,
                const uint32_t* __restrict__ A, const uint32_t* __restrict__ B, int n_rows,
                int L, int k, int NW, uint32_t* __restrict__ keys, int n_total, int row_offset) {
@@ -118,9 +118,10 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
             bd[i] = (h < H ? (double)B[h] : 0.0) + 5.0 + MH_2_52;
         }
     };
-    // the integer forms take their parameters from the doubles: these are all the loop has registers for
-    auto a_of = [&](int i) { return __double2uint_rz(ad[i]); };
-    auto b5_of = [&](int i) { return (uint64_t)(bd[i] - MH_2_52); };
+    // The integer forms take their parameters from the doubles: these are all the loop has registers for.  Added to 2^52, as bd
+    // is, an integer lies in the low bits: conversions for every 32 ids took 5 % of a row of ids from 2^20 on.
+    auto a_of = [&](int i) { return (uint32_t)__double2loint(ad[i] + MH_2_52); };
+    auto b5_of = [&](int i) { return (uint64_t)__double_as_longlong(bd[i]) - ((uint64_t)MH_2_52_HI << 32); };
     load_params(0);
 
     // the ids of a step are fetched a step ahead, the bounds of a row a row ahead
@@ -136,6 +137,7 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
         next_start = more ? indptr[row + gridDim.x] : 0;
         next_end = more ? indptr[row + gridDim.x + 1] : 0;
         const uint32_t short_col = end - start <= MH_SHORT_ROW ? MH_SHORT_COL : 0u;
+        bool shorts = false;  // the row has had ids below short_col
         for (int h0 = 0; h0 < H; h0 += 32 * PL) {
             const bool last = h0 + 32 * PL >= H;
             if (H > 32 * PL) load_params(h0);
@@ -154,6 +156,7 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
                     const bool have = lane < cnt, is_short = have && (uint32_t)mine < short_col;
                     const uint32_t m_short = __ballot_sync(0xFFFFFFFFu, is_short), m_long = __ballot_sync(0xFFFFFFFFu, have && !is_short);
                     const int n_short = __popc(m_short), n_long = __popc(m_long);
+                    shorts = shorts || n_short > 0;
                     if (have) {
                         double* const list = is_short ? ids_short : ids_long;
                         const int at = __popc((is_short ? m_short : m_long) & below);
@@ -184,7 +187,7 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
                     b[i] = b5_of(i);
                 }
                 if (__any_sync(0xFFFFFFFFu, (uint32_t)mine >= MH_FAST_COL)) {
-#pragma unroll 4
+#pragma unroll (PL <= 2 ? 4 : 2)
                     for (int s = 0; s < cnt; ++s) {
                         const uint32_t c = (uint32_t)__shfl_sync(0xFFFFFFFFu, mine, s);
 #pragma unroll
@@ -192,7 +195,7 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
                     }
                     continue;
                 }
-#pragma unroll 8
+#pragma unroll (PL <= 4 ? 8 : 4)
                 for (int s = 0; s < cnt; ++s) {
                     const uint32_t c = (uint32_t)__shfl_sync(0xFFFFFFFFu, mine, s);
 #pragma unroll
@@ -201,7 +204,7 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
             }
 #pragma unroll
             for (int i = 0; i < PL; ++i) {
-                uint32_t again = __ballot_sync(0xFFFFFFFFu, h0 + i * 32 + lane < H && m[i] < (short_col ? MH_AGAIN : 5u));
+                uint32_t again = __ballot_sync(0xFFFFFFFFu, h0 + i * 32 + lane < H && m[i] < (shorts ? MH_AGAIN : 5u));
                 while (again) {
                     const int src = __ffs(again) - 1;
                     again &= again - 1u;
