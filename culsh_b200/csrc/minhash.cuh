@@ -9,17 +9,19 @@
 #pragma once
 
 #include "common.cuh"
-#include "index_math.h"
 
 namespace culsh_b200 {
 
 constexpr uint32_t MINHASH_PRIME = 4294967291u;  // minhash/hash.cuh:17
 constexpr int MH_STEPS = 4;  // pairs of ids a turn of the loop
 // A warp is a CTA of its own: rows differ in length tenfold, and with eight warps a CTA held its place until the longest of their
-// rows was over.
+// rows was over.  Its rows lie next to one another: their bounds are one load, the ids of the next row follow those of this one,
+// and a line of ids or of keys has one user.  With rows a grid apart a row waited for its bounds and then for its ids, which short
+// rows do not cover (2M rows of 5 ids below 2^16 into 32 functions 541 us, 394 this way; eight warps a CTA, with twice the warps an SM,
+// 438; the whole pass of 2M sets of 20 to 200 ids 12,290 and 12,097).
 constexpr int MH_THREADS = 32;
-// Rows of a warp: many for what it sets up once, few for the last warps to end together, but no fewer warps than
-// MH_WARPS of an SM, eight turns (2M sets: 4 rows 4,525 us, 16 4,450, 64 4,497; 100,003: 4 rows 248, 16 269, 64 288).
+// Rows of a warp, at most (fewer than 32: a lane each for their bounds): many for what it sets up once, few for the last warps to
+// end together, but no fewer warps than MH_WARPS of an SM, eight turns (with rows a grid apart, 2M sets: 4 rows 4,525 us, 16 4,450, 64 4,497; 100,003: 4 rows 248, 16 269, 64 288).
 constexpr int MH_ROWS = 16;
 constexpr int MH_WARPS = 192;
 constexpr int MH_MAX_PER_LANE = 8;               // hashes per lane per sweep (H <= 256 in one sweep)
@@ -99,15 +101,17 @@ __device__ __forceinline__ uint32_t min_plus5_short(uint32_t m, double a, double
 // PL = hash functions per lane per sweep; a sweep covers 32*PL consecutive hash functions and
 // H > 256 takes several sweeps.  Slots past H hold a = b = 0, evaluate to 0 and are never stored,
 // so the inner loop carries no predicate.
+// Warps of an SM: as many as registers allow without spills that cost.
 template <int PL>
-__global__ void __launch_bounds__(MH_THREADS, PL <= 4 ? 24 : 18)
+__global__ void __launch_bounds__(MH_THREADS, PL <= 2 ? 32 : PL <= 4 ? 24 : 18)
 minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ indptr,
                const uint32_t* __restrict__ A, const uint32_t* __restrict__ B, int n_rows,
-               int L, int k, int NW, uint32_t* __restrict__ keys, int n_total, int row_offset) {
+               int L, int k, int NW, uint32_t* __restrict__ keys, int n_total, int row_offset, int rows) {
     const int lane = threadIdx.x & 31;
     const int H = L * k;
     const int pad_words = NW - k;  // leading zero words when 4k is not 4, 8, 16 or 32 bytes
     __shared__ __align__(16) double ids_short[34], ids_long[34];
+    __shared__ size_t key_at[32 * PL];  // word of a hash function in the first row's keys
     const uint32_t below = (1u << lane) - 1u;
     double ad[PL], bd[PL];
     auto load_params = [&](int h0) {
@@ -116,6 +120,8 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
             const int h = h0 + i * 32 + lane;
             ad[i] = h < H ? (double)A[h] : 0.0;
             bd[i] = (h < H ? (double)B[h] : 0.0) + 5.0 + MH_2_52;
+            const int t = h / k;
+            key_at[i * 32 + lane] = (size_t)t * n_total * NW + pad_words + (h - t * k);
         }
     };
     // The integer forms take their parameters from the doubles: these are all the loop has registers for.  Added to 2^52, as bd
@@ -124,18 +130,15 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
     auto b5_of = [&](int i) { return (uint64_t)__double_as_longlong(bd[i]) - ((uint64_t)MH_2_52_HI << 32); };
     load_params(0);
 
-    // the ids of a step are fetched a step ahead, the bounds of a row a row ahead
-    int start = 0, end = 0;
-    if (blockIdx.x < n_rows) {
-        start = indptr[blockIdx.x];
-        end = indptr[blockIdx.x + 1];
-    }
+    // the ids of a step are fetched a step ahead
+    const uint32_t row0 = blockIdx.x * (uint32_t)rows;
+    const int here = (int)min((uint32_t)rows, (uint32_t)n_rows - row0);
+    const int bound = lane <= here ? indptr[row0 + lane] : 0;
+    int start = __shfl_sync(0xFFFFFFFFu, bound, 0), end = __shfl_sync(0xFFFFFFFFu, bound, 1);
     int ahead = start + lane < end ? indices[start + lane] : 0;
-    int next_start, next_end;
-    walk_rows(blockIdx.x, gridDim.x, n_rows, [&](int row) {
-        const bool more = n_rows - row > (int)gridDim.x;
-        next_start = more ? indptr[row + gridDim.x] : 0;
-        next_end = more ? indptr[row + gridDim.x + 1] : 0;
+    for (int r = 0; r < here; ++r) {
+        const int row = row_offset + (int)row0 + r;
+        const int next_end = r + 1 < here ? __shfl_sync(0xFFFFFFFFu, bound, r + 2) : end;
         const uint32_t short_col = end - start <= MH_SHORT_ROW ? MH_SHORT_COL : 0u;
         bool shorts = false;  // the row has had ids below short_col
         for (int h0 = 0; h0 < H; h0 += 32 * PL) {
@@ -148,7 +151,7 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
                 const int mine = ahead;
                 // the next step's, then the row's first again for another sweep, or the next row's
                 const bool inside = base + 32 < end;
-                const int at = (inside ? base + 32 : last ? next_start : start) + lane;
+                const int at = (inside ? base + 32 : last ? end : start) + lane;
                 ahead = at < (inside || !last ? end : next_end) ? indices[at] : 0;
                 const int cnt = min(32, end - base);
                 if (!__any_sync(0xFFFFFFFFu, (uint32_t)mine >= MH_DOUBLE_COL)) {
@@ -220,24 +223,20 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
 #pragma unroll
             for (int i = 0; i < PL; ++i) {
                 int h = h0 + i * 32 + lane;
-                if (h < H) {
-                    int t = h / k, j = h - t * k;
-                    size_t item = (size_t)t * n_total + row_offset + row;
-                    keys[item * NW + pad_words + j] = __byte_perm(m[i], 0, 0x0123);
-                }
+                if (h < H) keys[key_at[i * 32 + lane] + (size_t)row * NW] = __byte_perm(m[i], 0, 0x0123);
             }
         }
-        if (end <= start) ahead = next_start + lane < next_end ? indices[next_start + lane] : 0;
+        if (end <= start) ahead = end + lane < next_end ? indices[end + lane] : 0;
         if (pad_words > 0) {
             for (int idx = lane; idx < L * pad_words; idx += 32) {
                 int t = idx / pad_words, j = idx - t * pad_words;
-                size_t item = (size_t)t * n_total + row_offset + row;
+                size_t item = (size_t)t * n_total + row;
                 keys[item * NW + j] = 0u;
             }
         }
-        start = next_start;
+        start = end;
         end = next_end;
-    });
+    }
 }
 
 inline void launch_minhash(const CtxPtr& c, cudaStream_t stream, const int32_t* indices,
@@ -245,14 +244,15 @@ inline void launch_minhash(const CtxPtr& c, cudaStream_t stream, const int32_t* 
                            int L, int k, const KeySpec& ks, uint32_t* keys, int n_total,
                            int row_offset) {
     if (n_rows == 0) return;
-    const size_t blocks = std::min<size_t>(n_rows, std::max<size_t>(ceil_div((size_t)n_rows, MH_ROWS), (size_t)c->sm_count * MH_WARPS));
+    const int rows = (int)std::min<size_t>(MH_ROWS, ceil_div((size_t)n_rows, (size_t)c->sm_count * MH_WARPS));
+    const size_t blocks = ceil_div((size_t)n_rows, (size_t)rows);
     const int H = L * k;
     const int sweeps = (int)ceil_div(H, 32 * MH_MAX_PER_LANE);
     const int per_lane = (int)ceil_div(H, 32 * sweeps);  // 1..MH_MAX_PER_LANE
 #define CULSH_MH_CASE(PLV)                                                                      \
     case PLV:                                                                                   \
         minhash_kernel<PLV><<<(unsigned)blocks, MH_THREADS, 0, stream>>>(                       \
-            indices, indptr, A, B, n_rows, L, k, ks.key_words, keys, n_total, row_offset);      \
+            indices, indptr, A, B, n_rows, L, k, ks.key_words, keys, n_total, row_offset, rows); \
         break;
     switch (per_lane) {
         CULSH_MH_CASE(1) CULSH_MH_CASE(2) CULSH_MH_CASE(3) CULSH_MH_CASE(4)

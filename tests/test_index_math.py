@@ -50,8 +50,8 @@ int main() {
 
 
 def test_row_walks_end(tmp_path):
-    """148 CTAs of 8 warps step by 1,184 rows: the last step of n = 2^31 - 1 rows ends beyond 2^31.  MinHash, with up to 16 rows
-    a warp, steps by a sixteenth of the rows."""
+    """148 CTAs of 8 warps step by 1,184 rows: the last step of n = 2^31 - 1 rows ends beyond 2^31.  So does one of a grid that
+    steps by a sixteenth of the rows."""
     top = (1 << 31) - 1
     cases = [(0, 1, 0), (0, 1184, 1), (5, 1184, 5), (7, 1184, 10_000), (1183, 1184, top), (0, 1184, top),
              (top - 1, 37_888, top), (top, 1184, top), (100, 37_888, top - 900),
