@@ -130,6 +130,7 @@ struct Ctx {
     cudaEvent_t ev[8] = {};
     cudaEvent_t ev_pass[2] = {};      // around the scatter launch of the last radix pass
     cudaEvent_t ev_dedupe[4] = {};    // around the window / bitmap dedupe launch of the last query batch and around its copy to the result
+    cudaEvent_t counted = nullptr;    // behind the raw counts of the last set of queries
     cudaEvent_t copy_done[2] = {};
     cudaEvent_t chunk_free[2] = {};
     uint64_t* pinned = nullptr;       // 64 x u64 words of pinned host memory: read_words' first, see HostSlot
@@ -157,6 +158,7 @@ struct Ctx {
         for (auto& e : ev) if (e) cudaEventDestroy(e);
         for (auto& e : ev_pass) if (e) cudaEventDestroy(e);
         for (auto& e : ev_dedupe) if (e) cudaEventDestroy(e);
+        if (counted) cudaEventDestroy(counted);
         for (auto& e : copy_done) if (e) cudaEventDestroy(e);
         for (auto& e : chunk_free) if (e) cudaEventDestroy(e);
         if (copy_stream) cudaStreamSynchronize(copy_stream);

@@ -91,8 +91,8 @@ def test_small_sets_are_gathered_once():
     launches = core.last_stats()["launches"]
     assert int(small.get_counts().max()) < 256
     got = core.query_float(mixed, 100, ix)
-    # the windows, the second scan of the counts and the copy of the pieces
-    assert core.last_stats()["launches"] == launches + 3
+    # the windows and the copy of the pieces
+    assert core.last_stats()["launches"] == launches + 2
     counts = got.get_counts()
     assert (counts[::10] >= 3000).all()
     for q in (1, 10, 55):
