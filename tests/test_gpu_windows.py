@@ -87,3 +87,35 @@ def test_result_inside_its_raw_array(bounce, monkeypatch):
     got = m.query(Q)
     for f in ("get_offsets", "get_indices", "get_counts"):
         assert np.array_equal(getattr(got, f)(), getattr(want, f)())
+
+
+def test_result_inside_its_raw_array_when_memory_is_short():
+    """No memory for a second array of the result's size, and enough for the buffer."""
+    import torch
+    import culsh_b200 as culsh
+    from culsh_b200 import _culsh_core as core_mod
+    n, L, k, nq = 1_000_000, 4, 2, 200
+    g = torch.Generator("cuda").manual_seed(4)
+    X = torch.randn(n, 8, device="cuda", generator=g)
+    Q = torch.randn(nq, 8, device="cuda", generator=g)
+    core = core_mod.RPLSHCore(L, k, 2)
+    m = culsh.RPLSH(L, k, seed=2).fit(X)
+    want = m.query(Q)
+    offsets, ids = want.get_offsets(), want.get_indices()
+    stats = core.last_stats()
+    raw, unique, launches = 4 * stats["raw_candidates"], 4 * stats["unique_candidates"], stats["launches"]
+    assert unique > 400 << 20
+    del want, X
+    core.trim_scratch(0)
+    torch.cuda.empty_cache()
+    spare = raw + (200 << 20)
+    ballast = torch.empty(torch.cuda.mem_get_info()[0] - spare, dtype=torch.uint8, device="cuda")
+    try:
+        got = m.query(Q)
+        assert core.last_stats()["launches"] > launches
+    finally:
+        del ballast
+        torch.cuda.empty_cache()
+    assert np.array_equal(got.get_offsets(), offsets) and np.array_equal(got.get_indices(), ids)
+    del got
+    core.trim_scratch(0)
