@@ -108,7 +108,7 @@ struct ParamKey {
 enum ScratchSlot {
     SL_STAGE0, SL_STAGE1, SL_CSR_INDPTR, SL_CSR_INDICES, SL_KEYS0, SL_KEYS1, SL_VALS, SL_HEADS,
     SL_STATUS, SL_COUNTER, SL_TILE_HEADS, SL_TILE_BASE, SL_SCAN, SL_RAW_CNT, SL_RAW_OFF,
-    SL_BIG_LIST, SL_TMP, SL_QKEYS, SL_QOVF, SL_MISC0, SL_MISC1, SL_MISC2, SL_CHAIN,
+    SL_BIG_LIST, SL_TMP, SL_QKEYS, SL_QOVF, SL_MISC0, SL_MISC1, SL_MISC2, SL_PIECES,
     SL_SLICES, SL_BOUNDS, SL_COUNT
 };
 
@@ -365,10 +365,8 @@ struct HashRange {
 
 // Device-side self-check word: kernels OR a code into it instead of trapping.
 enum DeviceErrorBits : int {
-    DEV_ERR_LOOKBACK_TIMEOUT = 1,  // a bounded wait on another tile's status ran out
     DEV_ERR_NARROW_OVERFLOW = 2,   // a p-stable hash value does not fit the narrow key width
-    DEV_ERR_MBAR_TIMEOUT = 4,      // a bounded mbarrier wait ran out (tensor-core projection)
-    DEV_ERR_RANGE = 8              // an index outside its array was skipped
+    DEV_ERR_MBAR_TIMEOUT = 4       // a bounded mbarrier wait ran out (tensor-core projection)
 };
 
 // A launch in clusters of `ctas` CTAs each; `grid` is a multiple of that.

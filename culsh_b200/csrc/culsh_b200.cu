@@ -145,11 +145,8 @@ void reset_error_word(const CtxPtr& c) {
 int read_error_word(const CtxPtr& c) { return c->seen_error; }
 
 void check_error_word(int e) {
-    if (e & DEV_ERR_LOOKBACK_TIMEOUT)
-        fail(CULSH_ERR_INTERNAL, "radix sort: a bounded wait on a preceding tile ran out");
     if (e & DEV_ERR_MBAR_TIMEOUT)
         fail(CULSH_ERR_INTERNAL, "projection: a bounded wait on a copy/MMA barrier ran out");
-    if (e & DEV_ERR_RANGE) fail(CULSH_ERR_INTERNAL, "a kernel skipped an out-of-range index");
 }
 
 // -----------------------------------------------------------------------------------------
@@ -717,7 +714,8 @@ int bitmap_window_bits(const CtxPtr& c, int n_rows) {
     return (int)std::min(want, cap);
 }
 
-// Tuning knobs of the window kernel, read from the environment at every call (tests vary them):
+// Tuning knobs of the window kernel, read from the environment at every call (tests vary them).  Their names are those of the
+// kernel before it, which chained the counts of its CTAs.
 //   CULSH_CHAIN_BITS    rows per window at most (default WINDOW_ROWS); the row range is cut into the fewest such
 //                       windows, each a multiple of 4096 rows
 //   CULSH_CHAIN_THREADS threads per CTA: 256, 384 (default) or 512
@@ -867,7 +865,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         room = c->slot_cap[SL_TMP] / sizeof(int32_t);
         launch_small(self_join ? dedupe_small_kernel<SMALL_MAX, true> : dedupe_small_kernel<SMALL_MAX, false>, 0, room);
         if (ahead_windows) {
-            pieces.reserve(c, SL_CHAIN, (size_t)n_q * n_win);
+            pieces.reserve(c, SL_PIECES, (size_t)n_q * n_win);
             if (c->profiling) cudaEventRecord(c->ev_dedupe[0], s);
             launch_windows((size_t)n_q * n_win, n_big, room);
             if (c->profiling) cudaEventRecord(c->ev_dedupe[1], s);
@@ -880,7 +878,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
     }
     const uint64_t raw_total = c->pinned[HS_RAW];
     const uint32_t nb = slot_words(c, HS_RAW)[0], nm = slot_words(c, HS_RAW)[1], n_long = slot_words(c, HS_RAW)[2];
-    c->seen_error = (int)slot_words(c, HS_RAW)[3];  // what follows has no waits that could run out
+    c->seen_error = (int)slot_words(c, HS_RAW)[3];  // what follows reports nothing
     tr.lap("count+scan+sync");
     if (raw_total > raw_limit) return false;
     const bool fits = ahead && raw_total <= room, done = fits && nm == 0 && (nb == 0 || ahead_windows);
@@ -936,7 +934,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
             KERNEL_CHECK();
         }
         if (windows) {
-            pieces.reserve(c, SL_CHAIN, n_pieces);
+            pieces.reserve(c, SL_PIECES, n_pieces);
             // list slices per window, precomputed when the table is small enough (<= 256 MB)
             if (env_long("CULSH_CHAIN_SLICES", 1) && n_win > 1 && n_pieces * (size_t)L <= ((size_t)32 << 20)) {
                 slices.reserve(c, SL_SLICES, n_pieces * (size_t)L);
@@ -1164,7 +1162,7 @@ void fit_query_dense(culsh_handle* h, int family, const T* X, int n, int d, int 
     tm.mark();
     query_from_matched(*ix, self_bounds(*ix, bounds.p), true, *res, tm);
     h->ctx->stats.gather_ms = tm.between(0, 1);
-    check_error_word(read_error_word(h->ctx));  // the gather's bounded waits report here
+    check_error_word(read_error_word(h->ctx));  // the projection's bounded waits report there
     *out = res.release();
 }
 
@@ -1482,7 +1480,7 @@ int culsh_minhash_fit_query(culsh_handle* h, const int32_t* indices, const int32
         tm.mark();
         query_from_matched(*ix, self_bounds(*ix, bounds.p), true, *res, tm);
         h->ctx->stats.gather_ms = tm.between(0, 1);
-        check_error_word(read_error_word(h->ctx));  // the gather's bounded waits report here
+        check_error_word(read_error_word(h->ctx));  // the projection's bounded waits report there
         *out = res.release();
     });
 }
