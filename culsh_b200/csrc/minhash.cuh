@@ -18,10 +18,11 @@ constexpr int MH_STEPS = 4;  // pairs of ids a turn of the loop
 // rows was over.  Its rows lie next to one another: their bounds are one load, the ids of the next row follow those of this one,
 // and a line of ids or of keys has one user.  With rows a grid apart a row waited for its bounds and then for its ids, which short
 // rows do not cover (2M rows of 5 ids below 2^16 into 32 functions 541 us, 394 this way; eight warps a CTA, with twice the warps an SM,
-// 438; the whole pass of 2M sets of 20 to 200 ids 12,290 and 12,097).
+// 438.  2M of 20 to 200 ids into 128 with 10,000 queries 4,450 and 4,244).
 constexpr int MH_THREADS = 32;
 // Rows of a warp, at most (fewer than 32: a lane each for their bounds): many for what it sets up once, few for the last warps to
-// end together, but no fewer warps than MH_WARPS of an SM, eight turns (with rows a grid apart, 2M sets: 4 rows 4,525 us, 16 4,450, 64 4,497; 100,003: 4 rows 248, 16 269, 64 288).
+// end together, but no fewer warps than MH_WARPS of an SM, eight turns (with rows a grid apart, 2M sets: 4 rows 4,525 us, 16
+// 4,450, 64 4,497; 100,003: 4 rows 248, 16 269, 64 288).
 constexpr int MH_ROWS = 16;
 constexpr int MH_WARPS = 192;
 constexpr int MH_MAX_PER_LANE = 8;               // hashes per lane per sweep (H <= 256 in one sweep)

@@ -15,7 +15,7 @@
 // A row of a few dozen features is over in two or three stages of a microsecond, and what surrounds them weighs as much: a CTA
 // then stays for many row blocks of its group of columns (see launch_project_f64) and, for sign bits, fetches the first stages of
 // the next block before it packs the keys of this one.  The bits of a step of eight columns are one byte a row, made from ballots.
-// 200,003 x 100 rows, 224 columns: 0.97 ms on the CUDA cores, with one block of rows a CTA and a branch before every instruction 0.46 (with 2,001 queries), now 0.367.
+// 200,003 x 100 rows, 224 columns: 0.97 ms on the CUDA cores, with one block of rows a CTA and a branch before every instruction 0.46 (with 2,001 queries), with CTAs that stay 0.367, now 0.353.
 #pragma once
 
 #include "common.cuh"
