@@ -455,7 +455,9 @@ def config_of(wl, spec):
 NCU_TRAFFIC = {
     ("c2", 1_000_000): {
         "sort": 264_078_336 + 203_595_776,     # profiles/radix_scatter_kernel_c2_1M.md (second pass)
-        "hash": 512_630_784 + 113_564_928,     # profiles/project_tc_kernel_c2_1M.md
+        "hash": 512_648_448 + 114_698_240,     # profiles/project_tc_kernel_c2_1M.md
+        # profiles/dedupe_window_kernel_c2_1M.md: the dedupe launch and the copy to the result
+        "gather": 282_976_768 + 681_946_368 + 738_435_328 + 685_722_368,
     },
 }
 
