@@ -860,9 +860,12 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
     // A self-join's rows for the windows need their lists in another form, the sort path its number of queries.
     const bool ahead = n_q <= AHEAD_QUERIES;
     const bool ahead_windows = ahead && may_window && !self_join && mid_max == 0 && (size_t)n_q * n_win <= AHEAD_PIECES;
+    // With the windows ahead nothing is left that the counts could ask for, as a rule, and the gather of a small self-join is over before
+    // the host has launched the scan of the new counts (1,000 rows 227 and 224 us): that goes ahead, too, and the host waits for it all.
+    const bool whole = ahead_windows || (ahead && self_join);
     uint64_t room = 0;
     if (ahead) {
-        CU_CHECK(cudaEventRecord(c->counted, s));
+        if (!whole) CU_CHECK(cudaEventRecord(c->counted, s));
         tmp.reserve(c, SL_TMP, AHEAD_IDS);
         room = c->slot_cap[SL_TMP] / sizeof(int32_t);
         launch_small(self_join ? dedupe_small_kernel<SMALL_MAX, true> : dedupe_small_kernel<SMALL_MAX, false>, 0, room);
@@ -872,12 +875,10 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
             launch_windows((size_t)n_q * n_win, n_big, room);
             if (c->profiling) cudaEventRecord(c->ev_dedupe[1], s);
         }
-        // the gather of a small self-join is over before the host has launched the scan (1,000 rows 227 and 224 us)
-        if (self_join) scan_unique();
-        CU_CHECK(cudaEventSynchronize(c->counted));
-    } else {
-        CU_CHECK(cudaStreamSynchronize(s));
+        if (whole) scan_unique();
     }
+    if (ahead && !whole) CU_CHECK(cudaEventSynchronize(c->counted));
+    else CU_CHECK(cudaStreamSynchronize(s));
     const uint64_t raw_total = c->pinned[HS_RAW];
     const uint32_t nb = slot_words(c, HS_RAW)[0], nm = slot_words(c, HS_RAW)[1], n_long = slot_words(c, HS_RAW)[2];
     c->seen_error = (int)slot_words(c, HS_RAW)[3];  // what follows reports nothing
@@ -902,10 +903,11 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
     const bool windows = nb && may_window && (uint64_t)nb * (uint64_t)n_win < (1ull << 31);
     const size_t n_pieces = (size_t)nb * n_win;
     const uint32_t n_other = (uint32_t)n_q - nb - nm;  // queries on the warp path (incl. empty ones)
-    if (done) {
-        if (!self_join) scan_unique();
+    if (done && !whole) {
+        scan_unique();
         CU_CHECK(cudaStreamSynchronize(s));
-    } else {
+    }
+    if (!done) {
         // The ids of a query land in its raw span first.  A large such array is a block of the result's kind: it goes
         // back when the call is done, and takes the result's place when there is no memory for both.
         const bool block = windows && raw_total * sizeof(int32_t) >= BIG_BLOCK_MIN;
