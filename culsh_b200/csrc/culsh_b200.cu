@@ -716,29 +716,40 @@ int bitmap_window_bits(const CtxPtr& c, int n_rows) {
 
 // Tuning knobs of the window kernel, read from the environment at every call (tests vary them).  Their names are those of the
 // kernel before it, which chained the counts of its CTAs.
-//   CULSH_CHAIN_BITS    rows per window at most (default WINDOW_ROWS); the row range is cut into the fewest such
+//   CULSH_CHAIN_BITS    rows per window at most (default: what windows_for gives); the row range is cut into the fewest such
 //                       windows, each a multiple of 4096 rows
 //   CULSH_CHAIN_THREADS threads per CTA: 256, 384 (default) or 512
 //   CULSH_CHAIN_LOADS   loads in flight per lane in the list walk: 4, 8 (default) or 16
-//   CULSH_CHAIN_SLICES  0 = CTAs search their list slices themselves (default 1: precomputed)
+//   CULSH_CHAIN_SLICES  0 = CTAs search their list slices themselves, 1 = precomputed (default: from WINDOW_SEARCH CTAs on)
 //   CULSH_COMPACT_BOUNCE ids of the buffer through which a result is brought together inside its raw array
 //                       (default 0: only if there is no memory for a second array)
-// The line to the form of a CTA for each query is older than this kernel, which was the faster one beyond it, too, wherever it was
-// measured (3M rows x 16 tables, one query of 49,000 entries 84 us in nine windows and 184, 2,000 of 15,000 579 and 1,166).
-constexpr int MAX_WINDOWS = 8;
 // 43 KB of bitmap: five CTAs of 384 threads share an SM (1M rows: three windows 820 us, four of 254,000 rows 889, two of 504,000
 // 909; 2M rows of sparser sets 670, 740, 750)
 constexpr long WINDOW_ROWS = 344064;
+// A few large sets leave most of the chip idle in such windows, and each of their CTAs takes long (1M rows, one set of 21,000
+// entries in 32 lists: three windows 16 us, 61 of them 8): smaller ones then, down to WINDOW_MIN_ROWS.
+constexpr long WINDOW_MIN_ROWS = 16384;
+constexpr size_t WINDOW_SEARCH = 512;  // CTAs that search their slices themselves: a launch less
 inline long env_long(const char* name, long dflt) {
     const char* e = getenv(name);
     return e && *e ? atol(e) : dflt;
 }
-int window_bits(int n_rows, int* n_win) {
-    const size_t cap_bits = std::max<size_t>(4096, (size_t)env_long("CULSH_CHAIN_BITS", WINDOW_ROWS) / 4096 * 4096);
+struct Windows {
+    int bits, n;
+};
+// Windows for `n_sets` large sets: as many rows as fit, but smaller ones as long as there are fewer than `ctas` of them in all.
+// However many there are, they are faster than a CTA for each set that visits windows of 2^20 rows in turn.  Whole calls, that way and
+// this: 3M rows x 16 tables, one set of 123,000 ids 290 and 78 us, 1,024 sets of 93,000 1,509 and 641; 8M x 8, 64 of
+// 380,000 2,492 and 270; 40M x 4, one of 9.8M 20,600 and 170, 256 of 5M 40,800 and 10,400.
+Windows windows_for(int n_rows, size_t n_sets, size_t ctas) {
+    const long env = env_long("CULSH_CHAIN_BITS", 0);
+    const size_t cap_bits = std::max<size_t>(4096, (size_t)(env > 0 ? env : WINDOW_ROWS) / 4096 * 4096);
     const size_t n = (size_t)std::max(n_rows, 1);
-    const size_t wins = ceil_div(n, cap_bits);
-    *n_win = (int)std::min<size_t>(wins, 1u << 20);
-    return (int)(ceil_div(ceil_div(n, wins), (size_t)4096) * 4096);
+    size_t wins = ceil_div(n, cap_bits);
+    if (env <= 0)
+        wins = std::max(wins, std::min(ctas / std::max<size_t>(n_sets, 1), ceil_div(n, (size_t)WINDOW_MIN_ROWS)));
+    const size_t bits = ceil_div(ceil_div(n, wins), (size_t)4096) * 4096;
+    return Windows{(int)bits, (int)ceil_div(n, bits)};
 }
 
 // Where the raw counts of a set of queries go.
@@ -759,6 +770,7 @@ struct RawCounts {
 constexpr int AHEAD_QUERIES = 4096;
 constexpr size_t AHEAD_IDS = (size_t)1 << 20;  // 4 MB that every handle has then
 constexpr int AHEAD_PIECES = 64;  // CTAs of the window kernel that may turn out to have nothing to do
+constexpr int WINDOW_CTAS = 2;    // for each SM: below that the windows of a few large sets are cut smaller
 
 // The result inside its raw array, when there is no memory for a second one: what a run of queries has goes
 // through a buffer to where it belongs, at or before where it was and before what the next run has.
@@ -818,9 +830,9 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         exclusive_scan<uint64_t, uint64_t>(s, raw_cnt.p, n_q, raw_off.p, scratch.p, host_raw);
     }
     // Large sets: a CTA for each (query, window of the rows) where that is a few windows, else one for each query.
-    int n_win = 1;
-    const int cbits = window_bits(ix.n, &n_win);
-    const bool may_window = n_win <= MAX_WINDOWS && L <= CW_MAX_L && window_smem_bytes(cbits) + 1024 <= c->smem_optin;
+    const bool ahead = n_q <= AHEAD_QUERIES;
+    Windows win = windows_for(ix.n, (size_t)n_q, ahead ? (size_t)AHEAD_PIECES : 0);
+    const bool may_window = L <= CW_MAX_L && window_smem_bytes(win.bits) + 1024 <= c->smem_optin;
     Scratch<int32_t> tmp;
     DevBuf<int32_t> raw_ids;
     Scratch<uint2> pieces;
@@ -834,11 +846,11 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         auto launch = [&](auto nt_tag, auto mk_tag) {
             constexpr int NT = decltype(nt_tag)::value;
             constexpr int MK = decltype(mk_tag)::value;
-            const size_t smem = window_smem_bytes(cbits);
+            const size_t smem = window_smem_bytes(win.bits);
             auto kern = dedupe_window_kernel<NT, MK>;
             CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-            kern<<<(unsigned)n_ctas, NT, smem, s>>>(big_list.p, bounds, ix.cand.p, raw_off.p, L, ix.n, cbits, n_win, self_join,
+            kern<<<(unsigned)n_ctas, NT, smem, s>>>(big_list.p, bounds, ix.cand.p, raw_off.p, L, ix.n, win.bits, win.n, self_join,
                                                     slices.p, n_slots, room, tmp.p, pieces.p,
                                                     reinterpret_cast<unsigned long long*>(out.counts.p));
             KERNEL_CHECK();
@@ -858,8 +870,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         exclusive_scan<uint64_t, uint64_t>(s, out.counts.p, n_q, out.offsets.p, scratch.p, host_words(c, HS_UNIQUE, nullptr, 0));
     };
     // A self-join's rows for the windows need their lists in another form, the sort path its number of queries.
-    const bool ahead = n_q <= AHEAD_QUERIES;
-    const bool ahead_windows = ahead && may_window && !self_join && mid_max == 0 && (size_t)n_q * n_win <= AHEAD_PIECES;
+    const bool ahead_windows = ahead && may_window && !self_join && mid_max == 0 && (size_t)n_q * win.n <= AHEAD_PIECES;
     // With the windows ahead nothing is left that the counts could ask for, as a rule, and the gather of a small self-join is over before
     // the host has launched the scan of the new counts (1,000 rows 227 and 224 us): that goes ahead, too, and the host waits for it all.
     const bool whole = ahead_windows || (ahead && self_join);
@@ -870,9 +881,9 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         room = c->slot_cap[SL_TMP] / sizeof(int32_t);
         launch_small(self_join ? dedupe_small_kernel<SMALL_MAX, true> : dedupe_small_kernel<SMALL_MAX, false>, 0, room);
         if (ahead_windows) {
-            pieces.reserve(c, SL_PIECES, (size_t)n_q * n_win);
+            pieces.reserve(c, SL_PIECES, (size_t)n_q * win.n);
             if (c->profiling) cudaEventRecord(c->ev_dedupe[0], s);
-            launch_windows((size_t)n_q * n_win, n_big, room);
+            launch_windows((size_t)n_q * win.n, n_big, room);
             if (c->profiling) cudaEventRecord(c->ev_dedupe[1], s);
         }
         if (whole) scan_unique();
@@ -900,8 +911,9 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         CU_CHECK(cudaStreamSynchronize(s));
         return true;
     }
-    const bool windows = nb && may_window && (uint64_t)nb * (uint64_t)n_win < (1ull << 31);
-    const size_t n_pieces = (size_t)nb * n_win;
+    if (!done) win = windows_for(ix.n, nb, (size_t)WINDOW_CTAS * c->sm_count);  // what went ahead stays as it is
+    const bool windows = nb && may_window && (uint64_t)nb * (uint64_t)win.n < (1ull << 31);
+    const size_t n_pieces = (size_t)nb * win.n;
     const uint32_t n_other = (uint32_t)n_q - nb - nm;  // queries on the warp path (incl. empty ones)
     if (done && !whole) {
         scan_unique();
@@ -940,10 +952,11 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         if (windows) {
             pieces.reserve(c, SL_PIECES, n_pieces);
             // list slices per window, precomputed when the table is small enough (<= 256 MB)
-            if (env_long("CULSH_CHAIN_SLICES", 1) && n_win > 1 && n_pieces * (size_t)L <= ((size_t)32 << 20)) {
+            const long pre = env_long("CULSH_CHAIN_SLICES", n_pieces > WINDOW_SEARCH);
+            if (pre && win.n > 1 && n_pieces * (size_t)L <= ((size_t)32 << 20)) {
                 slices.reserve(c, SL_SLICES, n_pieces * (size_t)L);
                 slice_lists_kernel<<<(unsigned)ceil_div(n_pieces * (size_t)L, 256), 256, 0, s>>>(
-                    big_list.p, bounds, ix.cand.p, (int)nb, L, cbits, n_win, slices.p);
+                    big_list.p, bounds, ix.cand.p, (int)nb, L, win.bits, win.n, slices.p);
                 KERNEL_CHECK();
             }
             if (c->profiling) cudaEventRecord(c->ev_dedupe[0], s);
@@ -976,7 +989,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
             KERNEL_CHECK();
         }
         if (windows) {
-            compact_windows_kernel<<<(unsigned)n_pieces, 256, 0, s>>>(big_list.p, tmp.p, raw_off.p, pieces.p, out.offsets.p, n_win,
+            compact_windows_kernel<<<(unsigned)n_pieces, 256, 0, s>>>(big_list.p, tmp.p, raw_off.p, pieces.p, out.offsets.p, win.n,
                                                                      (uint32_t)q_lo, (uint32_t)q_hi, first, dst);
             KERNEL_CHECK();
         }

@@ -851,21 +851,56 @@ inline size_t window_smem_bytes(int window_bits) {
     return (size_t)window_bits / 8 + (3 * CW_MAX_L + 1) * sizeof(int);  // bitmap, lists
 }
 
-// First position p in [lo, hi) with a[p] >= target (hi if there is none).  Called by a full warp.
-__device__ __forceinline__ int warp_lower_bound(const int32_t* __restrict__ a, int lo, int hi, int32_t target,
-                                                int lane) {
-    while (hi - lo > 32) {
-        const int len = hi - lo;
-        const int p = lo + (int)(((long long)(lane + 1) * len) / 33);  // 32 distinct probes inside (lo, hi)
-        const uint32_t below = __ballot_sync(0xFFFFFFFFu, a[p] < target);  // lanes 0..c-1
-        const int c = __popc(below);
-        const int p_prev = __shfl_sync(0xFFFFFFFFu, p, max(c - 1, 0));
-        const int p_next = __shfl_sync(0xFFFFFFFFu, p, min(c, 31));
-        if (c > 0) lo = p_prev + 1;
-        if (c < 32) hi = p_next;
+// Cuts the ascending lists [s_lo[t], s_we[t]) of `cand` down to their slices in [win_lo, win_hi); an open side of the window
+// (the first one's lower, the last one's upper) cuts nothing.  Eight lanes take a (list, side) and look at eight places a step,
+// and with two of them in turn a warp has eight searches in flight: what bounds a CTA that has few of them is how many reads wait for
+// one another.  Called
+// by all threads, with a barrier before and behind.
+template <int NT>
+__device__ __forceinline__ void cut_lists(const int32_t* __restrict__ cand, int* __restrict__ s_lo, int* __restrict__ s_we, int L,
+                                          int win_lo, int win_hi, bool open_lo, bool open_hi) {
+    constexpr int GROUPS = NT / 8;  // a multiple of four: the two sides of a list are in one warp
+    const int lane = threadIdx.x & 31, at = threadIdx.x & 7, group = threadIdx.x >> 3, shift = lane & 24;
+    for (int p0 = 0; p0 < 2 * L; p0 += 2 * GROUPS) {
+        int lo[2], hi[2], target[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int p = p0 + u * GROUPS + group, t = p >> 1;
+            const bool upper = p & 1, have = p < 2 * L;
+            lo[u] = have ? s_lo[t] : 0;
+            hi[u] = have ? s_we[t] : 0;
+            target[u] = upper ? win_hi : win_lo;
+            if (!upper && open_lo) hi[u] = lo[u];
+            if (upper && open_hi) lo[u] = hi[u];
+        }
+        while (__any_sync(0xFFFFFFFFu, hi[0] - lo[0] > 8 || hi[1] - lo[1] > 8)) {
+            int32_t v[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int len = hi[u] - lo[u];
+                v[u] = len > 8 ? cand[lo[u] + (at + 1) * (len / 9)] : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int len = hi[u] - lo[u], step = len / 9;
+                const int c = __popc((__ballot_sync(0xFFFFFFFFu, len > 8 && v[u] < target[u]) >> shift) & 0xFFu);  // lanes 0 .. c - 1
+                if (len > 8) {
+                    if (c < 8) hi[u] = lo[u] + (c + 1) * step;
+                    if (c > 0) lo[u] += c * step + 1;
+                }
+            }
+        }
+        int32_t v[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) v[u] = at < hi[u] - lo[u] ? cand[lo[u] + at] : 0;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int c = __popc((__ballot_sync(0xFFFFFFFFu, at < hi[u] - lo[u] && v[u] < target[u]) >> shift) & 0xFFu);
+            const int p = p0 + u * GROUPS + group;
+            if (at == 0 && p < 2 * L) ((p & 1) ? s_we : s_lo)[p >> 1] = lo[u] + c;
+        }
+        __syncwarp();
     }
-    const bool below = lo + lane < hi && a[lo + lane] < target;
-    return lo + __popc(__ballot_sync(0xFFFFFFFFu, below));
 }
 
 // Walk over the Lg lists [s_lo[t], s_lo[t] + len_t) laid end to end (s_pre[t] = exclusive prefix
@@ -945,7 +980,7 @@ slice_lists_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds, con
 // pieces[b * n_win + w]: x = where the piece starts inside the query's raw span, y = its ids.  A launch whose counts the
 // host has not seen covers all queries: n_big says how many there are to do, and `room` is as in dedupe_small_kernel.
 template <int NT, int MK>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, 1920 / NT)  // cut_lists would take it to 37 registers and to four CTAs of 384 threads an SM
 dedupe_window_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds, const int32_t* __restrict__ cand,
                      const uint64_t* __restrict__ raw_off, int L, int n_rows, int window_bits, int n_win, bool self_join,
                      const int2* __restrict__ slices /* or null */, const uint32_t* __restrict__ n_big /* or null: all */, uint64_t room,
@@ -985,14 +1020,7 @@ dedupe_window_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds, c
     if (!slices && n_win > 1) {
         if (tid < L) { s_lo[tid] = mine.x; s_we[tid] = mine.y; }
         __syncthreads();
-        for (int t = warp; t < L; t += NWARP) {
-            const int lo = s_lo[t], we = s_we[t];
-            if (lo >= we) continue;
-            int a = lo, b = we;
-            if (w > 0) a = warp_lower_bound(cand, lo, we, win_lo, lane);
-            if (w < n_win - 1) b = warp_lower_bound(cand, a, we, win_hi, lane);
-            if (lane == 0) { s_lo[t] = a; s_we[t] = b; }
-        }
+        cut_lists<NT>(cand, s_lo, s_we, L, win_lo, win_hi, w == 0, w == n_win - 1);
         __syncthreads();
         if (tid < L) mine = make_int2(s_lo[tid], s_we[tid]);
     }
@@ -1115,8 +1143,9 @@ compact_windows_kernel(const uint32_t* __restrict__ big_list, const int32_t* __r
     const int slot = blockIdx.x / n_win, w = blockIdx.x - slot * n_win;
     const uint32_t q = big_list[slot];
     if (q < q_lo || q >= q_hi) return;
-    uint64_t to = offsets[q] - first;
-    for (int i = 0; i < w; ++i) to += pieces[slot * (size_t)n_win + i].y;
+    uint32_t before = 0;  // ids of the pieces before this one: at most as many as rows
+    for (int i = threadIdx.x & 31; i < w; i += 32) before += pieces[slot * (size_t)n_win + i].y;
+    const uint64_t to = offsets[q] - first + __reduce_add_sync(0xFFFFFFFFu, before);
     const uint2 p = pieces[blockIdx.x];
     const int32_t* src = tmp + raw_off[q] + p.x;
     int32_t* dst = out + to;

@@ -119,3 +119,27 @@ def test_result_inside_its_raw_array_when_memory_is_short():
     assert np.array_equal(got.get_offsets(), offsets) and np.array_equal(got.get_indices(), ids)
     del got
     core.trim_scratch(0)
+
+
+@pytest.mark.parametrize("threads", [256, 384, 512])
+@pytest.mark.parametrize("L,n,bits", [(1, 20_000, 4096), (50, 20_000, 4096), (256, 9_000, 4096), (3, 300_000, 4096), (40, 300_000, None)])
+def test_lists_cut_by_their_own_windows(L, n, bits, threads, monkeypatch):
+    """Few sets: CTAs cut the lists themselves, more lists than they take at once, and more windows than sixty-four."""
+    import culsh_b200 as culsh
+    from culsh_b200 import _culsh_core as core_mod
+    if bits:
+        monkeypatch.setenv("CULSH_CHAIN_BITS", str(bits))
+    monkeypatch.setenv("CULSH_CHAIN_THREADS", str(threads))
+    rng = np.random.default_rng(L)
+    d, k = 6, 5
+    X = rng.standard_normal((n, d)).astype(np.float32)
+    X[rng.permutation(n)[:1500]] = X[7]
+    Q = np.concatenate([X[7:9], 1e3 * X[-1:]]).astype(np.float32)
+    core = core_mod.RPLSHCore(L, k, 3)
+    m = culsh.RPLSH(L, k, seed=3).fit(X)
+    sig = lambda Y: core.hash(Y, m.index).transpose(1, 0, 2)  # noqa: E731
+    want = _lists(m, sig(X), sig(Q), n, L)
+    assert max(len(w) for w in want) >= 1500
+    _assert_lists(m.query(Q), want)
+    for q in range(len(Q)):
+        _assert_lists(m.query(Q[q:q + 1]), want[q:q + 1])
