@@ -10,6 +10,7 @@
 #include "query.cuh"
 #include "radix_sort.cuh"
 #include "row_norm.cuh"
+#include "splitter_sort.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -503,7 +504,9 @@ struct SortBuffers {
         keys[1].reserve(c, SL_KEYS1, items * ks.key_words);
         vals_out.alloc(c, items);
         vals_tmp.reserve(c, SL_VALS, items);
-        tile_hist.reserve(c, SL_STATUS, radix_sort_tile_words(n, L, ks.key_words));
+        size_t words = radix_sort_tile_words(n, L, ks.key_words);
+        if (splitters_can(n, ks.key_words)) words = std::max(words, splitter_plan(n, L).words);
+        tile_hist.reserve(c, SL_STATUS, words);
     }
     // the last pass must write the row ids into vals_out
     void set_final(int buf) {
@@ -560,7 +563,9 @@ int build_index(culsh_index& ix, SortBuffers& sb, Scratch<uint32_t>* bounds, Sta
     // of the values itself, and the bucket arrays are made for as many buckets as there are items (1,000 rows x 8
     // tables: two waits less of seven in a self-join).
     const int* check = nullptr;
-    if (may_compress && radix_sort_is_small(c, n, L, NW, true)) {
+    if (may_compress && sort_by_splitters(c, n, L, NW, ix.ks.key_bytes, true)) {
+        // the keys are sorted as they are
+    } else if (may_compress && radix_sort_is_small(c, n, L, NW, true)) {
         compressed = true;
         check = c->d_error;
     } else if (may_compress) {
@@ -573,10 +578,20 @@ int build_index(culsh_index& ix, SortBuffers& sb, Scratch<uint32_t>* bounds, Sta
     uint32_t B = 0;
     int cur = 0, passes = 0;
     while (true) {
-        passes = radix_sort_passes(ix.ks.key_bytes, compressed);
-        sb.set_final(radix_sort_final(c, passes, n, L, NW, compressed));
+        const bool splitters = sort_by_splitters(c, n, L, NW, ix.ks.key_bytes, compressed);
+        passes = splitters ? 1 : radix_sort_passes(ix.ks.key_bytes, compressed);
+        sb.set_final(splitters ? 1 : radix_sort_final(c, passes, n, L, NW, compressed));
         uint32_t* vp[2] = {sb.vals[0], sb.vals[1]};
-        cur = radix_sort_tables(c, NW, kp, vp, n, L, ix.ks.key_bytes, sb.tile_hist.p, compressed, kc, check);
+        if (splitters) {
+            switch (NW) {
+                case 2: cur = splitter_sort_tables<2>(c, kp, vp, n, L, ix.ks.key_bytes, sb.tile_hist.p); break;
+                case 4: cur = splitter_sort_tables<4>(c, kp, vp, n, L, ix.ks.key_bytes, sb.tile_hist.p); break;
+                case 8: cur = splitter_sort_tables<8>(c, kp, vp, n, L, ix.ks.key_bytes, sb.tile_hist.p); break;
+                default: cur = splitter_sort_tables<16>(c, kp, vp, n, L, ix.ks.key_bytes, sb.tile_hist.p); break;
+            }
+        } else {
+            cur = radix_sort_tables(c, NW, kp, vp, n, L, ix.ks.key_bytes, sb.tile_hist.p, compressed, kc, check);
+        }
         tm.mark();
         CULSH_DISPATCH_NW(NW, launch_bucket_count<NW>(c->stream, kp[cur], n, L, tile_heads.p, heads.p));
         exclusive_scan<uint32_t, uint32_t>(c->stream, tile_heads.p, n_tiles, tile_base.p, scratch.p,
@@ -636,7 +651,7 @@ int build_index(culsh_index& ix, SortBuffers& sb, Scratch<uint32_t>* bounds, Sta
     c->stats.n_items = (uint64_t)n * L;
     c->stats.n_buckets = B;
     c->stats.sort_passes = passes;
-    c->stats.sort_ctas = radix_sort_short_ctas(c, n, L, NW, compressed);
+    c->stats.sort_ctas = sort_by_splitters(c, n, L, NW, ix.ks.key_bytes, compressed) ? -1 : radix_sort_short_ctas(c, n, L, NW, compressed);
     c->stats.key_words = NW;
     c->stats.elem_bytes = ix.ks.elem_bytes;
     return 0;

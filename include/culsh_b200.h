@@ -81,7 +81,8 @@ typedef struct culsh_stats {
     uint64_t n_items, n_buckets, raw_candidates, unique_candidates;
     int32_t sort_passes, key_words, elem_bytes, hash_path; /* hash_path: 0 SIMT, 1 tcgen05 */
     int32_t launches;  /* kernels of this library launched by the call */
-    int32_t sort_ctas; /* fit: CTAs that sorted a table in one launch, 0 where every pass has launches of its own */
+    int32_t sort_ctas; /* fit: CTAs that sorted a table in one launch, 0 where every pass has launches of its own,
+                          -1 where rows went into bins by sampled splitters (sort_passes is 1 then) */
 } culsh_stats;
 
 /* ---- handle -------------------------------------------------------------------------- */

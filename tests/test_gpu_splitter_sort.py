@@ -1,0 +1,74 @@
+"""Keys of four words and more are sorted by sampled splitters, word by word by radix passes or, as one bin, by one CTA: row
+counts on both sides of a bin, of the change from one to several chunks of samples and of a tile, keys that end inside
+their words, and collections in which all rows are alike, come in order, repeat with a period or differ in one hash only, so that bins
+are full of equal keys and some are sorted in pieces."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(core, ix, indices, indptr, n, L, k):
+    sig = core.hash(indices, indptr, n, ix)  # [L][n][k]
+    got, keys = ix.get_candidate_indices(), ix.get_bucket_signatures().reshape(-1, 4 * k)
+    off, tab = ix.get_bucket_candidate_offsets(), ix.get_table_bucket_offsets()
+    for t in range(L):
+        raw = np.ascontiguousarray(sig[t]).view(np.uint8).reshape(n, 4 * k)
+        big = raw.view(">u4")
+        order = np.lexsort(tuple(big[:, j] for j in range(k - 1, -1, -1)))
+        assert np.array_equal(got[t * n:(t + 1) * n], order)
+        srt = raw[order]
+        head = np.concatenate([[True], (srt[1:] != srt[:-1]).any(axis=1)])
+        assert np.array_equal(keys[tab[t]:tab[t + 1]], srt[head])
+        assert np.array_equal(off[tab[t]:tab[t + 1]], t * n + np.flatnonzero(head))
+
+
+def _rows(kind, n, rng):
+    if kind == "alike":
+        return np.tile(rng.integers(0, 400, 6), (n, 1))
+    if kind == "few":  # two sets, one of them rare
+        return rng.integers(0, 400, (2, 6))[(rng.random(n) < 0.01).astype(int)]
+    if kind == "period":
+        return rng.integers(0, 4000, (7, 6))[np.arange(n) % 7]
+    if kind == "last":  # every row starts with the same ids
+        return np.concatenate([np.tile(rng.integers(0, 50, 5), (n, 1)), rng.integers(0, 1 << 19, (n, 1))], axis=1)
+    rows = rng.integers(0, 1 << 19, (max(1, n // 40), 6))[rng.integers(0, max(1, n // 40), n)]
+    if kind == "sorted":
+        return rows[np.lexsort(rows.T)]
+    change = rng.random(n) < 0.4
+    rows[change, rng.integers(0, 6, int(change.sum()))] = rng.integers(0, 1 << 19, int(change.sum()))
+    return rows
+
+
+@pytest.mark.parametrize("splitters", [None, "1", "0"])
+@pytest.mark.parametrize("n,k,kind", [
+    (1, 3, "mixed"), (9, 4, "mixed"), (2047, 4, "mixed"), (2048, 16, "mixed"), (2048, 4, "alike"), (2049, 4, "mixed"), (3000, 9, "few"),
+    (16_384, 4, "mixed"), (16_385, 5, "period"), (20_000, 4, "alike"), (20_000, 4, "sorted"), (65_537, 3, "last"),
+    (1500, 2, "mixed"), (12_289, 2, "few"), (100_003, 2, "sorted"), (700_000, 2, "mixed"), (100_003, 8, "mixed"), (100_003, 4, "few"), (524_288, 4, "mixed"), (524_289, 4, "sorted"), (600_000, 6, "last"), (2_100_000, 3, "mixed")])
+def test_order(n, k, kind, splitters, monkeypatch):
+    from culsh_b200 import _culsh_core as core_mod
+    if splitters:
+        monkeypatch.setenv("CULSH_SORT_SPLITTERS", splitters)
+    rng = np.random.default_rng(n + k)
+    L = 2
+    indices = np.ascontiguousarray(_rows(kind, n, rng).astype(np.int32)).ravel()
+    indptr = (6 * np.arange(n + 1)).astype(np.int32)
+    core = core_mod.MinHashCore(L, k, 7)
+    _check(core, core.fit(indices, indptr, n, 1 << 19), indices, indptr, n, L, k)
+
+
+def test_wide_p_stable_keys_and_many_tables():
+    """Values of two bytes (keys of four words with zeros in front), in more tables than the chip has SMs, and of one byte that span too much for the
+    compressed sort."""
+    from culsh_b200 import _culsh_core as core_mod
+    rng = np.random.default_rng(1)
+    for n, L, k, scale in [(3000, 150, 5, 300), (50_000, 2, 12, 300), (1500, 3, 8, 6), (12_288, 40, 8, 6), (100_003, 2, 7, 6)]:
+        X = (scale * rng.standard_normal((n, 6))).astype(np.float32)
+        core = core_mod.PSLSHCore(L, k, 1, 3)
+        ix = core.fit_float(X, n, 6)
+        assert ix.elem_bytes == (2 if scale == 300 else 1)
+        sig, got = core.hash(X, ix), ix.get_candidate_indices()
+        for t in range(0, L, 37):
+            raw = np.ascontiguousarray(sig[t]).view(np.uint8).reshape(n, 4 * k)
+            order = np.lexsort(tuple(raw[:, j] for j in range(4 * k - 1, -1, -1)))
+            assert np.array_equal(got[t * n:(t + 1) * n], order)
