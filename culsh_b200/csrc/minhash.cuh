@@ -98,6 +98,36 @@ __device__ __forceinline__ uint32_t min_plus5_short(uint32_t m, double a, double
     return __viaddmin_u32(5u * (uint32_t)__double2hiint(x) + (uint32_t)__double2loint(x), 0u - 5u * MH_2_52_HI, m);
 }
 
+// Rows of MH_LIST_FROM to MH_LIST ids: two instructions and a share of others for an evaluation.  2^32 / p is a little above one, and with alpha
+// the nearest whole number to a * 2^32 / p, beta that to b * 2^32 / p, y(c) = alpha * c + beta mod 2^32, one multiply-add, is the value f of the hash
+// function up to an error that the id bounds:
+//     y = f + e  (mod 2^32),  e = 5 * f / p + delta * c + epsilon,  |delta|, |epsilon| <= 1/2.
+// A shift in beta makes e >= 0 for all ids of the row, and it stays below some e_max.  The least y of eight ids, with the number of the eight in its low bits,
+// and the second of these are what a lane keeps of a row.  Of the eight of the least one, that with the least y is evaluated in full, f*: it is the row's
+// minimum where every other y is at e_max or more above it, for f >= y - e_max whether y wrapped or not.  Where that does not hold (of 110 ids below
+// 2^20 for a minimum in 70 to 150, in proportion to the largest id) the warp evaluates the minimum again.  Up to 32 ids that and what is set up for
+// a row weigh more than is saved, and with more than four hash functions a lane registers are too few.
+// Issue and the pipes of multiply-add (two cycles) and minimum bound it.  The double forms below and this one, 128 functions: 2M Zipf sets of 20 to 200
+// ids below 2^20 4,199 and 2,970 us, 300,000 below 2^16 593 and 443, below 2^22 768 and 537; 20M uniform ids below 2^20 in rows of 33 812 and
+// 647, 110 705 and 344, 1,000 778 and 332.  Next to it the double forms take 8 % longer for 12 uniform ids below 2^20 a row (634 and 682),
+// between 3 % less and 2 % more for other short rows.
+constexpr int MH_LIST = 1024;
+constexpr int MH_LIST_FROM = 33;
+constexpr uint32_t MH_TAG = MH_LIST / 8 - 1;
+constexpr int MH_COL_BITS = 22;  // rows with ids from 2^MH_COL_BITS on take the general forms
+// What ids in the list are above themselves: the sum of some of them tells their number, too.
+constexpr uint32_t MH_LIST_ID = 1u << 26;
+struct NearParams {
+    uint32_t alpha, beta;  // for ids in the list, without the shift
+    uint32_t off, below;   // |delta| * p, and whether delta < 0
+};
+__device__ __forceinline__ NearParams near_params(uint32_t a, uint32_t b) {
+    // delta = ra - 5 * a / p, and whole numbers next to it do: ra is 5 * a / 2^32 to the nearest
+    const uint32_t ra = (uint32_t)((5ull * a + (1ull << 31)) >> 32), rb = (uint32_t)((5ull * b + (1ull << 31)) >> 32);
+    const long long off = (long long)((uint64_t)ra * MINHASH_PRIME) - (long long)(5ull * a);  // delta * p
+    return NearParams{a + ra, b + rb - (a + ra) * MH_LIST_ID, (uint32_t)llabs(off), off < 0 ? 1u : 0u};
+}
+
 // keys: [L][n_total][NW] with NW = round_key_words(4k); word j (right-aligned) = bswap32(min).
 // PL = hash functions per lane per sweep; a sweep covers 32*PL consecutive hash functions and
 // H > 256 takes several sweeps.  Slots past H hold a = b = 0, evaluate to 0 and are never stored,
@@ -108,10 +138,14 @@ __global__ void __launch_bounds__(MH_THREADS, PL <= 2 ? 32 : PL <= 4 ? 24 : 18)
 minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ indptr,
                const uint32_t* __restrict__ A, const uint32_t* __restrict__ B, int n_rows,
                int L, int k, int NW, uint32_t* __restrict__ keys, int n_total, int row_offset, int rows) {
+    constexpr bool NEAR = PL <= 4;  // more leave it too few registers
     const int lane = threadIdx.x & 31;
     const int H = L * k;
     const int pad_words = NW - k;  // leading zero words when 4k is not 4, 8, 16 or 32 bytes
     __shared__ __align__(16) double ids_short[34], ids_long[34];
+    __shared__ __align__(16) uint32_t ids_row[NEAR ? MH_LIST : 1];
+    __shared__ __align__(16) NearParams near[NEAR ? PL : 1][32];
+    bool have_near = false;
     __shared__ size_t key_at[32 * PL];  // word of a hash function in the first row's keys
     const uint32_t below = (1u << lane) - 1u;
     double ad[PL], bd[PL];
@@ -137,18 +171,99 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
     const int bound = lane <= here ? indptr[row0 + lane] : 0;
     int start = __shfl_sync(0xFFFFFFFFu, bound, 0), end = __shfl_sync(0xFFFFFFFFu, bound, 1);
     int ahead = start + lane < end ? indices[start + lane] : 0;
+    // ... and three more of a row for the near form, while the row before it is under way
+    int more[3] = {0, 0, 0};
+    auto fetch_more = [&](int from, int to) {
+        if (NEAR && to - from >= MH_LIST_FROM && to - from <= MH_LIST) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) more[q] = from + 32 * (q + 1) + lane < to ? indices[from + 32 * (q + 1) + lane] : 0;
+        }
+    };
+    fetch_more(start, end);
     for (int r = 0; r < here; ++r) {
         const int row = row_offset + (int)row0 + r;
         const int next_end = r + 1 < here ? __shfl_sync(0xFFFFFFFFu, bound, r + 2) : end;
         const uint32_t short_col = end - start <= MH_SHORT_ROW ? MH_SHORT_COL : 0u;
         bool shorts = false;  // the row has had ids below short_col
+        // Rows for the near form: all ids at once, the last one again to a whole number of eights.
+        const int n_ids = end - start, eights = (n_ids + 7) / 8;
+        bool listed = NEAR && n_ids >= MH_LIST_FROM && n_ids <= MH_LIST;
+        uint32_t largest = 0;
+        if (listed) listed = !__any_sync(0xFFFFFFFFu, (uint32_t)ahead >> MH_COL_BITS);
+        if (listed) {
+            largest = (uint32_t)ahead;
+            ids_row[lane] = largest + MH_LIST_ID;
+            auto put = [&](int at, uint32_t id) {
+                if (at < n_ids) {
+                    largest = max(largest, id);
+                    ids_row[at] = id + MH_LIST_ID;
+                }
+            };
+#pragma unroll
+            for (int q = 0; q < 3; ++q) put(32 * (q + 1) + lane, (uint32_t)more[q]);
+#pragma unroll 1
+            for (int at = 128 + lane; at < n_ids; at += 32) put(at, (uint32_t)indices[start + at]);
+            largest = __reduce_max_sync(0xFFFFFFFFu, largest);
+            listed = largest >> MH_COL_BITS == 0;
+            __syncwarp();
+            if (lane < eights * 8 - n_ids) ids_row[n_ids + lane] = ids_row[n_ids - 1];
+            __syncwarp();
+        }
+        if (r + 1 < here) fetch_more(end, next_end);
         for (int h0 = 0; h0 < H; h0 += 32 * PL) {
             const bool last = h0 + 32 * PL >= H;
             if (H > 32 * PL) load_params(h0);
             uint32_t m[PL];
 #pragma unroll
             for (int i = 0; i < PL; ++i) m[i] = 0xFFFFFFFFu;
-            for (int base = start; base < end; base += 32) {
+            if constexpr (NEAR) if (listed) {  // one sweep
+                if (last) ahead = end + lane < next_end ? indices[end + lane] : 0;  // the next row's first
+                if (!have_near) {
+#pragma unroll
+                    for (int i = 0; i < PL; ++i) near[i][lane] = near_params(a_of(i), (uint32_t)(b5_of(i) - 5ull));
+                    have_near = true;
+                }
+                auto span_of = [&](const NearParams& np) { return __umulhi(np.off, largest + 1u) + 3u; };  // |delta| * largest and a little more
+                uint32_t alpha[PL], beta[PL], second[PL];
+#pragma unroll
+                for (int i = 0; i < PL; ++i) {
+                    const NearParams np = near[i][lane];
+                    alpha[i] = np.alpha;
+                    beta[i] = np.beta + (np.below ? span_of(np) : 1u);
+                    second[i] = 0xFFFFFFFFu;
+                }
+                const uint4* four = reinterpret_cast<const uint4*>(ids_row);
+#pragma unroll 1
+                for (int j = 0; j < eights; ++j) {
+                    const uint4 u = four[2 * j], v = four[2 * j + 1];
+#pragma unroll
+                    for (int i = 0; i < PL; ++i) {
+                        auto y = [&](uint32_t c) { return alpha[i] * c + beta[i]; };
+                        uint32_t t = __vimin3_u32(y(u.x), y(u.y), y(u.z));
+                        t = __vimin3_u32(t, y(u.w), y(v.x));
+                        t = __vimin3_u32(t, y(v.y), y(v.z));
+                        t = (min(t, y(v.w)) & ~MH_TAG) | (uint32_t)j;
+                        second[i] = min(second[i], max(m[i], t));
+                        m[i] = min(m[i], t);
+                    }
+                }
+                const uint32_t last_id = ids_row[n_ids - 1], times = (uint32_t)(eights * 8 - n_ids) + 1u;  // in its eight
+#pragma unroll
+                for (int i = 0; i < PL; ++i) {
+                    const uint4 u = four[2 * (m[i] & MH_TAG)], v = four[2 * (m[i] & MH_TAG) + 1];
+                    const uint32_t slack = span_of(near[i][lane]) + 8u + MH_TAG + 1u;  // e_max and what the tag takes off
+                    const uint32_t base = beta[i] - (m[i] & ~MH_TAG);
+                    uint32_t close = 0;  // sum of those whose y is close to the least one
+                    auto look = [&](uint32_t c) { close += alpha[i] * c + base <= slack ? c : 0u; };
+                    look(u.x); look(u.y); look(u.z); look(u.w);
+                    look(v.x); look(v.y); look(v.z); look(v.w);
+                    if (close == last_id * times) close = last_id;
+                    const uint32_t t = hash_plus5(a_of(i), close & (MH_LIST_ID - 1u), b5_of(i));
+                    // 0 where it is too close to tell, and below 5 near the prime: evaluated again
+                    m[i] = close < 2u * MH_LIST_ID && t >= 5u && t <= 0xFFFFFFFFu - slack && second[i] >= t - 5u + slack ? t : 0u;
+                }
+            }
+            for (int base = listed ? end : start; base < end; base += 32) {
                 const int mine = ahead;
                 // the next step's, then the row's first again for another sweep, or the next row's
                 const bool inside = base + 32 < end;
@@ -174,11 +289,17 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
 #pragma unroll
                         for (int i = 0; i < PL; ++i) m[i] = min_plus5_short(min_plus5_short(m[i], ad[i], c.x, bd[i]), ad[i], c.y, bd[i]);
                     }
-                    for (int s = 0; s < n_long; s += 2) {
+                    auto two_long = [&](int s) {
                         const double2 c = *reinterpret_cast<const double2*>(ids_long + s);
 #pragma unroll
                         for (int i = 0; i < PL; ++i)
                             m[i] = __vimin3_u32(m[i], hash_plus5_double(ad[i], c.x, bd[i]), hash_plus5_double(ad[i], c.y, bd[i]));
+                    };
+                    if (NEAR && n_long == 32) {  // rows that are too long for the list, or their ids too large, have many of these
+#pragma unroll 2
+                        for (int s = 0; s < 32; s += 2) two_long(s);
+                    } else {
+                        for (int s = 0; s < n_long; s += 2) two_long(s);
                     }
                     __syncwarp();
                     continue;
@@ -215,9 +336,20 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
                     const uint32_t a = __shfl_sync(0xFFFFFFFFu, a_of(i), src);
                     const uint32_t b = __shfl_sync(0xFFFFFFFFu, (uint32_t)(b5_of(i) - 5ull), src);
                     uint32_t exact = 0xFFFFFFFFu;
-                    for (int e = start + lane; e < end; e += 32) exact = min(exact, hash_mod_prime(a, (uint32_t)indices[e], b));
-                    exact = __reduce_min_sync(0xFFFFFFFFu, exact);
-                    if (lane == src) m[i] = exact + 5u;
+                    uint32_t plus5 = 0;
+                    if constexpr (NEAR) if (listed) {  // four ids of a lane at once, the last one for those that are not there
+                        plus5 = 0xFFFFFFFFu;
+                        for (int e = lane; e - lane < n_ids; e += 128)
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                                plus5 = min(plus5, hash_plus5(a, ids_row[min(e + 32 * q, n_ids - 1)] - MH_LIST_ID, (uint64_t)b + 5u));
+                        plus5 = __reduce_min_sync(0xFFFFFFFFu, plus5);
+                    }
+                    if (plus5 < 5u) {
+                        for (int e = start + lane; e < end; e += 32) exact = min(exact, hash_mod_prime(a, (uint32_t)indices[e], b));
+                        plus5 = __reduce_min_sync(0xFFFFFFFFu, exact) + 5u;
+                    }
+                    if (lane == src) m[i] = plus5;
                 }
                 if (end > start) m[i] -= 5u;
             }
