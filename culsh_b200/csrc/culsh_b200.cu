@@ -839,7 +839,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         count(RawCounts{raw_cnt.p, raw_off.p, big_list.p, mid_list, n_big, mid_max, out.counts.p, host_raw});
     } else {
         CU_CHECK(cudaMemsetAsync(n_big, 0, 4 * sizeof(uint32_t), s));
-        raw_count_kernel<<<(unsigned)ceil_div(n_q, 256), 256, 0, s>>>(bounds, n_q, L, self_join, raw_cnt.p, big_list.p,
+        launch_next(s, raw_count_kernel, (unsigned)ceil_div(n_q, 256), 256, 0, bounds, n_q, L, self_join, raw_cnt.p, big_list.p,
                                                                      mid_list, n_big, mid_max, out.counts.p);
         KERNEL_CHECK();
         exclusive_scan<uint64_t, uint64_t>(s, raw_cnt.p, n_q, raw_off.p, scratch.p, host_raw);
@@ -854,7 +854,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
     Scratch<int2> slices;
     auto launch_small = [&](auto kernel, int above, uint64_t room) {
         const size_t blocks = std::min<size_t>(ceil_div(n_q, SM_WARPS), (size_t)c->sm_count * 32);
-        kernel<<<(unsigned)blocks, SM_THREADS, 0, s>>>(bounds, ix.cand.p, raw_cnt.p, raw_off.p, L, above, room, tmp.p, out.counts.p);
+        launch_next(s, kernel, (unsigned)blocks, SM_THREADS, 0, bounds, ix.cand.p, raw_cnt.p, raw_off.p, L, above, room, tmp.p, out.counts.p);
         KERNEL_CHECK();
     };
     auto launch_windows = [&](size_t n_ctas, const uint32_t* n_slots, uint64_t room) {
@@ -865,7 +865,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
             auto kern = dedupe_window_kernel<NT, MK>;
             CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-            kern<<<(unsigned)n_ctas, NT, smem, s>>>(big_list.p, bounds, ix.cand.p, raw_off.p, L, ix.n, win.bits, win.n, self_join,
+            launch_next(s, kern, (unsigned)n_ctas, NT, smem, big_list.p, bounds, ix.cand.p, raw_off.p, L, ix.n, win.bits, win.n, self_join,
                                                     slices.p, n_slots, room, tmp.p, pieces.p,
                                                     reinterpret_cast<unsigned long long*>(out.counts.p));
             KERNEL_CHECK();
@@ -970,7 +970,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
             const long pre = env_long("CULSH_CHAIN_SLICES", n_pieces > WINDOW_SEARCH);
             if (pre && win.n > 1 && n_pieces * (size_t)L <= ((size_t)32 << 20)) {
                 slices.reserve(c, SL_SLICES, n_pieces * (size_t)L);
-                slice_lists_kernel<<<(unsigned)ceil_div(n_pieces * (size_t)L, 256), 256, 0, s>>>(
+                launch_next(s, slice_lists_kernel, (unsigned)ceil_div(n_pieces * (size_t)L, 256), 256, 0, 
                     big_list.p, bounds, ix.cand.p, (int)nb, L, win.bits, win.n, slices.p);
                 KERNEL_CHECK();
             }
@@ -999,12 +999,12 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         if (n_other) {
             const int per = count >= (1 << 17) ? 32 : CS_ROWS;  // from here on full warps still fill the chip
             const size_t blocks = std::min<size_t>(ceil_div(ceil_div((size_t)count, per) * 32, 256), (size_t)c->sm_count * 32);
-            compact_small_kernel<<<(unsigned)blocks, 256, 0, s>>>(tmp.p, raw_cnt.p + q_lo, raw_off.p + q_lo, out.counts.p + q_lo,
+            launch_next(s, compact_small_kernel, (unsigned)blocks, 256, 0, tmp.p, raw_cnt.p + q_lo, raw_off.p + q_lo, out.counts.p + q_lo,
                                                                  out.offsets.p + q_lo, count, per, first, dst);
             KERNEL_CHECK();
         }
         if (windows) {
-            compact_windows_kernel<<<(unsigned)n_pieces, 256, 0, s>>>(big_list.p, tmp.p, raw_off.p, pieces.p, out.offsets.p, win.n,
+            launch_next(s, compact_windows_kernel, (unsigned)n_pieces, 256, 0, big_list.p, tmp.p, raw_off.p, pieces.p, out.offsets.p, win.n,
                                                                      (uint32_t)q_lo, (uint32_t)q_hi, first, dst);
             KERNEL_CHECK();
         }

@@ -31,6 +31,7 @@ template <int NW>
 __global__ void __launch_bounds__(IB_THREADS)
 bucket_count_kernel(const uint32_t* __restrict__ keys, int n, int tiles_per_table,
                     uint32_t* __restrict__ tile_heads, uint32_t* __restrict__ heads) {
+    behind_kernel_before(keys, tile_heads, heads);
     __shared__ uint32_t s_warp[32];
     const int t = blockIdx.x / tiles_per_table;
     const int lt = blockIdx.x - t * tiles_per_table;
@@ -61,6 +62,7 @@ bucket_write_kernel(const uint32_t* __restrict__ keys, int n, int L, int tiles_p
                     const uint32_t* __restrict__ tile_base, uint32_t n_tiles, const uint32_t* __restrict__ heads,
                     uint32_t* __restrict__ bucket_keys, int32_t* __restrict__ bucket_offsets,
                     int32_t* __restrict__ table_offsets) {
+    behind_kernel_before(keys, tile_base, heads, bucket_keys, bucket_offsets, table_offsets);
     constexpr int WORDS = IB_WORDS;
     __shared__ uint32_t s_bits[WORDS];
     __shared__ uint32_t s_pref[WORDS];
@@ -117,7 +119,7 @@ template <int NW>
 inline void launch_bucket_count(cudaStream_t s, const uint32_t* keys, int n, int L,
                                 uint32_t* tile_heads, uint32_t* heads) {
     int tpt = (int)ceil_div(n, IB_TILE);
-    bucket_count_kernel<NW><<<(unsigned)((size_t)tpt * L), IB_THREADS, 0, s>>>(keys, n, tpt, tile_heads, heads);
+    launch_next(s, bucket_count_kernel<NW>, (unsigned)((size_t)tpt * L), IB_THREADS, 0, keys, n, tpt, tile_heads, heads);
     KERNEL_CHECK();
 }
 
@@ -126,7 +128,7 @@ inline void launch_bucket_write(cudaStream_t s, const uint32_t* keys, int n, int
                                 uint32_t* bucket_keys, int32_t* bucket_offsets, int32_t* table_offsets) {
     int tpt = (int)ceil_div(n, IB_TILE);
     uint32_t n_tiles = (uint32_t)((size_t)tpt * L);
-    bucket_write_kernel<NW><<<n_tiles, IB_THREADS, 0, s>>>(keys, n, L, tpt, tile_base, n_tiles, heads, bucket_keys,
+    launch_next(s, bucket_write_kernel<NW>, n_tiles, IB_THREADS, 0, keys, n, L, tpt, tile_base, n_tiles, heads, bucket_keys,
                                                           bucket_offsets, table_offsets);
     KERNEL_CHECK();
 }

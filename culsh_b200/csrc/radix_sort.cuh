@@ -140,6 +140,7 @@ template <int NW, bool COMP0>
 __global__ void __launch_bounds__(RS_THREADS)
 radix_tile_hist_kernel(const uint32_t* __restrict__ keys, int n, int tiles_per_table, int p, uint32_t sub,
                        uint32_t* __restrict__ tile_hist) {
+    behind_kernel_before(keys, tile_hist);
     using Cfg = SortCfg<NW>;
     __shared__ uint32_t s_hist[256];
     const int tile = blockIdx.x;
@@ -176,6 +177,7 @@ constexpr int RS_SCAN_SEGS = RS_SCAN_THREADS / 256;
 
 __global__ void __launch_bounds__(RS_SCAN_THREADS)
 radix_tile_scan_kernel(uint32_t* __restrict__ tile_hist, int tiles_per_table) {
+    behind_kernel_before(tile_hist);
     __shared__ uint32_t s_seg[RS_SCAN_SEGS][256];
     __shared__ uint32_t s_base[256];
     __shared__ uint32_t s_warp[8];
@@ -226,6 +228,7 @@ constexpr int RS_CHUNK_MIN_TILES = 96;  // tables with fewer tiles keep the sing
 __global__ void __launch_bounds__(RS_SCAN_THREADS)
 radix_tile_scan_chunk_kernel(uint32_t* __restrict__ tile_hist, int tiles_per_table, int n_chunks,
                              uint32_t* __restrict__ chunk_tot /* [table][chunk][256] */) {
+    behind_kernel_before(tile_hist, chunk_tot);
     __shared__ uint32_t s_seg[RS_SCAN_SEGS][256];
     const int d = threadIdx.x & 255, seg = threadIdx.x >> 8;
     const int table = blockIdx.x / n_chunks, chunk = blockIdx.x - table * n_chunks;
@@ -257,6 +260,7 @@ radix_tile_scan_chunk_kernel(uint32_t* __restrict__ tile_hist, int tiles_per_tab
 // one block of 256 threads per table: chunk_tot -> chunk bases, in place
 __global__ void __launch_bounds__(256)
 radix_chunk_base_kernel(uint32_t* __restrict__ chunk_tot, int n_chunks) {
+    behind_kernel_before(chunk_tot);
     __shared__ uint32_t s_warp[8];
     const int d = threadIdx.x, lane = d & 31, w = d >> 5;
     uint32_t* ct = chunk_tot + (size_t)blockIdx.x * n_chunks * 256 + d;
@@ -318,6 +322,7 @@ radix_scatter_kernel(const uint32_t* __restrict__ keys_in, const uint32_t* __res
                      uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int n,
                      int tiles_per_table, int p, KeyComp kc, const uint32_t* __restrict__ tile_off,
                      const uint32_t* __restrict__ chunk_base /* or null */, int n_chunks) {
+    behind_kernel_before(keys_in, vals_in, keys_out, vals_out, tile_off, chunk_base);
     using Cfg = SortCfg<NW>;
     constexpr int IPT = Cfg::IPT;
     constexpr int TILE = Cfg::TILE;
@@ -538,6 +543,7 @@ template <int NW, bool PACK>
 __global__ void __launch_bounds__(RSS_THREADS, 1)
 radix_sort_small_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
                         uint32_t* __restrict__ vals_out, int n, int passes, bool compressed, KeyComp kc, const int* __restrict__ check) {
+    behind_kernel_before(keys_in, keys_out, vals_out, check);
     using Cfg = SmallSortCfg<NW, PACK>;
     constexpr int KW = Cfg::KW, IPT = Cfg::IPT;
     constexpr bool WORDS = NW >= 4;
@@ -708,6 +714,7 @@ __global__ void __launch_bounds__(RSC_THREADS, 1)
 radix_sort_cluster_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
                           uint32_t* __restrict__ vals_out, int n, int cta_rows, uint32_t cta_rows_inv, int passes, bool compressed,
                           KeyComp kc, const int* __restrict__ check) {
+    behind_kernel_before(keys_in, keys_out, vals_out, check);
     using Cfg = ClusterSortCfg<NW, PACK>;
     constexpr int KW = Cfg::KW, IPT = Cfg::IPT;
     constexpr bool WORDS = NW >= 4;
@@ -913,7 +920,7 @@ inline int radix_sort_small(const CtxPtr& c, uint32_t* keys[2], uint32_t* vals[2
     auto go = [&](auto kern, size_t smem) {
         CU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (c->profiling) cudaEventRecord(c->ev_pass[0], c->stream);
-        kern<<<(unsigned)L, RSS_THREADS, smem, c->stream>>>(keys[0], keys[1], vals[1], n, passes, compressed, kc, check);
+        launch_next(c->stream, kern, (unsigned)L, RSS_THREADS, smem, keys[0], keys[1], vals[1], n, passes, compressed, kc, check);
         KERNEL_CHECK();
         if (c->profiling) cudaEventRecord(c->ev_pass[1], c->stream);
     };
@@ -951,12 +958,12 @@ struct TileScan {
     uint32_t* chunk_base() const { return chunked() ? tile_hist + (size_t)tiles_per_table * L * 256 : nullptr; }
     void run() const {
         if (chunked()) {
-            radix_tile_scan_chunk_kernel<<<(unsigned)(L * n_chunks()), RS_SCAN_THREADS, 0, s>>>(
+            launch_next(s, radix_tile_scan_chunk_kernel, (unsigned)(L * n_chunks()), RS_SCAN_THREADS, 0, 
                 tile_hist, tiles_per_table, n_chunks(), chunk_base());
             KERNEL_CHECK();
-            radix_chunk_base_kernel<<<(unsigned)L, 256, 0, s>>>(chunk_base(), n_chunks());
+            launch_next(s, radix_chunk_base_kernel, (unsigned)L, 256, 0, chunk_base(), n_chunks());
         } else {
-            radix_tile_scan_kernel<<<(unsigned)L, RS_SCAN_THREADS, 0, s>>>(tile_hist, tiles_per_table);
+            launch_next(s, radix_tile_scan_kernel, (unsigned)L, RS_SCAN_THREADS, 0, tile_hist, tiles_per_table);
         }
         KERNEL_CHECK();
     }
@@ -987,10 +994,10 @@ inline int radix_sort_tables_nw(const CtxPtr& c, uint32_t* keys[2], uint32_t* va
     int cur = 0;
     for (int p = 0; p < passes; ++p) {
         if (compressed && p == 0)
-            radix_tile_hist_kernel<NW, true><<<(unsigned)total_tiles, RS_THREADS, 0, s>>>(
+            launch_next(s, radix_tile_hist_kernel<NW, true>, (unsigned)total_tiles, RS_THREADS, 0, 
                 keys[cur], n, tiles_per_table, p, kc.sub, tile_hist);
         else
-            radix_tile_hist_kernel<NW, false><<<(unsigned)total_tiles, RS_THREADS, 0, s>>>(
+            launch_next(s, radix_tile_hist_kernel<NW, false>, (unsigned)total_tiles, RS_THREADS, 0, 
                 keys[cur], n, tiles_per_table, pack ? p + 3 : p, 0u, tile_hist);
         KERNEL_CHECK();
         scan.run();
@@ -998,7 +1005,7 @@ inline int radix_sort_tables_nw(const CtxPtr& c, uint32_t* keys[2], uint32_t* va
         if (last && c->profiling) cudaEventRecord(c->ev_pass[0], s);
         auto kern = p == 0 ? (compressed ? k_first_c : k_first) : (compressed && last ? k_last_c : k_next);
         if (pack) kern = p == 0 ? k_first_p : (last ? k_last_p : k_next_p);
-        kern<<<(unsigned)total_tiles, RS_THREADS, Cfg::SMEM, s>>>(
+        launch_next(s, kern, (unsigned)total_tiles, RS_THREADS, Cfg::SMEM, 
             keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n, tiles_per_table, p, kc, tile_hist,
             scan.chunk_base(), scan.n_chunks());
         KERNEL_CHECK();
@@ -1041,12 +1048,12 @@ inline int radix_sort_words(const CtxPtr& c, uint32_t* keys[2], uint32_t* vals[2
             radix_word_gather_kernel<NW><<<(unsigned)total_tiles, RS_THREADS, 0, s>>>(keys[0], ids, n, tiles_per_table,
                                                                                    NW - 1 - (p >> 2), w_in, tile_hist);
         else
-            radix_tile_hist_kernel<1, false><<<(unsigned)total_tiles, RS_THREADS, 0, s>>>(w_in, n, tiles_per_table, p & 3, 0u, tile_hist);
+            launch_next(s, radix_tile_hist_kernel<1, false>, (unsigned)total_tiles, RS_THREADS, 0, w_in, n, tiles_per_table, p & 3, 0u, tile_hist);
         KERNEL_CHECK();
         scan.run();
         if (p == KB - 1 && c->profiling) cudaEventRecord(c->ev_pass[0], s);
         auto kern = p == 0 ? k_first : (word_end ? k_last : k_next);  // a key has nine bytes at least
-        kern<<<(unsigned)total_tiles, RS_THREADS, Cfg::SMEM, s>>>(w_in, ids, words[(p & 1) ^ 1], ids_of(p), n, tiles_per_table, p & 3,
+        launch_next(s, kern, (unsigned)total_tiles, RS_THREADS, Cfg::SMEM, w_in, ids, words[(p & 1) ^ 1], ids_of(p), n, tiles_per_table, p & 3,
                                                                KeyComp{0u, 0u}, tile_hist, scan.chunk_base(), scan.n_chunks());
         KERNEL_CHECK();
         if (p == KB - 1 && c->profiling) cudaEventRecord(c->ev_pass[1], s);
@@ -1122,6 +1129,7 @@ __device__ __forceinline__ TOut block_exclusive_scan(TOut v, TOut* s_warp, TOut&
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(SCAN_THREADS)
 scan_reduce_kernel(const TIn* __restrict__ in, size_t n, TOut* __restrict__ block_sums) {
+    behind_kernel_before(in, block_sums);
     __shared__ TOut s_warp[32];
     size_t base = (size_t)blockIdx.x * SCAN_TILE;
     TOut sum = 0;
@@ -1156,6 +1164,7 @@ struct HostWords {
 template <typename TOut>
 __global__ void __launch_bounds__(1024)
 scan_block_sums_kernel(TOut* __restrict__ block_sums, size_t n_blocks, TOut* __restrict__ total_out, HostWords host) {
+    behind_kernel_before(block_sums, total_out);
     __shared__ TOut s_warp[32];
     TOut carry = 0;
     for (size_t base = 0; base < n_blocks; base += 1024) {
@@ -1174,6 +1183,7 @@ template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(SCAN_THREADS)
 scan_apply_kernel(const TIn* __restrict__ in, size_t n, const TOut* __restrict__ block_sums, bool scanned,
                   TOut* __restrict__ out, HostWords host) {
+    behind_kernel_before(in, block_sums, out);
     __shared__ TOut s_warp[32];
     TOut before = 0;  // elements of the blocks before this one
     if (scanned) {
@@ -1223,6 +1233,7 @@ struct alignas(16) ScanVec {
 template <typename T>
 __global__ void __launch_bounds__(SCAN_ONE_THREADS)
 scan_one_kernel(const T* __restrict__ in, int n, T* __restrict__ out, HostWords host) {
+    behind_kernel_before(in, out);
     constexpr int PER = 16 / sizeof(T), VECS = SCAN_ONE_IPT / PER;
     __shared__ T s_warp[32];
     T carry = 0;
@@ -1270,20 +1281,20 @@ inline void exclusive_scan(cudaStream_t s, const TIn* in, size_t n, TOut* out, T
     }
     if constexpr (std::is_same<TIn, TOut>::value) {
         if (n <= SCAN_ONE_MAX && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
-            scan_one_kernel<TOut><<<1, SCAN_ONE_THREADS, 0, s>>>(in, (int)n, out, host);
+            launch_next(s, scan_one_kernel<TOut>, 1, SCAN_ONE_THREADS, 0, in, (int)n, out, host);
             KERNEL_CHECK();
             return;
         }
     }
     size_t n_blocks = ceil_div(n, SCAN_TILE);
-    scan_reduce_kernel<TIn, TOut><<<(unsigned)n_blocks, SCAN_THREADS, 0, s>>>(in, n, scratch);
+    launch_next(s, scan_reduce_kernel<TIn, TOut>, (unsigned)n_blocks, SCAN_THREADS, 0, in, n, scratch);
     KERNEL_CHECK();
     const bool scanned = n_blocks > SCAN_ADD_MAX;
     if (scanned) {
-        scan_block_sums_kernel<TOut><<<1, 1024, 0, s>>>(scratch, n_blocks, out + n, host);
+        launch_next(s, scan_block_sums_kernel<TOut>, 1, 1024, 0, scratch, n_blocks, out + n, host);
         KERNEL_CHECK();
     }
-    scan_apply_kernel<TIn, TOut><<<(unsigned)n_blocks, SCAN_THREADS, 0, s>>>(in, n, scratch, scanned, out, host);
+    launch_next(s, scan_apply_kernel<TIn, TOut>, (unsigned)n_blocks, SCAN_THREADS, 0, in, n, scratch, scanned, out, host);
     KERNEL_CHECK();
 }
 

@@ -232,6 +232,7 @@ template <int NW>
 __global__ void __launch_bounds__(SS_THREADS)
 splitter_sample_kernel(const uint32_t* __restrict__ keys, int n, int skip, int samples, int chunks, int bins, int over,
                        RowList<NW> sorted /* one chunk: the splitters */) {
+    behind_kernel_before(keys);
     extern __shared__ __align__(16) unsigned char ss_smem[];
     using Sort = BlockSort<NW>;
     auto& s = *reinterpret_cast<typename Sort::Smem*>(ss_smem);
@@ -263,6 +264,7 @@ splitter_sample_kernel(const uint32_t* __restrict__ keys, int n, int skip, int s
 template <int NW>
 __global__ void __launch_bounds__(256)
 splitter_rank_kernel(const uint32_t* __restrict__ keys, int n, int skip, int chunks, int bins, int total, RowList<NW> sorted, RowList<NW> splitters) {
+    behind_kernel_before(keys);
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= total) return;
     const int samples = chunks * SS_CAP, t = i / samples, own = (i - t * samples) / SS_CAP;
@@ -387,6 +389,7 @@ splitter_classify_kernel(const uint32_t* __restrict__ keys, int n, int skip, int
 constexpr int SS_SCAN_THREADS = 64;
 __global__ void __launch_bounds__(SS_SCAN_THREADS)
 splitter_scan_kernel(uint32_t* __restrict__ tile_hist, int tiles, int bins, int total, uint32_t* __restrict__ bin_total) {
+    behind_kernel_before(tile_hist, bin_total);
     const int i = blockIdx.x * SS_SCAN_THREADS + threadIdx.x;
     if (i >= total) return;
     const int t = i / bins, b = i - t * bins;
@@ -414,6 +417,7 @@ __global__ void __launch_bounds__(SS_TILE_THREADS)
 splitter_scatter_kernel(const uint16_t* __restrict__ bin_of, int n, int tile, int tiles, int bins, const uint32_t* __restrict__ tile_hist,
                         const uint32_t* __restrict__ bin_total, uint32_t* __restrict__ bin_start,
                         uint32_t* __restrict__ ids) {
+    behind_kernel_before(bin_of, tile_hist, bin_total, bin_start, ids);
     extern __shared__ __align__(16) unsigned char ss_smem[];
     uint16_t* s_row = reinterpret_cast<uint16_t*>(ss_smem);            // [tile] its rows, bin after bin
     uint16_t* s_bin = s_row + tile;                                    // [tile] their bins
@@ -831,11 +835,12 @@ inline int splitter_sort_tables(const CtxPtr& c, uint32_t* keys[2], uint32_t* va
         const RowList<NW> splitters = list(p.list, (size_t)L * p.bins), sorted = p.chunks > 1 ? list(p.sorted, (size_t)L * p.samples) : splitters;
         auto sample = splitter_sample_kernel<NW>;
         smem_of(sample, sort_smem);
-        sample<<<(unsigned)(L * p.chunks), SS_THREADS, sort_smem, s>>>(keys[0], n, skip, p.samples, p.chunks, p.bins, p.samples / p.bins, sorted);
+        launch_next(s, sample, (unsigned)(L * p.chunks), SS_THREADS, sort_smem, keys[0], n, skip, p.samples, p.chunks, p.bins,
+                    p.samples / p.bins, sorted);
         KERNEL_CHECK();
         if (p.chunks > 1) {
             const int total = L * p.samples;
-            splitter_rank_kernel<NW><<<(unsigned)ceil_div(total, 256), 256, 0, s>>>(keys[0], n, skip, p.chunks, p.bins, total, sorted, splitters);
+            launch_next(s, splitter_rank_kernel<NW>, (unsigned)ceil_div(total, 256), 256, 0, keys[0], n, skip, p.chunks, p.bins, total, sorted, splitters);
             KERNEL_CHECK();
         }
         uint16_t* bin_of = reinterpret_cast<uint16_t*>(keys[1]);  // until the keys come
@@ -844,12 +849,12 @@ inline int splitter_sort_tables(const CtxPtr& c, uint32_t* keys[2], uint32_t* va
         classify<<<(unsigned)(L * p.tiles), SS_TILE_THREADS, splitter_classify_smem(p.bins), s>>>(keys[0], n, skip, p.tile, p.tiles, p.bins, splitters,
                                                                                                 bin_of, scratch + p.hist);
         KERNEL_CHECK();
-        splitter_scan_kernel<<<(unsigned)ceil_div((size_t)L * p.bins, SS_SCAN_THREADS), SS_SCAN_THREADS, 0, s>>>(scratch + p.hist, p.tiles, p.bins,
+        launch_next(s, splitter_scan_kernel, (unsigned)ceil_div((size_t)L * p.bins, SS_SCAN_THREADS), SS_SCAN_THREADS, 0, scratch + p.hist, p.tiles, p.bins,
                                                                                                            L * p.bins, scratch + p.total);
         KERNEL_CHECK();
         ids = vals[0];
         smem_of(splitter_scatter_kernel, splitter_scatter_smem(p.tile, p.bins));
-        splitter_scatter_kernel<<<(unsigned)(L * p.tiles), SS_TILE_THREADS, splitter_scatter_smem(p.tile, p.bins), s>>>(
+        launch_next(s, splitter_scatter_kernel, (unsigned)(L * p.tiles), SS_TILE_THREADS, splitter_scatter_smem(p.tile, p.bins),
             bin_of, n, p.tile, p.tiles, p.bins, scratch + p.hist, scratch + p.total, scratch + p.start, ids);
         KERNEL_CHECK();
     }
