@@ -113,7 +113,7 @@ enum ScratchSlot {
 };
 
 // Where kernels leave what the host reads behind its next wait: words of Ctx::pinned, a total and up to eight 32-bit words.
-enum HostSlot { HS_BUCKETS = 32, HS_RAW = 40, HS_UNIQUE = 48 };
+enum HostSlot { HS_BUCKETS = 32, HS_RAW = 40, HS_UNIQUE = 48, HS_NORM = 56 };
 
 struct Ctx {
     int device = 0;
@@ -136,6 +136,7 @@ struct Ctx {
     uint64_t* pinned = nullptr;       // 64 x u64 words of pinned host memory: read_words' first, see HostSlot
     FeedRing feed_ring;               // for pageable host inputs, made on first use
     int* d_error = nullptr;           // device-side self-check word; [2], [3]: see HashRange
+    unsigned* d_ticket = nullptr;     // behind it: for kernels whose last CTA does more, zero between them
     int seen_error = 0;               // its value behind the last query
     unsigned long long* d_mma = nullptr;  // tensor-core projection: K-blocks issued / with the low-part MMA
     bool profiling = false;

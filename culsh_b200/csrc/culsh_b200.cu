@@ -1290,8 +1290,9 @@ int culsh_create(int device, culsh_handle** out) {
         for (auto& e : c->copy_done) CU_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         for (auto& e : c->chunk_free) CU_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         CU_CHECK(cudaMallocHost(&c->pinned, 64 * sizeof(uint64_t)));
-        CU_CHECK(cudaMalloc(&c->d_error, 4 * sizeof(int)));
-        CU_CHECK(cudaMemset(c->d_error, 0, 4 * sizeof(int)));
+        CU_CHECK(cudaMalloc(&c->d_error, 8 * sizeof(int)));
+        CU_CHECK(cudaMemset(c->d_error, 0, 8 * sizeof(int)));
+        c->d_ticket = reinterpret_cast<unsigned*>(c->d_error) + 4;
         CU_CHECK(cudaMalloc(&c->d_mma, 2 * sizeof(unsigned long long)));
         CU_CHECK(cudaMemset(c->d_mma, 0, 2 * sizeof(unsigned long long)));
         cudaDeviceProp prop{};

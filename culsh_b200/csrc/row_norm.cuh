@@ -15,11 +15,12 @@ constexpr int RN_MAX_BLOCKS = 592;  // four CTAs an SM
 constexpr int RN_LOADS = 8;          // of a lane in flight
 
 // A warp per row, sums in float64.  The last CTA to finish adds up the partial sums, in one order, so that
-// the result does not depend on which one that is.  `ticket` comes zeroed.
+// the result does not depend on which one that is, and leaves the mean in page-locked host memory, and the ticket zero, as it was
+// before.  (A word to clear before the kernel and a copy behind it took longer than the kernel: 1,000 x 100, the call 25.3 us, 17.2 now.)
 template <typename T>
 __global__ void __launch_bounds__(RN_THREADS)
 mean_row_norm_kernel(const T* __restrict__ X, int n, int d, double* __restrict__ partial, unsigned* __restrict__ ticket,
-                     double* __restrict__ mean) {
+                     double* mean) {
     __shared__ double s_sum[RN_THREADS / 32];
     __shared__ bool s_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -49,7 +50,7 @@ mean_row_norm_kernel(const T* __restrict__ X, int n, int d, double* __restrict__
         for (int w = 0; w < WARPS; ++w) s += s_sum[w];
         partial[blockIdx.x] = s;
         __threadfence();
-        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        s_last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
     }
     __syncthreads();
     if (s_last && warp == 0) {
@@ -65,13 +66,12 @@ mean_row_norm_kernel(const T* __restrict__ X, int n, int d, double* __restrict__
 template <typename T>
 inline double mean_row_norm(const CtxPtr& c, const T* X, int n, int d) {
     const int blocks = (int)std::min<size_t>(ceil_div(n, RN_THREADS / 32), RN_MAX_BLOCKS);
-    Scratch<double> buf(c, SL_MISC2, RN_MAX_BLOCKS + 2);  // mean, ticket, partial sums
-    CU_CHECK(cudaMemsetAsync(buf.p, 0, 2 * sizeof(double), c->stream));
-    mean_row_norm_kernel<T><<<blocks, RN_THREADS, 0, c->stream>>>(X, n, d, buf.p + 2, reinterpret_cast<unsigned*>(buf.p + 1), buf.p);
+    Scratch<double> partial(c, SL_MISC2, RN_MAX_BLOCKS);
+    double* const mean = reinterpret_cast<double*>(c->pinned + HS_NORM);
+    mean_row_norm_kernel<T><<<blocks, RN_THREADS, 0, c->stream>>>(X, n, d, partial.p, c->d_ticket, mean);
     KERNEL_CHECK();
-    double mean = 0.0;
-    read_words(c, buf.p, sizeof(double), &mean);
-    return mean;
+    CU_CHECK(cudaStreamSynchronize(c->stream));
+    return *mean;
 }
 
 }  // namespace culsh_b200
