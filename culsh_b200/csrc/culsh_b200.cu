@@ -1066,10 +1066,12 @@ bool query_batch(const culsh_index& ix, int n_q, HashFn&& hash_fn, culsh_candida
     if (pairs <= LS_MAX_PAIRS) {
         count = [&](const RawCounts& r) {
             const unsigned ctas = pairs <= LS_ONE_PAIRS ? 1u : LS_CTAS;
+            int group = 1;  // lanes of a pair
+            while (group < LS_GROUP && pairs * group * 2 <= (size_t)ctas * LS_THREADS) group *= 2;
             CULSH_DISPATCH_NW(NW, launch_cluster(c->stream, lookup_count_kernel<NW>, ctas, ctas, LS_THREADS, 0, (const uint32_t*)qkeys.p,
                                                  (const uint8_t*)ovf.p, n_q, ix.L, (const uint32_t*)ix.bucket_keys.p,
                                                  (const int32_t*)ix.bucket_offsets.p, (const int32_t*)ix.table_offsets.p, bounds.p, r.cnt, r.off,
-                                                 r.big_list, r.mid_list, r.counters, r.mid_max, r.uniq, r.host));
+                                                 r.big_list, r.mid_list, r.counters, r.mid_max, r.uniq, group, r.host));
         };
     } else {
         CULSH_DISPATCH_NW(NW, launch_lookup<NW>(c, qkeys.p, ovf.p, n_q, ix.L, ix.bucket_keys.p, ix.bucket_offsets.p,

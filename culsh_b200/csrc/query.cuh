@@ -29,23 +29,46 @@ __device__ __forceinline__ int compare_keys(const uint32_t* __restrict__ a,
 // bounds[t*n_q + q] = the matched bucket's list [x, y) in `cand`, (0, 0) when there is none.  Table
 // major, like the query keys: neighbouring threads (queries) read and write neighbouring words here,
 // in the count and in the warp path, and a self-join writes the same array from its buckets.
+//
+// `group` neighbouring lanes (a power of two) search for one pair, each looking at a bucket of its own in every step, so that a step leaves
+// 1 / (group + 1) of them.  idx is that of the group's pair, `have` whether it has one.  Called by whole warps.
 template <int NW>
 __device__ __forceinline__ int2 lookup_pair(const uint32_t* __restrict__ qkeys, const uint8_t* __restrict__ q_ovf, int n_q,
-                                            size_t idx, const uint32_t* __restrict__ bucket_keys,
+                                            size_t idx, bool have, int group, const uint32_t* __restrict__ bucket_keys,
                                             const int32_t* __restrict__ bucket_offsets, const int32_t* __restrict__ table_offsets) {
-    const int t = (int)(idx / n_q);
+    const int lane = threadIdx.x & 31, at = lane & (group - 1), first = lane - at;
+    const uint32_t mine = (group == 32 ? 0xFFFFFFFFu : (1u << group) - 1u) << first;
     uint32_t key[NW];
-    load_key<NW>(qkeys + idx * NW, key);
-    int lo = table_offsets[t], hi = table_offsets[t + 1] - 1;
-    int2 found = make_int2(0, 0);
-    if (q_ovf && q_ovf[idx]) hi = lo - 1;  // value outside the index's narrow range: no bucket
-    while (lo <= hi) {
-        int mid = lo + ((hi - lo) >> 1);
-        int c = compare_keys<NW>(key, bucket_keys + (size_t)mid * NW);
-        if (c == 0) { found = make_int2(bucket_offsets[mid], bucket_offsets[mid + 1]); break; }
-        if (c < 0) hi = mid - 1; else lo = mid + 1;
+    int lo = 0, hi = 0, found = -1;
+    if (have) {
+        const int t = (int)(idx / n_q);
+        load_key<NW>(qkeys + idx * NW, key);
+        lo = table_offsets[t];
+        hi = table_offsets[t + 1];
+        if (q_ovf && q_ovf[idx]) hi = lo;  // value outside the index's narrow range: no bucket
     }
-    return found;
+    while (__any_sync(0xFFFFFFFFu, lo < hi)) {
+        const int len = hi - lo;
+        const bool few = len <= group;
+        auto place = [&](int i) { return few ? lo + i : lo + (int)((int64_t)(i + 1) * len / (group + 1)); };
+        int c = 1;  // of the bucket and the key
+        if (few ? at < len : lo < hi) c = compare_keys<NW>(bucket_keys + (size_t)place(at) * NW, key);
+        const uint32_t below = __ballot_sync(0xFFFFFFFFu, c < 0) & mine, same = __ballot_sync(0xFFFFFFFFu, c == 0) & mine;
+        if (lo < hi) {
+            const int n = __popc(below);  // the first n of them
+            if (same) {
+                found = place(__ffs(same) - 1 - first);
+                hi = lo;
+            } else if (few) {
+                hi = lo;
+            } else {
+                const int end = n < group ? place(n) : hi;
+                if (n > 0) lo = place(n - 1) + 1;
+                hi = end;
+            }
+        }
+    }
+    return found < 0 ? make_int2(0, 0) : make_int2(bucket_offsets[found], bucket_offsets[found + 1]);
 }
 
 // A CTA takes a stretch of the queries of one table.  A search is a chain of dependent
@@ -183,23 +206,25 @@ raw_count_kernel(BoundsView bounds, int n_q, int L, bool self_join, uint64_t* __
 }
 
 // Few (table, query) pairs: lookup, raw counts, their scan and the counters in one launch
-// in place of five (memset, lookup, count, scan; one query against 32 tables, the whole call: 153 -> 143 us).  A
-// search is a chain of about twenty dependent reads of lines of their own, and what one SM can have in flight of them bounds
-// more than a few hundred: a cluster of eight CTAs then shares the pairs and adds the counts up in the shared memory of its
-// first CTA, which does the rest (1,600 pairs 18.1 -> 11.6 us).  At 512 pairs the two are alike, below them the cluster starts
-// 2 us later.  Up to 8,192 pairs the call as a whole is faster this way (1M rows x 32 tables, 2,080 pairs 71.3 -> 64.0 us, 8,192 86 ->
+// in place of five (memset, lookup, count, scan; one query against 32 tables, the whole call: 153 -> 143 us).  A thread's search is
+// a chain of about twenty dependent reads of lines of their own: as many lanes as there are threads for it share one, up to a warp (1M rows, the whole
+// call with a thread and with a warp: 32 pairs 75 and 66 us, 1,024 74 and 67, 3,200 76 and 72; eight lanes as good as 32, four 1 us worse).  Above
+// LS_ONE_PAIRS a cluster of eight CTAs shares the pairs and adds the counts up in the shared memory of its first CTA, which does the rest; it
+// starts 2 us later than one CTA, whose SM can have so many reads in flight (512 pairs in one CTA 75 us, 1,024 in the cluster 67).  Up to 8,192 pairs
+// the call as a whole is faster this way than with a launch for each step (1M rows x 32 tables, 2,080 pairs 71.3 -> 64.0 us, 8,192 86 ->
 // 67; 10M rows 102 -> 80 and 89 -> 85).
 constexpr int LS_THREADS = 1024;
 constexpr int LS_CTAS = 8;
-constexpr size_t LS_ONE_PAIRS = 512;
+constexpr size_t LS_ONE_PAIRS = 128;
 constexpr size_t LS_MAX_PAIRS = LS_CTAS * LS_THREADS;
+constexpr int LS_GROUP = 32;  // lanes that search for a pair, at most
 template <int NW>
 __global__ void __launch_bounds__(LS_THREADS)
 lookup_count_kernel(const uint32_t* __restrict__ qkeys, const uint8_t* __restrict__ q_ovf, int n_q, int L,
                     const uint32_t* __restrict__ bucket_keys, const int32_t* __restrict__ bucket_offsets,
                     const int32_t* __restrict__ table_offsets, int2* __restrict__ bounds, uint64_t* __restrict__ raw_cnt,
                     uint64_t* __restrict__ raw_off, uint32_t* __restrict__ big_list, uint32_t* __restrict__ mid_list,
-                    uint32_t* __restrict__ counters, int mid_max, uint64_t* __restrict__ uniq_cnt, HostWords host) {
+                    uint32_t* __restrict__ counters, int mid_max, uint64_t* __restrict__ uniq_cnt, int group, HostWords host) {
     behind_kernel_before(qkeys, q_ovf, bucket_keys, bucket_offsets, table_offsets, bounds, raw_cnt, raw_off, big_list, mid_list, counters, uniq_cnt);
     __shared__ uint32_t s_cnt[LS_MAX_PAIRS];  // at most as many queries as pairs
     __shared__ uint32_t s_counters[3];
@@ -212,10 +237,15 @@ lookup_count_kernel(const uint32_t* __restrict__ qkeys, const uint8_t* __restric
     const int rank = (int)cluster.block_rank(), share = (n_q * L + (int)cluster.num_blocks() - 1) / (int)cluster.num_blocks();
     uint32_t* const cnt = cluster.map_shared_rank(s_cnt, 0);
     cluster.sync();
-    for (int idx = rank * share + tid; idx < min(n_q * L, (rank + 1) * share); idx += LS_THREADS) {
-        const int2 b = lookup_pair<NW>(qkeys, q_ovf, n_q, idx, bucket_keys, bucket_offsets, table_offsets);
-        bounds[idx] = b;
-        if (b.y > b.x) atomicAdd(cnt + idx % n_q, (uint32_t)(b.y - b.x));
+    const int end = min(n_q * L, (rank + 1) * share), at_once = LS_THREADS / group;
+    for (int first = rank * share; first < end; first += at_once) {
+        const int idx = first + tid / group;
+        const bool have = idx < end;
+        const int2 b = lookup_pair<NW>(qkeys, q_ovf, n_q, idx, have, group, bucket_keys, bucket_offsets, table_offsets);
+        if (have && tid % group == 0) {
+            bounds[idx] = b;
+            if (b.y > b.x) atomicAdd(cnt + idx % n_q, (uint32_t)(b.y - b.x));
+        }
     }
     cluster.sync();
     if (rank > 0) return;
