@@ -10,14 +10,18 @@ from .utils import ensure_engine_array, get_array_info, get_logger, is_device_ar
 
 
 def _engine_takes_norms(xs) -> bool:
-    """Whether the engine's one-launch kernel or torch's norm gives the mean row norm.  The kernel saves the
-    conversion of float32 rows to float64, which counts from 256 columns on (10,000 x 256: 57 -> 46 us,
-    10,000 x 1,024: 91 -> 47), and two launches where a warp has one row (1,000 x 100: 41 -> 38); for
-    10,000 x 128 torch is as fast (42 against 45), for float64 rows, too (10,000 x 128: 36 against 41), and
-    for longer rows it spreads a row over more of the chip (50 x 200,000: 89 against 250)."""
+    """Whether the engine's one-launch kernel or torch's norm gives the mean row norm.  Up to 4,096 columns the
+    kernel is the faster one everywhere (1,000 x 100: 24 us and 42, 10,000 x 128: 27 and 36, 10,000 x 1,024: 31 and
+    82, float64 10,000 x 128: 26 and 35, 4,096 x 128: 25 and 26); it takes float32 rows that are few, many or long and
+    many float64 rows, and leaves the sizes between, where it gains least, to torch as before.  Longer rows torch
+    spreads over more of the chip (50 x 200,000: 83 against 324)."""
     import torch
     n, d = xs.shape
-    return xs.dtype == torch.float32 and xs.is_contiguous() and n > 0 and 0 < d <= 4096 and (n <= 1024 or d >= 256)
+    if not xs.is_contiguous() or n <= 0 or not 0 < d <= 4096:
+        return False
+    if xs.dtype == torch.float64:
+        return n >= 4096
+    return xs.dtype == torch.float32 and (n <= 1024 or n >= 4096 or d >= 256)
 
 
 class PStableLSH:

@@ -88,3 +88,14 @@ def test_pageable_memory_is_refused():
     X, out = np.ones((4, 4), np.float32), ctypes.c_double()
     h = get_handle()
     assert h.lib.culsh_mean_row_norm(h.ptr, X.ctypes.data, 4, 4, 0, ctypes.byref(out)) != 0
+
+
+@pytest.mark.parametrize("n,d,double,engine", [(4095, 63, False, False), (4096, 63, False, True), (4096, 63, True, True), (4095, 511, True, False),
+                                               (4096, 4097, False, False)])
+def test_many_rows_go_to_the_engine(n, d, double, engine, monkeypatch):
+    import torch
+    from culsh_b200 import PStableLSH, pstable_lsh
+    calls = []
+    monkeypatch.setattr(pstable_lsh, "mean_row_norm", lambda x: calls.append(x.shape) or 3.0)
+    PStableLSH._estimate_window_size(torch.ones((n, d), device="cuda", dtype=torch.float64 if double else torch.float32))
+    assert bool(calls) == engine
