@@ -1127,7 +1127,8 @@ dedupe_window_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds, c
         if (n_win == 1) uniq_cnt[q] = total;
         else if (total) atomicAdd(&uniq_cnt[q], (unsigned long long)total);
     }
-    // ---- 4. emit ----
+    // ---- 4. emit.  Most words have an id or none: the first goes without a loop (10,000 sets of 18,500 ids of a million rows: the whole case 2,331 ->
+    // 2,298 us; with two or three without one 2,296 and 2,317, and sparser sets slower). ----
     int32_t* out = tmp + raw_off[q] + skip + at;
     for (int g = g_begin; g < g_end; ++g) {
         const uint4 x = bm4[g * 32 + lane];
@@ -1144,10 +1145,10 @@ dedupe_window_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds, c
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             uint32_t bits = wv[j];
-            while (bits) {
-                *dst++ = id0 + j * 32 + (__ffs(bits) - 1);
-                bits &= bits - 1;
-            }
+            int32_t* const end = dst + __popc(bits);
+            if (bits) *dst = id0 + j * 32 + (__ffs(bits) - 1);
+            for (bits &= bits - 1; bits; bits &= bits - 1) *++dst = id0 + j * 32 + (__ffs(bits) - 1);
+            dst = end;
         }
         out += __shfl_sync(0xFFFFFFFFu, inc, 31);
     }
