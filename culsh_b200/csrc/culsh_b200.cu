@@ -1068,6 +1068,7 @@ bool query_batch(const culsh_index& ix, int n_q, HashFn&& hash_fn, culsh_candida
             const unsigned ctas = pairs <= LS_ONE_PAIRS ? 1u : LS_CTAS;
             int group = 1;  // lanes of a pair
             while (group < LS_GROUP && pairs * group * 2 <= (size_t)ctas * LS_THREADS) group *= 2;
+            if (group == 2) group = 1;  // two lanes are slower than one
             CULSH_DISPATCH_NW(NW, launch_cluster(c->stream, lookup_count_kernel<NW>, ctas, ctas, LS_THREADS, 0, (const uint32_t*)qkeys.p,
                                                  (const uint8_t*)ovf.p, n_q, ix.L, (const uint32_t*)ix.bucket_keys.p,
                                                  (const int32_t*)ix.bucket_offsets.p, (const int32_t*)ix.table_offsets.p, bounds.p, r.cnt, r.off,

@@ -30,10 +30,28 @@ __device__ __forceinline__ int compare_keys(const uint32_t* __restrict__ a,
 // major, like the query keys: neighbouring threads (queries) read and write neighbouring words here,
 // in the count and in the warp path, and a self-join writes the same array from its buckets.
 //
-// `group` neighbouring lanes (a power of two) search for one pair, each looking at a bucket of its own in every step, so that a step leaves
-// 1 / (group + 1) of them.  idx is that of the group's pair, `have` whether it has one.  Called by whole warps.
+// One thread for a pair, or `group` neighbouring lanes (a power of two), each looking at a bucket of its own in every step, so that a step leaves
+// 1 / (group + 1) of them: idx is that of the group's pair then, `have` whether it has one, and whole warps call.
 template <int NW>
 __device__ __forceinline__ int2 lookup_pair(const uint32_t* __restrict__ qkeys, const uint8_t* __restrict__ q_ovf, int n_q,
+                                            size_t idx, const uint32_t* __restrict__ bucket_keys,
+                                            const int32_t* __restrict__ bucket_offsets, const int32_t* __restrict__ table_offsets) {
+    const int t = (int)(idx / n_q);
+    uint32_t key[NW];
+    load_key<NW>(qkeys + idx * NW, key);
+    int lo = table_offsets[t], hi = table_offsets[t + 1] - 1;
+    int2 found = make_int2(0, 0);
+    if (q_ovf && q_ovf[idx]) hi = lo - 1;  // value outside the index's narrow range: no bucket
+    while (lo <= hi) {
+        int mid = lo + ((hi - lo) >> 1);
+        int c = compare_keys<NW>(key, bucket_keys + (size_t)mid * NW);
+        if (c == 0) { found = make_int2(bucket_offsets[mid], bucket_offsets[mid + 1]); break; }
+        if (c < 0) hi = mid - 1; else lo = mid + 1;
+    }
+    return found;
+}
+template <int NW>
+__device__ __forceinline__ int2 lookup_pair_together(const uint32_t* __restrict__ qkeys, const uint8_t* __restrict__ q_ovf, int n_q,
                                             size_t idx, bool have, int group, const uint32_t* __restrict__ bucket_keys,
                                             const int32_t* __restrict__ bucket_offsets, const int32_t* __restrict__ table_offsets) {
     const int lane = threadIdx.x & 31, at = lane & (group - 1), first = lane - at;
@@ -208,7 +226,7 @@ raw_count_kernel(BoundsView bounds, int n_q, int L, bool self_join, uint64_t* __
 // Few (table, query) pairs: lookup, raw counts, their scan and the counters in one launch
 // in place of five (memset, lookup, count, scan; one query against 32 tables, the whole call: 153 -> 143 us).  A thread's search is
 // a chain of about twenty dependent reads of lines of their own: as many lanes as there are threads for it share one, up to a warp (1M rows, the whole
-// call with a thread and with a warp: 32 pairs 75 and 66 us, 1,024 74 and 67, 3,200 76 and 72; eight lanes as good as 32, four 1 us worse).  Above
+// call with a thread and with a warp: 32 pairs 75 and 66 us, 1,024 74 and 67; eight lanes as good as 32, four 1 us worse; two lanes 2 to 4 us slower than one).  Above
 // LS_ONE_PAIRS a cluster of eight CTAs shares the pairs and adds the counts up in the shared memory of its first CTA, which does the rest; it
 // starts 2 us later than one CTA, whose SM can have so many reads in flight (512 pairs in one CTA 75 us, 1,024 in the cluster 67).  Up to 8,192 pairs
 // the call as a whole is faster this way than with a launch for each step (1M rows x 32 tables, 2,080 pairs 71.3 -> 64.0 us, 8,192 86 ->
@@ -241,7 +259,9 @@ lookup_count_kernel(const uint32_t* __restrict__ qkeys, const uint8_t* __restric
     for (int first = rank * share; first < end; first += at_once) {
         const int idx = first + tid / group;
         const bool have = idx < end;
-        const int2 b = lookup_pair<NW>(qkeys, q_ovf, n_q, idx, have, group, bucket_keys, bucket_offsets, table_offsets);
+        int2 b = make_int2(0, 0);
+        if (group > 1) b = lookup_pair_together<NW>(qkeys, q_ovf, n_q, idx, have, group, bucket_keys, bucket_offsets, table_offsets);
+        else if (have) b = lookup_pair<NW>(qkeys, q_ovf, n_q, idx, bucket_keys, bucket_offsets, table_offsets);
         if (have && tid % group == 0) {
             bounds[idx] = b;
             if (b.y > b.x) atomicAdd(cnt + idx % n_q, (uint32_t)(b.y - b.x));
