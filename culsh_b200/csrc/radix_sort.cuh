@@ -19,7 +19,8 @@
 // key and the row id travel PACKED in one 64-bit item (key << 24 | id) between the first and the
 // last pass: 8 bytes per item instead of 12 and no separate id array in the passes in between.
 //
-// Keys of four words and more (MinHash from three hashes on, wide p-stable keys) stay where they are: the
+// Keys of four words and more (MinHash from three hashes on, wide p-stable keys), in tables too long for the splitters
+// (see splitter_sort.cuh, which takes most of them), stay where they are: the
 // sort runs over one word of the key at a time, least significant first, and what it moves are
 // (word, row id) pairs.  See radix_sort_words.
 #pragma once
