@@ -66,3 +66,50 @@ def test_many_rows():
     lengths = rng.integers(33, 300, 6000)
     indices, indptr = _rows(lengths, 1 << 22, rng)
     _check(core_mod.MinHashCore(32, 4, 2), indices, indptr, 6000, 1 << 22, 32, 4)
+
+
+def _around_the_last_id(a, b, m, alike, rng):
+    """A row that ends with `m` ids whose mean is its last id and whose first forms are within 2^18 of each other, while that of the last id is far
+    from them.  With the last eight filled up by copies of the last id there are as many of it as of the ids around it, and their sums are the
+    same.  The values of all other ids are above those of both."""
+    p, alpha = oracle.MINHASH_PRIME, (int(a) * 2 ** 32 + oracle.MINHASH_PRIME // 2) // oracle.MINHASH_PRIME
+    f = lambda c: (int(a) * c + int(b)) % p  # noqa: E731
+    D = np.arange(1, 1 << 19, dtype=np.uint64)
+    y = D * np.uint64(alpha) & np.uint64(0xFFFFFFFF)
+    off = y * np.uint64(m) & np.uint64(0xFFFFFFFF)
+    off = np.minimum(off, np.uint64(2 ** 32) - off)
+    off[(y < 2 ** 28) | (y > 2 ** 32 - 2 ** 28)] = 2 ** 32
+    D = int(D[np.argmin(off)])
+    if off.min() >= 2 ** 18:
+        return None  # no such distance for this function
+    while True:
+        last = int(rng.integers(1 << 19, 1 << 20))
+        near = [last - D] * (m - 1) + [last + (m - 1) * D]
+        if f(near[0]) < 2 ** 30 and f(near[0]) + 2 ** 24 < f(last) < 0.95 * p:
+            break
+    others = []
+    while len(others) < 40 - 2 * m:  # 32, and those that leave room in the last eight for m, one and m - 1
+        c = int(rng.integers(0, 1 << 21))
+        if f(c) > f(last) + 2 ** 24:
+            others.append(c)
+    row = others[:1] * len(others) if alike else others
+    assert min(map(f, row + near + [last])) in map(f, near) and (len(row) + m + 1) % 8 == 9 - m
+    return row + near + [last]
+
+
+@pytest.mark.parametrize("alike", [False, True])
+@pytest.mark.parametrize("m", [2, 3, 4])
+def test_ids_around_the_last_one(m, alike):
+    """For each hash function a row whose least ones have the last id, which stands for the places behind it, in their middle."""
+    from culsh_b200 import _culsh_core as core_mod
+    L, k, d = 8, 4, 1 << 22
+    rng = np.random.default_rng(m)
+    for seed in (0, 42):
+        core = core_mod.MinHashCore(L, k, seed)
+        ix = core.fit(np.arange(40, dtype=np.int32), np.array([0, 40], np.int32), 1, d)
+        rows = [_around_the_last_id(a, b, m, alike, rng) for a, b in zip(ix.get_hash_a().ravel(), ix.get_hash_b().ravel())]
+        rows = [r for r in rows if r]
+        assert len(rows) > 3 * L * k // 4
+        indices = np.concatenate(rows).astype(np.int32)
+        indptr = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+        _check(core, indices, indptr, len(rows), d, L, k)
