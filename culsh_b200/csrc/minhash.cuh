@@ -111,7 +111,12 @@ __device__ __forceinline__ uint32_t min_plus5_short(uint32_t m, double a, double
 // ids below 2^20 4,199 and 2,970 us, 300,000 below 2^16 593 and 443, below 2^22 768 and 537; 20M uniform ids below 2^20 in rows of 33 812 and
 // 647, 110 705 and 344, 1,000 778 and 332.  Next to it the double forms take 8 % longer for 12 uniform ids below 2^20 a row (634 and 682),
 // between 3 % less and 2 % more for other short rows.
+//
+// An id that a row has twice is close to itself: rows of few different ids would have nearly all their minima evaluated again (300,000 rows of 20 to 200
+// ids, four different ones 4,670 us and 1,125 in the double forms, 16 4,570 and 1,195, 64 3,300 and 1,225, 200 1,760 and 1,390, 1,000
+// 855 and 894).  MH_ALIKE of the first 32 ids that the row has had before keep it from this form; to see that takes 10 us of 300,000 rows.
 constexpr int MH_LIST = 1024;
+constexpr int MH_ALIKE = 2;
 constexpr int MH_LIST_FROM = 33;
 constexpr uint32_t MH_TAG = MH_LIST / 8 - 1;
 constexpr int MH_COL_BITS = 22;  // rows with ids from 2^MH_COL_BITS on take the general forms
@@ -191,6 +196,10 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
         bool listed = NEAR && n_ids >= MH_LIST_FROM && n_ids <= MH_LIST;
         uint32_t largest = 0;
         if (listed) listed = !__any_sync(0xFFFFFFFFu, (uint32_t)ahead >> MH_COL_BITS);
+        if (listed) {  // rows that repeat their ids
+            const uint32_t alike = __match_any_sync(0xFFFFFFFFu, ahead);
+            listed = __popc(__ballot_sync(0xFFFFFFFFu, (alike & below) != 0u)) < MH_ALIKE;
+        }
         if (listed) {
             largest = (uint32_t)ahead;
             ids_row[lane] = largest + MH_LIST_ID;

@@ -113,3 +113,21 @@ def test_ids_around_the_last_one(m, alike):
         indices = np.concatenate(rows).astype(np.int32)
         indptr = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
         _check(core, indices, indptr, len(rows), d, L, k)
+
+
+@pytest.mark.parametrize("alike", [0, 1, 2, 3, 31])
+@pytest.mark.parametrize("late", [False, True])
+def test_rows_that_repeat_ids(alike, late):
+    """On both sides of the line from which rows that repeat ids keep to the other forms, with the repeated ones among a row's first 32 or behind them, next to
+    rows that do not."""
+    from culsh_b200 import _culsh_core as core_mod
+    rng = np.random.default_rng(alike)
+    rows = []
+    for n in [33, 34, 64, 65, 200, 1024] * 20:
+        ids = rng.permutation(1 << 20)[:n]
+        first = 32 if late else 0
+        for j in range(min(alike, n - first - 1)):
+            ids[first + 1 + j] = ids[rng.integers(0, first + 1 + j)]
+        rows += [ids, rng.permutation(1 << 20)[:int(rng.integers(20, 80))]]
+    indptr = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    _check(core_mod.MinHashCore(16, 8, 3), np.concatenate(rows).astype(np.int32), indptr, len(rows), 1 << 20, 16, 8)
