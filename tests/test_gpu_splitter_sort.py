@@ -1,7 +1,7 @@
-"""Keys of four words and more are sorted by sampled splitters, word by word by radix passes or, as one bin, by one CTA: row
+"""Keys of two words and more are sorted by sampled splitters, word by word by radix passes or, as one bin, by one CTA: row
 counts on both sides of a bin, of the change from one to several chunks of samples and of a tile, keys that end inside
 their words, and collections in which all rows are alike, come in order, repeat with a period or differ in one hash only, so that bins
-are full of equal keys and some are sorted in pieces."""
+are full of equal keys."""
 import numpy as np
 import pytest
 
@@ -32,6 +32,12 @@ def _rows(kind, n, rng):
         return rng.integers(0, 4000, (7, 6))[np.arange(n) % 7]
     if kind == "last":  # every row starts with the same ids
         return np.concatenate([np.tile(rng.integers(0, 50, 5), (n, 1)), rng.integers(0, 1 << 19, (n, 1))], axis=1)
+    if kind == "near":  # sets of 30 ids that differ in one: most hashes are the same in all rows
+        return np.concatenate([np.tile(np.arange(29), (n, 1)), rng.integers(0, max(2, n // 8), (n, 1))], axis=1)
+    if kind == "but one":  # in the last place, in the first or in the middle
+        rows = np.tile(rng.integers(0, 400, 6), (n, 1))
+        rows[rng.choice([0, n // 2, n - 1])] += 1
+        return rows
     rows = rng.integers(0, 1 << 19, (max(1, n // 40), 6))[rng.integers(0, max(1, n // 40), n)]
     if kind == "sorted":
         return rows[np.lexsort(rows.T)]
@@ -51,24 +57,51 @@ def test_order(n, k, kind, splitters, monkeypatch):
         monkeypatch.setenv("CULSH_SORT_SPLITTERS", splitters)
     rng = np.random.default_rng(n + k)
     L = 2
-    indices = np.ascontiguousarray(_rows(kind, n, rng).astype(np.int32)).ravel()
-    indptr = (6 * np.arange(n + 1)).astype(np.int32)
+    rows = _rows(kind, n, rng)
+    indices = np.ascontiguousarray(rows.astype(np.int32)).ravel()
+    indptr = (rows.shape[1] * np.arange(n + 1)).astype(np.int32)
     core = core_mod.MinHashCore(L, k, 7)
     _check(core, core.fit(indices, indptr, n, 1 << 19), indices, indptr, n, L, k)
 
 
-def test_wide_p_stable_keys_and_many_tables():
-    """Values of two bytes (keys of four words with zeros in front), in more tables than the chip has SMs, and of one byte that span too much for the
-    compressed sort."""
+@pytest.mark.parametrize("n,k,kind", [
+    (300, 5, "alike"), (300, 16, "but one"), (2048, 8, "alike"), (2048, 5, "near"), (2047, 9, "near"), (2048, 16, "but one"), (5000, 16, "alike"), (20_000, 5, "near"),
+    (20_000, 16, "near"), (20_000, 8, "alike"), (40_000, 7, "few"), (40_000, 12, "but one"), (300_000, 5, "few"), (300_000, 8, "near"), (300_000, 10, "period")])
+def test_wide_keys_that_repeat(n, k, kind, monkeypatch):
+    """Keys of eight and sixteen words whose first words are the same in all rows of a bin or in many: the words behind them are looked at only
+    where there are rows that are not alike."""
+    test_order(n, k, kind, "1", monkeypatch)
+
+
+def _largest_bin(order, n):
+    """Rows of the fullest bin of a table whose rows come in this order, from the rows that the sort takes as samples."""
+    bins = 1
+    while bins * 1024 < n:
+        bins *= 2
+    samples = max(512, 8 * bins)
+    g = np.arange(samples, dtype=np.uint64)
+    r0, r1 = g * np.uint64(n) // np.uint64(samples), (g + np.uint64(1)) * np.uint64(n) // np.uint64(samples)
+    h = (g.astype(np.uint32) + np.uint32(1)) * np.uint32(0x9E3779B9)
+    for shift, factor in ((16, 0x85EBCA6B), (13, 0xC2B2AE35), (16, 1)):
+        h = (h ^ (h >> np.uint32(shift))) * np.uint32(factor)
+    place = np.empty(n, np.int64)
+    place[order] = np.arange(n)
+    at = np.sort(place[(r0 + h % (r1 - r0)).astype(np.int64)])[samples // bins::samples // bins]
+    return int(np.diff(np.concatenate([[0], at, [n]])).max())
+
+
+@pytest.mark.parametrize("n,k,kind", [(524_288, 2, "mixed"), (1_048_576, 2, "mixed"), (524_288, 3, "last"), (524_288, 6, "mixed"), (524_288, 8, "near"), (524_288, 9, "last"), (524_288, 16, "near")])
+def test_bins_in_pieces(n, k, kind):
+    """Tables whose bins hold 1,024 rows on average, so that some hold more than the 2,048 that a CTA sorts at once.  (Not where
+    few keys differ: rows that are alike come in the order of their ids, which the samples cover evenly.)"""
     from culsh_b200 import _culsh_core as core_mod
-    rng = np.random.default_rng(1)
-    for n, L, k, scale in [(3000, 150, 5, 300), (50_000, 2, 12, 300), (1500, 3, 8, 6), (12_288, 40, 8, 6), (100_003, 2, 7, 6)]:
-        X = (scale * rng.standard_normal((n, 6))).astype(np.float32)
-        core = core_mod.PSLSHCore(L, k, 1, 3)
-        ix = core.fit_float(X, n, 6)
-        assert ix.elem_bytes == (2 if scale == 300 else 1)
-        sig, got = core.hash(X, ix), ix.get_candidate_indices()
-        for t in range(0, L, 37):
-            raw = np.ascontiguousarray(sig[t]).view(np.uint8).reshape(n, 4 * k)
-            order = np.lexsort(tuple(raw[:, j] for j in range(4 * k - 1, -1, -1)))
-            assert np.array_equal(got[t * n:(t + 1) * n], order)
+    rng = np.random.default_rng(k)
+    rows = _rows(kind, n, rng)
+    indices = np.ascontiguousarray(rows.astype(np.int32)).ravel()
+    indptr = (rows.shape[1] * np.arange(n + 1)).astype(np.int32)
+    core = core_mod.MinHashCore(2, k, 7)
+    ix = core.fit(indices, indptr, n, 1 << 19)
+    assert core.last_stats()["sort_ctas"] == -1
+    _check(core, ix, indices, indptr, n, 2, k)
+    order = ix.get_candidate_indices()  # as _check has found it to be
+    assert max(_largest_bin(order[t * n:(t + 1) * n], n) for t in range(2)) > 2048
