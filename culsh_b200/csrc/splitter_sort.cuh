@@ -26,6 +26,7 @@ constexpr int SS_CAP = SS_THREADS * SS_ITEMS;   // rows that a CTA sorts at once
 constexpr int SS_BIN_ROWS = 1024;               // rows of a bin on average, at most
 constexpr int SS_OVER = 8;                      // samples for each bin, at least
 constexpr int SS_MAX_BINS = 4096;
+constexpr int SS_FROM = 12288, SS_FROM_12 = 16384;  // see sort_by_splitters
 constexpr int SS_TILE = 16384, SS_SHORT_TILE = 4096;  // rows of a CTA that classifies or scatters, and where these would be few
 constexpr int SS_TILE_THREADS = 512;
 
@@ -829,6 +830,10 @@ inline bool splitters_can(int n, int NW) { return NW >= 2 && splitter_bins(n) <=
 // passes and this way: 32 tables of 16-byte keys, 1,000 rows 53 and 22 us, 12,000 104 and 103, 30,000 316 and 132, 100,003 570 and 265,
 // 500,000 1,789 and 1,051, 2M 6,061 and 4,134; 16 tables of 9-byte keys, 1M rows 1,070 and 926; of 8-byte keys, 100,003 rows 214 and 125, 1M
 // 1,143 and 853, compressed 558 and 879; of 5-byte keys, 1M 741 and 826.
+// In those longer tables the radix sort is the faster one where keys repeat, and the more so the fewer bytes a key has.  8 tables, all keys different, groups of
+// near duplicates, ten different keys: 12,289 of 12 bytes 74 and 69 us, 60 and 75, 54 and 84, so that these go this way above SS_FROM_12 rows, 20,000 93 and
+// 75, 70 and 79, 62 and 79; 12,289 of 16 bytes 95 and 69, 74 and 77, 68 and 85; of 20 bytes 115 and 67, 91 and 118, 84 and 145; 40,000 of 20
+// bytes 236 and 74, 160 and 132, 140 and 161.
 // CULSH_SORT_SPLITTERS=0 / 1: never / wherever it can.
 inline bool sort_by_splitters(const CtxPtr& c, int n, int L, int NW, int KB, bool compressed) {
     if (!splitters_can(n, NW)) return false;
@@ -836,7 +841,7 @@ inline bool sort_by_splitters(const CtxPtr& c, int n, int L, int NW, int KB, boo
     if (e && *e) return atoi(e) != 0;
     if (n <= SS_CAP) return true;
     if (compressed || KB < 7) return false;
-    return (NW >= 4 && n > RSS_THREADS * 12) || !radix_sort_is_small(c, n, L, NW, compressed);
+    return (NW >= 4 && n > (KB <= 12 ? SS_FROM_12 : SS_FROM)) || !radix_sort_is_small(c, n, L, NW, compressed);
 }
 
 // keys[0] -> keys[1], row ids to vals[1]; vals[0] is scratch.

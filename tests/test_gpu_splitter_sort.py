@@ -105,3 +105,31 @@ def test_bins_in_pieces(n, k, kind):
     _check(core, ix, indices, indptr, n, 2, k)
     order = ix.get_candidate_indices()  # as _check has found it to be
     assert max(_largest_bin(order[t * n:(t + 1) * n], n) for t in range(2)) > 2048
+
+
+@pytest.mark.parametrize("n,k,route", [(16_384, 3, 4), (16_385, 3, -1), (12_288, 4, 4), (12_289, 4, -1), (12_289, 8, -1), (2048, 3, -1), (2049, 3, 1)])
+def test_which_sort(n, k, route):
+    """Lines between the sorts, in 32 tables: clusters of four CTAs, one CTA and splitters."""
+    from culsh_b200 import _culsh_core as core_mod
+    rng = np.random.default_rng(n)
+    indices, indptr = rng.integers(0, 1 << 19, 6 * n).astype(np.int32), (6 * np.arange(n + 1)).astype(np.int32)
+    core = core_mod.MinHashCore(32, k, 7)
+    core.fit(indices, indptr, n, 1 << 19)
+    assert core.last_stats()["sort_ctas"] == route
+
+
+def test_wide_p_stable_keys_and_many_tables():
+    """Values of two bytes (keys of four words with zeros in front), in more tables than the chip has SMs, and of one byte that span too much for the
+    compressed sort."""
+    from culsh_b200 import _culsh_core as core_mod
+    rng = np.random.default_rng(1)
+    for n, L, k, scale in [(3000, 150, 5, 300), (50_000, 2, 12, 300), (1500, 3, 8, 6), (12_288, 40, 8, 6), (100_003, 2, 7, 6)]:
+        X = (scale * rng.standard_normal((n, 6))).astype(np.float32)
+        core = core_mod.PSLSHCore(L, k, 1, 3)
+        ix = core.fit_float(X, n, 6)
+        assert ix.elem_bytes == (2 if scale == 300 else 1)
+        sig, got = core.hash(X, ix), ix.get_candidate_indices()
+        for t in range(0, L, 37):
+            raw = np.ascontiguousarray(sig[t]).view(np.uint8).reshape(n, 4 * k)
+            order = np.lexsort(tuple(raw[:, j] for j in range(4 * k - 1, -1, -1)))
+            assert np.array_equal(got[t * n:(t + 1) * n], order)
