@@ -504,9 +504,7 @@ struct SortBuffers {
         keys[1].reserve(c, SL_KEYS1, items * ks.key_words);
         vals_out.alloc(c, items);
         vals_tmp.reserve(c, SL_VALS, items);
-        size_t words = radix_sort_tile_words(n, L, ks.key_words);
-        if (splitters_can(n, ks.key_words)) words = std::max(words, splitter_plan(n, L).words);
-        tile_hist.reserve(c, SL_STATUS, words);
+        tile_hist.reserve(c, SL_STATUS, radix_sort_tile_words(n, L, ks.key_words));
     }
     // the last pass must write the row ids into vals_out
     void set_final(int buf) {
@@ -582,7 +580,8 @@ int build_index(culsh_index& ix, SortBuffers& sb, Scratch<uint32_t>* bounds, Sta
         passes = splitters ? 1 : radix_sort_passes(ix.ks.key_bytes, compressed);
         sb.set_final(splitters ? 1 : radix_sort_final(c, passes, n, L, NW, compressed));
         uint32_t* vp[2] = {sb.vals[0], sb.vals[1]};
-        if (splitters) {
+        if (splitters) {  // only now: their counts grow with the square of the rows (4M rows 4 MB a table)
+            sb.tile_hist.reserve(c, SL_STATUS, splitter_plan(n, L).words);
             switch (NW) {
                 case 2: cur = splitter_sort_tables<2>(c, kp, vp, n, L, ix.ks.key_bytes, sb.tile_hist.p); break;
                 case 4: cur = splitter_sort_tables<4>(c, kp, vp, n, L, ix.ks.key_bytes, sb.tile_hist.p); break;

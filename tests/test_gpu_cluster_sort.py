@@ -37,14 +37,21 @@ def test_order_of_the_host(n, L, family, k, scale):
 
 @pytest.mark.parametrize("n,L", SHAPES)
 @pytest.mark.parametrize("k", [3, 5, 9])
-def test_wide_keys(n, L, k):
+@pytest.mark.parametrize("splitters", [None, "0"])
+def test_wide_keys(n, L, k, splitters, monkeypatch):
+    """As they come, which is by splitters up to 2,048 and from 12,289 or 16,385 rows on, and without them."""
     from culsh_b200 import _culsh_core as core_mod
+    if splitters:
+        monkeypatch.setenv("CULSH_SORT_SPLITTERS", splitters)
     rng = np.random.default_rng(n + k)
     sets = rng.integers(0, 400, (n // 3 + 1, 6)).astype(np.int32)
     indices = np.ascontiguousarray(sets[rng.integers(0, len(sets), n)]).ravel()
     indptr = (6 * np.arange(n + 1)).astype(np.int32)
     core = core_mod.MinHashCore(L, k, 7)
     ix = core.fit(indices, indptr, n, 400)
+    if splitters:
+        ctas = 8 if L <= 13 and 4096 <= n <= 49_152 else 4 if L <= 32 and 8192 <= n <= 24_576 else int(n <= 12_288 and L <= 148)
+        assert core.last_stats()["sort_ctas"] == ctas
     _check(ix, core.hash(indices, indptr, n, ix), n, L)
 
 

@@ -1,5 +1,5 @@
-"""Keys of four words and more are sorted word by word, tables of more than 12,288 rows and, with the one-CTA sort
-switched off, shorter ones: row counts on both sides of the 4096-item tile, of the 96 tiles from which tile offsets
+"""Keys of four words and more are sorted word by word in tables of more than four million rows and, with splitters and
+the sorts in one launch switched off, in shorter ones: row counts on both sides of the 4096-item tile, of the 96 tiles from which tile offsets
 are scanned in chunks, and of whole chunks of 64 tiles, key lengths that end inside a word (16 to 64
 bytes, 8-word keys among them), and collections where the rows agree in the leading, the trailing or all hashes, so that
 the order depends on every word and equal keys keep their row order.  The chunked scan of one- and
@@ -20,8 +20,8 @@ TILE = 4096
                                  (128 * TILE + 1, 4), (2_097_153, 3)])
 def test_index_equals_oracle_order(n, k, monkeypatch):
     from culsh_b200 import _culsh_core as core_mod
-    if n <= 12_288:
-        monkeypatch.setenv("CULSH_SORT_NO_PACK", "1")
+    monkeypatch.setenv("CULSH_SORT_SPLITTERS", "0")  # which take all of these, as a rule
+    monkeypatch.setenv("CULSH_SORT_NO_PACK", "1")
     rng = np.random.default_rng(n)
     L = 2
     # row r of block b has b's set of ids with a few of the positions changed: many equal hashes
@@ -33,6 +33,7 @@ def test_index_equals_oracle_order(n, k, monkeypatch):
     indptr = (6 * np.arange(n + 1)).astype(np.int32)
     core = core_mod.MinHashCore(L, k, 7)
     ix = core.fit(indices, indptr, n, 400)
+    assert core.last_stats()["sort_ctas"] == 0 and core.last_stats()["sort_passes"] == 4 * k
     sig = core.hash(indices, indptr, n, ix)  # [L][n][k]
     # the order of the engine: unsigned bytes in memory order, ties by row
     got_c, got_b = ix.get_candidate_indices(), ix.get_bucket_signatures().reshape(-1, 4 * k)

@@ -133,3 +133,23 @@ def test_wide_p_stable_keys_and_many_tables():
             raw = np.ascontiguousarray(sig[t]).view(np.uint8).reshape(n, 4 * k)
             order = np.lexsort(tuple(raw[:, j] for j in range(4 * k - 1, -1, -1)))
             assert np.array_equal(got[t * n:(t + 1) * n], order)
+
+
+def test_no_scratch_where_another_sort_runs():
+    """Four million keys of eight bytes that are sorted in compressed form: the handle holds no more for them than for one row more, which the splitters do not
+    take in any form."""
+    import torch
+    from culsh_b200 import _culsh_core as core_mod
+    held = []
+    X = torch.randn(4_194_305, 4, device="cuda", generator=torch.Generator("cuda").manual_seed(2))
+    core = core_mod.PSLSHCore(16, 8, 2, 3)
+    for n in (4_194_304, 4_194_305):
+        core.trim_scratch(0)
+        ix = core.fit_float(X[:n], n, 4)
+        assert core.last_stats()["sort_ctas"] == 0 and core.last_stats()["sort_passes"] == 5
+        del ix
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        core.trim_scratch(0)
+        held.append(torch.cuda.mem_get_info()[0] - free)
+    assert held[0] <= held[1], held
