@@ -718,12 +718,18 @@ BoundsView self_bounds(const culsh_index& ix, const uint32_t* packed) {
 // -----------------------------------------------------------------------------------------
 // Query from the matched buckets' lists (bounds[t*n_q + q])
 // -----------------------------------------------------------------------------------------
+inline long env_long(const char* name, long dflt) {
+    const char* e = getenv(name);
+    return e && *e ? atol(e) : dflt;
+}
+
+// Rows of a window of the bitmap kernel: 2^20, or CULSH_BITMAP_BITS, read at every call (tests vary it).
 int bitmap_window_bits(const CtxPtr& c, int n_rows) {
     size_t fixed = bitmap_smem_bytes(0) + 1024;
     // a multiple of 4096 bits: the emission walks the window in 128-word groups
     size_t max_bits = ((c->smem_optin > fixed ? c->smem_optin - fixed : 0) * 8) / 4096 * 4096;
     size_t want = ((size_t)n_rows + 4095) / 4096 * 4096;
-    static const size_t cap_bits = [] { const char* e = getenv("CULSH_BITMAP_BITS"); return e ? (size_t)atol(e) : ((size_t)1 << 20); }();
+    const size_t cap_bits = std::max<size_t>(4096, (size_t)std::max(env_long("CULSH_BITMAP_BITS", 1 << 20), 0l) / 4096 * 4096);
     size_t cap = std::min<size_t>(max_bits, cap_bits);
     return (int)std::min(want, cap);
 }
@@ -744,17 +750,15 @@ constexpr long WINDOW_ROWS = 344064;
 // entries in 32 lists: three windows 16 us, 61 of them 8): smaller ones then, down to WINDOW_MIN_ROWS.
 constexpr long WINDOW_MIN_ROWS = 16384;
 constexpr size_t WINDOW_SEARCH = 512;  // CTAs that search their slices themselves: a launch less
-inline long env_long(const char* name, long dflt) {
-    const char* e = getenv(name);
-    return e && *e ? atol(e) : dflt;
-}
 struct Windows {
     int bits, n;
 };
 // Windows for `n_sets` large sets: as many rows as fit, but smaller ones as long as there are fewer than `ctas` of them in all.
-// However many there are, they are faster than a CTA for each set that visits windows of 2^20 rows in turn.  Whole calls, that way and
+// They are faster than a CTA for each set that visits windows of 2^20 rows in turn, wherever that was measured.  Whole calls, that way and
 // this: 3M rows x 16 tables, one set of 123,000 ids 290 and 78 us, 1,024 sets of 93,000 1,509 and 641; 8M x 8, 64 of
-// 380,000 2,492 and 270; 40M x 4, one of 9.8M 20,600 and 170, 256 of 5M 40,800 and 10,400.
+// 380,000 2,492 and 270; 40M x 4, one of 9.8M 20,600 and 170, 256 of 5M 40,800 and 10,400.  Sets of few ids for each window, the least that come here: 10M x
+// 16, 14,000 ids in 30 windows, one 257 and 85, 1,024 1,408 and 642, 40,000 49,300 and 21,300; 40M x 16, 12,600 in 117, 1,024 3,956 and 2,083, 40,000
+// (more slices than are precomputed) 144,000 and 91,600; 40M x 48, 17,400, 12,000 sets (too) 46,300 and 30,200; 100M x 16, 17,200 in 291, 1,024 8,660 and 4,937.
 Windows windows_for(int n_rows, size_t n_sets, size_t ctas) {
     const long env = env_long("CULSH_CHAIN_BITS", 0);
     const size_t cap_bits = std::max<size_t>(4096, (size_t)(env > 0 ? env : WINDOW_ROWS) / 4096 * 4096);
@@ -843,7 +847,7 @@ bool query_from_matched(const culsh_index& ix, const BoundsView& bounds, bool se
         KERNEL_CHECK();
         exclusive_scan<uint64_t, uint64_t>(s, raw_cnt.p, n_q, raw_off.p, scratch.p, host_raw);
     }
-    // Large sets: a CTA for each (query, window of the rows) where that is a few windows, else one for each query.
+    // Large sets: a CTA for each (query, window of the rows), or one for each query where there are more than CW_MAX_L tables or 2^31 pieces.
     const bool ahead = n_q <= AHEAD_QUERIES;
     Windows win = windows_for(ix.n, (size_t)n_q, ahead ? (size_t)AHEAD_PIECES : 0);
     const bool may_window = L <= CW_MAX_L && window_smem_bytes(win.bits) + 1024 <= c->smem_optin;
