@@ -139,9 +139,9 @@ __device__ __forceinline__ void decomp_key(uint32_t* k, KeyComp kc) {
 // ---------------------------------------------------------------------------------------
 template <int NW, bool COMP0>
 __global__ void __launch_bounds__(RS_THREADS)
-radix_tile_hist_kernel(const uint32_t* __restrict__ keys, int n, int tiles_per_table, int p, uint32_t sub,
+radix_tile_hist_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ keys, int n, int tiles_per_table, int p, uint32_t sub,
                        uint32_t* __restrict__ tile_hist) {
-    behind_kernel_before(keys, tile_hist);
+    kernel_before.wait(keys, tile_hist);
     using Cfg = SortCfg<NW>;
     __shared__ uint32_t s_hist[256];
     const int tile = blockIdx.x;
@@ -177,8 +177,8 @@ constexpr int RS_SCAN_THREADS = 1024;
 constexpr int RS_SCAN_SEGS = RS_SCAN_THREADS / 256;
 
 __global__ void __launch_bounds__(RS_SCAN_THREADS)
-radix_tile_scan_kernel(uint32_t* __restrict__ tile_hist, int tiles_per_table) {
-    behind_kernel_before(tile_hist);
+radix_tile_scan_kernel(KernelBefore kernel_before, uint32_t* __restrict__ tile_hist, int tiles_per_table) {
+    kernel_before.wait(tile_hist);
     __shared__ uint32_t s_seg[RS_SCAN_SEGS][256];
     __shared__ uint32_t s_base[256];
     __shared__ uint32_t s_warp[8];
@@ -227,9 +227,9 @@ constexpr int RS_CHUNK_TILES = 64;
 constexpr int RS_CHUNK_MIN_TILES = 96;  // tables with fewer tiles keep the single-launch scan
 
 __global__ void __launch_bounds__(RS_SCAN_THREADS)
-radix_tile_scan_chunk_kernel(uint32_t* __restrict__ tile_hist, int tiles_per_table, int n_chunks,
+radix_tile_scan_chunk_kernel(KernelBefore kernel_before, uint32_t* __restrict__ tile_hist, int tiles_per_table, int n_chunks,
                              uint32_t* __restrict__ chunk_tot /* [table][chunk][256] */) {
-    behind_kernel_before(tile_hist, chunk_tot);
+    kernel_before.wait(tile_hist, chunk_tot);
     __shared__ uint32_t s_seg[RS_SCAN_SEGS][256];
     const int d = threadIdx.x & 255, seg = threadIdx.x >> 8;
     const int table = blockIdx.x / n_chunks, chunk = blockIdx.x - table * n_chunks;
@@ -260,8 +260,8 @@ radix_tile_scan_chunk_kernel(uint32_t* __restrict__ tile_hist, int tiles_per_tab
 
 // one block of 256 threads per table: chunk_tot -> chunk bases, in place
 __global__ void __launch_bounds__(256)
-radix_chunk_base_kernel(uint32_t* __restrict__ chunk_tot, int n_chunks) {
-    behind_kernel_before(chunk_tot);
+radix_chunk_base_kernel(KernelBefore kernel_before, uint32_t* __restrict__ chunk_tot, int n_chunks) {
+    kernel_before.wait(chunk_tot);
     __shared__ uint32_t s_warp[8];
     const int d = threadIdx.x, lane = d & 31, w = d >> 5;
     uint32_t* ct = chunk_tot + (size_t)blockIdx.x * n_chunks * 256 + d;
@@ -319,11 +319,11 @@ constexpr int RS_PACK_ID_BITS = 24;
 
 template <int NW, bool FIRST, int COMP, bool PACK = false>
 __global__ void __launch_bounds__(RS_THREADS, 4)
-radix_scatter_kernel(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
+radix_scatter_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                      uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int n,
                      int tiles_per_table, int p, KeyComp kc, const uint32_t* __restrict__ tile_off,
                      const uint32_t* __restrict__ chunk_base /* or null */, int n_chunks) {
-    behind_kernel_before(keys_in, vals_in, keys_out, vals_out, tile_off, chunk_base);
+    kernel_before.wait(keys_in, vals_in, keys_out, vals_out, tile_off, chunk_base);
     using Cfg = SortCfg<NW>;
     constexpr int IPT = Cfg::IPT;
     constexpr int TILE = Cfg::TILE;
@@ -542,9 +542,9 @@ struct SmallSortCfg {
 // wait for; where they cannot the items go through in row order, and the host, which sees that later, sorts again.
 template <int NW, bool PACK>
 __global__ void __launch_bounds__(RSS_THREADS, 1)
-radix_sort_small_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
+radix_sort_small_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
                         uint32_t* __restrict__ vals_out, int n, int passes, bool compressed, KeyComp kc, const int* __restrict__ check) {
-    behind_kernel_before(keys_in, keys_out, vals_out, check);
+    kernel_before.wait(keys_in, keys_out, vals_out, check);
     using Cfg = SmallSortCfg<NW, PACK>;
     constexpr int KW = Cfg::KW, IPT = Cfg::IPT;
     constexpr bool WORDS = NW >= 4;
@@ -712,10 +712,10 @@ struct ClusterSortCfg {
 
 template <int NW, bool PACK>
 __global__ void __launch_bounds__(RSC_THREADS, 1)
-radix_sort_cluster_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
+radix_sort_cluster_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
                           uint32_t* __restrict__ vals_out, int n, int cta_rows, uint32_t cta_rows_inv, int passes, bool compressed,
                           KeyComp kc, const int* __restrict__ check) {
-    behind_kernel_before(keys_in, keys_out, vals_out, check);
+    kernel_before.wait(keys_in, keys_out, vals_out, check);
     using Cfg = ClusterSortCfg<NW, PACK>;
     constexpr int KW = Cfg::KW, IPT = Cfg::IPT;
     constexpr bool WORDS = NW >= 4;
@@ -1129,8 +1129,8 @@ __device__ __forceinline__ TOut block_exclusive_scan(TOut v, TOut* s_warp, TOut&
 
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(SCAN_THREADS)
-scan_reduce_kernel(const TIn* __restrict__ in, size_t n, TOut* __restrict__ block_sums) {
-    behind_kernel_before(in, block_sums);
+scan_reduce_kernel(KernelBefore kernel_before, const TIn* __restrict__ in, size_t n, TOut* __restrict__ block_sums) {
+    kernel_before.wait(in, block_sums);
     __shared__ TOut s_warp[32];
     size_t base = (size_t)blockIdx.x * SCAN_TILE;
     TOut sum = 0;
@@ -1164,8 +1164,8 @@ struct HostWords {
 
 template <typename TOut>
 __global__ void __launch_bounds__(1024)
-scan_block_sums_kernel(TOut* __restrict__ block_sums, size_t n_blocks, TOut* __restrict__ total_out, HostWords host) {
-    behind_kernel_before(block_sums, total_out);
+scan_block_sums_kernel(KernelBefore kernel_before, TOut* __restrict__ block_sums, size_t n_blocks, TOut* __restrict__ total_out, HostWords host) {
+    kernel_before.wait(block_sums, total_out);
     __shared__ TOut s_warp[32];
     TOut carry = 0;
     for (size_t base = 0; base < n_blocks; base += 1024) {
@@ -1182,9 +1182,9 @@ scan_block_sums_kernel(TOut* __restrict__ block_sums, size_t n_blocks, TOut* __r
 
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(SCAN_THREADS)
-scan_apply_kernel(const TIn* __restrict__ in, size_t n, const TOut* __restrict__ block_sums, bool scanned,
+scan_apply_kernel(KernelBefore kernel_before, const TIn* __restrict__ in, size_t n, const TOut* __restrict__ block_sums, bool scanned,
                   TOut* __restrict__ out, HostWords host) {
-    behind_kernel_before(in, block_sums, out);
+    kernel_before.wait(in, block_sums, out);
     __shared__ TOut s_warp[32];
     TOut before = 0;  // elements of the blocks before this one
     if (scanned) {
@@ -1233,8 +1233,8 @@ struct alignas(16) ScanVec {
 // in and out on 16-byte boundaries
 template <typename T>
 __global__ void __launch_bounds__(SCAN_ONE_THREADS)
-scan_one_kernel(const T* __restrict__ in, int n, T* __restrict__ out, HostWords host) {
-    behind_kernel_before(in, out);
+scan_one_kernel(KernelBefore kernel_before, const T* __restrict__ in, int n, T* __restrict__ out, HostWords host) {
+    kernel_before.wait(in, out);
     constexpr int PER = 16 / sizeof(T), VECS = SCAN_ONE_IPT / PER;
     __shared__ T s_warp[32];
     T carry = 0;
