@@ -371,12 +371,13 @@ enum DeviceErrorBits : int {
 };
 
 // A kernel that takes this as its first parameter may be set up while the one in front of it in the stream still runs, and starts with wait(): that lets the
-// next one do the same, and waits until the one before is done and what it wrote can be read.  launch_next and launch_cluster take no other kernels.  The
+// next one do the same, and waits until the one before is done and what it wrote can be read.  launch_next and launch_cluster take no others but KernelDone's.  The
 // pointers come back as ones that the compiler knows nothing of: a load through one that it takes for the only way to its memory could move to the front
 // of the wait (members of structs are not such; the wait is a barrier to them as it is).  A chain of short
 // kernels takes 0.6 us less for each of them (2.1 to 3.0 us in place of 2.6 to 3.7): one query 109 -> 101 us, 333,337 x 50 in 33 launches
 // 445 -> 409.  Kernels that fill the chip for long and are short of registers are launched as usual: what the compiler no longer knows
-// made the search among splitters 13 % slower and the sort of the bins 7 %.
+// made the search among splitters 13 % slower and the sort of the bins 7 %.  So are kernels with a CTA or two for each SM behind one whose CTAs have an SM
+// each: they gather on the SMs that are free first (148 tables of 3,000 keys of 64 bytes, the buckets' count behind the sort 36 us, 142 when launched early).
 struct KernelBefore {
     template <typename... T>
     __device__ __forceinline__ void wait(T&... pointers) const {
@@ -389,38 +390,44 @@ struct KernelBefore {
         (..., anew(pointers));
     }
 };
-template <typename... P, typename... A>
-inline void launch_next(cudaStream_t stream, void (*kern)(KernelBefore, P...), size_t grid, unsigned block, size_t smem, A... args) {
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+// For forms of a kernel that are launched as usual.
+struct KernelDone {
+    template <typename... T>
+    __device__ __forceinline__ void wait(T&...) const {}
+};
+template <bool EARLY>
+using EarlyIf = std::conditional_t<EARLY, KernelBefore, KernelDone>;
+
+// A launch in clusters of `ctas` CTAs each, `grid` is a multiple of that; one CTA is none.  `early`: as a KernelBefore allows.
+template <typename Before, typename... P, typename... A>
+inline void launch_with(bool early, cudaStream_t stream, void (*kern)(Before, P...), size_t grid, unsigned ctas, unsigned threads, size_t smem, A... args) {
+    static_assert(std::is_same<Before, KernelBefore>::value || std::is_same<Before, KernelDone>::value, "");
+    cudaLaunchAttribute attr[2]{};
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    CU_CHECK(cudaLaunchKernelEx(&cfg, kern, KernelBefore{}, static_cast<P>(args)...));
-}
-
-// A launch in clusters of `ctas` CTAs each; `grid` is a multiple of that.
-template <typename... P, typename... A>
-inline void launch_cluster(cudaStream_t stream, void (*kern)(KernelBefore, P...), unsigned grid, unsigned ctas, unsigned threads, size_t smem, A... args) {
-    cudaLaunchAttribute attr[2]{};
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = ctas;
-    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = attr;
-    cfg.numAttrs = ctas > 1 ? 2 : 1;  // an ordinary launch starts 2 us earlier
-    CU_CHECK(cudaLaunchKernelEx(&cfg, kern, KernelBefore{}, static_cast<P>(args)...));
+    if (early && std::is_same<Before, KernelBefore>::value) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (ctas > 1) {  // an ordinary launch starts 2 us earlier
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = ctas;
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
+    }
+    CU_CHECK(cudaLaunchKernelEx(&cfg, kern, Before{}, static_cast<P>(args)...));
+}
+template <typename Before, typename... P, typename... A>
+inline void launch_next(cudaStream_t stream, void (*kern)(Before, P...), size_t grid, unsigned threads, size_t smem, A... args) {
+    launch_with(true, stream, kern, grid, 1u, threads, smem, args...);
+}
+template <typename Before, typename... P, typename... A>
+inline void launch_cluster(cudaStream_t stream, void (*kern)(Before, P...), size_t grid, unsigned ctas, unsigned threads, size_t smem, A... args) {
+    launch_with(true, stream, kern, grid, ctas, threads, smem, args...);
     KERNEL_CHECK();
 }
 

@@ -592,7 +592,7 @@ int build_index(culsh_index& ix, SortBuffers& sb, Scratch<uint32_t>* bounds, Sta
             cur = radix_sort_tables(c, NW, kp, vp, n, L, ix.ks.key_bytes, sb.tile_hist.p, compressed, kc, check);
         }
         tm.mark();
-        CULSH_DISPATCH_NW(NW, launch_bucket_count<NW>(c->stream, kp[cur], n, L, tile_heads.p, heads.p));
+        CULSH_DISPATCH_NW(NW, launch_bucket_count<NW>(c, kp[cur], n, L, splitters ? 0 : radix_sort_short_ctas(c, n, L, NW, compressed), tile_heads.p, heads.p));
         exclusive_scan<uint32_t, uint32_t>(c->stream, tile_heads.p, n_tiles, tile_base.p, scratch.p,
                                            host_words(c, HS_BUCKETS, reinterpret_cast<const uint32_t*>(c->d_error) + 2, 2));
         // the one host round trip of the build: bucket total, range and self-check word

@@ -115,11 +115,16 @@ bucket_write_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ key
     }
 }
 
+// sort_ctas: CTAs for each table that sorted in the one launch in front, if there was one.  They leave their SMs one by one, and this kernel's CTAs, a
+// few for each SM, gather on the first where they are launched early.  With long keys and many tables that costs more than it saves.  Whole fits before early
+// launches, with all of them, and as it is: 148 tables of 3,000 keys of 64 bytes 400, 499 and 396 us, 32 of 8,192 486, 581 and 480, 48 of 5,000
+// 415, 435 and 414, 148 of 3,000 keys of 12 bytes 119, 120 and 115.
 template <int NW>
-inline void launch_bucket_count(cudaStream_t s, const uint32_t* keys, int n, int L,
+inline void launch_bucket_count(const CtxPtr& c, const uint32_t* keys, int n, int L, int sort_ctas,
                                 uint32_t* tile_heads, uint32_t* heads) {
     int tpt = (int)ceil_div(n, IB_TILE);
-    launch_next(s, bucket_count_kernel<NW>, (unsigned)((size_t)tpt * L), IB_THREADS, 0, keys, n, tpt, tile_heads, heads);
+    const bool early = NW < 4 || (size_t)std::max(sort_ctas, 0) * L * NW < 2 * (size_t)c->sm_count;
+    launch_with(early, c->stream, bucket_count_kernel<NW>, (size_t)tpt * L, 1u, IB_THREADS, 0, keys, n, tpt, tile_heads, heads);
     KERNEL_CHECK();
 }
 
