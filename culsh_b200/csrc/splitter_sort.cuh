@@ -27,7 +27,7 @@ constexpr int SS_BIN_ROWS = 1024;               // rows of a bin on average, at 
 constexpr int SS_OVER = 8;                      // samples for each bin, at least
 constexpr int SS_MAX_BINS = 4096;
 constexpr int SS_FROM = 12288, SS_FROM_12 = 16384;  // see sort_by_splitters
-constexpr int SS_TILE = 16384, SS_SHORT_TILE = 4096;  // rows of a CTA that classifies or scatters, and where these would be few
+constexpr int SS_TILE = 16384, SS_SHORT_TILE = 4096;  // rows of a CTA that classifies or scatters, and where these would be few, at least
 constexpr int SS_TILE_THREADS = 512;
 
 inline int splitter_bins(int n) {
@@ -804,7 +804,9 @@ inline SplitterPlan splitter_plan(int n, int L) {
     p.bins = splitter_bins(n);
     p.samples = std::max(512, p.bins * SS_OVER);  // powers of two
     p.chunks = (int)ceil_div(p.samples, SS_CAP);
-    p.tile = (size_t)L * ceil_div(n, SS_TILE) < 1024 ? SS_SHORT_TILE : SS_TILE;
+    // Short tiles fill the chip, but have as many counts as there are bins each: eight rows a bin at least (4 tables of 4M keys of 8 bytes, the sort with
+    // tiles of 4,096 1,570 us, of 16,384 1,115; one table of 100,003 97 and 106, of 1M 165, with 8,192 160, and 176).
+    p.tile = (size_t)L * ceil_div(n, SS_TILE) < 1024 ? std::min(std::max(SS_SHORT_TILE, 8 * p.bins), SS_TILE) : SS_TILE;
     p.tiles = (int)ceil_div(n, p.tile);
     constexpr size_t row_words = 5;  // of a RowList
     auto take = [&](size_t words) {
@@ -829,7 +831,8 @@ inline bool splitters_can(int n, int NW) { return NW >= 2 && splitter_bins(n) <=
 // radix sort does not take the table in one launch, and for keys of four words also in longer tables that it does.  The sort stage by radix
 // passes and this way: 32 tables of 16-byte keys, 1,000 rows 53 and 22 us, 12,000 104 and 103, 30,000 316 and 132, 100,003 570 and 265,
 // 500,000 1,789 and 1,051, 2M 6,061 and 4,134; 16 tables of 9-byte keys, 1M rows 1,070 and 926; of 8-byte keys, 100,003 rows 214 and 125, 1M
-// 1,143 and 853, compressed 558 and 879; of 5-byte keys, 1M 741 and 826.
+// 1,143 and 853, compressed 558 and 879; of 5-byte keys, 1M 741 and 826; of 8-byte keys, 4M rows x one table 372 and 416, x two 634 and 678, x four 1,182
+// and 1,117 (2M x one 268 and 242).
 // In those longer tables the radix sort is the faster one where keys repeat, and the more so the fewer bytes a key has.  8 tables, all keys different, groups of
 // near duplicates, ten different keys: 12,289 of 12 bytes 74 and 69 us, 60 and 75, 54 and 84, so that these go this way above SS_FROM_12 rows, 20,000 93 and
 // 75, 70 and 79, 62 and 79; 12,289 of 16 bytes 95 and 69, 74 and 77, 68 and 85; of 20 bytes 115 and 67, 91 and 118, 84 and 145; 40,000 of 20
@@ -840,7 +843,7 @@ inline bool sort_by_splitters(const CtxPtr& c, int n, int L, int NW, int KB, boo
     const char* e = getenv("CULSH_SORT_SPLITTERS");
     if (e && *e) return atoi(e) != 0;
     if (n <= SS_CAP) return true;
-    if (compressed || KB < 7) return false;
+    if (compressed || KB < 7 || (NW == 2 && L < 4 && splitter_bins(n) == SS_MAX_BINS)) return false;
     return (NW >= 4 && n > (KB <= 12 ? SS_FROM_12 : SS_FROM)) || !radix_sort_is_small(c, n, L, NW, compressed);
 }
 

@@ -107,13 +107,14 @@ def test_bins_in_pieces(n, k, kind):
     assert max(_largest_bin(order[t * n:(t + 1) * n], n) for t in range(2)) > 2048
 
 
-@pytest.mark.parametrize("n,k,route", [(16_384, 3, 4), (16_385, 3, -1), (12_288, 4, 4), (12_289, 4, -1), (12_289, 8, -1), (2048, 3, -1), (2049, 3, 1)])
-def test_which_sort(n, k, route):
-    """Lines between the sorts, in 32 tables: clusters of four CTAs, one CTA and splitters."""
+@pytest.mark.parametrize("n,k,L,route", [(16_384, 3, 32, 4), (16_385, 3, 32, -1), (12_288, 4, 32, 4), (12_289, 4, 32, -1), (12_289, 8, 32, -1), (2048, 3, 32, -1), (2049, 3, 32, 1),
+                                         (2_097_152, 2, 3, -1), (2_097_153, 2, 3, 0), (2_097_153, 2, 4, -1), (2_097_153, 3, 1, -1)])
+def test_which_sort(n, k, L, route):
+    """Lines between the sorts: clusters of four CTAs, one CTA, passes with launches of their own and splitters."""
     from culsh_b200 import _culsh_core as core_mod
     rng = np.random.default_rng(n)
     indices, indptr = rng.integers(0, 1 << 19, 6 * n).astype(np.int32), (6 * np.arange(n + 1)).astype(np.int32)
-    core = core_mod.MinHashCore(32, k, 7)
+    core = core_mod.MinHashCore(L, k, 7)
     core.fit(indices, indptr, n, 1 << 19)
     assert core.last_stats()["sort_ctas"] == route
 
