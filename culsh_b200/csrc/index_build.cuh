@@ -29,8 +29,8 @@ __device__ __forceinline__ bool keys_differ(const uint32_t* __restrict__ a,
 // heads per tile, and a bit per item that is one: heads[tile][IB_WORDS].  A tile covers IB_TILE consecutive items of one table
 template <int NW>
 __global__ void __launch_bounds__(IB_THREADS)
-bucket_count_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ keys, int n, int tiles_per_table,
-                    uint32_t* __restrict__ tile_heads, uint32_t* __restrict__ heads) {
+bucket_count_kernel(const uint32_t* __restrict__ keys, int n, int tiles_per_table,
+                    uint32_t* __restrict__ tile_heads, uint32_t* __restrict__ heads, KernelBefore kernel_before) {
     kernel_before.wait(keys, tile_heads, heads);
     __shared__ uint32_t s_warp[32];
     const int t = blockIdx.x / tiles_per_table;
@@ -58,10 +58,10 @@ bucket_count_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ key
 // keys / offsets go to consecutive addresses.  (With the keys read and compared once more instead of the bits: 12.5M x 16 keys of two words 660 -> 469 us, with the count 967 -> 779; 10M x 48 of one 925 -> 582, with the count 1,425 -> 1,143.)
 template <int NW>
 __global__ void __launch_bounds__(IB_THREADS)
-bucket_write_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ keys, int n, int L, int tiles_per_table,
+bucket_write_kernel(const uint32_t* __restrict__ keys, int n, int L, int tiles_per_table,
                     const uint32_t* __restrict__ tile_base, uint32_t n_tiles, const uint32_t* __restrict__ heads,
                     uint32_t* __restrict__ bucket_keys, int32_t* __restrict__ bucket_offsets,
-                    int32_t* __restrict__ table_offsets) {
+                    int32_t* __restrict__ table_offsets, KernelBefore kernel_before) {
     kernel_before.wait(keys, tile_base, heads, bucket_keys, bucket_offsets, table_offsets);
     constexpr int WORDS = IB_WORDS;
     __shared__ uint32_t s_bits[WORDS];

@@ -97,9 +97,9 @@ __device__ __forceinline__ int2 lookup_pair_together(const uint32_t* __restrict_
 constexpr int LU_THREADS = 256;
 template <int NW>
 __global__ void __launch_bounds__(LU_THREADS)
-lookup_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ qkeys, const uint8_t* __restrict__ q_ovf, int n_q, int chunks,
+lookup_kernel(const uint32_t* __restrict__ qkeys, const uint8_t* __restrict__ q_ovf, int n_q, int chunks,
               const uint32_t* __restrict__ bucket_keys, const int32_t* __restrict__ bucket_offsets,
-              const int32_t* __restrict__ table_offsets, int2* __restrict__ bounds) {
+              const int32_t* __restrict__ table_offsets, int2* __restrict__ bounds, KernelBefore kernel_before) {
     kernel_before.wait(qkeys, q_ovf, bucket_keys, bucket_offsets, table_offsets, bounds);
     constexpr int SPLIT = LU_THREADS / NW;  // a power of two
     __shared__ __align__(16) uint32_t s_split[SPLIT * NW];
@@ -179,9 +179,9 @@ constexpr int RC_BATCH = 8;
 // shared-memory sort path (mid_list; only used when mid_max > SMALL_MAX), counters[2] = queries for
 // the long form of the warp path
 __global__ void __launch_bounds__(256)
-raw_count_kernel(KernelBefore kernel_before, BoundsView bounds, int n_q, int L, bool self_join, uint64_t* __restrict__ raw_cnt,
+raw_count_kernel(BoundsView bounds, int n_q, int L, bool self_join, uint64_t* __restrict__ raw_cnt,
                  uint32_t* __restrict__ big_list, uint32_t* __restrict__ mid_list, uint32_t* __restrict__ counters,
-                 int mid_max, uint64_t* __restrict__ uniq_cnt) {
+                 int mid_max, uint64_t* __restrict__ uniq_cnt, KernelBefore kernel_before) {
     kernel_before.wait(raw_cnt, big_list, mid_list, counters, uniq_cnt);
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;  // unsigned: the last CTA may reach past 2^31
     if (q >= (uint32_t)n_q) return;
@@ -238,11 +238,11 @@ constexpr size_t LS_MAX_PAIRS = LS_CTAS * LS_THREADS;
 constexpr int LS_GROUP = 32;  // lanes that search for a pair, at most
 template <int NW>
 __global__ void __launch_bounds__(LS_THREADS)
-lookup_count_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ qkeys, const uint8_t* __restrict__ q_ovf, int n_q, int L,
+lookup_count_kernel(const uint32_t* __restrict__ qkeys, const uint8_t* __restrict__ q_ovf, int n_q, int L,
                     const uint32_t* __restrict__ bucket_keys, const int32_t* __restrict__ bucket_offsets,
                     const int32_t* __restrict__ table_offsets, int2* __restrict__ bounds, uint64_t* __restrict__ raw_cnt,
                     uint64_t* __restrict__ raw_off, uint32_t* __restrict__ big_list, uint32_t* __restrict__ mid_list,
-                    uint32_t* __restrict__ counters, int mid_max, uint64_t* __restrict__ uniq_cnt, int group, HostWords host) {
+                    uint32_t* __restrict__ counters, int mid_max, uint64_t* __restrict__ uniq_cnt, int group, HostWords host, KernelBefore kernel_before) {
     kernel_before.wait(qkeys, q_ovf, bucket_keys, bucket_offsets, table_offsets, bounds, raw_cnt, raw_off, big_list, mid_list, counters, uniq_cnt);
     __shared__ uint32_t s_cnt[LS_MAX_PAIRS];  // at most as many queries as pairs
     __shared__ uint32_t s_counters[3];
@@ -406,9 +406,9 @@ struct WarpLists {
 // together have more than `room` ids: a launch whose counts the host has not seen says how many `tmp` holds.
 template <int CAP, bool SELF>
 __global__ void __launch_bounds__(SM_THREADS, CAP == SHORT_MAX ? 6 : 4)
-dedupe_small_kernel(KernelBefore kernel_before, BoundsView bounds, const int32_t* __restrict__ cand, const uint64_t* __restrict__ raw_cnt,
+dedupe_small_kernel(BoundsView bounds, const int32_t* __restrict__ cand, const uint64_t* __restrict__ raw_cnt,
                     const uint64_t* __restrict__ raw_off, int L, int above, uint64_t room, int32_t* __restrict__ tmp,
-                    uint64_t* __restrict__ uniq_cnt) {
+                    uint64_t* __restrict__ uniq_cnt, KernelBefore kernel_before) {
     kernel_before.wait(cand, raw_cnt, raw_off, tmp, uniq_cnt);
     __shared__ int32_t s_buf[SM_WARPS][CAP];
     __shared__ WarpLists s_lists[SELF ? 1 : SM_WARPS];
@@ -1010,8 +1010,8 @@ struct ListWalk {
 // with a million independent searches in flight the dependent loads cost nothing, whereas
 // inside the window kernel they would sit on the critical path of every CTA.
 __global__ void __launch_bounds__(256)
-slice_lists_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ big_list, BoundsView bounds, const int32_t* __restrict__ cand, int n_big, int L,
-                   int window_bits, int n_win, int2* __restrict__ slices) {
+slice_lists_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds, const int32_t* __restrict__ cand, int n_big, int L,
+                   int window_bits, int n_win, int2* __restrict__ slices, KernelBefore kernel_before) {
     kernel_before.wait(big_list, cand, slices);
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)n_big * L * n_win) return;
@@ -1036,10 +1036,10 @@ slice_lists_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ big_
 // host has not seen covers all queries: n_big says how many there are to do, and `room` is as in dedupe_small_kernel.
 template <int NT, int MK>
 __global__ void __launch_bounds__(NT, 1920 / NT)  // cut_lists would take it to 37 registers and to four CTAs of 384 threads an SM
-dedupe_window_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ big_list, BoundsView bounds, const int32_t* __restrict__ cand,
+dedupe_window_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds, const int32_t* __restrict__ cand,
                      const uint64_t* __restrict__ raw_off, int L, int n_rows, int window_bits, int n_win, bool self_join,
                      const int2* __restrict__ slices /* or null */, const uint32_t* __restrict__ n_big /* or null: all */, uint64_t room,
-                     int32_t* __restrict__ tmp, uint2* __restrict__ pieces, unsigned long long* __restrict__ uniq_cnt) {
+                     int32_t* __restrict__ tmp, uint2* __restrict__ pieces, unsigned long long* __restrict__ uniq_cnt, KernelBefore kernel_before) {
     kernel_before.wait(big_list, cand, raw_off, slices, n_big, tmp, pieces, uniq_cnt);
     constexpr int NWARP = NT / 32;
     extern __shared__ __align__(16) uint32_t s_dyn[];
@@ -1194,9 +1194,9 @@ compact_big_kernel(const uint32_t* __restrict__ big_list, const int32_t* __restr
 // out[offsets[q] - first ...].  Bound by the 8 bytes an id moves.
 constexpr int CWN_LOADS = 8;
 __global__ void __launch_bounds__(256)
-compact_windows_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ big_list, const int32_t* __restrict__ tmp, const uint64_t* __restrict__ raw_off,
+compact_windows_kernel(const uint32_t* __restrict__ big_list, const int32_t* __restrict__ tmp, const uint64_t* __restrict__ raw_off,
                        const uint2* __restrict__ pieces, const uint64_t* __restrict__ offsets, int n_win, uint32_t q_lo, uint32_t q_hi,
-                       uint64_t first, int32_t* __restrict__ out) {
+                       uint64_t first, int32_t* __restrict__ out, KernelBefore kernel_before) {
     kernel_before.wait(big_list, tmp, raw_off, pieces, offsets, out);
     const int slot = blockIdx.x / n_win, w = blockIdx.x - slot * n_win;
     const uint32_t q = big_list[slot];
@@ -1224,9 +1224,9 @@ compact_windows_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ 
 // left the copy of the 10M-row self-join's 1.8 GB at 1.6 TB/s.
 constexpr int CS_ROWS = 4;
 __global__ void __launch_bounds__(256)
-compact_small_kernel(KernelBefore kernel_before, const int32_t* __restrict__ tmp, const uint64_t* __restrict__ raw_cnt,
+compact_small_kernel(const int32_t* __restrict__ tmp, const uint64_t* __restrict__ raw_cnt,
                      const uint64_t* __restrict__ raw_off, const uint64_t* __restrict__ uniq_cnt,
-                     const uint64_t* __restrict__ offsets, int n_q, int per, uint64_t first, int32_t* __restrict__ out) {
+                     const uint64_t* __restrict__ offsets, int n_q, int per, uint64_t first, int32_t* __restrict__ out, KernelBefore kernel_before) {
     kernel_before.wait(tmp, raw_cnt, raw_off, uniq_cnt, offsets, out);
     const int lane = threadIdx.x & 31;
     const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;

@@ -139,8 +139,8 @@ __device__ __forceinline__ void decomp_key(uint32_t* k, KeyComp kc) {
 // ---------------------------------------------------------------------------------------
 template <int NW, bool COMP0>
 __global__ void __launch_bounds__(RS_THREADS)
-radix_tile_hist_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ keys, int n, int tiles_per_table, int p, uint32_t sub,
-                       uint32_t* __restrict__ tile_hist) {
+radix_tile_hist_kernel(const uint32_t* __restrict__ keys, int n, int tiles_per_table, int p, uint32_t sub,
+                       uint32_t* __restrict__ tile_hist, KernelBefore kernel_before) {
     kernel_before.wait(keys, tile_hist);
     using Cfg = SortCfg<NW>;
     __shared__ uint32_t s_hist[256];
@@ -177,7 +177,7 @@ constexpr int RS_SCAN_THREADS = 1024;
 constexpr int RS_SCAN_SEGS = RS_SCAN_THREADS / 256;
 
 __global__ void __launch_bounds__(RS_SCAN_THREADS)
-radix_tile_scan_kernel(KernelBefore kernel_before, uint32_t* __restrict__ tile_hist, int tiles_per_table) {
+radix_tile_scan_kernel(uint32_t* __restrict__ tile_hist, int tiles_per_table, KernelBefore kernel_before) {
     kernel_before.wait(tile_hist);
     __shared__ uint32_t s_seg[RS_SCAN_SEGS][256];
     __shared__ uint32_t s_base[256];
@@ -227,8 +227,8 @@ constexpr int RS_CHUNK_TILES = 64;
 constexpr int RS_CHUNK_MIN_TILES = 96;  // tables with fewer tiles keep the single-launch scan
 
 __global__ void __launch_bounds__(RS_SCAN_THREADS)
-radix_tile_scan_chunk_kernel(KernelBefore kernel_before, uint32_t* __restrict__ tile_hist, int tiles_per_table, int n_chunks,
-                             uint32_t* __restrict__ chunk_tot /* [table][chunk][256] */) {
+radix_tile_scan_chunk_kernel(uint32_t* __restrict__ tile_hist, int tiles_per_table, int n_chunks,
+                             uint32_t* __restrict__ chunk_tot /* [table][chunk][256] */, KernelBefore kernel_before) {
     kernel_before.wait(tile_hist, chunk_tot);
     __shared__ uint32_t s_seg[RS_SCAN_SEGS][256];
     const int d = threadIdx.x & 255, seg = threadIdx.x >> 8;
@@ -260,7 +260,7 @@ radix_tile_scan_chunk_kernel(KernelBefore kernel_before, uint32_t* __restrict__ 
 
 // one block of 256 threads per table: chunk_tot -> chunk bases, in place
 __global__ void __launch_bounds__(256)
-radix_chunk_base_kernel(KernelBefore kernel_before, uint32_t* __restrict__ chunk_tot, int n_chunks) {
+radix_chunk_base_kernel(uint32_t* __restrict__ chunk_tot, int n_chunks, KernelBefore kernel_before) {
     kernel_before.wait(chunk_tot);
     __shared__ uint32_t s_warp[8];
     const int d = threadIdx.x, lane = d & 31, w = d >> 5;
@@ -319,10 +319,10 @@ constexpr int RS_PACK_ID_BITS = 24;
 
 template <int NW, bool FIRST, int COMP, bool PACK = false>
 __global__ void __launch_bounds__(RS_THREADS, 4)
-radix_scatter_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
+radix_scatter_kernel(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                      uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int n,
                      int tiles_per_table, int p, KeyComp kc, const uint32_t* __restrict__ tile_off,
-                     const uint32_t* __restrict__ chunk_base /* or null */, int n_chunks) {
+                     const uint32_t* __restrict__ chunk_base /* or null */, int n_chunks, KernelBefore kernel_before) {
     kernel_before.wait(keys_in, vals_in, keys_out, vals_out, tile_off, chunk_base);
     using Cfg = SortCfg<NW>;
     constexpr int IPT = Cfg::IPT;
@@ -543,8 +543,8 @@ struct SmallSortCfg {
 // Keys of eight and sixteen words are launched as usual: with pointers that the compiler knows nothing of their passes take 2.5 % longer.
 template <int NW, bool PACK>
 __global__ void __launch_bounds__(RSS_THREADS, 1)
-radix_sort_small_kernel(EarlyIf<(NW <= 4)> kernel_before, const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
-                        uint32_t* __restrict__ vals_out, int n, int passes, bool compressed, KeyComp kc, const int* __restrict__ check) {
+radix_sort_small_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
+                        uint32_t* __restrict__ vals_out, int n, int passes, bool compressed, KeyComp kc, const int* __restrict__ check, EarlyIf<(NW <= 4)> kernel_before) {
     kernel_before.wait(keys_in, keys_out, vals_out, check);
     using Cfg = SmallSortCfg<NW, PACK>;
     constexpr int KW = Cfg::KW, IPT = Cfg::IPT;
@@ -713,9 +713,9 @@ struct ClusterSortCfg {
 
 template <int NW, bool PACK>
 __global__ void __launch_bounds__(RSC_THREADS, 1)
-radix_sort_cluster_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
+radix_sort_cluster_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
                           uint32_t* __restrict__ vals_out, int n, int cta_rows, uint32_t cta_rows_inv, int passes, bool compressed,
-                          KeyComp kc, const int* __restrict__ check) {
+                          KeyComp kc, const int* __restrict__ check, KernelBefore kernel_before) {
     kernel_before.wait(keys_in, keys_out, vals_out, check);
     using Cfg = ClusterSortCfg<NW, PACK>;
     constexpr int KW = Cfg::KW, IPT = Cfg::IPT;
@@ -1130,7 +1130,7 @@ __device__ __forceinline__ TOut block_exclusive_scan(TOut v, TOut* s_warp, TOut&
 
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(SCAN_THREADS)
-scan_reduce_kernel(KernelBefore kernel_before, const TIn* __restrict__ in, size_t n, TOut* __restrict__ block_sums) {
+scan_reduce_kernel(const TIn* __restrict__ in, size_t n, TOut* __restrict__ block_sums, KernelBefore kernel_before) {
     kernel_before.wait(in, block_sums);
     __shared__ TOut s_warp[32];
     size_t base = (size_t)blockIdx.x * SCAN_TILE;
@@ -1165,7 +1165,7 @@ struct HostWords {
 
 template <typename TOut>
 __global__ void __launch_bounds__(1024)
-scan_block_sums_kernel(KernelBefore kernel_before, TOut* __restrict__ block_sums, size_t n_blocks, TOut* __restrict__ total_out, HostWords host) {
+scan_block_sums_kernel(TOut* __restrict__ block_sums, size_t n_blocks, TOut* __restrict__ total_out, HostWords host, KernelBefore kernel_before) {
     kernel_before.wait(block_sums, total_out);
     __shared__ TOut s_warp[32];
     TOut carry = 0;
@@ -1183,8 +1183,8 @@ scan_block_sums_kernel(KernelBefore kernel_before, TOut* __restrict__ block_sums
 
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(SCAN_THREADS)
-scan_apply_kernel(KernelBefore kernel_before, const TIn* __restrict__ in, size_t n, const TOut* __restrict__ block_sums, bool scanned,
-                  TOut* __restrict__ out, HostWords host) {
+scan_apply_kernel(const TIn* __restrict__ in, size_t n, const TOut* __restrict__ block_sums, bool scanned,
+                  TOut* __restrict__ out, HostWords host, KernelBefore kernel_before) {
     kernel_before.wait(in, block_sums, out);
     __shared__ TOut s_warp[32];
     TOut before = 0;  // elements of the blocks before this one
@@ -1234,7 +1234,7 @@ struct alignas(16) ScanVec {
 // in and out on 16-byte boundaries
 template <typename T>
 __global__ void __launch_bounds__(SCAN_ONE_THREADS)
-scan_one_kernel(KernelBefore kernel_before, const T* __restrict__ in, int n, T* __restrict__ out, HostWords host) {
+scan_one_kernel(const T* __restrict__ in, int n, T* __restrict__ out, HostWords host, KernelBefore kernel_before) {
     kernel_before.wait(in, out);
     constexpr int PER = 16 / sizeof(T), VECS = SCAN_ONE_IPT / PER;
     __shared__ T s_warp[32];

@@ -260,8 +260,8 @@ struct RowList {
 // them is scrambled: rows that repeat with some period are sampled like any others.
 template <int NW>
 __global__ void __launch_bounds__(SS_THREADS)
-splitter_sample_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ keys, int n, int skip, int samples, int chunks, int bins, int over,
-                       RowList<NW> sorted /* one chunk: the splitters */) {
+splitter_sample_kernel(const uint32_t* __restrict__ keys, int n, int skip, int samples, int chunks, int bins, int over,
+                       RowList<NW> sorted /* one chunk: the splitters */, KernelBefore kernel_before) {
     kernel_before.wait(keys);
     extern __shared__ __align__(16) unsigned char ss_smem[];
     using Sort = BlockSort<NW>;
@@ -291,7 +291,7 @@ splitter_sample_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ 
 // A thread for each sample: its rank among the table's samples.  Every SS_OVER-th becomes a splitter.  samples = chunks * SS_CAP.
 template <int NW>
 __global__ void __launch_bounds__(256)
-splitter_rank_kernel(KernelBefore kernel_before, const uint32_t* __restrict__ keys, int n, int skip, int chunks, int bins, int total, RowList<NW> sorted, RowList<NW> splitters) {
+splitter_rank_kernel(const uint32_t* __restrict__ keys, int n, int skip, int chunks, int bins, int total, RowList<NW> sorted, RowList<NW> splitters, KernelBefore kernel_before) {
     kernel_before.wait(keys);
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= total) return;
@@ -416,7 +416,7 @@ splitter_classify_kernel(const uint32_t* __restrict__ keys, int n, int skip, int
 // A thread for each (table, bin): its counts become those of the tiles before, and bin_total theirs.
 constexpr int SS_SCAN_THREADS = 64;
 __global__ void __launch_bounds__(SS_SCAN_THREADS)
-splitter_scan_kernel(KernelBefore kernel_before, uint32_t* __restrict__ tile_hist, int tiles, int bins, int total, uint32_t* __restrict__ bin_total) {
+splitter_scan_kernel(uint32_t* __restrict__ tile_hist, int tiles, int bins, int total, uint32_t* __restrict__ bin_total, KernelBefore kernel_before) {
     kernel_before.wait(tile_hist, bin_total);
     const int i = blockIdx.x * SS_SCAN_THREADS + threadIdx.x;
     if (i >= total) return;
@@ -442,9 +442,9 @@ inline size_t splitter_scatter_smem(int tile, int bins) { return (size_t)tile * 
 // A CTA for each tile: its rows in the order of their bins through shared memory, out in runs.  The first tile of a table leaves where its
 // bins start in bin_start[t * (bins + 1) ...].
 __global__ void __launch_bounds__(SS_TILE_THREADS)
-splitter_scatter_kernel(KernelBefore kernel_before, const uint16_t* __restrict__ bin_of, int n, int tile, int tiles, int bins, const uint32_t* __restrict__ tile_hist,
+splitter_scatter_kernel(const uint16_t* __restrict__ bin_of, int n, int tile, int tiles, int bins, const uint32_t* __restrict__ tile_hist,
                         const uint32_t* __restrict__ bin_total, uint32_t* __restrict__ bin_start,
-                        uint32_t* __restrict__ ids) {
+                        uint32_t* __restrict__ ids, KernelBefore kernel_before) {
     kernel_before.wait(bin_of, tile_hist, bin_total, bin_start, ids);
     extern __shared__ __align__(16) unsigned char ss_smem[];
     uint16_t* s_row = reinterpret_cast<uint16_t*>(ss_smem);            // [tile] its rows, bin after bin

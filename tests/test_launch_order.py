@@ -27,7 +27,7 @@ def test_kernels_launched_early_wait_first():
             if "KernelBefore" not in params and "EarlyIf" not in params:
                 continue
             early += 1
-            assert re.match(r"\s*(?:KernelBefore|EarlyIf<\([^()]*\)>)\s+kernel_before\s*,", params), head.group(1)
+            assert re.search(r",\s*(?:KernelBefore|EarlyIf<\([^()]*\)>)\s+kernel_before\s*$", params), head.group(1)
             wait = re.compile(r"\s*\{\s*kernel_before\s*\.\s*wait\s*\(").match(text, end)
             assert wait, head.group(1)
             given = re.findall(r"\w+", text[wait.end():_closing(text, wait.end()) - 1])
