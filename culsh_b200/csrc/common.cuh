@@ -370,7 +370,7 @@ enum DeviceErrorBits : int {
     DEV_ERR_MBAR_TIMEOUT = 4       // a bounded mbarrier wait ran out (tensor-core projection)
 };
 
-// A kernel that takes this as its last parameter may be set up while the one in front of it in the stream still runs, and starts with wait(): that lets the
+// A kernel that takes this as its last parameter may be set up while the one in front of it in the stream still runs, and starts with behind_kernel_before(): that lets the
 // next one do the same, and waits until the one before is done and what it wrote can be read.  launch_next and launch_cluster take no others but KernelDone's.  The
 // pointers come back as ones that the compiler knows nothing of: a load through one that it takes for the only way to its memory could move to the front
 // of the wait (members of structs are not such; the wait is a barrier to them as it is).  A chain of short
@@ -378,23 +378,9 @@ enum DeviceErrorBits : int {
 // 445 -> 409.  Kernels that fill the chip for long and are short of registers are launched as usual: what the compiler no longer knows
 // made the search among splitters 13 % slower and the sort of the bins 7 %.  So are kernels with a CTA or two for each SM behind one whose CTAs have an SM
 // each: they gather on the SMs that are free first (148 tables of 3,000 keys of 64 bytes, the buckets' count behind the sort 36 us, 142 when launched early).
-struct KernelBefore {
-    template <typename... T>
-    __device__ __forceinline__ void wait(T&... pointers) const {
-        asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
-        auto anew = [](auto& p) {  // but that they point to global memory
-            size_t g = __cvta_generic_to_global(p);
-            asm volatile("" : "+l"(g) : : "memory");
-            p = static_cast<std::remove_reference_t<decltype(p)>>(__cvta_global_to_generic(g));
-        };
-        (..., anew(pointers));
-    }
-};
+struct KernelBefore {};
 // For forms of a kernel that are launched as usual.
-struct KernelDone {
-    template <typename... T>
-    __device__ __forceinline__ void wait(T&...) const {}
-};
+struct KernelDone {};
 template <bool EARLY>
 using EarlyIf = std::conditional_t<EARLY, KernelBefore, KernelDone>;
 
@@ -403,6 +389,25 @@ template <typename T, typename... P>
 struct LastOf { using type = typename LastOf<P...>::type; };
 template <typename T>
 struct LastOf<T> { using type = T; };
+
+template <typename T>
+__device__ __forceinline__ void pointer_anew(T& p) {  // but that it points to global memory
+    if constexpr (!std::is_same<T, KernelBefore>::value) {
+        size_t g = __cvta_generic_to_global(p);
+        asm volatile("" : "+l"(g) : : "memory");
+        p = static_cast<T>(__cvta_global_to_generic(g));
+    }
+}
+// A kernel's pointers and, behind them, that parameter.
+template <typename... T>
+__device__ __forceinline__ void behind_kernel_before(T&... pointers) {
+    if constexpr (std::is_same<typename LastOf<T...>::type, KernelBefore>::value) {
+        asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+        (..., pointer_anew(pointers));
+    } else {
+        static_assert(std::is_same<typename LastOf<T...>::type, KernelDone>::value, "");
+    }
+}
 template <typename... P, typename... A>
 inline cudaError_t launch_cast(const cudaLaunchConfig_t& cfg, void (*kern)(P...), A... args) {
     return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);

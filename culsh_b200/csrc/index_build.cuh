@@ -31,7 +31,7 @@ template <int NW>
 __global__ void __launch_bounds__(IB_THREADS)
 bucket_count_kernel(const uint32_t* __restrict__ keys, int n, int tiles_per_table,
                     uint32_t* __restrict__ tile_heads, uint32_t* __restrict__ heads, KernelBefore kernel_before) {
-    kernel_before.wait(keys, tile_heads, heads);
+    behind_kernel_before(keys, tile_heads, heads, kernel_before);
     __shared__ uint32_t s_warp[32];
     const int t = blockIdx.x / tiles_per_table;
     const int lt = blockIdx.x - t * tiles_per_table;
@@ -62,7 +62,7 @@ bucket_write_kernel(const uint32_t* __restrict__ keys, int n, int L, int tiles_p
                     const uint32_t* __restrict__ tile_base, uint32_t n_tiles, const uint32_t* __restrict__ heads,
                     uint32_t* __restrict__ bucket_keys, int32_t* __restrict__ bucket_offsets,
                     int32_t* __restrict__ table_offsets, KernelBefore kernel_before) {
-    kernel_before.wait(keys, tile_base, heads, bucket_keys, bucket_offsets, table_offsets);
+    behind_kernel_before(keys, tile_base, heads, bucket_keys, bucket_offsets, table_offsets, kernel_before);
     constexpr int WORDS = IB_WORDS;
     __shared__ uint32_t s_bits[WORDS];
     __shared__ uint32_t s_pref[WORDS];

@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(LU_THREADS)
 lookup_kernel(const uint32_t* __restrict__ qkeys, const uint8_t* __restrict__ q_ovf, int n_q, int chunks,
               const uint32_t* __restrict__ bucket_keys, const int32_t* __restrict__ bucket_offsets,
               const int32_t* __restrict__ table_offsets, int2* __restrict__ bounds, KernelBefore kernel_before) {
-    kernel_before.wait(qkeys, q_ovf, bucket_keys, bucket_offsets, table_offsets, bounds);
+    behind_kernel_before(qkeys, q_ovf, bucket_keys, bucket_offsets, table_offsets, bounds, kernel_before);
     constexpr int SPLIT = LU_THREADS / NW;  // a power of two
     __shared__ __align__(16) uint32_t s_split[SPLIT * NW];
     const int t = blockIdx.x / chunks;
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(256)
 raw_count_kernel(BoundsView bounds, int n_q, int L, bool self_join, uint64_t* __restrict__ raw_cnt,
                  uint32_t* __restrict__ big_list, uint32_t* __restrict__ mid_list, uint32_t* __restrict__ counters,
                  int mid_max, uint64_t* __restrict__ uniq_cnt, KernelBefore kernel_before) {
-    kernel_before.wait(raw_cnt, big_list, mid_list, counters, uniq_cnt);
+    behind_kernel_before(raw_cnt, big_list, mid_list, counters, uniq_cnt, kernel_before);
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;  // unsigned: the last CTA may reach past 2^31
     if (q >= (uint32_t)n_q) return;
     uint32_t c = self_join ? 1u : 0u;  // at most n * L < 2^31
@@ -243,7 +243,7 @@ lookup_count_kernel(const uint32_t* __restrict__ qkeys, const uint8_t* __restric
                     const int32_t* __restrict__ table_offsets, int2* __restrict__ bounds, uint64_t* __restrict__ raw_cnt,
                     uint64_t* __restrict__ raw_off, uint32_t* __restrict__ big_list, uint32_t* __restrict__ mid_list,
                     uint32_t* __restrict__ counters, int mid_max, uint64_t* __restrict__ uniq_cnt, int group, HostWords host, KernelBefore kernel_before) {
-    kernel_before.wait(qkeys, q_ovf, bucket_keys, bucket_offsets, table_offsets, bounds, raw_cnt, raw_off, big_list, mid_list, counters, uniq_cnt);
+    behind_kernel_before(qkeys, q_ovf, bucket_keys, bucket_offsets, table_offsets, bounds, raw_cnt, raw_off, big_list, mid_list, counters, uniq_cnt, kernel_before);
     __shared__ uint32_t s_cnt[LS_MAX_PAIRS];  // at most as many queries as pairs
     __shared__ uint32_t s_counters[3];
     __shared__ uint64_t s_warp[32];
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(SM_THREADS, CAP == SHORT_MAX ? 6 : 4)
 dedupe_small_kernel(BoundsView bounds, const int32_t* __restrict__ cand, const uint64_t* __restrict__ raw_cnt,
                     const uint64_t* __restrict__ raw_off, int L, int above, uint64_t room, int32_t* __restrict__ tmp,
                     uint64_t* __restrict__ uniq_cnt, KernelBefore kernel_before) {
-    kernel_before.wait(cand, raw_cnt, raw_off, tmp, uniq_cnt);
+    behind_kernel_before(cand, raw_cnt, raw_off, tmp, uniq_cnt, kernel_before);
     __shared__ int32_t s_buf[SM_WARPS][CAP];
     __shared__ WarpLists s_lists[SELF ? 1 : SM_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1012,7 +1012,7 @@ struct ListWalk {
 __global__ void __launch_bounds__(256)
 slice_lists_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds, const int32_t* __restrict__ cand, int n_big, int L,
                    int window_bits, int n_win, int2* __restrict__ slices, KernelBefore kernel_before) {
-    kernel_before.wait(big_list, cand, slices);
+    behind_kernel_before(big_list, cand, slices, kernel_before);
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)n_big * L * n_win) return;
     const int w = (int)(idx % n_win);
@@ -1040,7 +1040,7 @@ dedupe_window_kernel(const uint32_t* __restrict__ big_list, BoundsView bounds, c
                      const uint64_t* __restrict__ raw_off, int L, int n_rows, int window_bits, int n_win, bool self_join,
                      const int2* __restrict__ slices /* or null */, const uint32_t* __restrict__ n_big /* or null: all */, uint64_t room,
                      int32_t* __restrict__ tmp, uint2* __restrict__ pieces, unsigned long long* __restrict__ uniq_cnt, KernelBefore kernel_before) {
-    kernel_before.wait(big_list, cand, raw_off, slices, n_big, tmp, pieces, uniq_cnt);
+    behind_kernel_before(big_list, cand, raw_off, slices, n_big, tmp, pieces, uniq_cnt, kernel_before);
     constexpr int NWARP = NT / 32;
     extern __shared__ __align__(16) uint32_t s_dyn[];
     const int n32 = window_bits / 32;                        // a multiple of 128
@@ -1197,7 +1197,7 @@ __global__ void __launch_bounds__(256)
 compact_windows_kernel(const uint32_t* __restrict__ big_list, const int32_t* __restrict__ tmp, const uint64_t* __restrict__ raw_off,
                        const uint2* __restrict__ pieces, const uint64_t* __restrict__ offsets, int n_win, uint32_t q_lo, uint32_t q_hi,
                        uint64_t first, int32_t* __restrict__ out, KernelBefore kernel_before) {
-    kernel_before.wait(big_list, tmp, raw_off, pieces, offsets, out);
+    behind_kernel_before(big_list, tmp, raw_off, pieces, offsets, out, kernel_before);
     const int slot = blockIdx.x / n_win, w = blockIdx.x - slot * n_win;
     const uint32_t q = big_list[slot];
     if (q < q_lo || q >= q_hi) return;
@@ -1227,7 +1227,7 @@ __global__ void __launch_bounds__(256)
 compact_small_kernel(const int32_t* __restrict__ tmp, const uint64_t* __restrict__ raw_cnt,
                      const uint64_t* __restrict__ raw_off, const uint64_t* __restrict__ uniq_cnt,
                      const uint64_t* __restrict__ offsets, int n_q, int per, uint64_t first, int32_t* __restrict__ out, KernelBefore kernel_before) {
-    kernel_before.wait(tmp, raw_cnt, raw_off, uniq_cnt, offsets, out);
+    behind_kernel_before(tmp, raw_cnt, raw_off, uniq_cnt, offsets, out, kernel_before);
     const int lane = threadIdx.x & 31;
     const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const size_t n_warps = ((size_t)gridDim.x * blockDim.x) >> 5;

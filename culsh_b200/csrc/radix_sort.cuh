@@ -141,7 +141,7 @@ template <int NW, bool COMP0>
 __global__ void __launch_bounds__(RS_THREADS)
 radix_tile_hist_kernel(const uint32_t* __restrict__ keys, int n, int tiles_per_table, int p, uint32_t sub,
                        uint32_t* __restrict__ tile_hist, KernelBefore kernel_before) {
-    kernel_before.wait(keys, tile_hist);
+    behind_kernel_before(keys, tile_hist, kernel_before);
     using Cfg = SortCfg<NW>;
     __shared__ uint32_t s_hist[256];
     const int tile = blockIdx.x;
@@ -178,7 +178,7 @@ constexpr int RS_SCAN_SEGS = RS_SCAN_THREADS / 256;
 
 __global__ void __launch_bounds__(RS_SCAN_THREADS)
 radix_tile_scan_kernel(uint32_t* __restrict__ tile_hist, int tiles_per_table, KernelBefore kernel_before) {
-    kernel_before.wait(tile_hist);
+    behind_kernel_before(tile_hist, kernel_before);
     __shared__ uint32_t s_seg[RS_SCAN_SEGS][256];
     __shared__ uint32_t s_base[256];
     __shared__ uint32_t s_warp[8];
@@ -229,7 +229,7 @@ constexpr int RS_CHUNK_MIN_TILES = 96;  // tables with fewer tiles keep the sing
 __global__ void __launch_bounds__(RS_SCAN_THREADS)
 radix_tile_scan_chunk_kernel(uint32_t* __restrict__ tile_hist, int tiles_per_table, int n_chunks,
                              uint32_t* __restrict__ chunk_tot /* [table][chunk][256] */, KernelBefore kernel_before) {
-    kernel_before.wait(tile_hist, chunk_tot);
+    behind_kernel_before(tile_hist, chunk_tot, kernel_before);
     __shared__ uint32_t s_seg[RS_SCAN_SEGS][256];
     const int d = threadIdx.x & 255, seg = threadIdx.x >> 8;
     const int table = blockIdx.x / n_chunks, chunk = blockIdx.x - table * n_chunks;
@@ -261,7 +261,7 @@ radix_tile_scan_chunk_kernel(uint32_t* __restrict__ tile_hist, int tiles_per_tab
 // one block of 256 threads per table: chunk_tot -> chunk bases, in place
 __global__ void __launch_bounds__(256)
 radix_chunk_base_kernel(uint32_t* __restrict__ chunk_tot, int n_chunks, KernelBefore kernel_before) {
-    kernel_before.wait(chunk_tot);
+    behind_kernel_before(chunk_tot, kernel_before);
     __shared__ uint32_t s_warp[8];
     const int d = threadIdx.x, lane = d & 31, w = d >> 5;
     uint32_t* ct = chunk_tot + (size_t)blockIdx.x * n_chunks * 256 + d;
@@ -323,7 +323,7 @@ radix_scatter_kernel(const uint32_t* __restrict__ keys_in, const uint32_t* __res
                      uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int n,
                      int tiles_per_table, int p, KeyComp kc, const uint32_t* __restrict__ tile_off,
                      const uint32_t* __restrict__ chunk_base /* or null */, int n_chunks, KernelBefore kernel_before) {
-    kernel_before.wait(keys_in, vals_in, keys_out, vals_out, tile_off, chunk_base);
+    behind_kernel_before(keys_in, vals_in, keys_out, vals_out, tile_off, chunk_base, kernel_before);
     using Cfg = SortCfg<NW>;
     constexpr int IPT = Cfg::IPT;
     constexpr int TILE = Cfg::TILE;
@@ -545,7 +545,7 @@ template <int NW, bool PACK>
 __global__ void __launch_bounds__(RSS_THREADS, 1)
 radix_sort_small_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
                         uint32_t* __restrict__ vals_out, int n, int passes, bool compressed, KeyComp kc, const int* __restrict__ check, EarlyIf<(NW <= 4)> kernel_before) {
-    kernel_before.wait(keys_in, keys_out, vals_out, check);
+    behind_kernel_before(keys_in, keys_out, vals_out, check, kernel_before);
     using Cfg = SmallSortCfg<NW, PACK>;
     constexpr int KW = Cfg::KW, IPT = Cfg::IPT;
     constexpr bool WORDS = NW >= 4;
@@ -716,7 +716,7 @@ __global__ void __launch_bounds__(RSC_THREADS, 1)
 radix_sort_cluster_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
                           uint32_t* __restrict__ vals_out, int n, int cta_rows, uint32_t cta_rows_inv, int passes, bool compressed,
                           KeyComp kc, const int* __restrict__ check, KernelBefore kernel_before) {
-    kernel_before.wait(keys_in, keys_out, vals_out, check);
+    behind_kernel_before(keys_in, keys_out, vals_out, check, kernel_before);
     using Cfg = ClusterSortCfg<NW, PACK>;
     constexpr int KW = Cfg::KW, IPT = Cfg::IPT;
     constexpr bool WORDS = NW >= 4;
@@ -1131,7 +1131,7 @@ __device__ __forceinline__ TOut block_exclusive_scan(TOut v, TOut* s_warp, TOut&
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(SCAN_THREADS)
 scan_reduce_kernel(const TIn* __restrict__ in, size_t n, TOut* __restrict__ block_sums, KernelBefore kernel_before) {
-    kernel_before.wait(in, block_sums);
+    behind_kernel_before(in, block_sums, kernel_before);
     __shared__ TOut s_warp[32];
     size_t base = (size_t)blockIdx.x * SCAN_TILE;
     TOut sum = 0;
@@ -1166,7 +1166,7 @@ struct HostWords {
 template <typename TOut>
 __global__ void __launch_bounds__(1024)
 scan_block_sums_kernel(TOut* __restrict__ block_sums, size_t n_blocks, TOut* __restrict__ total_out, HostWords host, KernelBefore kernel_before) {
-    kernel_before.wait(block_sums, total_out);
+    behind_kernel_before(block_sums, total_out, kernel_before);
     __shared__ TOut s_warp[32];
     TOut carry = 0;
     for (size_t base = 0; base < n_blocks; base += 1024) {
@@ -1185,7 +1185,7 @@ template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(SCAN_THREADS)
 scan_apply_kernel(const TIn* __restrict__ in, size_t n, const TOut* __restrict__ block_sums, bool scanned,
                   TOut* __restrict__ out, HostWords host, KernelBefore kernel_before) {
-    kernel_before.wait(in, block_sums, out);
+    behind_kernel_before(in, block_sums, out, kernel_before);
     __shared__ TOut s_warp[32];
     TOut before = 0;  // elements of the blocks before this one
     if (scanned) {
@@ -1235,7 +1235,7 @@ struct alignas(16) ScanVec {
 template <typename T>
 __global__ void __launch_bounds__(SCAN_ONE_THREADS)
 scan_one_kernel(const T* __restrict__ in, int n, T* __restrict__ out, HostWords host, KernelBefore kernel_before) {
-    kernel_before.wait(in, out);
+    behind_kernel_before(in, out, kernel_before);
     constexpr int PER = 16 / sizeof(T), VECS = SCAN_ONE_IPT / PER;
     __shared__ T s_warp[32];
     T carry = 0;

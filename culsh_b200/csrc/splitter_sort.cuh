@@ -262,7 +262,7 @@ template <int NW>
 __global__ void __launch_bounds__(SS_THREADS)
 splitter_sample_kernel(const uint32_t* __restrict__ keys, int n, int skip, int samples, int chunks, int bins, int over,
                        RowList<NW> sorted /* one chunk: the splitters */, KernelBefore kernel_before) {
-    kernel_before.wait(keys);
+    behind_kernel_before(keys, kernel_before);
     extern __shared__ __align__(16) unsigned char ss_smem[];
     using Sort = BlockSort<NW>;
     auto& s = *reinterpret_cast<typename Sort::Smem*>(ss_smem);
@@ -292,7 +292,7 @@ splitter_sample_kernel(const uint32_t* __restrict__ keys, int n, int skip, int s
 template <int NW>
 __global__ void __launch_bounds__(256)
 splitter_rank_kernel(const uint32_t* __restrict__ keys, int n, int skip, int chunks, int bins, int total, RowList<NW> sorted, RowList<NW> splitters, KernelBefore kernel_before) {
-    kernel_before.wait(keys);
+    behind_kernel_before(keys, kernel_before);
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= total) return;
     const int samples = chunks * SS_CAP, t = i / samples, own = (i - t * samples) / SS_CAP;
@@ -417,7 +417,7 @@ splitter_classify_kernel(const uint32_t* __restrict__ keys, int n, int skip, int
 constexpr int SS_SCAN_THREADS = 64;
 __global__ void __launch_bounds__(SS_SCAN_THREADS)
 splitter_scan_kernel(uint32_t* __restrict__ tile_hist, int tiles, int bins, int total, uint32_t* __restrict__ bin_total, KernelBefore kernel_before) {
-    kernel_before.wait(tile_hist, bin_total);
+    behind_kernel_before(tile_hist, bin_total, kernel_before);
     const int i = blockIdx.x * SS_SCAN_THREADS + threadIdx.x;
     if (i >= total) return;
     const int t = i / bins, b = i - t * bins;
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(SS_TILE_THREADS)
 splitter_scatter_kernel(const uint16_t* __restrict__ bin_of, int n, int tile, int tiles, int bins, const uint32_t* __restrict__ tile_hist,
                         const uint32_t* __restrict__ bin_total, uint32_t* __restrict__ bin_start,
                         uint32_t* __restrict__ ids, KernelBefore kernel_before) {
-    kernel_before.wait(bin_of, tile_hist, bin_total, bin_start, ids);
+    behind_kernel_before(bin_of, tile_hist, bin_total, bin_start, ids, kernel_before);
     extern __shared__ __align__(16) unsigned char ss_smem[];
     uint16_t* s_row = reinterpret_cast<uint16_t*>(ss_smem);            // [tile] its rows, bin after bin
     uint16_t* s_bin = s_row + tile;                                    // [tile] their bins

@@ -37,22 +37,34 @@ def test_order_of_the_host(n, L, family, k, scale):
 
 @pytest.mark.parametrize("n,L", SHAPES)
 @pytest.mark.parametrize("k", [3, 5, 9])
-@pytest.mark.parametrize("splitters", [None, "0"])
-def test_wide_keys(n, L, k, splitters, monkeypatch):
-    """As they come, which is by splitters up to 2,048 and from 12,289 or 16,385 rows on, and without them."""
+def test_wide_keys(n, L, k):
     from culsh_b200 import _culsh_core as core_mod
-    if splitters:
-        monkeypatch.setenv("CULSH_SORT_SPLITTERS", splitters)
     rng = np.random.default_rng(n + k)
     sets = rng.integers(0, 400, (n // 3 + 1, 6)).astype(np.int32)
     indices = np.ascontiguousarray(sets[rng.integers(0, len(sets), n)]).ravel()
     indptr = (6 * np.arange(n + 1)).astype(np.int32)
     core = core_mod.MinHashCore(L, k, 7)
     ix = core.fit(indices, indptr, n, 400)
-    if splitters:
-        ctas = 8 if L <= 13 and 4096 <= n <= 49_152 else 4 if L <= 32 and 8192 <= n <= 24_576 else int(n <= 12_288 and L <= 148)
-        assert core.last_stats()["sort_ctas"] == ctas
     _check(ix, core.hash(indices, indptr, n, ix), n, L)
+
+
+@pytest.mark.parametrize("n,L", SHAPES)
+@pytest.mark.parametrize("k", [3, 5, 9])
+def test_wide_keys_without_splitters(n, L, k, monkeypatch):
+    """Splitters take wide keys of up to 2,048 and from 12,289 or 16,385 rows on as a rule."""
+    from culsh_b200 import _culsh_core as core_mod
+    monkeypatch.setenv("CULSH_SORT_SPLITTERS", "0")
+    stats = []
+
+    class Core(core_mod.MinHashCore):
+        def fit(self, *args, **kw):
+            ix = super().fit(*args, **kw)
+            stats.append(self.last_stats())
+            return ix
+    monkeypatch.setattr(core_mod, "MinHashCore", Core)
+    test_wide_keys(n, L, k)
+    ctas = 8 if L <= 13 and 4096 <= n <= 49_152 else 4 if L <= 32 and 8192 <= n <= 24_576 else int(n <= 12_288 and L <= 148)
+    assert [s["sort_ctas"] for s in stats] == [ctas]
 
 
 @pytest.mark.parametrize("n,L,ctas", [(1000, 8, 1), (10_000, 13, 8), (24_576, 32, 4), (49_152, 13, 8), (49_153, 13, 0)])

@@ -390,7 +390,7 @@ def test_warp_path_sorts_up_to_1024_ids(eng):
     assert seen.all(), seen
 
 
-def test_large_buckets_of_few_tables(eng):
+def test_large_buckets_use_the_bitmap_path(eng):
     """k = 2 sign bits -> four buckets per table of ~n/4 rows: raw candidate counts far above
     the warp path's limit; heavy cross-table duplication."""
     culsh, core_mod = eng
@@ -404,8 +404,8 @@ def test_large_buckets_of_few_tables(eng):
     _assert_candidates_equal(model.query(Q), oracle.query_index(oracle.fit_index(sig, L, k), sig[:16]))
 
 
-def test_more_rows_than_two_to_the_twenty(eng):
-    """More rows than the bitmap of one CTA covers: large sets in windows."""
+def test_bitmap_windows_beyond_one_window(eng):
+    """More rows than one shared-memory bitmap window covers (2^20 ids)."""
     culsh, core_mod = eng
     rng = np.random.RandomState(8)
     n, d, L, k = (1 << 20) + 300000, 8, 3, 3
@@ -446,7 +446,7 @@ def test_sort_path_for_mid_sized_sets_on_a_large_index(eng):
     (None, None, None, None),   # defaults: one window at this size
     (131072, 256, 1, 16),       # 3 windows
     (65536, 512, 0, 4),         # 5 windows, whose CTAs search their slices themselves
-    (8192, 256, 1, 16),         # 37 windows
+    (8192, 256, 1, 16),         # too many windows: a CTA for each query
     (65536, 256, 1, 8),         # 5 windows, slices precomputed
     (131072, 384, 0, 8),
     (1 << 20, 384, 1, 4),       # one window

@@ -1,5 +1,5 @@
-"""Keys of four words and more are sorted word by word in tables of more than four million rows and, with splitters and
-the sorts in one launch switched off, in shorter ones: row counts on both sides of the 4096-item tile, of the 96 tiles from which tile offsets
+"""Keys of four words and more are sorted word by word, tables of more than 12,288 rows and, with the one-CTA sort
+switched off, shorter ones: row counts on both sides of the 4096-item tile, of the 96 tiles from which tile offsets
 are scanned in chunks, and of whole chunks of 64 tiles, key lengths that end inside a word (16 to 64
 bytes, 8-word keys among them), and collections where the rows agree in the leading, the trailing or all hashes, so that
 the order depends on every word and equal keys keep their row order.  The chunked scan of one- and
@@ -20,8 +20,8 @@ TILE = 4096
                                  (128 * TILE + 1, 4), (2_097_153, 3)])
 def test_index_equals_oracle_order(n, k, monkeypatch):
     from culsh_b200 import _culsh_core as core_mod
-    monkeypatch.setenv("CULSH_SORT_SPLITTERS", "0")  # which take all of these, as a rule
-    monkeypatch.setenv("CULSH_SORT_NO_PACK", "1")
+    if n <= 12_288:
+        monkeypatch.setenv("CULSH_SORT_NO_PACK", "1")
     rng = np.random.default_rng(n)
     L = 2
     # row r of block b has b's set of ids with a few of the positions changed: many equal hashes
@@ -33,7 +33,6 @@ def test_index_equals_oracle_order(n, k, monkeypatch):
     indptr = (6 * np.arange(n + 1)).astype(np.int32)
     core = core_mod.MinHashCore(L, k, 7)
     ix = core.fit(indices, indptr, n, 400)
-    assert core.last_stats()["sort_ctas"] == 0 and core.last_stats()["sort_passes"] == 4 * k
     sig = core.hash(indices, indptr, n, ix)  # [L][n][k]
     # the order of the engine: unsigned bytes in memory order, ties by row
     got_c, got_b = ix.get_candidate_indices(), ix.get_bucket_signatures().reshape(-1, 4 * k)
@@ -67,3 +66,23 @@ def test_scan_of_many_tiles(k, tile, tiles, extra):
     for t in range(L):
         key = (sig[t].astype(np.uint64) << np.arange(k - 1, -1, -1, dtype=np.uint64)).sum(axis=1, dtype=np.uint64)
         assert np.array_equal(cand[t * n:(t + 1) * n], np.argsort(key, kind="stable"))
+
+
+@pytest.mark.parametrize("n,k", [(1, 3), (31, 16), (4095, 3), (4096, 4), (4097, 5), (8193, 8), (12_289, 9), (12_289, 5), (20_000, 16),
+                                 (20_000, 8), (95 * TILE, 5), (95 * TILE + 1, 3), (96 * TILE + 1, 8), (128 * TILE, 3),
+                                 (128 * TILE + 1, 4), (2_097_153, 3)])
+def test_word_by_word(n, k, monkeypatch):
+    """As above with splitters, which take keys of two words and more in up to four million rows as a rule, and the sorts in one launch switched off."""
+    from culsh_b200 import _culsh_core as core_mod
+    monkeypatch.setenv("CULSH_SORT_SPLITTERS", "0")
+    monkeypatch.setenv("CULSH_SORT_NO_PACK", "1")
+    stats = []
+
+    class Core(core_mod.MinHashCore):
+        def fit(self, *args, **kw):
+            ix = super().fit(*args, **kw)
+            stats.append(self.last_stats())
+            return ix
+    monkeypatch.setattr(core_mod, "MinHashCore", Core)
+    test_index_equals_oracle_order(n, k, monkeypatch)
+    assert len(stats) == 1 and stats[0]["sort_ctas"] == 0 and stats[0]["sort_passes"] == 4 * k

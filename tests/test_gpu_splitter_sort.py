@@ -1,7 +1,7 @@
 """Keys of two words and more are sorted by sampled splitters, word by word by radix passes or, as one bin, by one CTA: row
 counts on both sides of a bin, of the change from one to several chunks of samples and of a tile, keys that end inside
 their words, and collections in which all rows are alike, come in order, repeat with a period or differ in one hash only, so that bins
-are full of equal keys."""
+are full of equal keys and some are sorted in pieces."""
 import numpy as np
 import pytest
 
@@ -57,9 +57,8 @@ def test_order(n, k, kind, splitters, monkeypatch):
         monkeypatch.setenv("CULSH_SORT_SPLITTERS", splitters)
     rng = np.random.default_rng(n + k)
     L = 2
-    rows = _rows(kind, n, rng)
-    indices = np.ascontiguousarray(rows.astype(np.int32)).ravel()
-    indptr = (rows.shape[1] * np.arange(n + 1)).astype(np.int32)
+    indices = np.ascontiguousarray(_rows(kind, n, rng).astype(np.int32)).ravel()
+    indptr = (6 * np.arange(n + 1)).astype(np.int32)
     core = core_mod.MinHashCore(L, k, 7)
     _check(core, core.fit(indices, indptr, n, 1 << 19), indices, indptr, n, L, k)
 
@@ -70,7 +69,14 @@ def test_order(n, k, kind, splitters, monkeypatch):
 def test_wide_keys_that_repeat(n, k, kind, monkeypatch):
     """Keys of eight and sixteen words whose first words are the same in all rows of a bin or in many: the words behind them are looked at only
     where there are rows that are not alike."""
-    test_order(n, k, kind, "1", monkeypatch)
+    from culsh_b200 import _culsh_core as core_mod
+    monkeypatch.setenv("CULSH_SORT_SPLITTERS", "1")
+    rng = np.random.default_rng(n + k)
+    rows = _rows(kind, n, rng)
+    indices = np.ascontiguousarray(rows.astype(np.int32)).ravel()
+    indptr = (rows.shape[1] * np.arange(n + 1)).astype(np.int32)
+    core = core_mod.MinHashCore(2, k, 7)
+    _check(core, core.fit(indices, indptr, n, 1 << 19), indices, indptr, n, 2, k)
 
 
 def _largest_bin(order, n):
