@@ -1,6 +1,6 @@
 // Sort of a table's (key, row id) pairs by sampled splitters: the rows go into bins of about a thousand, a bin
 // is sorted by one CTA in shared memory.  It takes keys that a radix sort would need many passes for - seven bytes and more, up to SS_CAP
-// rows all of two words and more - in tables that a CTA or a cluster does not sort faster as a whole: see sort_by_splitters.
+// rows all of two words and more - in tables that a CTA or a cluster does not sort faster as a whole, and that are not too long: see sort_by_splitters.
 //
 //   1. splitter_sample_kernel   sorts SS_OVER rows a bin and more, drawn from all of the table, SS_CAP a CTA
 //      splitter_rank_kernel     (tables of several such chunks) ranks the samples among all of the table's
@@ -26,7 +26,6 @@ constexpr int SS_CAP = SS_THREADS * SS_ITEMS;   // rows that a CTA sorts at once
 constexpr int SS_BIN_ROWS = 1024;               // rows of a bin on average, at most
 constexpr int SS_OVER = 8;                      // samples for each bin, at least
 constexpr int SS_MAX_BINS = 4096;
-constexpr int SS_FROM = 12288, SS_FROM_12 = 16384;  // see sort_by_splitters
 constexpr int SS_TILE = 16384, SS_SHORT_TILE = 4096;  // rows of a CTA that classifies or scatters, and where these would be few, at least
 constexpr int SS_TILE_THREADS = 512;
 
@@ -823,28 +822,47 @@ inline SplitterPlan splitter_plan(int n, int L) {
     }
     return p;
 }
-// Keys this sort takes: of two words and more, in tables of up to four million rows.
+// Keys this sort takes: of two words and more, in tables of up to 2^22 rows.  (8 tables of 16-byte keys, by radix passes and this way: 2^22 rows 3,712
+// and 2,535 us, one more 3,737 by radix passes.)
 inline bool splitters_can(int n, int NW) { return NW >= 2 && splitter_bins(n) <= SS_MAX_BINS; }
 
 // What sorts the tables: splitters, or the radix sorts.  What a radix sort costs grows with the bytes of a key, what this costs with the logarithm
-// of the rows.  Up to SS_CAP rows a table is one bin.  Above, it pays for keys of seven bytes that are not sorted in compressed form, where the
-// radix sort does not take the table in one launch, and for keys of four words also in longer tables that it does.  The sort stage by radix
-// passes and this way: 32 tables of 16-byte keys, 1,000 rows 53 and 22 us, 12,000 104 and 103, 30,000 316 and 132, 100,003 570 and 265,
-// 500,000 1,789 and 1,051, 2M 6,061 and 4,134; 16 tables of 9-byte keys, 1M rows 1,070 and 926; of 8-byte keys, 100,003 rows 214 and 125, 1M
-// 1,143 and 853, compressed 558 and 879; of 5-byte keys, 1M 741 and 826; of 8-byte keys, 4M rows x one table 372 and 416, x two 634 and 678, x four 1,182
-// and 1,117 (2M x one 268 and 242).
-// In those longer tables the radix sort is the faster one where keys repeat, and the more so the fewer bytes a key has.  8 tables, all keys different, groups of
-// near duplicates, ten different keys: 12,289 of 12 bytes 74 and 69 us, 60 and 75, 54 and 84, so that these go this way above SS_FROM_12 rows, 20,000 93 and
-// 75, 70 and 79, 62 and 79; 12,289 of 16 bytes 95 and 69, 74 and 77, 68 and 85; of 20 bytes 115 and 67, 91 and 118, 84 and 145; 40,000 of 20
-// bytes 236 and 74, 160 and 132, 140 and 161.
+// of the rows; up to SS_CAP rows a table is one bin.  Above, this pays for keys of seven bytes and more that are not sorted in compressed form.  The sort stage by
+// radix passes and this way: 32 tables of 16-byte keys, 1,000 rows 53 and 22 us, 30,000 316 and 132, 100,003 570 and 265, 500,000 1,789 and 1,051, 2M
+// 6,061 and 4,134; 5-byte keys, 16 tables of 1M 741 and 826.
 // CULSH_SORT_SPLITTERS=0 / 1: never / wherever it can.
+//
+// Rows of a table that the radix sort takes in one launch (one CTA or a cluster) and sorts faster or as fast.  It gains where keys repeat, and the more so
+// the fewer bytes they have.  8 tables, all keys different, twenty rows to a key, ten keys in all: 12,289 rows of 16 bytes 95 and 69 us, 74 and 77, 68 and 85;
+// 16,385 of 12 bytes in 0.71, 1.20 and 1.22 of the radix sort's time; 24,576 of 10 bytes 0.92, 1.26 and 1.48, 40,000 0.74, 1.05 and 1.20; of 11 bytes
+// 0.81, 1.19 and 1.42, 0.65, 0.96 and 1.17; of 9 bytes 1.07, 1.37 and 1.62, 0.83, 1.12 and 1.39, of 8 and 7 alike.
+inline int64_t splitters_from(int KB) { return KB >= 13 ? 12288 : KB == 12 ? 16384 : KB >= 10 ? 32768 : INT32_MAX; }
+// Rows of a table up to which this is faster than radix passes with launches of their own, or as fast.  They gain with the rows, most of all beyond 2^21, where
+// 4,096 splitters leave an SM no second CTA of the search, and with fewer tables.  Times by radix passes and this way:
+//   7 bytes (this way with the 17 us of a look for a compressed form): 8 tables of 100,003 136 and 116 us, 131,072 138 and 143, 250,000 181 and 180, 1M 416
+//   and 475, 2^22 1,516 and 2,249
+//   8 bytes: 4 tables of 500,000 191 and 187 (twenty rows to a key 180 and 189), 786,432 with twenty rows to a key 213 and 240, 2^21 509 and 543, 2^22 966
+//   and 1,140; 8 of 1M 483 and 460, 2^21 964 and 908, 3M 1,333 and 1,577
+//   9 bytes: 4 of 1M 335 and 326, 2^21 569 and 597; 8 of 2^21 1,050 and 982, 3M 1,548 and 1,753; 10 bytes: 2 of 1M 246 and 234, 2^21 358 and 369; 8 of 2^21
+//   1,130 and 1,018, 3M 1,662 and 1,733
+//   11 bytes: 2 of 2^21 384 and 363, 3M 527 and 556; 8 of 3M 1,784 and 1,746, 2^22 2,568 and 2,398; 12 bytes: one of 3M 348 and 359
+inline int64_t splitters_to(int KB, int L) {
+    switch (KB) {
+        case 7: return 7 << 14;
+        case 8: return L < 8 ? 1 << 19 : 1 << 21;
+        case 9: return L < 8 ? 1 << 20 : 1 << 21;
+        case 10: return L < 4 ? 1 << 20 : 1 << 21;
+        case 11: return L < 4 ? 1 << 21 : 1 << 22;
+        default: return KB < 7 ? 0 : 1 << 22;
+    }
+}
 inline bool sort_by_splitters(const CtxPtr& c, int n, int L, int NW, int KB, bool compressed) {
     if (!splitters_can(n, NW)) return false;
     const char* e = getenv("CULSH_SORT_SPLITTERS");
     if (e && *e) return atoi(e) != 0;
     if (n <= SS_CAP) return true;
-    if (compressed || KB < 7 || (NW == 2 && L < 4 && splitter_bins(n) == SS_MAX_BINS)) return false;
-    return (NW >= 4 && n > (KB <= 12 ? SS_FROM_12 : SS_FROM)) || !radix_sort_is_small(c, n, L, NW, compressed);
+    if (compressed || n > splitters_to(KB, L)) return false;
+    return n > splitters_from(KB) || !radix_sort_is_small(c, n, L, NW, compressed);
 }
 
 // keys[0] -> keys[1], row ids to vals[1]; vals[0] is scratch.

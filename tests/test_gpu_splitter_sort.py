@@ -97,10 +97,11 @@ def _largest_bin(order, n):
 
 
 @pytest.mark.parametrize("n,k,kind", [(524_288, 2, "mixed"), (1_048_576, 2, "mixed"), (524_288, 3, "last"), (524_288, 6, "mixed"), (524_288, 8, "near"), (524_288, 9, "last"), (524_288, 16, "near")])
-def test_bins_in_pieces(n, k, kind):
+def test_bins_in_pieces(n, k, kind, monkeypatch):
     """Tables whose bins hold 1,024 rows on average, so that some hold more than the 2,048 that a CTA sorts at once.  (Not where
     few keys differ: rows that are alike come in the order of their ids, which the samples cover evenly.)"""
     from culsh_b200 import _culsh_core as core_mod
+    monkeypatch.setenv("CULSH_SORT_SPLITTERS", "1")  # two long tables of short keys are not theirs as a rule
     rng = np.random.default_rng(k)
     rows = _rows(kind, n, rng)
     indices = np.ascontiguousarray(rows.astype(np.int32)).ravel()
@@ -114,7 +115,7 @@ def test_bins_in_pieces(n, k, kind):
 
 
 @pytest.mark.parametrize("n,k,L,route", [(16_384, 3, 32, 4), (16_385, 3, 32, -1), (12_288, 4, 32, 4), (12_289, 4, 32, -1), (12_289, 8, 32, -1), (2048, 3, 32, -1), (2049, 3, 32, 1),
-                                         (2_097_152, 2, 3, -1), (2_097_153, 2, 3, 0), (2_097_153, 2, 4, -1), (2_097_153, 3, 1, -1)])
+                                         (524_288, 2, 7, -1), (524_289, 2, 7, 0), (2_097_152, 2, 8, -1), (2_097_153, 2, 8, 0), (2_097_153, 3, 1, -1)])
 def test_which_sort(n, k, L, route):
     """Lines between the sorts: clusters of four CTAs, one CTA, passes with launches of their own and splitters."""
     from culsh_b200 import _culsh_core as core_mod
@@ -140,6 +141,19 @@ def test_wide_p_stable_keys_and_many_tables():
             raw = np.ascontiguousarray(sig[t]).view(np.uint8).reshape(n, 4 * k)
             order = np.lexsort(tuple(raw[:, j] for j in range(4 * k - 1, -1, -1)))
             assert np.array_equal(got[t * n:(t + 1) * n], order)
+
+@pytest.mark.parametrize("n,k,L,route", [(114_688, 7, 8, -1), (114_689, 7, 8, 0), (49_152, 9, 8, 8), (49_153, 9, 8, -1), (32_768, 10, 8, 8), (32_769, 10, 8, -1), (32_769, 11, 8, -1),
+                                         (1_048_576, 9, 7, -1), (1_048_577, 9, 7, 0), (1_048_577, 9, 8, -1), (2_097_152, 10, 4, -1), (2_097_153, 10, 4, 0), (2_097_153, 11, 3, 0), (2_097_153, 11, 4, -1)])
+def test_which_sort_of_one_byte_values(n, k, L, route):
+    """As above, for keys of as many bytes as hashes, whose values span too much for the compressed form."""
+    import torch
+    from culsh_b200 import _culsh_core as core_mod
+    X = 9 * torch.randn(n, 4, device="cuda", generator=torch.Generator("cuda").manual_seed(n))
+    torch.cuda.synchronize()
+    core = core_mod.PSLSHCore(L, k, 2, 3)
+    assert core.fit_float(X, n, 4).elem_bytes == 1
+    assert core.last_stats()["sort_ctas"] == route
+
 
 
 def test_no_scratch_where_another_sort_runs():
