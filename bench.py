@@ -651,13 +651,14 @@ def line_of(torch, args, wl, spec, world, m, peaks, tf32):
     passes = max(1, sf["sort_passes"])
     items, kb = sf["n_items"], 4 * sf["key_words"]
     # keys of four words and more: the last pass reads (word, row id) and writes the ids; short tables: one launch
-    # reads the keys and writes keys and ids; by splitters: the launch over the bins reads their ids besides
+    # reads the keys and writes keys and ids; by splitters: the launch over the bins reads their ids besides, where a table (n rows) has several
     ctas = sf["sort_ctas"]
     split = ctas < 0
     short = ctas > 0
     wide = sf["key_words"] >= 4
-    item_bytes = 2.0 * kb + 8.0 if split else 2.0 * kb + 4.0 if short else (12.0 if wide else (kb + 4) * 2.0)
-    item_note = (f"row id and key ({kb} B) read, key and row id written per item" if split else f"key {kb} B read, key and row id written per item, one launch for all passes" if short else
+    bins = split and items > 2048 * spec["L"]
+    item_bytes = 2.0 * kb + 8.0 if bins else 2.0 * kb + 4.0 if short or split else (12.0 if wide else (kb + 4) * 2.0)
+    item_note = (f"row id and key ({kb} B) read, key and row id written per item" if bins else f"key {kb} B read, key and row id written per item, one launch for all passes" if short or split else
                  "key word and row id read, row id written per item, one launch" if wide else
                  f"(key {kb} B + row id 4 B) read + written per item, one launch")
     roof = {}
@@ -685,9 +686,9 @@ def line_of(torch, args, wl, spec, world, m, peaks, tf32):
     if scatter_ms > 0:
         roof["sort"] = {"bound": "hbm", "achieved": items * item_bytes / (scatter_ms * 1e-3) / 1e9,
                         "peak": peaks["hbm_gbs"], "unit": "GB/s", "traffic": None,
-                        "kernel": ("splitter_short_bin_kernel" if split else "radix_sort_cluster_kernel" if ctas > 1 else "radix_sort_small_kernel" if short else
+                        "kernel": (("splitter_short_bin_kernel" if sf["key_words"] <= 4 else "splitter_bin_kernel") if split else "radix_sort_cluster_kernel" if ctas > 1 else "radix_sort_small_kernel" if short else
                                    "radix_scatter_kernel"),
-                        "note": item_note + (" (the launches over the bins)" if split else "" if short else f" (the scatter of the last of {passes} passes)") +
+                        "note": item_note + (" (the launches over the bins)" if bins else "" if split else "" if short else f" (the scatter of the last of {passes} passes)") +
                                 f", timed with CUDA events; peak {peaks['source']}"}
     dedupe_ms = mean("dedupe_ms", "query")
     if dedupe_ms > 0:

@@ -106,7 +106,10 @@ __device__ __forceinline__ uint32_t min_plus5_short(uint32_t m, double a, double
 // and the second of these are what a lane keeps of a row.  Of the eight of the least one, that with the least y is evaluated in full, f*: it is the row's
 // minimum where every other y is at e_max or more above it, for f >= y - e_max whether y wrapped or not.  Where that does not hold (of 110 ids below
 // 2^20 for a minimum in 70 to 150, in proportion to the largest id) the warp evaluates the minimum again.  Up to 32 ids that and what is set up for
-// a row weigh more than is saved, and with more than four hash functions a lane registers are too few.
+// a row weigh more than is saved.  Ids from 2^MH_COL_BITS on and more than four hash functions a lane keep to the forms below, which is where the form has
+// been tried out, not where it stops paying.  Those forms and this one, uniform ids, 300,000 rows of 20 to 200, 600,000 of 33, 20,000 of 1,000: 128 functions below
+// 2^23 1,474 and 826 us, 967 and 765, 832 and 705, below 2^24 1,475 and 1,055, 966 and 877, 832 and 950; 160 functions below 2^16 1,002 and 772, 810
+// and 948, 665 and 332, below 2^20 1,477 and 814, 1,056 and 964, 946 and 413.
 // Issue and the pipes of multiply-add (two cycles) and minimum bound it.  The double forms below and this one, 128 functions: 2M Zipf sets of 20 to 200
 // ids below 2^20 4,199 and 2,970 us, 300,000 below 2^16 593 and 443, below 2^22 768 and 537; 20M uniform ids below 2^20 in rows of 33 812 and
 // 647, 110 705 and 344, 1,000 778 and 332.  Next to it the double forms take 8 % longer for 12 uniform ids below 2^20 a row (634 and 682),
@@ -119,7 +122,7 @@ constexpr int MH_LIST = 1024;
 constexpr int MH_ALIKE = 2;
 constexpr int MH_LIST_FROM = 33;
 constexpr uint32_t MH_TAG = MH_LIST / 8 - 1;
-constexpr int MH_COL_BITS = 22;  // rows with ids from 2^MH_COL_BITS on take the general forms
+constexpr int MH_COL_BITS = 22;  // rows with ids from 2^MH_COL_BITS on take the general forms, see above
 // What ids in the list are above themselves: the sum of some of them tells their number, too.
 constexpr uint32_t MH_LIST_ID = 1u << 26;
 struct NearParams {
@@ -144,7 +147,7 @@ __global__ void __launch_bounds__(MH_THREADS, PL <= 2 ? 32 : PL <= 4 ? 22 : 18)
 minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ indptr,
                const uint32_t* __restrict__ A, const uint32_t* __restrict__ B, int n_rows,
                int L, int k, int NW, uint32_t* __restrict__ keys, int n_total, int row_offset, int rows) {
-    constexpr bool NEAR = PL <= 4;  // more leave it too few registers
+    constexpr bool NEAR = PL <= 4;
     const int lane = threadIdx.x & 31;
     const int H = L * k;
     const int pad_words = NW - k;  // leading zero words when 4k is not 4, 8, 16 or 32 bytes

@@ -908,8 +908,7 @@ inline size_t window_smem_bytes(int window_bits) {
 // Cuts the ascending lists [s_lo[t], s_we[t]) of `cand` down to their slices in [win_lo, win_hi); an open side of the window
 // (the first one's lower, the last one's upper) cuts nothing.  Eight lanes take a (list, side) and look at eight places a step,
 // and with two of them in turn a warp has eight searches in flight: what bounds a CTA that has few of them is how many reads wait for
-// one another.  Called
-// by all threads, with a barrier before and behind.
+// one another.  Called by all threads, with a barrier before and behind.
 template <int NT>
 __device__ __forceinline__ void cut_lists(const int32_t* __restrict__ cand, int* __restrict__ s_lo, int* __restrict__ s_we, int L,
                                           int win_lo, int win_hi, bool open_lo, bool open_hi) {

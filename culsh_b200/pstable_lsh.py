@@ -11,10 +11,12 @@ from .utils import ensure_engine_array, get_array_info, get_logger, is_device_ar
 
 def _engine_takes_norms(xs) -> bool:
     """Whether the engine's one-launch kernel or torch's norm gives the mean row norm.  Up to 4,096 columns the
-    kernel is the faster one everywhere (1,000 x 100: 24 us and 42, 10,000 x 128: 27 and 36, 10,000 x 1,024: 31 and
-    82, float64 10,000 x 128: 26 and 35, 4,096 x 128: 25 and 26); it takes float32 rows that are few, many or long and
-    many float64 rows, and leaves the sizes between, where it gains least, to torch as before.  Longer rows torch
-    spreads over more of the chip (50 x 200,000: 83 against 324)."""
+    kernel is the faster one wherever both were timed, engine and torch (float32 1,000 x 100 24 us and 32, 2,000 x 128
+    23 and 32, 10,000 x 128 27 and 36, 10,000 x 1,024 31 and 82; float64 1,000 x 100 22 and 25, 4,000 x 250 24 and 25,
+    10,000 x 128 26 and 35).  float64 rows below 4,096, and float32 rows from 1,025 to 4,095 of less than 256 columns,
+    stay with torch for what it returns, not for its time: where all rows have the same whole norm, the last bit of
+    the mean decides the window, and torch's is now and then below it (float64 rows of one norm: 6 sets of 200, the
+    engine's none).  Longer rows torch spreads over more of the chip (50 x 200,000: 83 against 324)."""
     import torch
     n, d = xs.shape
     if not xs.is_contiguous() or n <= 0 or not 0 < d <= 4096:
