@@ -111,7 +111,7 @@ __device__ __forceinline__ uint32_t min_plus5_short(uint32_t m, double a, double
 // 2^23 1,474 and 826 us, 967 and 765, 832 and 705, below 2^24 1,475 and 1,055, 966 and 877, 832 and 950; 160 functions below 2^16 1,002 and 772, 810
 // and 948, 665 and 332, below 2^20 1,477 and 814, 1,056 and 964, 946 and 413.
 // Issue and the pipes of multiply-add (two cycles) and minimum bound it.  The double forms below and this one, 128 functions: 2M Zipf sets of 20 to 200
-// ids below 2^20 4,199 and 2,970 us, 300,000 below 2^16 593 and 443, below 2^22 768 and 537; 20M uniform ids below 2^20 in rows of 33 812 and
+// ids below 2^20 4,199 and 3,030 us, 300,000 below 2^16 593 and 443, below 2^22 768 and 537; 20M uniform ids below 2^20 in rows of 33 812 and
 // 647, 110 705 and 344, 1,000 778 and 332.  Next to it the double forms take 8 % longer for 12 uniform ids below 2^20 a row (634 and 682),
 // between 3 % less and 2 % more for other short rows.
 //
