@@ -115,13 +115,15 @@ __device__ __forceinline__ uint32_t min_plus5_short(uint32_t m, double a, double
 // 647, 110 705 and 344, 1,000 778 and 332.  Next to it the double forms take 8 % longer for 12 uniform ids below 2^20 a row (634 and 682),
 // between 3 % less and 2 % more for other short rows.
 //
-// An id that a row has twice is close to itself: rows of few different ids would have nearly all their minima evaluated again (300,000 rows of 20 to 200
-// ids, four different ones 4,670 us and 1,125 in the double forms, 16 4,570 and 1,195, 64 3,300 and 1,225, 200 1,760 and 1,390, 1,000
-// 855 and 894).  MH_ALIKE of the first 32 ids that the row has had before keep it from this form; to see that takes 10 us of 300,000 rows.
+// An id that a row has twice is close to itself: where rows repeat their ids nearly all minima would be evaluated again, each in more time than the double form
+// takes for five functions.  A row with MH_TOO_CLOSE of them among its first 32 functions, and twice as many more as ids so many and as large lead to, is
+// done in the double forms instead, and so are the warp's rows behind it.  300,000 rows of 80 ids, 128 functions, without that, with it, in the double forms
+// alone: 40 ids below 2^16 twice 3,840 us, 621 and 585, below 2^20 3,849, 903 and 832, 55 and 25 of them again 2,013, 909 and 838; all different 465, 468 and 846;
+// 32 functions 961, 260 and 230, all different 171, 180 and 234.
 constexpr int MH_LIST = 1024;
-constexpr int MH_ALIKE = 2;
 constexpr int MH_LIST_FROM = 33;
 constexpr uint32_t MH_TAG = MH_LIST / 8 - 1;
+constexpr int MH_TOO_CLOSE = 6;  // of the first 32 functions
 constexpr int MH_COL_BITS = 22;  // rows with ids from 2^MH_COL_BITS on take the general forms, see above
 // What ids in the list are above themselves: the sum of some of them tells their number, too.
 constexpr uint32_t MH_LIST_ID = 1u << 26;
@@ -154,7 +156,7 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
     __shared__ __align__(16) double ids_short[34], ids_long[34];
     __shared__ __align__(16) uint32_t ids_row[NEAR ? MH_LIST : 1];
     __shared__ __align__(16) NearParams near[NEAR ? PL : 1][32];
-    bool have_near = false;
+    bool have_near = false, repeats = false;  // the rows repeat their ids
     __shared__ size_t key_at[32 * PL];  // word of a hash function in the first row's keys
     const uint32_t below = (1u << lane) - 1u;
     double ad[PL], bd[PL];
@@ -196,13 +198,9 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
         bool shorts = false;  // the row has had ids below short_col
         // Rows for the near form: all ids at once, the last one again to a whole number of eights.
         const int n_ids = end - start, eights = (n_ids + 7) / 8;
-        bool listed = NEAR && n_ids >= MH_LIST_FROM && n_ids <= MH_LIST;
+        bool listed = NEAR && !repeats && n_ids >= MH_LIST_FROM && n_ids <= MH_LIST;
         uint32_t largest = 0;
         if (listed) listed = !__any_sync(0xFFFFFFFFu, (uint32_t)ahead >> MH_COL_BITS);
-        if (listed) {  // rows that repeat their ids
-            const uint32_t alike = __match_any_sync(0xFFFFFFFFu, ahead);
-            listed = __popc(__ballot_sync(0xFFFFFFFFu, (alike & below) != 0u)) < MH_ALIKE;
-        }
         if (listed) {
             largest = (uint32_t)ahead;
             ids_row[lane] = largest + MH_LIST_ID;
@@ -276,6 +274,14 @@ minhash_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ 
                     const uint32_t t = hash_plus5(a_of(i), close & (MH_LIST_ID - 1u), b5_of(i));
                     // 0 where it is too close to tell, and below 5 near the prime: evaluated again
                     m[i] = close < 2u * MH_LIST_ID && t >= 5u && t <= 0xFFFFFFFFu - slack && second[i] >= t - 5u + slack ? t : 0u;
+                }
+                // n_ids * largest / 2^29 is what to expect
+                if (__popc(__ballot_sync(0xFFFFFFFFu, m[0] == 0u && lane < H)) >= MH_TOO_CLOSE + (int)((uint32_t)n_ids * (largest >> 10) >> 18)) {
+                    repeats = true;
+                    listed = false;
+                    ahead = indices[start + lane];
+#pragma unroll
+                    for (int i = 0; i < PL; ++i) m[i] = 0xFFFFFFFFu;
                 }
             }
             for (int base = listed ? end : start; base < end; base += 32) {

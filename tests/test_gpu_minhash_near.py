@@ -115,11 +115,11 @@ def test_ids_around_the_last_one(m, alike):
         _check(core, indices, indptr, len(rows), d, L, k)
 
 
-@pytest.mark.parametrize("alike", [0, 1, 2, 3, 31])
+@pytest.mark.parametrize("alike", [0, 1, 3, 8, 31, 1000])
 @pytest.mark.parametrize("late", [False, True])
 def test_rows_that_repeat_ids(alike, late):
-    """On both sides of the line from which rows that repeat ids keep to the other forms, with the repeated ones among a row's first 32 or behind them, next to
-    rows that do not."""
+    """On both sides of the line from which rows that repeat ids, and those behind them, are done in the other forms, with the repeated ones among a row's first
+    32 or behind them, next to rows that do not."""
     from culsh_b200 import _culsh_core as core_mod
     rng = np.random.default_rng(alike)
     rows = []
